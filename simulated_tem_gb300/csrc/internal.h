@@ -168,6 +168,7 @@ struct ColumnJob {
   ColumnParams p;
   int tile_base[kRingShapes];
   int pad;
+  int64_t sample_base;  // first field sample of the image in the batch's sample sequence (32 per patch and slice)
 };
 int column_tiles(const ColumnParams& p, int shape = 0);  // warp tiles of one image in `shape`
 // The slab-ring launch.  `tiles`: the pass's warp tiles in each shape (host array).
@@ -206,12 +207,49 @@ extern template cudaError_t ring3_launch_np<8>(const Ring3Args&);
 extern template cudaError_t ring3_launch_np<16>(const Ring3Args&);
 }  // namespace ring3
 cudaError_t launch_column_fp64(const ColumnParams& p, cudaStream_t st);
-// The FP64 slab-ring launch (k_column_f64ring.cu) over the jobs of one pass of at most 4
-// precession angles; slab tiers 0, 1, 2 stage 128, 192, 256 atoms; `four`: every job's
-// steps of four slices fit the ring (four_slices_fit).
-cudaError_t launch_column_fp64_ring(const ColumnJob* d_jobs, int n_jobs, int tiles, int max_np, int slab_tier,
-                                    bool masked, bool four, unsigned* work, const unsigned long long* counters,
-                                    int64_t cap, cudaStream_t st);
+// The voxel field of a range of patches (warp tiles of 32 columns) of a batch, in a workspace of
+// samples: patch by patch in job order, slice by slice, 32 lanes.  The work is handed out in units
+// of one patch and `chunk` slices, so that few patches still fill the GPU.
+struct FieldRange {
+  void* samples = nullptr;  // the field x of a voxel (times rho with density): double2
+  double* rho64 = nullptr;  // with density: rho
+  int64_t origin = 0;       // index of the workspace's first sample in the batch's sample sequence
+  int patch_lo = 0, patch_hi = 0;
+  int n_chunks = 1;         // per patch: ceil(deepest image / chunk)
+  int chunk = 0;            // slices per unit, a multiple of 4
+  unsigned* work = nullptr;
+  const unsigned long long* counters = nullptr;
+  int64_t cap = 0;
+  __host__ __device__ int units() const { return (patch_hi - patch_lo) * n_chunks; }
+};
+// The job of patch `g` (in the batch's patch sequence of tile shape 0) and its number in the job.
+__device__ __forceinline__ const ColumnJob& field_patch(const ColumnJob* __restrict__ jobs, int n_jobs, int g,
+                                                        int& patch) {
+  int lo = 0, hi = n_jobs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (jobs[mid].tile_base[0] <= g)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  patch = g - jobs[lo].tile_base[0];
+  return jobs[lo];
+}
+inline int sm_count() {
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+// The FP64 path's field and integration of one range (k_field64.cu); slab tiers 0, 1, 2 stage
+// 128, 192, 256 atoms; `four`: every job's steps of four slices fit the ring (four_slices_fit);
+// d_gauss: gauss64_table's values.
+constexpr int kGauss64Size = 3 * 1024 + 16;
+constexpr int kField64Blocks = 2;  // CTAs of four warps per SM at tier 0
+void gauss64_table(double* t);
+cudaError_t launch_field64(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, int slab_tier,
+                           bool density, bool masked, bool four, const double* d_gauss, cudaStream_t st);
 // Whether every step of four slices (z = 0, 4, 8 ...) of an image has home z cells that
 // rise by at most one cell without wrapping, so that the cells the step needs (one more on
 // either side) fit the slab ring's four slots.

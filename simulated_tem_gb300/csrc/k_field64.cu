@@ -1,0 +1,631 @@
+// K2+K3, FP64: the voxel field of the plain FP64 path on the slab ring, and its column
+// integrator.
+//
+// The pixel loop of computeD2BI_img (Lib_DynamicalTwoBeamImaging.f90:1870-1900) with the
+// neighbour search of Lib_LinkCell3D.f90:1515-1605 (k_field64) and the integrator of
+// :2316-2480 (k_integrate64).  The field samples of a column pass through device memory
+// (16 bytes a voxel), so that the field kernel splits a column's depth over warps (an image
+// of a few hundred patches still fills the GPU) and is computed once however many precession
+// angles integrate over it.
+//
+// The field kernel: one warp per 8 x 4 pixel columns and range of slices, four slices per
+// step (two where some image's steps of four do not fit the ring), the atoms of the link-cell
+// slabs staged in warp-private shared memory and ordered by z bin (slab_ring.cuh).
+//
+// What bounds it is the FP64 pipe: one warp instruction per 76 cycles and SM sub-partition
+// (measured; predicated-off lanes, fully predicated-off instructions and FP64 <-> FP32
+// conversions cost the same), against one FP32 or integer instruction per cycle.  So FP64 is
+// spent only where the result needs it:
+// * The accept decision is the reference's, d.d <= (3 sigma)^2 in its rounded operations
+//   (d_a = a_aa (f_a + (k_a - zi_frac_a)), the fractions f of the FP64 binning, the unwrapped
+//   27-cell offsets k).  An FP32 distance decides every pair further than kGuard64 from the
+//   cutoff; the others (2 % of the warp's atoms have one) are decided in FP64, so the accepted
+//   set equals the reference's.
+// * The weight is a product of three Gaussians, one per axis: exp(-d_x^2 / 2 sigma^2) depends on
+//   the atom and one of the patch's 8 columns, the y factor on one of its 4 rows, the z factor
+//   (times the phasor) on the slice.  The warp evaluates these 16 values per buffered atom as
+//   one flat list of tasks over its lanes instead of one exp per lane.
+// * The Gaussian itself is a table value times a short polynomial (gauss64): 9 FP64 operations.
+// * A lane then spends one multiplication per atom and two fused multiply-adds per slice that
+//   some lane of the warp accepts.
+// Measured (GB300, whole calls): 128k atoms with density 29.0 -> 7.4 ms, 28k atoms 6.75 -> 0.86 ms,
+// 16k atoms with six precession angles 13.6 -> 1.35 ms (before: one exp, the divisions of the
+// reference's integrator and hypot in every lane, a whole column per warp, the field once per four
+// angles).
+//
+// Precision: gauss64 is within 2.4 units of 2^-53 of the exact value (root mean square 0.57;
+// exp of the rounded d.d / 2 sigma^2, up to 4.5, is within 13.5, 2.1 in the mean square: the rounding of
+// its argument); the weight takes two more products, the sums and the integrator are fused.  Images
+// against a 64-bit evaluation of the same sums: relative 2-norm 0.4 to 1.2e-15 (before 0.5 to 1.6e-15).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cfloat>
+#include <cmath>
+
+#include "internal.h"
+#include "slab_ring.cuh"
+
+namespace stem {
+namespace field64 {
+
+using slab::Geo;
+using slab::kBins;
+using slab::kRing;
+using slab::load_slab;
+
+constexpr int kWarps = 4;
+// Scaled r^2 (cutoff 6.49): the FP32 distance decides outside this distance of the cutoff.  Its
+// error is below 1e-4 for voxels up to a lattice constant; the reject side of the FP32 test always
+// had this margin.
+constexpr float kGuard64 = 1e-3f;
+constexpr int kN = 64;            // step buffer: flushed at 32, before a round of 32 may add more
+constexpr float kOff = -1e30f;    // hmax of a slice the slab does not serve
+
+#define DM __dmul_rn
+#define DA __dadd_rn
+#define DS __dsub_rn
+#define DF __fma_rn
+
+template <int CAPS, int SL>
+struct WarpSmem {
+  static_assert(CAPS % 32 == 0, "the z sort holds CAPS / 32 atoms per lane");
+  float4 p[kRing][CAPS];  // X', Y', z (scaled FP32), cell code
+  int gi[kRing][CAPS];    // index of the kept atom
+  int bin[kRing][kBins + 1];
+  int count[kRing];
+  alignas(16) float hm[kN][SL];  // per slice: the largest accepted in-plane r^2 (FP32, scaled)
+  float2 xy[kN];          // X', Y'
+  int2 ref[kN];           // kept atom, cell code | slab number within the step << 16
+  double exy[kN][12];     // the patch's 8 column and 4 row factors of the Gaussian
+  double2 be[SL][kN];     // per slice: z factor times (cos, sin)
+  double off[12][3];      // k - zi_frac of the patch's columns and rows, k = -1, 0, 1
+  double zoff[kRing][SL]; // the same for the step's slices, per slab
+  float cx[12];           // X' of the columns, Y' of the rows
+  int hc[12];             // their home cells in the atoms' cell code
+};
+
+// exp(-d^2 / 2 sigma^2) for d >= 0, given jf = d / (sigma / 1024) to within about one unit: with
+// d_c = j sigma / 1024 (exact: a power of two and an integer), d^2 - d_c^2 = (d - d_c)(d + d_c)
+// is small, so its exponential is a polynomial, and exp(-d_c^2 / 2 sigma^2) does not depend on
+// sigma: one table for every image, exact to half a unit.  |u| <= 0.003: the degree-4 Taylor
+// polynomial is within 2e-17 where jf is rounded right.  (Table-driven evaluation after Tang,
+// ACM TOMS 15 (1989) 144, here on the distance instead of the exponent.)
+__device__ __forceinline__ double gauss64(double d, float jf, const double* __restrict__ T, double s1024,
+                                          double ni2s2) {
+  jf = fminf(rintf(jf), (float)(kGauss64Size - 1));
+  const int b = __float_as_int(jf);
+  // the FP64 bits of an FP32 integer (a conversion instruction runs on the FP64 pipe); 0 becomes 2^-127
+  const double jd = __hiloint2double((b >> 3) + 0x38000000, b << 29);
+  const double t = __ldg(T + (int)jf);
+  const double del = DF(-jd, s1024, d);
+  const double s = DF(2.0, d, -del);
+  const double u = DM(DM(del, s), ni2s2);
+  double q = DF(u, 1.0 / 24.0, 1.0 / 6.0);
+  q = DF(u, q, 0.5);
+  q = DF(u, q, 1.0);
+  return DF(t, DM(u, q), t);
+}
+
+template <int SL>
+struct Acc {
+  double sr[SL], si[SL];
+  float rm[SL];  // FP32 min of (r^2 - cutoff^2), scaled (density)
+};
+
+// Exact squared distance of kept atom gi (cell code `code`) and this lane's column at slice k of
+// the step, in the reference's operations; +inf outside the lane's 27 cells.
+template <int CAPS, int SL>
+__device__ __forceinline__ double exact_dd(const ColumnParams& p, const WarpSmem<CAPS, SL>& W, int gi, int code, int us,
+                                           int k, int lane) {
+  const int c = lane & 7, r = 8 + (lane >> 3);
+  const int kx = (code & 255) - W.hc[c], ky = ((code >> 8) & 255) - W.hc[r];
+  if (kx < -1 || kx > 1 || ky < -1 || ky > 1) return (double)INFINITY;
+  const double4_32a f = p.f64[gi];
+  const double d0 = DM(p.a11, DA(f.x, W.off[c][kx + 1]));
+  const double d1 = DM(p.a22, DA(f.y, W.off[r][ky + 1]));
+  const double d2 = DM(p.a33, DA(f.z, W.zoff[us][k]));
+  return DA(DA(DM(d0, d0), DM(d1, d1)), DM(d2, d2));
+}
+
+// The buffered atoms: their Gaussian factors (tasks over the lanes), then every lane's sums.
+template <int CAPS, int SL, bool kDens>
+__device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL>& W, int n, float Xv, float Yv,
+                                        float cut2f, const double* __restrict__ T, double s1024, double ni2s2,
+                                        Acc<SL>& A, unsigned& n_acc, int lane) {
+  constexpr float kGrid = 1.1774100225f * 1024.f;  // scaled length -> sigma / 1024
+  __syncwarp();
+  for (int t = lane; t < 12 * n; t += 32) {
+    const int i = t / 12, c = t - 12 * i;
+    const bool x = c < 8;
+    const int2 r = W.ref[i];
+    const int k = min(1, max(-1, (x ? r.y & 255 : (r.y >> 8) & 255) - W.hc[c]));
+    const double f = reinterpret_cast<const double*>(p.f64 + r.x)[x ? 0 : 1];
+    const float2 q = W.xy[i];
+    const float df = fabsf((x ? q.x : q.y) - W.cx[c]);
+    const double d = fabs(DM(x ? p.a11 : p.a22, DA(f, W.off[c][k + 1])));
+    W.exy[i][c] = gauss64(d, df * kGrid, T, s1024, ni2s2);
+  }
+  for (int t = lane; t < SL * n; t += 32) {
+    const int i = t / SL, k = t - SL * i;
+    const int2 r = W.ref[i];
+    const double f = reinterpret_cast<const double*>(p.f64 + r.x)[2];
+    const double2 cs = p.cs64[r.x];
+    const float df = sqrtf(fmaxf(0.f, cut2f - W.hm[i][k]));
+    const double d = fabs(DM(p.a33, DA(f, W.zoff[r.y >> 16][k])));
+    const double e = gauss64(d, df * kGrid, T, s1024, ni2s2);
+    W.be[k][i] = make_double2(DM(e, cs.x), DM(e, cs.y));
+  }
+  __syncwarp();
+  const int c = lane & 7, row = 8 + (lane >> 3);
+  for (int i = 0; i < n; ++i) {
+    const float2 q = W.xy[i];
+    const float dx = q.x - Xv, dy = q.y - Yv;
+    const float h = fmaf(dx, dx, dy * dy);
+    bool acc[SL], near = false;
+    float g[SL];
+#pragma unroll
+    for (int k = 0; k < SL; ++k) {
+      g[k] = h - W.hm[i][k];
+      acc[k] = g[k] <= 0.f;
+      near = near || fabsf(g[k]) <= kGuard64;
+    }
+    if (__any_sync(0xffffffffu, near)) {
+      if (near) {
+        const int2 r = W.ref[i];
+#pragma unroll
+        for (int k = 0; k < SL; ++k)
+          if (fabsf(g[k]) <= kGuard64) acc[k] = exact_dd(p, W, r.x, r.y, r.y >> 16, k, lane) <= p.cut2;
+      }
+      __syncwarp();
+    }
+    unsigned m[SL], any = 0;
+#pragma unroll
+    for (int k = 0; k < SL; ++k) {
+      m[k] = __ballot_sync(0xffffffffu, acc[k]);
+      any |= m[k];
+    }
+    if (!any) continue;
+    const double w = DM(W.exy[i][c], W.exy[i][row]);
+#pragma unroll
+    for (int k = 0; k < SL; ++k) {
+      if (m[k]) {  // the same branch in every lane: a slice no lane accepts costs no FP64
+        const double2 e = W.be[k][i];
+        const double wk = acc[k] ? w : 0.0;
+        A.sr[k] = DF(wk, e.x, A.sr[k]);
+        A.si[k] = DF(wk, e.y, A.si[k]);
+        n_acc += acc[k];
+        if (kDens) A.rm[k] = fminf(A.rm[k], acc[k] ? g[k] : 0.f);
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// rho of convertScaledRangeToRho (:1973-1994), the reference's operations.
+__device__ __forceinline__ double rho64(double r2min, double sig) {
+  if (r2min < DM(sig, sig)) return 1.0;
+  if (r2min > DM(DM(4.0, sig), sig)) return 0.0;
+  const double xx = DS(__ddiv_rn(__dsqrt_rn(r2min), sig), 1.0);
+  const double poly = DA(DS(10.0, DM(15.0, xx)), DM(DM(6.0, xx), xx));
+  return DS(1.0, DM(DM(DM(xx, xx), xx), poly));
+}
+
+// The slices [z_lo, z_hi) of one patch (the 8 x 4 columns of warp tile `tile`): samples to `out`
+// (slice z, lane at out[(z << 5) + lane]).  False when a slab overflows its staging.
+template <int CAPS, int SL, bool kDens, bool kMasked>
+__device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL>& W, int tile, int z_lo, int z_hi,
+                                        double2* __restrict__ out, double* __restrict__ out_rho,
+                                        const double* __restrict__ T, int lane) {
+  constexpr int TX = 8, TY = 4;
+  const int Wd = p.ix1 - p.ix0;
+  const int tiles_x = (Wd + TX - 1) / TX;
+  const int tx = tile % tiles_x, ty = tile / tiles_x;
+  const int ix = p.ix0 + tx * TX + (lane % TX);
+  const int iy = p.iy0 + ty * TY + lane / TX;
+  const bool active = ix < p.ix1 && iy < p.iy1;
+  if constexpr (kMasked) {
+    const bool wanted =
+        active && (!p.tile_mask || p.tile_mask[(iy / p.mask_T) * p.mask_ntx + ix / p.mask_T] != 0);
+    if (!__any_sync(0xffffffffu, wanted)) return true;
+  }
+
+  const double sd = sqrt(p.i2s2 * 1.4426950408889634);
+  Geo G;
+  G.scale = (float)sd;
+  const int ixc = min(ix, p.ix1 - 1), iyc = min(iy, p.iy1 - 1);
+  const int hx = p.xtab[ixc].x, hy = p.ytab[iyc].x;
+  const double fvx = p.xfv[ixc], fvy = p.yfv[iyc];
+  float Xv, Yv;
+  slab::patch_frame(p, G, sd, active, hx, hy, fvx, fvy, Xv, Yv);
+  const float cut2f = (float)(p.cut2 * sd * sd);
+  const float r3 = sqrtf(cut2f) * 1.0001f + 1e-3f;  // z-window half width, rounded up
+  G.pre2 = cut2f * 1.0002f + 1e-2f;
+  const float inv_bin = kBins / G.a33s;
+  const unsigned lt = (1u << lane) - 1;
+  const double s1024 = p.sigma * (1.0 / 1024.0), ni2s2 = -p.i2s2;
+  __syncwarp();  // a previous unit's reads of the tables are done
+  if (lane < 8) {  // k - zi_frac for k = -1, 0, 1 (:1576-1588), per column ...
+    W.cx[lane] = Xv;
+    W.hc[lane] = hx - G.ux_ref + 8;
+    for (int k = 0; k < 3; ++k) W.off[lane][k] = DS((double)(k - 1), fvx);
+  }
+  if ((lane & 7) == 0) {  // ... and row
+    const int r = 8 + (lane >> 3);
+    W.cx[r] = Yv;
+    W.hc[r] = hy - G.uy_ref + 8;
+    for (int k = 0; k < 3; ++k) W.off[r][k] = DS((double)(k - 1), fvy);
+  }
+  // rho changes between sigma and 2 sigma (scaled r^2 - cutoff^2; margins for the FP32 distance)
+  const float sig2 = (float)(p.sigma * p.sigma * sd * sd);
+  const float rm_lo = sig2 - cut2f - kGuard64, rm_hi = 4.f * sig2 - cut2f + kGuard64;
+
+  int ring_lo = 1 << 30, ring_hi = (1 << 30) - 1;
+  unsigned n_acc = 0;
+  unsigned long long n_tst = 0;
+  for (int z0 = z_lo; z0 < z_hi; z0 += SL) {
+    // the step's slices: home z cells, FP32 depths in the frame of home cell hz[0] (the
+    // table gives each pair's from its even slice's home cell)
+    int hz[SL];
+    float zv[SL];
+    bool has[SL];
+#pragma unroll
+    for (int k = 0; k < SL; ++k) {
+      has[k] = z0 + k < p.Mz;
+      const int2 e = p.ztab[has[k] ? z0 + k : z0];
+      hz[k] = has[k] ? e.x : hz[0];
+      zv[k] = has[k] ? __int_as_float(e.y) : 0.f;
+    }
+#pragma unroll
+    for (int k = 2; k < SL; ++k)
+      if (has[k]) zv[k] = __fadd_rn(zv[k], __fmul_rn(G.a33s, (float)(hz[k & ~1] - hz[0])));
+    int hz_last = hz[0];
+#pragma unroll
+    for (int k = 1; k < SL; ++k)
+      if (has[k]) hz_last = hz[k];
+    const int need_lo = hz[0] - 1, need_hi = hz_last + 1;
+    if (need_hi - need_lo + 1 > kRing) {  // the host takes four slices only where they fit
+      if (lane == 0) atomicExch(&p.counters[4], 1ull);
+      return false;
+    }
+    if (need_lo > ring_hi || need_hi < ring_lo) {
+      ring_lo = need_lo;
+      ring_hi = need_lo - 1;
+    }
+    if (ring_lo < need_lo) ring_lo = need_lo;
+    bool ok = true;
+    while (ring_hi < need_hi && ok) {
+      ++ring_hi;
+      ok = load_slab<CAPS, true, true>(p, G, ring_hi, W, lane);
+    }
+    if (!ok) {
+      if (lane == 0) atomicExch(&p.counters[4], 1ull);
+      return false;
+    }
+    __syncwarp();
+    for (int t = lane; t < kRing * SL; t += 32) {
+      const int us = t / SL, k = t - SL * us, z = min(z0 + k, p.Mz - 1);
+      W.zoff[us][k] = DS((double)(need_lo + us - p.ztab[z].x), p.zfv[z]);
+    }
+    Acc<SL> A;
+#pragma unroll
+    for (int k = 0; k < SL; ++k) {
+      A.sr[k] = A.si[k] = 0.0;
+      A.rm[k] = FLT_MAX;
+    }
+    int nb = 0;
+    // per slab of the step: the bins that overlap the depth window of the slices it serves
+    auto window = [&](int u, float* t, bool* v, int& lo, int& hi) {
+      const int slot = u & (kRing - 1);
+      const float zo = __fmul_rn(G.a33s, (float)(u - hz[0]));
+      // the reference's 27 cells in z: slab u serves slice k within one cell of its home cell
+      float w_lo = 1e30f, w_hi = -1e30f;
+#pragma unroll
+      for (int k = 0; k < SL; ++k) {
+        t[k] = __fsub_rn(zv[k], zo);
+        v[k] = has[k] && u - hz[k] >= -1 && u - hz[k] <= 1;
+        if (v[k]) {
+          w_lo = fminf(w_lo, t[k]);
+          w_hi = fmaxf(w_hi, t[k]);
+        }
+      }
+      lo = hi = 0;
+      if (w_lo > w_hi) return;
+      lo = W.bin[slot][max(0, min(kBins, (int)floorf((w_lo - r3) * inv_bin)))];
+      hi = W.bin[slot][max(0, min(kBins, (int)ceilf((w_hi + r3) * inv_bin)))];
+    };
+    for (int u = need_lo; u <= need_hi; ++u) {
+      const int slot = u & (kRing - 1);
+      float t[SL];
+      bool v[SL];
+      int lo, hi;
+      window(u, t, v, lo, hi);
+      for (int b = lo; b < hi; b += 32) {
+        // one atom per lane: kept if some column of the patch can accept it at some slice
+        const int j = b + lane;
+        bool keep = false;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        float hm[SL];
+        if (j < hi) {
+          q = W.p[slot][j];
+          float hmax = kOff;
+#pragma unroll
+          for (int k = 0; k < SL; ++k) {
+            const float dz = q.z - t[k];
+            hm[k] = v[k] ? cut2f - dz * dz : kOff;
+            hmax = fmaxf(hmax, hm[k]);
+          }
+          const float dxr = fmaxf(0.f, fmaxf(G.xmin - q.x, q.x - G.xmax));
+          const float dyr = fmaxf(0.f, fmaxf(G.ymin - q.y, q.y - G.ymax));
+          keep = fmaf(dxr, dxr, dyr * dyr) <= hmax + 2.f * kGuard64;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const int d = nb + __popc(m & lt);
+          W.xy[d] = make_float2(q.x, q.y);
+          W.ref[d] = make_int2(W.gi[slot][j], __float_as_int(q.w) | ((u - need_lo) << 16));
+#pragma unroll
+          for (int k = 0; k < SL; ++k) W.hm[d][k] = hm[k];
+        }
+        nb += __popc(m);
+        if (nb >= kN - 32) {
+          consume<CAPS, SL, kDens>(p, W, nb, Xv, Yv, cut2f, T, s1024, ni2s2, A, n_acc, lane);
+          n_tst += (unsigned long long)nb;
+          nb = 0;
+        }
+      }
+    }
+    if (nb > 0) {
+      consume<CAPS, SL, kDens>(p, W, nb, Xv, Yv, cut2f, T, s1024, ni2s2, A, n_acc, lane);
+      n_tst += (unsigned long long)nb;
+    }
+    // density: where the FP32 minimum lies in rho's range, the exact minimum over the atoms the
+    // FP32 distance cannot tell from the nearest
+    double rho[SL];
+    if constexpr (kDens) {
+      bool want[SL], any = false;
+#pragma unroll
+      for (int k = 0; k < SL; ++k) {
+        rho[k] = !p.use_density || A.rm[k] < rm_lo ? 1.0 : 0.0;
+        want[k] = active && has[k] && p.use_density && A.rm[k] >= rm_lo && A.rm[k] <= fminf(rm_hi, 0.f);
+        any = any || want[k];
+      }
+      if (__any_sync(0xffffffffu, any)) {
+        double best[SL];
+#pragma unroll
+        for (int k = 0; k < SL; ++k) best[k] = DBL_MAX;
+        for (int u = need_lo; u <= need_hi; ++u) {
+          const int slot = u & (kRing - 1);
+          float t[SL];
+          bool v[SL];
+          int lo, hi;
+          window(u, t, v, lo, hi);
+          for (int j = lo; j < hi; ++j) {
+            const float4 q = W.p[slot][j];
+            const float dx = q.x - Xv, dy = q.y - Yv;
+            const float h = fmaf(dx, dx, dy * dy);
+#pragma unroll
+            for (int k = 0; k < SL; ++k) {
+              const float dz = q.z - t[k];
+              if (want[k] && v[k] && h + dz * dz - cut2f <= A.rm[k] + 2.f * kGuard64) {
+                const double dd = exact_dd(p, W, W.gi[slot][j], __float_as_int(q.w), u - need_lo, k, lane);
+                if (dd <= p.cut2 && dd < best[k]) best[k] = dd;
+              }
+            }
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < SL; ++k)
+          if (want[k]) rho[k] = rho64(best[k], p.sigma);
+        __syncwarp();
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < SL; ++k) {
+      if (z0 + k >= z_hi) break;
+      // x = S / max(1e-16, |S|) (:1877-1892); with density, rho x and rho are stored
+      double inv = rsqrt(fmax(DF(A.sr[k], A.sr[k], DM(A.si[k], A.si[k])), 1e-32));
+      if constexpr (kDens) {
+        inv = DM(inv, rho[k]);
+        out_rho[((int64_t)(z0 + k) << 5) + lane] = rho[k];
+      }
+      out[((int64_t)(z0 + k) << 5) + lane] = make_double2(DM(A.sr[k], inv), DM(A.si[k], inv));
+    }
+  }
+  if (p.want_stats) {
+    unsigned long long acc_w = active ? n_acc : 0u, tst_w = active ? (unsigned long long)SL * n_tst : 0u;
+    for (int o = 16; o > 0; o >>= 1) {
+      acc_w += __shfl_xor_sync(0xffffffffu, acc_w, o);
+      tst_w += __shfl_xor_sync(0xffffffffu, tst_w, o);
+    }
+    if (lane == 0) {
+      atomicAdd(&p.counters[2], tst_w);
+      atomicAdd(&p.counters[3], acc_w);
+    }
+  }
+  return true;
+}
+
+template <int CAPS, int SL, bool kDens, bool kMasked, int kMinBlocks>
+__global__ void __launch_bounds__(kWarps * 32, kMinBlocks)
+    k_field64(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R, const double* __restrict__ T) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  WarpSmem<CAPS, SL>& W = reinterpret_cast<WarpSmem<CAPS, SL>*>(smem_raw)[warp];
+  if ((int64_t)R.counters[0] > R.cap) return;  // the binning overflowed: the host retries
+  for (;;) {
+    int unit = 0;
+    if (lane == 0) unit = (int)atomicAdd(R.work, 1u);
+    unit = __shfl_sync(0xffffffffu, unit, 0);
+    if (unit >= R.units()) break;
+    if (R.counters[4] != 0) break;  // a slab overflowed: the host recomputes with larger slabs
+    int patch;
+    const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + unit / R.n_chunks, patch);
+    const int z_lo = unit % R.n_chunks * R.chunk, z_hi = min(J.p.Mz, z_lo + R.chunk);
+    if (z_lo >= z_hi) continue;  // an image less deep than the batch's deepest
+    const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32;
+    if (!field_tile<CAPS, SL, kDens, kMasked>(J.p, W, patch, z_lo, z_hi, (double2*)R.samples + o, R.rho64 + o, T, lane))
+      break;
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// The column integrator
+// ------------------------------------------------------------------------------------------
+
+struct S64 {
+  double c0, cgr, cgi;
+};
+
+// d/dz (phi_0, phi_g) of the two-beam equations (:2375-2380, 2393-2396), fused
+__device__ __forceinline__ void deriv64(const S64& s, double ca, const double* ph, double* d) {
+  d[0] = DF(-s.cgr, ph[3], DF(-s.cgi, ph[2], -DM(s.c0, ph[1])));
+  d[1] = DF(-s.cgi, ph[3], DF(s.cgr, ph[2], DM(s.c0, ph[0])));
+  d[2] = DF(-ca, ph[3], DF(-s.cgr, ph[1], DM(s.cgi, ph[0])));
+  d[3] = DF(ca, ph[2], DF(s.cgi, ph[1], DM(s.cgr, ph[0])));
+}
+
+// One RK4 double step (:2389-2464): phi + dz/3 (k1 + 2 k2 + 2 k3 + k4), dz/3 in two parts so
+// that its rounding does not add up along the column.
+__device__ __forceinline__ void rk4_64(const S64& s0, const S64& s1, const S64& s2, double a, double dz, double dz3h,
+                                       double dz3l, double* ph) {
+  double k1[4], k2[4], k[4], q[4];
+  const double ca1 = DA(s1.c0, a);
+  deriv64(s0, DA(s0.c0, a), ph, k1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) q[i] = DF(k1[i], dz, ph[i]);
+  deriv64(s1, ca1, q, k2);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) q[i] = DF(k2[i], dz, ph[i]);
+  deriv64(s1, ca1, q, k);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    k2[i] = DA(k2[i], k[i]);
+    q[i] = DF(k[i], 2.0 * dz, ph[i]);
+  }
+  deriv64(s2, DA(s2.c0, a), q, k);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double t = DF(2.0, k2[i], DA(k1[i], k[i]));
+    ph[i] = DF(t, dz3h, DF(t, dz3l, ph[i]));
+  }
+}
+
+// A warp per patch and angle (warp w of the CTA takes angles w, w + warps, ...), one lane per
+// column.  Bound by the FP64 pipe: about 90 operations per double step.  The equations are
+// linear, so the reference's renormalisation after every double step (:2466-2472) only
+// scales phi: it is done every 8 steps, and at the end through the quotient (every step when a
+// step could grow phi by more than a small factor).
+template <bool kDens>
+__global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R) {
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x, warp = threadIdx.y, nw = blockDim.y;
+  if ((int64_t)R.counters[0] > R.cap || R.counters[4] != 0) return;
+  int patch;
+  const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + blockIdx.x, patch);
+  const ColumnParams& p = J.p;
+  const int tiles_x = (p.ix1 - p.ix0 + 7) / 8;
+  const int ix = p.ix0 + (patch % tiles_x) * 8 + (lane & 7), iy = p.iy0 + (patch / tiles_x) * 4 + (lane >> 3);
+  const bool active = ix < p.ix1 && iy < p.iy1;
+  bool wanted = active;
+  if (p.tile_mask) wanted = active && p.tile_mask[(iy / p.mask_T) * p.mask_ntx + ix / p.mask_T] != 0;
+  if (!__any_sync(0xffffffffu, wanted)) return;
+  const int64_t o = J.sample_base - R.origin + (int64_t)patch * p.Mz * 32 + lane;
+  const double2* __restrict__ X = (const double2*)R.samples + o;
+  const double* __restrict__ RH = R.rho64 + o;
+  const double dz = p.dz, dz3h = __ddiv_rn(dz, 3.0), dz3l = __ddiv_rn(DF(-3.0, dz3h, dz), 3.0);
+  auto sample = [&](int z) {
+    const double2 x = X[(int64_t)z << 5];
+    const double c0 = kDens ? DM(p.b0, RH[(int64_t)z << 5]) : p.b0;
+    return S64{c0, DM(p.bg, x.x), DM(p.bg, x.y)};
+  };
+  double total = 0.0;
+  for (int k0 = 0; k0 < p.n_prec; k0 += nw) {
+    const int k = k0 + warp;
+    if (k < p.n_prec) {
+      const double a = p.aa[k];
+      const int every = 2.0 * dz * (fabs(p.b0) + fabs(p.bg) + fabs(a)) < 1.0 ? 8 : 1;
+      double ph[4] = {1.0, 0.0, 0.0, 0.0};
+      S64 s0 = sample(0);
+      int n = 0;
+      for (int z = 2; z <= p.Mz; z += 2) {  // the last sample of an even column is the first (:1898-1899)
+        const S64 s1 = sample(z - 1), s2 = sample(z < p.Mz ? z : 0);
+        rk4_64(s0, s1, s2, a, dz, dz3h, dz3l, ph);
+        s0 = s2;
+        if (++n == every) {
+          n = 0;
+          const double inv = rsqrt(DF(ph[3], ph[3], DF(ph[2], ph[2], DF(ph[1], ph[1], DM(ph[0], ph[0])))));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) ph[i] = DM(ph[i], inv);
+        }
+      }
+      const double ig = DF(ph[2], ph[2], DM(ph[3], ph[3]));
+      part[warp][lane] = __ddiv_rn(ig, DF(ph[0], ph[0], DF(ph[1], ph[1], ig)));
+    }
+    __syncthreads();
+    if (warp == 0)
+      for (int w = 0; w < min(nw, p.n_prec - k0); ++w) total = DA(total, part[w][lane]);
+    __syncthreads();
+  }
+  if (warp == 0 && wanted) {
+    if (p.finalize) {  // the precession average and the bright-field flip
+      total = __ddiv_rn(total, p.fin_scale);
+      if (p.fin_bright) total = DS(1.0, total);
+    }
+    p.img[ix + (int64_t)p.Mx * iy] = total;
+  }
+}
+
+template <int CAPS, int SL, bool kDens, bool kMasked, int B>
+cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, const double* T, cudaStream_t st) {
+  const size_t smem = sizeof(WarpSmem<CAPS, SL>) * kWarps;
+  auto kernel = k_field64<CAPS, SL, kDens, kMasked, B>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int grid = sm_count() * B;
+  grid = std::max(1, std::min(grid, (R.units() + kWarps - 1) / kWarps));
+  ++launch_count();
+  kernel<<<grid, kWarps * 32, smem, st>>>(jobs, n_jobs, R, T);
+  return cudaGetLastError();
+}
+
+template <int SL, bool kDens, bool kMasked>
+cudaError_t launch_tier(int tier, const ColumnJob* jobs, int n_jobs, const FieldRange& R, const double* T,
+                        cudaStream_t st) {
+  if (tier >= 2) return launch<256, SL, kDens, kMasked, 1>(jobs, n_jobs, R, T, st);
+  if (tier == 1) return launch<192, SL, kDens, kMasked, 1>(jobs, n_jobs, R, T, st);
+  return launch<128, SL, kDens, kMasked, kField64Blocks>(jobs, n_jobs, R, T, st);
+}
+
+}  // namespace field64
+
+// exp(-(j / 1024)^2 / 2), j = 0 .. kGauss64Size - 1 (the library's exp: correctly rounded but for
+// one value in a few thousand)
+void gauss64_table(double* t) {
+  for (int j = 0; j < kGauss64Size; ++j) t[j] = std::exp(-0.5 * ((double)j / 1024.0) * ((double)j / 1024.0));
+}
+
+cudaError_t launch_field64(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, int slab_tier,
+                           bool density, bool masked, bool four, const double* d_gauss, cudaStream_t st) {
+  using namespace field64;
+  cudaError_t e = cudaMemsetAsync(R.work, 0, sizeof(unsigned), st);
+  if (e != cudaSuccess || R.units() <= 0) return e;
+#define STEM_F64(SL)                                                                                        \
+  (masked ? (density ? launch_tier<SL, true, true>(slab_tier, d_jobs, n_jobs, R, d_gauss, st)               \
+                     : launch_tier<SL, false, true>(slab_tier, d_jobs, n_jobs, R, d_gauss, st))             \
+          : (density ? launch_tier<SL, true, false>(slab_tier, d_jobs, n_jobs, R, d_gauss, st)              \
+                     : launch_tier<SL, false, false>(slab_tier, d_jobs, n_jobs, R, d_gauss, st)))
+  e = four ? STEM_F64(4) : STEM_F64(2);
+#undef STEM_F64
+  if (e != cudaSuccess) return e;
+  const dim3 block(32, std::min(8, max_np));
+  ++launch_count();
+  if (density)
+    k_integrate64<true><<<R.patch_hi - R.patch_lo, block, 0, st>>>(d_jobs, n_jobs, R);
+  else
+    k_integrate64<false><<<R.patch_hi - R.patch_lo, block, 0, st>>>(d_jobs, n_jobs, R);
+  return cudaGetLastError();
+}
+
+}  // namespace stem

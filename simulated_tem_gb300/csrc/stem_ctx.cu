@@ -43,6 +43,9 @@ struct st_ctx {
   ColumnJob* d_coljobs = nullptr;
   size_t cap_coljobs = 0;
   unsigned* d_work = nullptr;
+  void* d_samples = nullptr;  // field samples of one range of patches
+  size_t cap_samples = 0;     // bytes
+  double* d_gauss = nullptr;  // gauss64_table
   double* d_bx = nullptr;  // st_batch: packed atoms of the distinct atom arrays
   size_t cap_bx = 0;
   double* d_bimg = nullptr;  // st_batch: images
@@ -414,6 +417,63 @@ bool ring_eligible(const ColumnParams& cp, bool stats) {
   return cp.a11 >= r3 && cp.a22 >= r3 && cp.Ez <= cp.Mz;
 }
 
+// The sample workspace: `want` bytes, at most kSampleBytes (an image's or batch's columns then run
+// in several ranges); less where the device has no room for that, but at least `least`, one patch.
+constexpr size_t kSampleBytes = (size_t)2 << 30, kMinSampleBytes = (size_t)32 << 20;
+cudaError_t sample_workspace(st_ctx* c, size_t want, size_t least, size_t& room) {
+  room = std::max(std::min(want, kSampleBytes), least);
+  if (c->d_samples && c->cap_samples >= room) return cudaSuccess;
+  if (c->d_samples) cudaFree(c->d_samples);
+  c->d_samples = nullptr;
+  c->cap_samples = 0;
+  for (;;) {
+    const cudaError_t e = cudaMalloc(&c->d_samples, room);
+    if (e == cudaSuccess) {
+      c->cap_samples = room;
+      return e;
+    }
+    if (e != cudaErrorMemoryAllocation || room <= std::max(kMinSampleBytes, least)) return e;
+    cudaGetLastError();
+    room = std::max(room / 2, least);
+  }
+}
+
+// Splits the patches of a batch into ranges of at most `samples` samples.  A unit of work is one
+// patch and `chunk` slices: whole columns where these keep `warps_per_sm` warps on every SM busy
+// four times over (the last ones to finish then cost little), shorter pieces, down to
+// `min_chunk`, where they do not.
+void field_ranges(const std::vector<ColumnJob>& jobs, int n_jobs, int patches, int64_t samples, int deepest,
+                  int warps_per_sm, int min_chunk, std::vector<FieldRange>& out) {
+  out.clear();
+  int chunk = (deepest + 3) & ~3;
+  const int64_t want = 4ll * sm_count() * warps_per_sm;
+  while ((int64_t)patches * ((deepest + chunk - 1) / chunk) < want && chunk > min_chunk)
+    chunk = std::max(min_chunk, (chunk / 2 + 3) & ~3);
+  int job = 0;
+  for (int lo = 0; lo < patches;) {
+    FieldRange R;
+    R.patch_lo = lo;
+    R.chunk = chunk;
+    R.n_chunks = (deepest + chunk - 1) / chunk;
+    auto end_of = [&](int j) { return j + 1 < n_jobs ? jobs[j + 1].tile_base[0] : patches; };
+    while (end_of(job) <= lo) ++job;
+    R.origin = jobs[job].sample_base + (int64_t)(lo - jobs[job].tile_base[0]) * jobs[job].p.Mz * 32;
+    int64_t left = samples;
+    int hi = lo;
+    for (int j = job; j < n_jobs; ++j) {
+      const int64_t per = (int64_t)jobs[j].p.Mz * 32;
+      const int begin = std::max(lo, jobs[j].tile_base[0]), n = end_of(j) - begin;
+      const int64_t fit = std::min<int64_t>(n, left / per);
+      hi = begin + (int)fit;
+      left -= fit * per;
+      if (fit < n) break;
+    }
+    R.patch_hi = std::max(hi, lo + 1);
+    lo = R.patch_hi;
+    out.push_back(R);
+  }
+}
+
 // A recorded call (st_plan): the instantiated graph and what its kernels were recorded with.
 struct GraphOut {
   cudaGraphExec_t exec = nullptr;
@@ -524,8 +584,11 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   }
   const bool ring = !ring_jobs.empty();
   const int n_ring = (int)ring_jobs.size();
-  const int width = fp32 ? 16 : 4;
+  // the FP32 ring marches up to 16 angles per pass; the FP64 field serves any number of angles
+  const int width = fp32 ? 16 : std::max(1, ring_np);
   const int passes = (ring_np + width - 1) / width;
+  int64_t total_samples = 0;
+  int deepest = 1;
   std::vector<ColumnJob> cj;
   std::vector<int> pass_tiles((size_t)passes * kRingShapes, 0);  // per pass, per tile shape
   if (ring) {
@@ -546,6 +609,11 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
         J.p.fin_scale = (double)J.p.n_prec;
         J.p.fin_bright = (flags & ST_FLAG_BRIGHT) ? 1 : 0;
         J.pad = 0;
+        J.sample_base = total_samples;
+        if (!fp32) {
+          total_samples += (int64_t)column_tiles(J.p, 0) * J.p.Mz * 32;
+          deepest = std::max(deepest, J.p.Mz);
+        }
         for (int sh = 0; sh < kRingShapes; ++sh) {
           J.tile_base[sh] = tiles[sh];
           if (J.p.prec_offset < J.p.n_prec) tiles[sh] += column_tiles(J.p, sh);  // fewer angles: none this pass
@@ -609,6 +677,20 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   if (!c->ev_stage) cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming);
   if (c->ev_stage) cudaEventRecord(c->ev_stage, st);
 
+  // ---- ranges of patches whose field samples share one workspace
+  std::vector<FieldRange> ranges;
+  if (ring && !fp32 && total_samples > 0) {
+    const size_t per = dens ? 3 * sizeof(double) : 2 * sizeof(double);
+    size_t room = 0;
+    e = sample_workspace(c, (size_t)total_samples * per, (size_t)deepest * 32 * per, room);
+    if (e != cudaSuccess) return cuda_fail(c, e, "allocating field samples");
+    field_ranges(cj, n_ring, pass_tiles[0], (int64_t)(room / per), deepest, kField64Blocks * 4, 4, ranges);
+    for (FieldRange& R : ranges) {
+      R.samples = c->d_samples;
+      R.rho64 = (double*)c->d_samples + 2 * (room / per);
+    }
+  }
+
   // ---- per-image column launches (general FP32 or FP64 kernel), epilogues, image clearing
   auto columns_per_image = [&](int64_t kept_cap, bool all) -> cudaError_t {
     cudaError_t ce = cudaSuccess;
@@ -617,7 +699,8 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
       ColumnParams cp = cps[i];
       cp.cap = kept_cap;
       if (cp.ix1 <= cp.ix0 || cp.iy1 <= cp.iy0) continue;
-      for (int off = 0; off < cp.n_prec && ce == cudaSuccess; off += width) {
+      const int per_pass = fp32 ? 16 : 4;
+      for (int off = 0; off < cp.n_prec && ce == cudaSuccess; off += per_pass) {
         cp.prec_offset = off;
         cp.accumulate = off > 0 ? 1 : 0;
         ce = fp32 ? launch_column_fp32(cp, st) : launch_column_fp64(cp, st);
@@ -690,10 +773,17 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     for (int pass = 0; ring_ok && pass < passes && ce == cudaSuccess; ++pass) {
       const int np_pass = std::min(width, ring_np - pass * width);
       auto ring_launch = [&](int v) {
-        if (!fp32)
-          return launch_column_fp64_ring(c->d_coljobs + (size_t)pass * n_ring, n_ring,
-                                         pass_tiles[(size_t)pass * kRingShapes], np_pass, big, masked, four64,
-                                         c->d_work, c->s.counters, cap, st);
+        if (!fp32) {
+          cudaError_t le = cudaSuccess;
+          for (FieldRange R : ranges) {
+            R.work = c->d_work;
+            R.counters = c->s.counters;
+            R.cap = cap;
+            if (le == cudaSuccess)
+              le = launch_field64(c->d_coljobs, n_ring, R, ring_np, big, dens, masked, four64, c->d_gauss, st);
+          }
+          return le;
+        }
         return launch_column_fp32_ring(c->d_coljobs + (size_t)pass * n_ring, n_ring,
                                        pass_tiles.data() + (size_t)pass * kRingShapes, np_pass,
                                        dens, stats, v, big, masked, c->d_work, c->s.counters, cap, st);
@@ -865,6 +955,15 @@ extern "C" int st_create(st_ctx** out, int device) {
   c->fp64_general = kv64 && std::strcmp(kv64, "general") == 0;
   const char* ks = std::getenv("STEM_RING_SLABS");
   c->min_slab_tier = !ks ? 0 : std::strcmp(ks, "256") == 0 ? 2 : std::strcmp(ks, "192") == 0 ? 1 : 0;
+  std::vector<double> gauss(kGauss64Size);
+  gauss64_table(gauss.data());
+  e = cudaMalloc((void**)&c->d_gauss, gauss.size() * sizeof(double));
+  if (e == cudaSuccess)
+    e = cudaMemcpy(c->d_gauss, gauss.data(), gauss.size() * sizeof(double), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    st_destroy(c);
+    return ST_ERR_CUDA;
+  }
   *out = c;
   return ST_OK;
 }
@@ -876,7 +975,7 @@ extern "C" void st_destroy(st_ctx* c) {
   void* dev_ptrs[] = {c->s.tmp_key, c->s.tmp_cell, c->s.tmp_slot, c->s.tmp_f, c->s.perm, c->s.block_sums,
                       c->s.counters, c->s.xtab, c->s.xfv, c->s.ytab, c->s.yfv, c->s.ztab, c->s.zfv, c->s.aa,
                       c->s.aaf, c->b.cell_start, c->b.cell_count, c->b.f64, c->b.cs64, c->b.p32, c->b.cs32,
-                      c->b.fr32, c->b.ph32, c->d_x, c->d_img, c->d_blur, c->d_kern, c->d_binjobs, c->d_coljobs, c->d_work, c->d_bx, c->d_bimg,
+                      c->b.fr32, c->b.ph32, c->d_x, c->d_img, c->d_blur, c->d_kern, c->d_binjobs, c->d_coljobs, c->d_work, c->d_samples, c->d_gauss, c->d_bx, c->d_bimg,
                       c->d_lvaux, c->d_levels, c->d_text, c->d_pseg, c->d_pstart, c->d_pbad, c->d_geom, c->d_tilt, c->d_keys, c->d_species};
   for (void* p : dev_ptrs)
     if (p) cudaFree(p);
