@@ -82,11 +82,11 @@ struct Scratch {
   size_t cap_cells = 0;
   size_t cap_blocks = 0;
   // per-image tables of the voxel columns
-  int2* xtab = nullptr;  // (home cell, unused) per ix
+  int2* xtab = nullptr;  // (home cell, FP32 bits of the scaled offset in it) per ix
   double* xfv = nullptr; // fractional voxel offset per ix
   int2* ytab = nullptr;
   double* yfv = nullptr;
-  int2* ztab = nullptr;  // (home cell, FP32 bits of the slab-ring kernel's scaled slice depth) per iz
+  int2* ztab = nullptr;  // (home cell, FP32 bits of the scaled slice depth) per iz
   double* zfv = nullptr;
   size_t cap_x = 0, cap_y = 0, cap_z = 0;
   double* aa = nullptr;
@@ -99,13 +99,13 @@ struct ColumnParams {
   int ix0, ix1, iy0, iy1;
   int Ex, Ey, Ez;
   int n_prec;
-  int prec_offset;  // first precession angle of this pass
-  int accumulate;   // add into img instead of overwriting
+  int prec_offset;  // general kernels: first precession angle of this pass
+  int accumulate;   // general kernels: add into img instead of overwriting
   int use_density;
   int check_cells;  // restrict to the 27 cells around the home cell (needed when a cell is < 3 sigma)
   int trunc_z;      // the z cells are shorter than 3 sigma (the slab ring applies the 27-cell rule in z)
   int want_stats;
-  int finalize;          // the slab ring's last pass: write (sum) / fin_scale, or 1 - that when fin_bright
+  int finalize;          // the slab ring's integrator: write (sum) / fin_scale, or 1 - that when fin_bright
   int fin_bright;
   double fin_scale;
   double a11, a22, a33;  // link-cell sides (cuboid)
@@ -113,6 +113,8 @@ struct ColumnParams {
   double i2s2;           // 1 / (2 sigma^2)
   double sigma;
   double b0, bg, dz;
+  // FP32 scaled lengths (s = sqrt(log2 e / 2 sigma^2)): s, the link-cell sides, (3 sigma)^2, and back to A^2
+  float scale, a11s, a22s, a33s, cut2s, r2_to_A2;
   const int* cell_start;
   const double4_32a* f64;
   const double2* cs64;
@@ -161,79 +163,49 @@ cudaError_t launch_bin_finalize(const BinParams* d_jobs, int n_jobs, int64_t tot
                                 BinnedAtoms& b, bool fp32, cudaStream_t st);
 cudaError_t launch_column_fp32(const ColumnParams& p, cudaStream_t st);
 
-// A job of the persistent slab-ring FP32 column kernels: an image and the first warp
-// tile it owns in the batch's tile sequence, for each tile shape (8 x 4, 4 x 8, 16 x 2).
-constexpr int kRingShapes = 3;
+// A job of the slab-ring field kernels: an image, the first patch (32 pixel columns) it owns in the
+// batch's patch sequence, and its first field sample in the batch's sample sequence (32 per patch
+// and slice).
 struct ColumnJob {
   ColumnParams p;
-  int tile_base[kRingShapes];
+  int patch_base;
   int pad;
-  int64_t sample_base;  // first field sample of the image in the batch's sample sequence (32 per patch and slice)
+  int64_t sample_base;
 };
-int column_tiles(const ColumnParams& p, int shape = 0);  // warp tiles of one image in `shape`
-// The slab-ring launch.  `tiles`: the pass's warp tiles in each shape (host array).
-// `variant` 0 .. ring_variant_count() - 1 selects the kernel, its tile shape, slab
-// capacity and CTAs per SM (ring_variant_name); the images of different variants agree to
-// FP32 rounding, those of one variant to the last bit.  `slab_tier` 1, 2: 192, 256 atoms
-// per slab (dense footprints), with variant 0's 8 x 4 tiles, so at those tiers every
-// variant gives variant 0's bits.  `masked`: some jobs carry a tile mask (then max_np must
-// be 1 and stats false).
-cudaError_t launch_column_fp32_ring(const ColumnJob* d_jobs, int n_jobs, const int* tiles, int max_np, bool density,
-                                    bool stats, int variant, int slab_tier, bool masked, unsigned* work,
-                                    const unsigned long long* counters, int64_t cap, cudaStream_t st);
-int ring_variant_count();
-const char* ring_variant_name(int variant);
-int ring_variant_slab(int variant);  // atoms per slab of the variant's first tier
-int ring_np_bucket(int max_np);  // the kernel template (angles per pass) serving max_np angles
-namespace ring3 {
-// third generation (k_column_v3.cuh), one instance set per angle bucket NP
-struct Ring3Args {
-  const ColumnJob* jobs;
-  int n_jobs;
-  const int* tiles;  // per shape
-  bool density, stats, masked;
-  int variant, tier;
-  unsigned* work;
-  const unsigned long long* counters;
-  int64_t cap;
-  cudaStream_t st;
-};
-template <int NP>
-cudaError_t ring3_launch_np(const Ring3Args& a);
-extern template cudaError_t ring3_launch_np<1>(const Ring3Args&);
-extern template cudaError_t ring3_launch_np<2>(const Ring3Args&);
-extern template cudaError_t ring3_launch_np<4>(const Ring3Args&);
-extern template cudaError_t ring3_launch_np<8>(const Ring3Args&);
-extern template cudaError_t ring3_launch_np<16>(const Ring3Args&);
-}  // namespace ring3
+int field32_patches(const ColumnParams& p);  // 16 x 8 tiles of four patches
+int field64_patches(const ColumnParams& p);  // 8 x 4 patches
 cudaError_t launch_column_fp64(const ColumnParams& p, cudaStream_t st);
 // The voxel field of a range of patches (warp tiles of 32 columns) of a batch, in a workspace of
 // samples: patch by patch in job order, slice by slice, 32 lanes.  The work is handed out in units
 // of one patch and `chunk` slices, so that few patches still fill the GPU.
 struct FieldRange {
-  void* samples = nullptr;  // the field x of a voxel (times rho with density): double2
-  double* rho64 = nullptr;  // with density: rho
+  void* samples = nullptr;  // the field x of a voxel (times rho with density): float2 or double2
+  float* rho32 = nullptr;   // with density: rho
+  double* rho64 = nullptr;
   int64_t origin = 0;       // index of the workspace's first sample in the batch's sample sequence
   int patch_lo = 0, patch_hi = 0;
   int n_chunks = 1;         // per patch: ceil(deepest image / chunk)
   int chunk = 0;            // slices per unit, a multiple of 4
+  int job_lo = 0, n_jobs = 0;  // the range's jobs in the call's job table
+  bool four = true;         // four slices per step (else two)
+  int64_t rho_at = 0;       // where rho starts in the workspace, in values
   unsigned* work = nullptr;
   const unsigned long long* counters = nullptr;
   int64_t cap = 0;
   __host__ __device__ int units() const { return (patch_hi - patch_lo) * n_chunks; }
 };
-// The job of patch `g` (in the batch's patch sequence of tile shape 0) and its number in the job.
+// The job of patch `g` of the batch's patch sequence and its number in the job.
 __device__ __forceinline__ const ColumnJob& field_patch(const ColumnJob* __restrict__ jobs, int n_jobs, int g,
                                                         int& patch) {
   int lo = 0, hi = n_jobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (jobs[mid].tile_base[0] <= g)
+    if (jobs[mid].patch_base <= g)
       lo = mid;
     else
       hi = mid - 1;
   }
-  patch = g - jobs[lo].tile_base[0];
+  patch = g - jobs[lo].patch_base;
   return jobs[lo];
 }
 inline int sm_count() {
@@ -242,6 +214,19 @@ inline int sm_count() {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return sms;
 }
+// The FP32 path's field and integration of one range (k_field32.cu).  `variant` 0 ..
+// ring_variant_count() - 1 selects the patch shape and the slab capacity of tier 0 (named per 8 x 4
+// patch: "slab96" stages 160 atoms per 16 x 8 tile, "slab128" 192); `slab_tier` 1: 352 atoms per tile,
+// 2: 256 atoms per patch, the tiles split into their patches.  Variants of
+// one patch shape give the same image to the last bit; the shapes agree to FP32 rounding.  `four` as
+// below; `masked`: some jobs carry a tile mask (then stats must be false).
+constexpr int kField32Blocks = 5;  // CTAs of four warps per SM at tier 0
+cudaError_t launch_field32(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, bool density,
+                           bool stats, bool masked, bool four, int variant, int slab_tier, cudaStream_t st);
+int ring_variant_count();
+const char* ring_variant_name(int variant);
+int ring_variant_slab(int variant);  // the capacity in the variant's name
+bool ring_variant_same(int variant);  // gives variant 0's image to the last bit
 // The FP64 path's field and integration of one range (k_field64.cu); slab tiers 0, 1, 2 stage
 // 128, 192, 256 atoms; `four`: every job's steps of four slices fit the ring (four_slices_fit);
 // d_gauss: gauss64_table's values.

@@ -600,6 +600,11 @@ cudaError_t launch_tier(int tier, const ColumnJob* jobs, int n_jobs, const Field
 
 }  // namespace field64
 
+int field64_patches(const ColumnParams& p) {
+  const int Wd = p.ix1 - p.ix0, Hd = p.iy1 - p.iy0;
+  return Wd <= 0 || Hd <= 0 ? 0 : ((Wd + 7) / 8) * ((Hd + 3) / 4);
+}
+
 // exp(-(j / 1024)^2 / 2), j = 0 .. kGauss64Size - 1 (the library's exp: correctly rounded but for
 // one value in a few thousand)
 void gauss64_table(double* t) {

@@ -157,6 +157,12 @@ int __float_as_int_host(float v) {
   return b;
 }
 
+// The field kernels' length scale s = sqrt(log2 e / (2 sigma^2)): exp(-r^2 / 2 sigma^2) = 2^-(s r)^2.
+double length_scale(const st_geom* g) {
+  const double i2s2 = 1 / (2 * g->sigma * g->sigma);
+  return std::sqrt(i2s2 * 1.4426950408889634);
+}
+
 bool is_cuboid(const double* m) {
   return m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0 && m[5] == 0.0 && m[6] == 0.0 && m[7] == 0.0;
 }
@@ -164,15 +170,17 @@ bool is_cuboid(const double* m) {
 // Home link cell and fractional offset of voxel index i along one axis:
 // zi = ia * (a_vox * i - lc_delta); h = mod(floor(zi) + 16 N, N); fv = zi - h
 // (Lib_DynamicalTwoBeamImaging.f90:1878-1879, Lib_LinkCell3D.f90:1547-1560).
-void axis_table(int n, double a_vox, double lcd, double ia, int N, int2* tab, double* fv) {
+// The table's .y: the offset within the home cell times a_scaled (the cell side in the field
+// kernels' scaled lengths), as FP32 bits.
+void axis_table(int n, double a_vox, double lcd, double ia, int N, double a_scaled, int2* tab, double* fv) {
   for (int i = 0; i < n; ++i) {
     const double xx = a_vox * (double)i - lcd;
     const double zi = ia * xx;
     int h = (int)std::floor(zi) + 16 * N;
     h = h % N;
     if (h < 0) h += N;  // the reference's mod of a non-negative value
-    tab[i] = make_int2(h, 0);
     fv[i] = zi - (double)h;
+    tab[i] = make_int2(h, __float_as_int_host((float)(a_scaled * fv[i])));
   }
 }
 
@@ -181,8 +189,7 @@ void axis_table(int n, double a_vox, double lcd, double ia, int N, int2* tab, do
 // origin of the home cell of the even slice of its pair (z & ~1), which is the frame the
 // kernel marches in.  Computed in FP64 exactly as a33 (fv + dh) s, rounded once to FP32.
 void depth_table(const st_geom* g, int2* tab, const double* fv) {
-  const double i2s2 = 1 / (2 * g->sigma * g->sigma);
-  const double sd = std::sqrt(i2s2 * 1.4426950408889634);
+  const double sd = length_scale(g);
   const double a33 = g->a_col[8];
   for (int z = 0; z < g->Mz; ++z) {
     const int h_even = tab[z & ~1].x;
@@ -194,7 +201,7 @@ void depth_table(const st_geom* g, int2* tab, const double* fv) {
 bool four_slices_fit(const st_geom* g) {
   std::vector<int2> tab((size_t)g->Mz);
   std::vector<double> fv((size_t)g->Mz);
-  axis_table(g->Mz, g->a_vox[8], g->lc_delta[2], g->ia_col[8], g->Ez, tab.data(), fv.data());
+  axis_table(g->Mz, g->a_vox[8], g->lc_delta[2], g->ia_col[8], g->Ez, 0.0, tab.data(), fv.data());
   for (int z0 = 0; z0 < g->Mz; z0 += 4) {
     const int last = std::min(z0 + 3, g->Mz - 1);
     for (int z = z0 + 1; z <= last; ++z)
@@ -342,6 +349,13 @@ ColumnParams column_params(st_ctx* c, const Job& j, int64_t cell_base, size_t xo
   cp.b0 = g->b0;
   cp.bg = g->bg;
   cp.dz = g->deltaz;
+  const double sd = length_scale(g);
+  cp.scale = (float)sd;
+  cp.a11s = (float)(cp.a11 * sd);
+  cp.a22s = (float)(cp.a22 * sd);
+  cp.a33s = (float)(cp.a33 * sd);
+  cp.cut2s = (float)(cp.cut2 * sd * sd);
+  cp.r2_to_A2 = (float)(1.0 / (sd * sd));
   // link cells narrower than 3 sigma truncate the search to 27 cells: test the cell offsets too
   const double r3 = 3 * g->sigma * (1.0 + 1e-6) + 1e-6;
   cp.check_cells = (cp.a11 < r3 || cp.a22 < r3 || cp.a33 < r3) ? 1 : 0;
@@ -364,11 +378,12 @@ ColumnParams column_params(st_ctx* c, const Job& j, int64_t cell_base, size_t xo
   return cp;
 }
 
-// Times every slab-ring variant once on the same pass (each overwrites the pass's
+// Times the slab-ring variants that give variant 0's image (the others differ from it by FP32
+// rounding, and an image must not depend on a timing) once on the same work (each overwrites the
 // images) and returns the fastest in `best`, or -1 when the binning overflowed (the
 // timings mean nothing then).  A variant whose slabs overflowed its staging is left out
-// (its counter is cleared for the next trial).  The variants' images agree to FP32
-// rounding, not to the bit, so the pass ends with the chosen variant's own output.
+// (its counter is cleared for the next trial), and the launch ends with the chosen variant's
+// output (the last trial's may be incomplete).
 template <typename F>
 cudaError_t tune_ring(st_ctx* c, F&& launch_variant, int64_t cap, cudaStream_t st, int& best) {
   best = -1;
@@ -381,6 +396,7 @@ cudaError_t tune_ring(st_ctx* c, F&& launch_variant, int64_t cap, cudaStream_t s
   unsigned long long h[5];
   int last = -1;  // the last trial that ran (its output, whole or partial, is in the images)
   for (int v = 0; v < nv && e == cudaSuccess; ++v) {
+    if (!ring_variant_same(v)) continue;
     cudaEventRecord(c->tev[0], st);
     e = launch_variant(v);
     last = v;
@@ -438,37 +454,46 @@ cudaError_t sample_workspace(st_ctx* c, size_t want, size_t least, size_t& room)
   }
 }
 
-// Splits the patches of a batch into ranges of at most `samples` samples.  A unit of work is one
-// patch and `chunk` slices: whole columns where these keep `warps_per_sm` warps on every SM busy
-// four times over (the last ones to finish then cost little), shorter pieces, down to
-// `min_chunk`, where they do not.
-void field_ranges(const std::vector<ColumnJob>& jobs, int n_jobs, int patches, int64_t samples, int deepest,
-                  int warps_per_sm, int min_chunk, std::vector<FieldRange>& out) {
-  out.clear();
+// Slices per unit of work (a multiple of 4) of `tiles` tiles up to `deepest` slices deep, `per_sm` of
+// which an SM works on at a time: whole columns where these keep the GPU busy four times over (the
+// last ones to finish then cost little), else shorter pieces.  Every piece stages its own slabs, so
+// pieces below 16 slices are only taken while the GPU is not full once.
+int depth_chunk(int64_t tiles, int deepest, int per_sm) {
+  const int64_t full = (int64_t)sm_count() * per_sm;
   int chunk = (deepest + 3) & ~3;
-  const int64_t want = 4ll * sm_count() * warps_per_sm;
-  while ((int64_t)patches * ((deepest + chunk - 1) / chunk) < want && chunk > min_chunk)
-    chunk = std::max(min_chunk, (chunk / 2 + 3) & ~3);
+  for (;;) {
+    const int64_t units = tiles * ((deepest + chunk - 1) / chunk);
+    const bool enough = chunk > 16 ? units >= 4 * full : units >= full;
+    if (enough || chunk <= 4) return chunk;
+    chunk = (chunk / 2 + 3) & ~3;
+  }
+}
+
+// Splits the patches of a batch into ranges of at most `samples` samples, cut at multiples of
+// `align` patches of an image.
+void field_ranges(const ColumnJob* jobs, int n_jobs, int patches, int64_t samples, int align, int chunk,
+                  int deepest, std::vector<FieldRange>& out) {
+  out.clear();
   int job = 0;
   for (int lo = 0; lo < patches;) {
     FieldRange R;
     R.patch_lo = lo;
     R.chunk = chunk;
     R.n_chunks = (deepest + chunk - 1) / chunk;
-    auto end_of = [&](int j) { return j + 1 < n_jobs ? jobs[j + 1].tile_base[0] : patches; };
+    auto end_of = [&](int j) { return j + 1 < n_jobs ? jobs[j + 1].patch_base : patches; };
     while (end_of(job) <= lo) ++job;
-    R.origin = jobs[job].sample_base + (int64_t)(lo - jobs[job].tile_base[0]) * jobs[job].p.Mz * 32;
+    R.origin = jobs[job].sample_base + (int64_t)(lo - jobs[job].patch_base) * jobs[job].p.Mz * 32;
     int64_t left = samples;
     int hi = lo;
     for (int j = job; j < n_jobs; ++j) {
       const int64_t per = (int64_t)jobs[j].p.Mz * 32;
-      const int begin = std::max(lo, jobs[j].tile_base[0]), n = end_of(j) - begin;
-      const int64_t fit = std::min<int64_t>(n, left / per);
+      const int begin = std::max(lo, jobs[j].patch_base), n = end_of(j) - begin;
+      const int64_t fit = std::min<int64_t>(n, left / per / align * align);
       hi = begin + (int)fit;
       left -= fit * per;
       if (fit < n) break;
     }
-    R.patch_hi = std::max(hi, lo + 1);
+    R.patch_hi = std::max(hi, lo + align);  // the workspace holds at least `align` of the deepest
     lo = R.patch_hi;
     out.push_back(R);
   }
@@ -582,44 +607,40 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
       for (int r : ring_jobs) dens = dens || cps[r].use_density;
     }
   }
+  // images whose steps of four slices fit the slab ring first: the others march two per step, in
+  // launches of their own, so that an image's result does not depend on the rest of its batch
+  const int n_four = (int)(std::stable_partition(ring_jobs.begin(), ring_jobs.end(),
+                                                 [&](int i) { return four_slices_fit(jobs[i].g); }) -
+                           ring_jobs.begin());
   const bool ring = !ring_jobs.empty();
   const int n_ring = (int)ring_jobs.size();
-  // the FP32 ring marches up to 16 angles per pass; the FP64 field serves any number of angles
-  const int width = fp32 ? 16 : std::max(1, ring_np);
-  const int passes = (ring_np + width - 1) / width;
-  int64_t total_samples = 0;
-  int deepest = 1;
+  // the jobs of the field kernels, with the first patch and field sample of each; the integrator
+  // takes all angles of an image at once
   std::vector<ColumnJob> cj;
-  std::vector<int> pass_tiles((size_t)passes * kRingShapes, 0);  // per pass, per tile shape
+  int64_t tune_tiles = 0;  // 8 x 4 tiles
+  int64_t total_samples[2] = {0, 0}, total_patches[2] = {0, 0};  // four, two slices per step
+  int deepest[2] = {1, 1};
   if (ring) {
     // the density variant of the kernel serves every image of the launch when any image uses it;
     // an image without the density field then gets rho = 1 from use_density = 0 in the sample
-    cj.resize((size_t)n_ring * passes);
-    for (int pass = 0; pass < passes; ++pass) {
-      int tiles[kRingShapes] = {0, 0, 0};
-      for (int r = 0; r < n_ring; ++r) {
-        ColumnJob& J = cj[(size_t)pass * n_ring + r];
-        J.p = cps[ring_jobs[r]];
-        J.p.prec_offset = pass * width;
-        J.p.accumulate = pass > 0 ? 1 : 0;
-        // the average (and bright-field flip) in the store of the image's last pass, unless
-        // the image is tile-masked (its epilogue also covers the columns the mask leaves)
-        J.p.finalize = (flags & ST_FLAG_AVERAGE) && !J.p.tile_mask && J.p.prec_offset < J.p.n_prec &&
-                       J.p.prec_offset + width >= J.p.n_prec;
-        J.p.fin_scale = (double)J.p.n_prec;
-        J.p.fin_bright = (flags & ST_FLAG_BRIGHT) ? 1 : 0;
-        J.pad = 0;
-        J.sample_base = total_samples;
-        if (!fp32) {
-          total_samples += (int64_t)column_tiles(J.p, 0) * J.p.Mz * 32;
-          deepest = std::max(deepest, J.p.Mz);
-        }
-        for (int sh = 0; sh < kRingShapes; ++sh) {
-          J.tile_base[sh] = tiles[sh];
-          if (J.p.prec_offset < J.p.n_prec) tiles[sh] += column_tiles(J.p, sh);  // fewer angles: none this pass
-        }
-      }
-      for (int sh = 0; sh < kRingShapes; ++sh) pass_tiles[(size_t)pass * kRingShapes + sh] = tiles[sh];
+    cj.resize((size_t)n_ring);
+    for (int r = 0; r < n_ring; ++r) {
+      ColumnJob& J = cj[r];
+      J.p = cps[ring_jobs[r]];
+      // the average (and bright-field flip) in the integrator's store, unless the image is
+      // tile-masked (its epilogue also covers the columns the mask leaves)
+      J.p.finalize = (flags & ST_FLAG_AVERAGE) && !J.p.tile_mask;
+      J.p.fin_scale = (double)J.p.n_prec;
+      J.p.fin_bright = (flags & ST_FLAG_BRIGHT) ? 1 : 0;
+      J.pad = 0;
+      const int grp = r < n_four ? 0 : 1;
+      J.patch_base = (int)total_patches[grp];
+      J.sample_base = total_samples[grp];
+      const int np = fp32 ? field32_patches(J.p) : field64_patches(J.p);
+      total_patches[grp] += np;
+      tune_tiles += field64_patches(J.p);
+      total_samples[grp] += (int64_t)np * J.p.Mz * 32;
+      deepest[grp] = std::max(deepest[grp], J.p.Mz);
     }
   }
 
@@ -649,9 +670,10 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   ColumnJob* hcj = (ColumnJob*)(hjobs + (size_t)n * sizeof(BinParams));
   for (int i = 0; i < n; ++i) {
     const st_geom* g = jobs[i].g;
-    axis_table(g->Mx, g->a_vox[0], g->lc_delta[0], g->ia_col[0], g->Ex, hxt + xoff[i], hxf + xoff[i]);
-    axis_table(g->My, g->a_vox[4], g->lc_delta[1], g->ia_col[4], g->Ey, hyt + yoff[i], hyf + yoff[i]);
-    axis_table(g->Mz, g->a_vox[8], g->lc_delta[2], g->ia_col[8], g->Ez, hzt + zoff[i], hzf + zoff[i]);
+    const double sd = length_scale(g);
+    axis_table(g->Mx, g->a_vox[0], g->lc_delta[0], g->ia_col[0], g->Ex, g->a_col[0] * sd, hxt + xoff[i], hxf + xoff[i]);
+    axis_table(g->My, g->a_vox[4], g->lc_delta[1], g->ia_col[4], g->Ey, g->a_col[4] * sd, hyt + yoff[i], hyf + yoff[i]);
+    axis_table(g->Mz, g->a_vox[8], g->lc_delta[2], g->ia_col[8], g->Ez, g->a_col[8] * sd, hzt + zoff[i], hzf + zoff[i]);
     depth_table(g, hzt + zoff[i], hzf + zoff[i]);
     for (int k = 0; k < jobs[i].n_prec; ++k) {
       haa[aoff[i] + k] = jobs[i].aa[k];
@@ -679,15 +701,27 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
 
   // ---- ranges of patches whose field samples share one workspace
   std::vector<FieldRange> ranges;
-  if (ring && !fp32 && total_samples > 0) {
-    const size_t per = dens ? 3 * sizeof(double) : 2 * sizeof(double);
+  for (int grp = 0; grp < 2; ++grp) {
+    if (total_samples[grp] == 0) continue;
+    const size_t value = fp32 ? sizeof(float) : sizeof(double), per = (dens ? 3 : 2) * value;
+    const int align = fp32 ? 4 : 1;  // patches of an FP32 tile stay together
+    const size_t least = (size_t)deepest[grp] * 32 * align * per;
     size_t room = 0;
-    e = sample_workspace(c, (size_t)total_samples * per, (size_t)deepest * 32 * per, room);
+    e = sample_workspace(c, (size_t)std::max(total_samples[0], total_samples[1]) * per, least, room);
     if (e != cudaSuccess) return cuda_fail(c, e, "allocating field samples");
-    field_ranges(cj, n_ring, pass_tiles[0], (int64_t)(room / per), deepest, kField64Blocks * 4, 4, ranges);
-    for (FieldRange& R : ranges) {
-      R.samples = c->d_samples;
-      R.rho64 = (double*)c->d_samples + 2 * (room / per);
+    const int64_t n_room = (int64_t)(room / per) & ~(int64_t)31;
+    const int lo = grp ? n_four : 0, hi = grp ? n_ring : n_four;
+    std::vector<FieldRange> part;
+    field_ranges(cj.data() + lo, hi - lo, (int)total_patches[grp], n_room, align,
+                 fp32 ? depth_chunk(total_patches[grp] / 4, deepest[grp], kField32Blocks)
+                      : depth_chunk(total_patches[grp], deepest[grp], 4 * kField64Blocks),
+                 deepest[grp], part);
+    for (FieldRange& R : part) {
+      R.job_lo = lo;
+      R.n_jobs = hi - lo;
+      R.four = grp == 0;
+      R.rho_at = 2 * n_room;
+      ranges.push_back(R);
     }
   }
 
@@ -715,7 +749,7 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     for (int i = 0; i < n && ce == cudaSuccess; ++i) {
       const st_geom* g = jobs[i].g;
       if (g->ix1 <= g->ix0 || g->iy1 <= g->iy0) continue;
-      if (ring_ok && on_ring[i] && !cps[i].tile_mask) continue;  // finished by the ring's last pass
+      if (ring_ok && on_ring[i] && !cps[i].tile_mask) continue;  // finished by the ring's integrator
       ce = launch_epilogue(jobs[i].d_img, g->Mx, g->My, g->ix0, g->ix1, g->iy0, g->iy1, (double)jobs[i].n_prec,
                            (flags & ST_FLAG_BRIGHT) ? 1 : 0, st);
     }
@@ -737,29 +771,20 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   // epilogues and the read-back of the counters.  `capturing`: no events, no tuning
   // (the variants and the kernel choice of the eager run are replayed).
   const bool stats = (flags & ST_FLAG_STATS) != 0;
-  std::vector<int> pass_variant(passes, 0);
-  // a pass's kind (angles per pass, density, precision) and the shape of its images (the first
-  // ring image's image and link-cell dimensions): the key of the slab tier an earlier call of
-  // this context needed, and of the variant it tuned
-  auto big_key = [&](int pass) -> uint64_t {
-    uint64_t h = (uint64_t)(ring_np_bucket(std::min(width, ring_np - pass * width)) * 2 + (dens ? 1 : 0)) +
-                 (fp32 ? 0u : 1000u);
-    if (!ring_jobs.empty()) {
-      const st_geom* g = jobs[ring_jobs[0]].g;
-      const int dims[6] = {g->Mx, g->My, g->Mz, g->Ex, g->Ey, g->Ez};
-      for (int d : dims) h = h * 1000003ull + (uint64_t)d;
-    }
-    return h;
-  };
-  int big = c->min_slab_tier;  // slab tier: 128, 192, 256 atoms
-  for (int pass = 0; pass < passes; ++pass) {
-    auto it = c->ring_big.find(big_key(pass));
-    if (it != c->ring_big.end()) big = std::max(big, it->second);
+  int ring_variant = 0;
+  // the launch's kind (density, precision) and the shape of its images (the first ring image's
+  // image and link-cell dimensions): the key of the slab tier an earlier call of this context
+  // needed, and of the variant it tuned
+  uint64_t key = (dens ? 1u : 0u) + (fp32 ? 0u : 2u);
+  if (!ring_jobs.empty()) {
+    const st_geom* g = jobs[ring_jobs[0]].g;
+    const int dims[6] = {g->Mx, g->My, g->Mz, g->Ex, g->Ey, g->Ez};
+    for (int d : dims) key = key * 1000003ull + (uint64_t)d;
   }
+  int big = c->min_slab_tier;  // slab tier: 128, 192, 256 atoms
+  if (auto it = c->ring_big.find(key); it != c->ring_big.end()) big = std::max(big, it->second);
   bool masked = false;  // tile-masked ring jobs take the masked kernel instances
   for (int r : ring_jobs) masked = masked || cps[r].tile_mask != nullptr;
-  bool four64 = !fp32 && !ring_jobs.empty();  // the FP64 ring marches four slices per step where all fit
-  for (int r : ring_jobs) four64 = four64 && four_slices_fit(jobs[r].g);
   // with_bin false: the column phase only, on the binning already in place
   auto enqueue = [&](bool capturing, bool with_bin) -> cudaError_t {
     cudaError_t ce = cudaSuccess;
@@ -770,52 +795,46 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     }
     if (ce == cudaSuccess) ce = clear_images();
     if (!capturing) cudaEventRecord(c->ev[1], st);
-    for (int pass = 0; ring_ok && pass < passes && ce == cudaSuccess; ++pass) {
-      const int np_pass = std::min(width, ring_np - pass * width);
-      auto ring_launch = [&](int v) {
-        if (!fp32) {
-          cudaError_t le = cudaSuccess;
-          for (FieldRange R : ranges) {
-            R.work = c->d_work;
-            R.counters = c->s.counters;
-            R.cap = cap;
-            if (le == cudaSuccess)
-              le = launch_field64(c->d_coljobs, n_ring, R, ring_np, big, dens, masked, four64, c->d_gauss, st);
-          }
-          return le;
-        }
-        return launch_column_fp32_ring(c->d_coljobs + (size_t)pass * n_ring, n_ring,
-                                       pass_tiles.data() + (size_t)pass * kRingShapes, np_pass,
-                                       dens, stats, v, big, masked, c->d_work, c->s.counters, cap, st);
-      };
-      if (capturing) {
-        ce = ring_launch(pass_variant[pass]);
-        continue;
+    auto ring_launch = [&](int v) {
+      cudaError_t le = cudaSuccess;
+      for (FieldRange R : ranges) {
+        R.samples = c->d_samples;
+        R.rho32 = (float*)c->d_samples + R.rho_at;
+        R.rho64 = (double*)c->d_samples + R.rho_at;
+        R.work = c->d_work;
+        R.counters = c->s.counters;
+        R.cap = cap;
+        if (le != cudaSuccess) break;
+        const ColumnJob* dj = c->d_coljobs + R.job_lo;
+        le = fp32 ? launch_field32(dj, R.n_jobs, R, ring_np, dens, stats, masked, R.four, v, big, st)
+                  : launch_field64(dj, R.n_jobs, R, ring_np, big, dens, masked, R.four, c->d_gauss, st);
       }
-      // the variant tuned for this kind of pass (angles, density) on images of this shape
-      const uint64_t key = big_key(pass);
-      int v = 0;
-      if (c->tune_mode >= 0 && fp32) {
-        v = c->tune_mode;
-      } else if (c->tune_mode == ST_TUNE_AUTO && !stats && fp32) {  // the FP64 ring has one variant
-        auto it = c->ring_tuned.find(key);
-        if (it != c->ring_tuned.end()) {
-          v = it->second;
-        } else if (pass == 0 && pass_tiles[0] >= 4096 && !big && !masked) {
-          // autotune on the real work: the first pass overwrites its images, and the tuner
-          // ends with the chosen variant's output; keep it for the later calls of this context
-          ce = tune_ring(c, ring_launch, cap, st, v);
-          if (ce == cudaSuccess && v >= 0) {
-            c->ring_tuned[key] = v;
-            pass_variant[pass] = v;
-            continue;
+      return le;
+    };
+    if (ring_ok && ce == cudaSuccess) {
+      int v = ring_variant;
+      bool done = false;
+      if (!capturing) {  // a recorded launch replays the eager run's variant
+        v = 0;
+        if (c->tune_mode >= 0 && fp32) {
+          v = c->tune_mode;
+        } else if (c->tune_mode == ST_TUNE_AUTO && !stats && fp32) {  // the FP64 path has one variant
+          auto it = c->ring_tuned.find(key);
+          if (it != c->ring_tuned.end()) {
+            v = it->second;
+          } else if (tune_tiles >= 4096 && !big && !masked) {
+            // autotune on the real work: the launch overwrites its images, and the tuner
+            // ends with the chosen variant's output; keep it for the later calls of this context
+            ce = tune_ring(c, ring_launch, cap, st, v);
+            done = ce == cudaSuccess && v >= 0;
+            if (done) c->ring_tuned[key] = v;
+            else v = 0;
           }
-          v = 0;
         }
+        ring_variant = v;
+        c->last_ring_variant = stats ? 0 : v;
       }
-      if (ce == cudaSuccess) ce = ring_launch(v);
-      pass_variant[pass] = v;
-      c->last_ring_variant = stats ? 0 : v;
+      if (!done && ce == cudaSuccess) ce = ring_launch(v);
     }
     if (ce == cudaSuccess && (!ring_ok || n_ring < n)) ce = columns_per_image(cap, !ring_ok);
     if (ce == cudaSuccess) ce = epilogues();
@@ -851,7 +870,7 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
       // (192, then 256 atoms), and this context keeps it for these kinds of pass on images
       // of this shape
       ++big;
-      for (int pass = 0; pass < passes; ++pass) c->ring_big[big_key(pass)] = big;
+      c->ring_big[key] = big;
       cudaMemsetAsync(c->s.counters + 2, 0, 3 * sizeof(unsigned long long), st);
       e = enqueue(false, false);
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);
