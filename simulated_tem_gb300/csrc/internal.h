@@ -77,7 +77,7 @@ struct Scratch {
   double4_32a* tmp_f = nullptr; // fx, fy, fz, g.y (FP64 path); Rec32 (FP32 path)
   int* perm = nullptr;      // position-in-cell -> tmp index
   int* block_sums = nullptr;
-  unsigned long long* counters = nullptr;  // [0] kept, [1] max cell count, [2] tests, [3] accepted, [4] slab overflow
+  unsigned long long* counters = nullptr;  // [0] kept, [1] max cell count, [2] tests, [3] accepted, [4] slab overflow, [5] units of field work handed out
   size_t cap_candidates = 0;
   size_t cap_cells = 0;
   size_t cap_blocks = 0;
@@ -88,10 +88,8 @@ struct Scratch {
   double* yfv = nullptr;
   int2* ztab = nullptr;  // (home cell, FP32 bits of the scaled slice depth) per iz
   double* zfv = nullptr;
-  size_t cap_x = 0, cap_y = 0, cap_z = 0;
   double* aa = nullptr;
   float* aaf = nullptr;
-  size_t cap_prec = 0;
 };
 
 struct ColumnParams {
@@ -189,7 +187,7 @@ struct FieldRange {
   int job_lo = 0, n_jobs = 0;  // the range's jobs in the call's job table
   bool four = true;         // four slices per step (else two)
   int64_t rho_at = 0;       // where rho starts in the workspace, in values
-  unsigned* work = nullptr;
+  unsigned* work = nullptr;  // units handed out: zero before the field kernel, zeroed again by the integrator
   const unsigned long long* counters = nullptr;
   int64_t cap = 0;
   __host__ __device__ int units() const { return (patch_hi - patch_lo) * n_chunks; }

@@ -32,6 +32,8 @@
 // insertion order, so the result is deterministic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "internal.h"
 
 namespace stem {
@@ -214,7 +216,10 @@ __device__ __forceinline__ bool decide(const BinParams& p, const AtomFix& a, int
   return keep;
 }
 
-// FP32 path: one thread per atom, all replicas.  Warps stay converged: every lane runs
+// FP32 path: one thread per atom and share of the replicas (blockIdx.y of gridDim.y; all of them
+// where the atoms alone fill the GPU twice over: the FP64 part is done once per thread).  A few
+// thousand atoms are bound by the chain of replicas, each with its atomics.  Warps stay converged:
+// every lane runs
 // the same replica loop, lanes past the end or past their job's replicas keep nothing.
 // (Counting first and claiming one compaction range per block halves the atomics on the
 // kept-atom counter but decides every candidate twice: slower.)
@@ -258,7 +263,7 @@ __global__ void __launch_bounds__(256) k_bin_atoms_fp32(const BinParams* __restr
     a.v1 = (float)(int)(a.q1 >> 20) * 1.52587890625e-05f;
     a.v2 = (float)(int)(a.q2 >> 20) * 1.52587890625e-05f;
     const int nmax = __reduce_max_sync(0xffffffffu, nrep);
-    for (int nn = 0; nn < nmax; ++nn) {
+    for (int nn = blockIdx.y; nn < nmax; nn += gridDim.y) {
       const bool cand = nn < nrep && prefilter(p, a, nn);
       if (__any_sync(0xffffffffu, cand)) {
         long long c[3] = {0, 0, 0}, gt = 0;
@@ -328,25 +333,74 @@ __global__ void __launch_bounds__(256) k_scan_blocks(const int* __restrict__ cou
   }
 }
 
-__global__ void __launch_bounds__(1024) k_scan_top(int* __restrict__ block_sums, int nb) {
-  __shared__ int buf[1024];
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
+// The whole scan in one CTA, for up to kSmallScan cells: each thread sums and then writes a run
+// of consecutive counts.  Three launches of a few microseconds each become one; with the shares of
+// k_bin_atoms_fp32 the binning of a 1.6k-atom image goes from 76 to 33 us.
+constexpr int kSmallScan = 1024 * 16;
+__global__ void __launch_bounds__(1024) k_scan_small(const int* __restrict__ counts, int n, int* __restrict__ start,
+                                                     unsigned long long* __restrict__ counters) {
+  __shared__ int warp_sums[32];
+  __shared__ int warp_max[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (n + 1023) / 1024, base = threadIdx.x * per;
+  int v[kSmallScan / 1024], s = 0, m = 0;
+#pragma unroll
+  for (int i = 0; i < kSmallScan / 1024; ++i) {
+    v[i] = i < per && base + i < n ? counts[base + i] : 0;
+    s += v[i];
+    m = max(m, v[i]);
+  }
+  int incl = s;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += a;
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (lane == 31) warp_sums[warp] = incl;
+  if (lane == 0) warp_max[warp] = m;
   __syncthreads();
+  const int w = warp_sums[lane];  // every warp scans the 32 warp sums
+  int wi = w;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, wi, o);
+    if (lane >= o) wi += a;
+  }
+  int run = __shfl_sync(0xffffffffu, wi - w, warp) + incl - s;
+#pragma unroll
+  for (int i = 0; i < kSmallScan / 1024; ++i) {
+    if (i < per && base + i < n) start[base + i] = run;
+    run += v[i];
+  }
+  if (threadIdx.x == 1023) start[n] = run;
+  if (warp == 0) {
+    const int mm = __reduce_max_sync(0xffffffffu, warp_max[lane]);
+    if (lane == 0) counters[1] = (unsigned long long)mm;
+  }
+}
+
+__global__ void __launch_bounds__(1024) k_scan_top(int* __restrict__ block_sums, int nb) {
+  __shared__ int warp_sums[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int carry = 0;
   for (int off = 0; off < nb; off += 1024) {
     const int i = off + threadIdx.x;
     const int v = (i < nb) ? block_sums[i] : 0;
-    buf[threadIdx.x] = v;
-    __syncthreads();
-    for (int d = 1; d < 1024; d <<= 1) {
-      const int a = (threadIdx.x >= d) ? buf[threadIdx.x - d] : 0;
-      __syncthreads();
-      buf[threadIdx.x] += a;
-      __syncthreads();
+    int incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += a;
     }
-    if (i < nb) block_sums[i] = carry + buf[threadIdx.x] - v;  // exclusive
+    if (lane == 31) warp_sums[warp] = incl;
     __syncthreads();
-    if (threadIdx.x == 1023) carry += buf[1023];
+    const int w = warp_sums[lane];
+    int wi = w;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= o) wi += a;
+    }
+    const int before = __shfl_sync(0xffffffffu, wi - w, warp);
+    if (i < nb) block_sums[i] = carry + before + incl - v;  // exclusive
+    carry += __shfl_sync(0xffffffffu, wi, 31);
     __syncthreads();
   }
 }
@@ -459,18 +513,25 @@ cudaError_t launch_bin(const BinParams* d_jobs, int n_jobs, int64_t total_atoms,
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // shares of the replicas: until there are two waves of threads
+  const int64_t want = (int64_t)sms * 2048 * 2;
+  const int shares = (int)std::max<int64_t>(1, std::min<int64_t>(27, want / std::max<int64_t>(1, total_atoms)));
   if (fp32)
-    k_bin_atoms_fp32<<<grid_for(total_atoms, 256, sms * 16), 256, 0, st>>>(
+    k_bin_atoms_fp32<<<dim3(grid_for(total_atoms, 256, sms * 16), shares), 256, 0, st>>>(
         d_jobs, n_jobs, total_atoms, cap, b.cell_count, s.tmp_key, s.tmp_cell, s.tmp_slot,
         reinterpret_cast<Rec32*>(s.tmp_f), s.counters);
   else
     k_bin_transform_exact<<<grid_for(total_cand, 256, sms * 16), 256, 0, st>>>(
         d_jobs, n_jobs, total_cand, cap, b.cell_count, s.tmp_key, s.tmp_cell, s.tmp_slot, s.tmp_f, s.counters);
   const int nb = (int)((total_cells + kScanBlock - 1) / kScanBlock);
-  launch_count() += 5;  // the kernel above, three scans and the placement
-  k_scan_blocks<<<nb, 256, 0, st>>>(b.cell_count, total_cells, s.block_sums, s.counters);
-  k_scan_top<<<1, 1024, 0, st>>>(s.block_sums, nb);
-  k_scan_final<<<nb, 256, 0, st>>>(b.cell_count, total_cells, s.block_sums, b.cell_start);
+  launch_count() += total_cells <= kSmallScan ? 3 : 5;  // the kernel above, the scans and the placement
+  if (total_cells <= kSmallScan) {
+    k_scan_small<<<1, 1024, 0, st>>>(b.cell_count, (int)total_cells, b.cell_start, s.counters);
+  } else {
+    k_scan_blocks<<<nb, 256, 0, st>>>(b.cell_count, total_cells, s.block_sums, s.counters);
+    k_scan_top<<<1, 1024, 0, st>>>(s.block_sums, nb);
+    k_scan_final<<<nb, 256, 0, st>>>(b.cell_count, total_cells, s.block_sums, b.cell_start);
+  }
   k_bin_place<<<sms * 8, 256, 0, st>>>(s.tmp_cell, s.tmp_slot, b.cell_start, s.counters, cap, s.perm);
   return cudaGetLastError();
 }

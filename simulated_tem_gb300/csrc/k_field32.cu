@@ -825,6 +825,7 @@ __device__ __forceinline__ int renorm_every(const ColumnParams& p, float a_max) 
 template <int TX, bool kDens>
 __global__ void __launch_bounds__(128) k_integrate32(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R) {
   const int lane = threadIdx.x, g = R.patch_lo + blockIdx.x * 4 + threadIdx.y;
+  if (g == R.patch_lo && lane == 0) *R.work = 0;  // for the next field kernel
   if ((int64_t)R.counters[0] > R.cap || R.counters[4] != 0 || g >= R.patch_hi) return;
   int patch;
   const ColumnJob& J = field_patch(jobs, n_jobs, g, patch);
@@ -845,6 +846,7 @@ __global__ void __launch_bounds__(128) k_integrate32_multi(const ColumnJob* __re
                                                            FieldRange R) {
   __shared__ float part[16][32];
   const int lane = threadIdx.x, warp = threadIdx.y;
+  if (blockIdx.x == 0 && warp == 0 && lane == 0) *R.work = 0;  // for the next field kernel
   if ((int64_t)R.counters[0] > R.cap || R.counters[4] != 0) return;
   int patch;
   const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + blockIdx.x, patch);
@@ -961,8 +963,8 @@ const char* ring_variant_name(int variant) {
 cudaError_t launch_field32(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, bool density,
                            bool stats, bool masked, bool four, int variant, int slab_tier, cudaStream_t st) {
   if (masked && stats) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(R.work, 0, sizeof(unsigned), st);
-  if (e != cudaSuccess || R.units() <= 0) return e;
+  cudaError_t e = cudaSuccess;
+  if (R.units() <= 0) return e;
   using namespace field32;
   if (four)
     return density ? dispatch2<4, true>(d_jobs, n_jobs, R, max_np, variant, slab_tier, stats, masked, st)

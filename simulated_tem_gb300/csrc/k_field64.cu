@@ -521,6 +521,7 @@ template <bool kDens>
 __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R) {
   __shared__ double part[8][32];
   const int lane = threadIdx.x, warp = threadIdx.y, nw = blockDim.y;
+  if (blockIdx.x == 0 && warp == 0 && lane == 0) *R.work = 0;  // for the next field kernel
   if ((int64_t)R.counters[0] > R.cap || R.counters[4] != 0) return;
   int patch;
   const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + blockIdx.x, patch);
@@ -614,8 +615,8 @@ void gauss64_table(double* t) {
 cudaError_t launch_field64(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, int slab_tier,
                            bool density, bool masked, bool four, const double* d_gauss, cudaStream_t st) {
   using namespace field64;
-  cudaError_t e = cudaMemsetAsync(R.work, 0, sizeof(unsigned), st);
-  if (e != cudaSuccess || R.units() <= 0) return e;
+  cudaError_t e = cudaSuccess;
+  if (R.units() <= 0) return e;
 #define STEM_F64(SL)                                                                                        \
   (masked ? (density ? launch_tier<SL, true, true>(slab_tier, d_jobs, n_jobs, R, d_gauss, st)               \
                      : launch_tier<SL, false, true>(slab_tier, d_jobs, n_jobs, R, d_gauss, st))             \
