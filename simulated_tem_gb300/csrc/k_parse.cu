@@ -3,11 +3,12 @@
 // line is ignored).
 //
 // The block's bytes are in device memory.  Line starts: each block of threads owns a
-// 64 KB segment and counts its newlines (16-byte loads, coalesced); an exclusive scan over
+// 16 KB segment and counts its newlines (16-byte loads, coalesced); an exclusive scan over
 // the segments gives each segment's first line number; each segment then writes the starts
 // of its lines (the byte after each newline) in order, 4 KB per step with a block-wide scan
-// of the threads' newline counts.  Then one thread per atom line reads five tokens:
-// two integers and three reals, each correctly rounded (parse_number.cuh), separated by
+// of the threads' newline counts.  Then one thread per atom line reads five tokens (from shared
+// memory, where each block copies its lines with 16-byte loads: bytes read one by one from global
+// memory cost a sector per lane): two integers and three reals, each correctly rounded (parse_number.cuh), separated by
 // blanks or commas.  A line with fewer than five tokens, a malformed token or a number
 // outside the exact parser's range records its line number (the smallest such line wins)
 // and nothing is guessed.
@@ -20,7 +21,7 @@
 namespace stem {
 namespace {
 
-constexpr int kSeg = 65536;   // bytes per segment (one block)
+constexpr int kSeg = 16384;   // bytes per segment (one block)
 constexpr int kChunk = 4096;  // bytes per block-wide step: 256 threads x 16 bytes
 
 // newlines among the 16 bytes at t[i0, i0 + 16) (bytes at or past n are not newlines),
@@ -63,24 +64,28 @@ __global__ void __launch_bounds__(256) k_count_lines(const char* __restrict__ t,
 
 // exclusive scan of nseg counts in place (one block)
 __global__ void __launch_bounds__(1024) k_scan_segments(long long* __restrict__ v, int64_t nseg) {
-  __shared__ long long buf[1024];
-  __shared__ long long carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
+  __shared__ long long warp_sums[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long carry = 0;
   for (int64_t off = 0; off < nseg; off += 1024) {
     const int64_t i = off + threadIdx.x;
     const long long x = i < nseg ? v[i] : 0;
-    buf[threadIdx.x] = x;
-    __syncthreads();
-    for (int d = 1; d < 1024; d <<= 1) {
-      const long long a = threadIdx.x >= d ? buf[threadIdx.x - d] : 0;
-      __syncthreads();
-      buf[threadIdx.x] += a;
-      __syncthreads();
+    long long incl = x;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long a = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += a;
     }
-    if (i < nseg) v[i] = carry + buf[threadIdx.x] - x;
+    if (lane == 31) warp_sums[warp] = incl;
     __syncthreads();
-    if (threadIdx.x == 1023) carry += buf[1023];
+    const long long w = warp_sums[lane];
+    long long wi = w;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long a = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= o) wi += a;
+    }
+    const long long before = __shfl_sync(0xffffffffu, wi - w, warp);
+    if (i < nseg) v[i] = carry + before + incl - x;
+    carry += __shfl_sync(0xffffffffu, wi, 31);
     __syncthreads();
   }
 }
@@ -132,35 +137,74 @@ __device__ __forceinline__ bool token_end(const char* p, const char* end) {
   return p >= end || pn::is_blank(*p) || *p == '\n';
 }
 
-__global__ void __launch_bounds__(256) k_parse_atoms(const char* __restrict__ t, int64_t n,
-                                                     const long long* __restrict__ starts, int64_t n_atoms,
-                                                     double* __restrict__ x, int64_t ldx, int* __restrict__ types,
-                                                     unsigned long long* __restrict__ bad) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_atoms;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const char* end = t + n;
-    const long long st = starts[i];
-    if (st < 0 || st > n) {  // the block has fewer lines than atoms
-      atomicMin(bad, (unsigned long long)i);
-      continue;
-    }
-    const char* p = t + st;
-    bool ok = true;
-    long long id = 0, ty = 0;
-    double v[3] = {0.0, 0.0, 0.0};
-    int used = 0;
+// The five tokens of one atom line.
+__device__ __forceinline__ bool parse_atom(const char* p, const char* end, int& type, double* v) {
+  long long id = 0, ty = 0;
+  int used = 0;
+  p = skip_blanks(p, end);
+  bool ok = pn::parse_int(p, end, id, used) && token_end(p + used, end);
+  p += used;
+  if (ok) {
     p = skip_blanks(p, end);
-    ok = pn::parse_int(p, end, id, used) && token_end(p + used, end);
+    ok = pn::parse_int(p, end, ty, used) && token_end(p + used, end);
     p += used;
+  }
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    double r = 0.0;
     if (ok) {
       p = skip_blanks(p, end);
-      ok = pn::parse_int(p, end, ty, used) && token_end(p + used, end);
+      ok = pn::parse_real(p, end, r, used) && token_end(p + used, end);
       p += used;
     }
-    for (int c = 0; c < 3 && ok; ++c) {
-      p = skip_blanks(p, end);
-      ok = pn::parse_real(p, end, v[c], used) && token_end(p + used, end);
-      p += used;
+    if (c == 0) v[0] = r;
+    else if (c == 1) v[1] = r;
+    else v[2] = r;
+  }
+  type = (int)ty;
+  return ok;
+}
+
+__device__ __noinline__ bool parse_atom_global(const char* p, const char* end, int& type, double* v) {
+  return parse_atom(p, end, type, v);
+}
+
+// One thread per line, kLines lines per block.  A line that the staged bytes hold whole (its successor
+// starts within them: parsing never passes a newline) is parsed from shared memory, any other (the
+// last line, lines longer than 112 bytes on average) from global memory.
+constexpr int kLines = 128;
+constexpr int kLineBytes = kLines * 112;
+__global__ void __launch_bounds__(kLines) k_parse_atoms(const char* __restrict__ t, int64_t n,
+                                                        const long long* __restrict__ starts, int64_t n_atoms,
+                                                        double* __restrict__ x, int64_t ldx, int* __restrict__ types,
+                                                        unsigned long long* __restrict__ bad) {
+  __shared__ __align__(16) char stage[kLineBytes + 16];
+  for (int64_t first = (int64_t)blockIdx.x * kLines; first < n_atoms; first += (int64_t)gridDim.x * kLines) {
+    const int64_t i = first + threadIdx.x, last = min(first + kLines, n_atoms);
+    // bytes [lo, hi): from the first line's start to the last line's, at most kLineBytes
+    const long long s0 = starts[first], s1 = last < n_atoms ? starts[last] : (long long)n;
+    const int64_t lo = s0, hi = s0 < 0 || s1 < s0 ? s0 : min((long long)s1, s0 + kLineBytes);
+    // 16-byte loads from the aligned address at or below t + lo (within its 256-byte aligned allocation)
+    const int pad = (int)((uintptr_t)(t + lo) & 15);
+    __syncthreads();  // the previous lines are parsed
+    if (hi > lo) {
+      const char* src = t + lo - pad;
+      const int bytes = (int)(hi - lo) + pad, whole = bytes & ~15;
+      for (int k = 16 * threadIdx.x; k < whole; k += 16 * kLines)
+        *reinterpret_cast<uint4*>(stage + k) = *reinterpret_cast<const uint4*>(src + k);
+      for (int k = whole + threadIdx.x; k < bytes; k += kLines) stage[k] = src[k];
+    }
+    __syncthreads();
+    if (i >= n_atoms) continue;
+    const long long st = starts[i], next = i + 1 < n_atoms ? starts[i + 1] : -1;
+    bool ok = st >= 0 && st <= n;  // else the block has fewer lines than atoms
+    int type = 0;
+    double v[3] = {0.0, 0.0, 0.0};
+    if (ok) {
+      if (next > st && next <= hi)
+        ok = parse_atom(stage + pad + (int)(st - lo), stage + pad + (int)(next - lo), type, v);
+      else
+        ok = parse_atom_global(t + st, t + n, type, v);
     }
     if (!ok) {
       atomicMin(bad, (unsigned long long)i);
@@ -169,8 +213,7 @@ __global__ void __launch_bounds__(256) k_parse_atoms(const char* __restrict__ t,
     x[i * ldx + 0] = v[0];
     x[i * ldx + 1] = v[1];
     x[i * ldx + 2] = v[2];
-    if (types) types[i] = (int)ty;
-    (void)id;
+    if (types) types[i] = type;
   }
 }
 
@@ -432,9 +475,9 @@ cudaError_t launch_parse_atoms(const char* d_text, int64_t n_bytes, int64_t n_at
   if (nseg <= 0 || n_atoms <= 0) return cudaSuccess;
   cudaError_t e = launch_line_starts(d_text, n_bytes, n_atoms, d_seg, d_starts, d_bad, st);
   if (e != cudaSuccess) return e;
-  const int64_t pb = (n_atoms + 255) / 256;
-  k_parse_atoms<<<(int)(pb < 16384 ? pb : 16384), 256, 0, st>>>(d_text, n_bytes, d_starts, n_atoms, d_x, ldx,
-                                                                 d_types, d_bad);
+  const int64_t pb = (n_atoms + kLines - 1) / kLines;
+  k_parse_atoms<<<(int)(pb < 32768 ? pb : 32768), kLines, 0, st>>>(d_text, n_bytes, d_starts, n_atoms, d_x, ldx,
+                                                                    d_types, d_bad);
   return cudaGetLastError();
 }
 

@@ -6,7 +6,10 @@
 // form an integer W (< 2^127) with a decimal exponent q: the value is W 10^q (digits beyond
 // the 38th set a sticky flag).  When W <= 2^53 and |q| <= 22 both W and 10^|q| are exact
 // FP64 numbers and one IEEE multiplication or division is the correctly rounded result
-// (Clinger's fast path).  Otherwise the result is exact by construction:
+// (Clinger's fast path).  Up to 19 digits and |q| <= 40 (17-digit coordinates among them), the
+// 128 leading bits of W 10^q from a 128-bit power of five decide the rounding unless they lie within
+// two units of a midpoint (scaled_round, after Lemire, "Number parsing at a gigabyte per second",
+// Software: Practice and Experience 51, 2021).  Otherwise the result is exact by construction:
 //   * an FP64 estimate of W 10^q (within a few ulp) gives a candidate m 2^e (m of 53 bits);
 //   * the candidate is moved until w 10^q lies between its lower and upper midpoints,
 //     decided by exact comparisons of 256-bit integers (W 10^q against a midpoint num 2^sh,
@@ -24,8 +27,10 @@
 
 #ifdef __CUDACC__
 #define PN_HD __host__ __device__ __forceinline__
+#define PN_SLOW static __host__ __device__ __noinline__
 #else
 #define PN_HD inline
+#define PN_SLOW inline
 #endif
 
 namespace stem {
@@ -105,6 +110,111 @@ PN_HD bool mul_pow10(U256& a, int k) {
     if (!mul_small(a, p)) return false;
     k -= s;
   }
+  return true;
+}
+
+// 5^q for |q| <= kPow5 as a 128-bit significand t in [2^127, 2^128), truncated, and its exponent:
+// 5^q = t 2^e (1 + r), 0 <= r < 2^-127.  Built at compile time by exact integer arithmetic.
+constexpr int kPow5 = 40;
+struct Pow5 {
+  uint64_t hi[2 * kPow5 + 1] = {}, lo[2 * kPow5 + 1] = {};
+  int e[2 * kPow5 + 1] = {};
+  constexpr Pow5() {
+    uint64_t h = 0, l = 1;  // 5^k, up to 93 bits
+    for (int k = 0; k <= kPow5; ++k) {
+      if (k > 0) {  // times 5
+        const uint64_t l4 = l << 2, h4 = (h << 2) | (l >> 62);
+        const uint64_t nl = l4 + l;
+        h = h4 + h + (nl < l4 ? 1 : 0);
+        l = nl;
+      }
+      // q = k: shifted up to 128 bits
+      uint64_t a = h, b = l;
+      int sh = 0;
+      while (!(a >> 63)) {
+        a = (a << 1) | (b >> 63);
+        b <<= 1;
+        ++sh;
+      }
+      hi[kPow5 + k] = a;
+      lo[kPow5 + k] = b;
+      e[kPow5 + k] = -sh;
+      // q = -k: the first 128 bits of 1 / 5^k by long division
+      const int bits = 128 - sh;   // of 5^k
+      uint64_t qh = 0, ql = 0, rh = 0, rl = 1;  // quotient, remainder (below 5^k)
+      int made = 0, p = 0;         // quotient bits from its leading one on; position of the last bit
+      if (k == 0) {
+        qh = 1ULL << 63;
+        made = 128;
+        p = 127;
+      }
+      while (made < 128) {
+        rh = (rh << 1) | (rl >> 63);
+        rl <<= 1;
+        ++p;
+        const bool ge = rh > h || (rh == h && rl >= l);
+        if (ge) {
+          const uint64_t nl = rl - l;
+          rh = rh - h - (rl < l ? 1 : 0);
+          rl = nl;
+        }
+        if (ge || made > 0) {
+          qh = (qh << 1) | (ql >> 63);
+          ql = (ql << 1) | (ge ? 1 : 0);
+          ++made;
+        }
+      }
+      (void)bits;
+      hi[kPow5 - k] = qh;
+      lo[kPow5 - k] = ql;
+      e[kPow5 - k] = -p;
+    }
+  }
+};
+#ifdef __CUDACC__
+static __device__ const Pow5 d_pow5{};
+#endif
+static const constexpr Pow5 h_pow5{};
+
+PN_HD int clz64(uint64_t v) {
+#ifdef __CUDA_ARCH__
+  return __clzll((long long)v);
+#else
+  return __builtin_clzll(v);
+#endif
+}
+
+// w 10^q rounded to FP64 (w > 0, |q| <= kPow5); false when the 128 leading bits do not decide (a
+// midpoint, or within two units of one) or the result is not a normal number.
+PN_HD bool scaled_round(uint64_t w, int q, double& out) {
+#ifdef __CUDA_ARCH__
+  const Pow5& T = d_pow5;
+#else
+  const Pow5& T = h_pow5;
+#endif
+  const int l = clz64(w);
+  w <<= l;
+  uint64_t h1, l1, h2, l2;
+  mul64(w, T.hi[kPow5 + q], h1, l1);
+  mul64(w, T.lo[kPow5 + q], h2, l2);
+  l1 += h2;  // P = floor(w t / 2^64), up to one less; the value is in [P, P + 2) 2^x
+  h1 += l1 < h2 ? 1 : 0;
+  int x = 64 - l + T.e[kPow5 + q] + q;
+  // m: the 53 leading bits, and what is left of h1 above l1
+  const int s = h1 >> 63 ? 11 : 10;
+  uint64_t m = h1 >> s;
+  const uint64_t rest = h1 & ((1ULL << s) - 1), half = 1ULL << (s - 1);
+  if (rest == half && l1 == 0) return false;
+  if (rest == half - 1 && l1 >= ~1ULL) return false;
+  x += 64 + s;  // value = m 2^x
+  if (rest >= half && ++m == (1ULL << 53)) {
+    m >>= 1;
+    ++x;
+  }
+  const int be = x + 52 + 1023;
+  if (be < 1 || be > 2046) return false;
+  const uint64_t bits = ((uint64_t)be << 52) | (m & ((1ULL << 52) - 1));
+  memcpy(&out, &bits, 8);
   return true;
 }
 
@@ -213,6 +323,39 @@ PN_HD bool round_exact(const U256& W, double est, int q, double& out) {
   return true;
 }
 
+// The exact comparisons, for the numbers the fast paths leave (out of line: its 256-bit integers would
+// cost every caller its registers): |value| of w1 10^n2 + w2 (more digits when sticky) times 10^q.
+PN_SLOW bool parse_exact(uint64_t w1, uint64_t w2, int n2, int q, bool sticky, double& out) {
+  // W = w1 10^n2 + w2, and its FP64 estimate
+  U256 W = u256(w1);
+  if (!mul_pow10(W, n2)) return false;
+  {
+    uint64_t c = 0;
+    uint64_t s0 = W.w[0] + w2;
+    c = s0 < W.w[0] ? 1 : 0;
+    W.w[0] = s0;
+    for (int i = 1; i < 4 && c; ++i) {
+      W.w[i] += 1;
+      c = W.w[i] == 0 ? 1 : 0;
+    }
+  }
+  const double est = (double)w1 * pow10_est(n2) + (double)w2;
+  double r;
+  if (!round_exact(W, est, q, r)) return false;
+  if (sticky) {  // the value lies strictly between W 10^q and (W + 1) 10^q
+    U256 W1 = W;
+    uint64_t c = 1;
+    for (int i = 0; i < 4 && c; ++i) {
+      W1.w[i] += 1;
+      c = W1.w[i] == 0 ? 1 : 0;
+    }
+    double r2;
+    if (!round_exact(W1, est, q, r2) || r2 != r) return false;
+  }
+  out = r;
+  return true;
+}
+
 // Parse one number from [p, end); used = characters consumed.  Returns false on malformed
 // text or outside the exact range.
 PN_HD bool parse_real(const char* p, const char* end, double& out, int& used) {
@@ -281,32 +424,15 @@ PN_HD bool parse_real(const char* p, const char* end, double& out, int& used) {
     out = neg ? -r : r;
     return true;
   }
-  // W = w1 10^n2 + w2, and its FP64 estimate
-  U256 W = u256(w1);
-  if (!mul_pow10(W, n2)) return false;
-  {
-    uint64_t c = 0;
-    uint64_t s0 = W.w[0] + w2;
-    c = s0 < W.w[0] ? 1 : 0;
-    W.w[0] = s0;
-    for (int i = 1; i < 4 && c; ++i) {
-      W.w[i] += 1;
-      c = W.w[i] == 0 ? 1 : 0;
+  if (n2 == 0 && !sticky && q >= -kPow5 && q <= kPow5) {
+    double r;
+    if (scaled_round(w1, q, r)) {
+      out = neg ? -r : r;
+      return true;
     }
   }
-  const double est = (double)w1 * pow10_est(n2) + (double)w2;
   double r;
-  if (!round_exact(W, est, q, r)) return false;
-  if (sticky) {  // the value lies strictly between W 10^q and (W + 1) 10^q
-    U256 W1 = W;
-    uint64_t c = 1;
-    for (int i = 0; i < 4 && c; ++i) {
-      W1.w[i] += 1;
-      c = W1.w[i] == 0 ? 1 : 0;
-    }
-    double r2;
-    if (!round_exact(W1, est, q, r2) || r2 != r) return false;
-  }
+  if (!parse_exact(w1, w2, n2, q, sticky, r)) return false;
   out = neg ? -r : r;
   return true;
 }
