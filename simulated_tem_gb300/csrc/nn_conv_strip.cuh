@@ -237,12 +237,30 @@ __global__ void __launch_bounds__(kThreads) k_conv_strip(const StripArgs a, cons
       const int xw = sp.xt * kTileX + 32 * warp + lane;
       for (int j = 0; j < nsteps; ++j, ++k) {
         const int buf = k & 1;
+        // the step's mask values, all loads in flight before the accumulators are waited for (one
+        // load per 8 channels, each between two stores: 8 x 256 x 256 pixels of 64 channels 172 us, so 129)
+        constexpr bool kAhead = BN >= 64;  // (two CTAs per SM at BN = 32: one row's at a time)
+        uint4 mk[kAhead ? RP : 1][BN / 8];
+        auto load_mask = [&](int r) {
+          const int yy = sp.y0 + j * RP + r;
+          const bool in = a.mask && xw < a.W && yy < sp.y1;
+          const size_t p = ((size_t)sp.img * a.H + yy) * a.W + xw;
+#pragma unroll
+          for (int c = 0; c < BN / 8; ++c)
+            if (in && 8 * c < a.Cout) mk[kAhead ? r : 0][c] = *reinterpret_cast<const uint4*>(a.mask + p * a.Cout + 8 * c);
+        };
+        if constexpr (kAhead) {
+#pragma unroll
+          for (int r = 0; r < RP; ++r) load_mask(r);
+        }
         if (!wait_bar(tc::smem_addr(&S.acc_full[buf]), (k >> 1) & 1, abort)) {
           ok = false;
           break;
         }
         tc::fence_after_sync();
+#pragma unroll
         for (int r = 0; r < RP; ++r) {
+          if constexpr (!kAhead) load_mask(r);
           float v[BN];
           {
             uint32_t reg[BN];
@@ -273,7 +291,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_strip(const StripArgs a, cons
                 if (a.relu) vv[i] = fmaxf(vv[i], 0.f);
               }
               if (a.mask) {
-                const uint4 mv = *reinterpret_cast<const uint4*>(a.mask + p * a.Cout + n);
+                const uint4 mv = mk[kAhead ? r : 0][col / 8];
                 const __nv_bfloat16* m = reinterpret_cast<const __nv_bfloat16*>(&mv);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
