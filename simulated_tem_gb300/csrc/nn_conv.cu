@@ -38,6 +38,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "nn.h"
 #include "tc_sm100.cuh"
@@ -49,8 +50,7 @@ __device__ int g_nn_error = 0;  // first failure code of a corrector kernel (0 =
 
 namespace {
 
-constexpr int kThreads = 128;              // weight-gradient kernel
-constexpr int kTileThreads = 192;          // persistent forward kernel: 4 epilogue warps, producer, issuer
+constexpr int kTileThreads = 192;          // forward and weight-gradient kernels: 4 epilogue warps, producer, issuer
 constexpr uint32_t kWaitLimit = 1u << 20;  // polls of an mbarrier before giving up (about a second)
 constexpr int kTileX = 128;                // output pixels per tile (one image row)
 constexpr int kHalo = kTileX + 2;          // input pixels per halo row
@@ -347,6 +347,17 @@ bool make_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same with the 128-byte swizzle (a box of 64 BF16 innermost).
+bool make_map_128(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
+                  const cuuint32_t* box) {
+  PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
+  if (!fn) return false;
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides_bytes, box,
+            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Blocked weights: wb[nt][c][tap][g][n][8] = w[nt BN + n][tap][c KC + 8 g + 0..7] (zero for
 // output channels past Cout), one 16-byte vector per thread.
 __global__ void k_block_weights(const uint4* __restrict__ w, int Cout, int taps, int Cin, int BN, int KC,
@@ -481,194 +492,204 @@ namespace {
 // ---------------------------------------------------------------------------
 // Weight gradient: gw[co, t, ci] += sum_p gy[p, co] x[p + d_t, ci]
 // ---------------------------------------------------------------------------
-// GEMM per tap with K = pixels: A[co, p] = gy[p, co], B_t[ci, p] = x[p + d_t, ci], both
-// transposed while staged (K-major tiles, p along K).  A CTA owns 128 output channels x
-// BN input channels x TG taps (TG x BN TMEM columns) for one range of pixels, in chunks
-// of 64 pixels; the A tile of a chunk serves all TG taps.  Partial sums over the CTA's
-// pixels go to the CTA's slice of a workspace (one slice per pixel split), which a second
-// kernel adds to the FP32 gradient in split order: the result does not depend on the
-// order in which CTAs finish (training is reproducible).
+// GEMM per tap with K = pixels: A[co, p] = gy[p, co], B_t[ci, p] = x[p + d_t, ci].  NHWC activations are
+// such operands as they lie, with the channel index contiguous: a TMA box of 64 channels x P pixels
+// of one image row, 128-byte swizzled, is an MN-major tile, and no thread touches it (transposing
+// the operands into K-major tiles while staging them, with 2-byte stores, took 539 us for 8 x 256 x
+// 256 pixels and 64 x 64 channels, this takes 61: 630 TFLOP/s).  A chunk is P consecutive pixels of a row
+// (P a multiple of 16 up to 64); for a 3 x 3 convolution a CTA owns one tap row dy: its x tile is row
+// y + dy, pixels x0 - 1 .. x0 + P, and the three taps read it shifted by 0, 1, 2 pixels (128 bytes
+// each).  Outside the image the boxes are zero-filled, in gy past the row's end, in x on every side.
+// A CTA owns 128 output channels (one 64-channel atom twice when Cout <= 64: the upper half of
+// the accumulator is not read) x BN input channels x TG taps (TG BN TMEM columns) for a range of
+// chunks.  Partial sums over the CTA's pixels go to its slice of a workspace (one slice per pixel
+// split), which a second kernel adds to the FP32 gradient in split order: the result does not depend
+// on the order in which CTAs finish (training is reproducible).
+// Roles (192 threads): warps 0-3 read TMEM at the end, warp 4 lane 0 loads, warp 5 lane 0 issues.
 struct WgradArgs {
-  const __nv_bfloat16* x;   // [B][H][W][Cin]
-  const __nv_bfloat16* gy;  // [B][H][W][Cout]
   float* ws;                // [splits][Cout][taps][Cin] partial sums
   int B, H, W, Cin, Cout, taps;
-  int chunks_per_cta;       // 64-pixel chunks per CTA (pixel split)
+  int P, nx;                // pixels per chunk, chunks per row
+  int chunks, chunks_per_cta;
 };
 
-template <int BN, int TG>
+constexpr int kWStages = 4;
+constexpr int kWAtom = 8192;   // 64 pixels x 128 bytes
+constexpr int kWAtomB = 9216;  // 66 pixels, rounded to the swizzle's 1024 bytes
+
+// MA, NB: 64-channel atoms of the output and input channels
+template <int MA, int NB>
 struct WSmem {
-  alignas(1024) unsigned char a[2][128 * 64 * 2];
-  alignas(1024) unsigned char b[2][TG][BN * 64 * 2];
-  alignas(8) unsigned long long mbar[2];
+  alignas(1024) unsigned char a[kWStages][MA * kWAtom];
+  alignas(1024) unsigned char b[kWStages][NB * kWAtomB];
+  alignas(8) unsigned long long full[kWStages], empty[kWStages], done;
   uint32_t tmem;
+  int abort;
 };
 
 __host__ __device__ constexpr int tmem_cols(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512; }
 
-// Stage 8 consecutive channels of pixel p (or zeros) as column kp of rows r0 .. r0 + 7.
-__device__ __forceinline__ void put_column8(unsigned char* tile, int r0, int kp, const __nv_bfloat16* src) {
-  uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  if (src) v = *reinterpret_cast<const uint4*>(src);
-  const unsigned short* h = reinterpret_cast<const unsigned short*>(&v);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) *reinterpret_cast<unsigned short*>(tile + tc::tile_offset(r0 + i, kp, 64)) = h[i];
-}
-
-template <int BN, int TG>
-__global__ void __launch_bounds__(kThreads) k_conv_wgrad(const WgradArgs a) {
+// BN = 32, 64 or 128 input channels, TG taps (3: a tap row; 1: a 1 x 1 convolution)
+template <int MA, int BN, int TG>
+__global__ void __launch_bounds__(kTileThreads) k_conv_wgrad(const WgradArgs a, const __grid_constant__ CUtensorMap tmg,
+                                                             const __grid_constant__ CUtensorMap tmx) {
+  constexpr int NB = BN > 64 ? 2 : 1;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  WSmem<BN, TG>& S = *reinterpret_cast<WSmem<BN, TG>*>(smem_raw + ((1024 - ((uintptr_t)smem_raw & 1023)) & 1023));
-  const int t = threadIdx.x, warp = t >> 5;
+  WSmem<MA, NB>& S = *reinterpret_cast<WSmem<MA, NB>*>(smem_raw + ((1024 - ((uintptr_t)smem_raw & 1023)) & 1023));
+  constexpr uint32_t kCols = tmem_cols(TG * BN);
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  volatile int* abort = &S.abort;
   const int m0 = blockIdx.y * 128;                    // output channels
   const int n_ctiles = (a.Cin + BN - 1) / BN;
   const int c0 = (blockIdx.z % n_ctiles) * BN;        // input channels
-  const int t0 = (blockIdx.z / n_ctiles) * TG;        // first tap of the group
-  const int ntap = min(TG, a.taps - t0);
-  const int npix = a.B * a.H * a.W;
+  const int dyi = blockIdx.z / n_ctiles;              // tap row
   const int chunk0 = blockIdx.x * a.chunks_per_cta;
-  const int nchunks = max(0, min(a.chunks_per_cta, (npix + 63) / 64 - chunk0));
-  constexpr int kCols = tmem_cols(TG * BN);
+  const int n = max(0, min(a.chunks_per_cta, a.chunks - chunk0));
 
-  if (warp == 0) tc::tmem_alloc(tc::smem_addr(&S.tmem), kCols);
+  if (warp == 5) tc::tmem_alloc(tc::smem_addr(&S.tmem), kCols);
   if (t == 0) {
-    tc::mbar_init(tc::smem_addr(&S.mbar[0]), 1);
-    tc::mbar_init(tc::smem_addr(&S.mbar[1]), 1);
+    for (int i = 0; i < kWStages; ++i) {
+      tc::mbar_init(tc::smem_addr(&S.full[i]), 1);
+      tc::mbar_init(tc::smem_addr(&S.empty[i]), 1);
+    }
+    tc::mbar_init(tc::smem_addr(&S.done), 1);
+    S.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = S.tmem;
-  constexpr uint32_t idesc = tc::make_idesc_bf16(128, BN);
 
-  const int kp = t & 63, half = t >> 6;
-  bool ok = true;
-  int issued = 0;
-  for (int c = 0; c < nchunks; ++c) {
-    const int st = c & 1;
-    if (c >= 2) ok = tc::mbar_wait(tc::smem_addr(&S.mbar[st]), ((c - 2) >> 1) & 1, kWaitLimit);
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
-    const int p = (chunk0 + c) * 64 + kp;
-    int b = 0, yh = 0, xw = 0;
-    if (p < npix) {
-      xw = p % a.W;
-      const int rest = p / a.W;
-      yh = rest % a.H;
-      b = rest / a.H;
-    }
-    // A: 128 output channels x 64 pixels
-    for (int g = half; g < 16; g += 2) {
-      const int co = m0 + 8 * g;
-      const __nv_bfloat16* src = (p < npix && co < a.Cout) ? a.gy + (size_t)p * a.Cout + co : nullptr;
-      put_column8(S.a[st], 8 * g, kp, src);
-    }
-    // B_t: BN input channels x 64 pixels, one tile per tap of the group
-    for (int j = 0; j < TG; ++j) {
-      const int tap = t0 + j;
-      const int dy = a.taps == 9 ? tap / 3 - 1 : 0, dx = a.taps == 9 ? tap % 3 - 1 : 0;
-      const int yy = yh + dy, xx = xw + dx;
-      const bool in = j < ntap && p < npix && yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
-      for (int g = half; g < BN / 8; g += 2) {
-        const int ci = c0 + 8 * g;
-        const __nv_bfloat16* src =
-            (in && ci < a.Cin) ? a.x + (((size_t)b * a.H + yy) * a.W + xx) * a.Cin + ci : nullptr;
-        put_column8(S.b[st][j], 8 * g, kp, src);
+  if (warp == 4) {
+    if (lane == 0) {
+      // ---- producer
+      const uint32_t bytes = (uint32_t)(MA * a.P + NB * (a.P + TG - 1)) * 128u;
+      int armed = 0;
+      for (int c = 0; c < n; ++c, ++armed) {
+        const int st = c % kWStages;
+        if (c >= kWStages && !wait_or_abort(tc::smem_addr(&S.empty[st]), (c / kWStages - 1) & 1, abort)) break;
+        const int ch = chunk0 + c, xi = ch % a.nx, row = ch / a.nx, y = row % a.H, img = row / a.H;
+        const uint32_t f = tc::smem_addr(&S.full[st]);
+        tc::mbar_arrive_expect_tx(f, bytes);
+        for (int j = 0; j < MA; ++j)
+          tc::tma_load_4d(tc::smem_addr(S.a[st] + j * kWAtom), &tmg, m0 + 64 * j, xi * a.P, y, img, f);
+        for (int j = 0; j < NB; ++j)
+          tc::tma_load_4d(tc::smem_addr(S.b[st] + j * kWAtomB), &tmx, c0 + 64 * j, xi * a.P - (TG == 3 ? 1 : 0),
+                          y + (TG == 3 ? dyi - 1 : 0), img, f);
       }
+      // every load issued has landed before the CTA may leave (bounded)
+      for (int st = 0; st < kWStages; ++st)
+        if (armed > st && !tc::mbar_wait(tc::smem_addr(&S.full[st]), ((armed - 1 - st) / kWStages) & 1, kWaitLimit))
+          *abort = 1;
     }
-    tc::fence_proxy_async_smem();
-    __syncthreads();
-    if (t == 0) {
-      tc::fence_after_sync();
-      const uint32_t sa = tc::smem_addr(S.a[st]);
-      for (int j = 0; j < ntap; ++j) {
-        const uint32_t sb = tc::smem_addr(S.b[st][j]);
+  } else if (warp == 5) {
+    if (lane == 0) {
+      // ---- MMA issuer
+      constexpr uint32_t idesc = tc::make_idesc_bf16_mn(128, BN);
+      for (int c = 0; c < n; ++c) {
+        const int st = c % kWStages;
+        if (!wait_or_abort(tc::smem_addr(&S.full[st]), (c / kWStages) & 1, abort)) break;
+        tc::fence_after_sync();
+        // start addresses in 16-byte units: 16 pixels are 2048 bytes, one pixel 128.  With one atom of
+        // output channels the second one's rows (any shared memory behind it) are not read back.
+        uint64_t ad = tc::make_desc_mn128(tc::smem_addr(S.a[st]), kWAtom);
+        uint64_t bd = tc::make_desc_mn128(tc::smem_addr(S.b[st]), kWAtomB);
+        for (int s = 0; s < a.P / 16; ++s) {
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
-          tc::mma_bf16(tmem + (uint32_t)(j * BN), tc::make_desc(sa + 256 * s, 128, 64 * 16),
-                       tc::make_desc(sb + 256 * s, 128, 64 * 16), idesc, (c > 0 || s > 0) ? 1u : 0u);
+          for (int tap = 0; tap < TG; ++tap)
+            tc::mma_bf16(tmem + (uint32_t)(tap * BN), ad, bd + (uint64_t)(8 * tap), idesc, (c > 0 || s > 0) ? 1u : 0u);
+          ad += 128;
+          bd += 128;
+        }
+        tc::mma_commit(tc::smem_addr(&S.empty[st]));
       }
-      tc::mma_commit(tc::smem_addr(&S.mbar[st]));
+      tc::mma_commit(tc::smem_addr(&S.done));  // arrives when every MMA issued above has completed
+      if (!tc::mbar_wait(tc::smem_addr(&S.done), 0, kWaitLimit)) *abort = 1;
     }
-    issued = c + 1;
-  }
-  if (issued > 0) {
-    const int last = issued - 1;
-    bool done = tc::mbar_wait(tc::smem_addr(&S.mbar[last & 1]), (last >> 1) & 1, kWaitLimit);
-    done = __syncthreads_and(done);
-    if (!done) tc::mbar_wait(tc::smem_addr(&S.mbar[last & 1]), (last >> 1) & 1, kWaitLimit);
-    ok = ok && done;
-  }
-  if (!ok && t == 0) atomicCAS(&g_nn_error, 0, 1);
-  tc::fence_after_sync();
-
-  if (ok && issued > 0) {
-    const int co = m0 + 32 * warp + (t & 31);
-    for (int j = 0; j < ntap; ++j) {
-      for (int col = 0; col < BN; col += 8) {
-        float v[8];
-        tc::tmem_ld8(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(j * BN + col), v);
-        const int ci = c0 + col;
-        if (co < a.Cout && ci < a.Cin) {
-          float* dst = a.ws + (size_t)blockIdx.x * a.Cout * a.taps * a.Cin + ((size_t)co * a.taps + t0 + j) * a.Cin + ci;
-          reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-          reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  } else if (n > 0 && wait_or_abort(tc::smem_addr(&S.done), 0, abort)) {
+    // ---- the accumulators: TMEM lanes 32 warp .. 32 warp + 31 = output channels
+    tc::fence_after_sync();
+    const int co = m0 + 32 * warp + lane;
+    float* dst0 = a.ws + (size_t)blockIdx.x * a.Cout * a.taps * a.Cin + ((size_t)co * a.taps + dyi * TG) * a.Cin + c0;
+    for (int tap = 0; tap < TG; ++tap) {
+#pragma unroll 1
+      for (int col = 0; col < BN; col += 32) {
+        uint32_t r[32];
+        tc::tmem_ld32_nowait(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(tap * BN + col), r);
+        tc::tmem_wait_ld();
+        if (co < a.Cout) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            if (c0 + col + i < a.Cin)
+              *reinterpret_cast<uint4*>(dst0 + (size_t)tap * a.Cin + col + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
         }
       }
     }
+    tc::fence_before_sync();
   }
-  tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem, kCols);
+  if (t == 0 && S.abort) atomicCAS(&g_nn_error, 0, 1);
+  tc::fence_after_sync();
+  if (warp == 5) tc::tmem_dealloc(tmem, kCols);
 }
 
 // gw[i] += sum over splits s (in order) of ws[s][i]
 __global__ void k_wgrad_reduce(const float* __restrict__ ws, int splits, long long n, float* __restrict__ gw) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float s = 0.f;
+#pragma unroll 8
     for (int k = 0; k < splits; ++k) s += ws[(size_t)k * n + i];
     gw[i] += s;
   }
 }
 
-// Pixel split of a weight-gradient launch: about two waves of CTAs, at least 8 chunks per
-// CTA so the partial sums amortise.
-template <int BN, int TG>
-void wgrad_split(int B, int H, int W, int Cin, int Cout, int taps, int& splits, int& chunks_per_cta) {
-  int dev = 0, sms = 148;
+// The launch: chunks of P pixels (as even as multiples of 16 up to 64 make them), and as many pixel
+// splits as fill the GPU once (two CTAs per SM where TMEM and shared memory allow two: up to 64 x 64
+// channels), at least four chunks each.
+struct WgradPlan {
+  int P, nx, chunks, chunks_per_cta, splits, bn, tg, ma;
+};
+WgradPlan wgrad_plan(int B, int H, int W, int Cin, int Cout, int taps) {
+  WgradPlan p;
+  p.nx = (W + 63) / 64;
+  p.P = ((W + p.nx - 1) / p.nx + 15) / 16 * 16;
+  p.nx = (W + p.P - 1) / p.P;
+  p.chunks = B * H * p.nx;
+  p.bn = Cin <= 32 ? 32 : Cin <= 64 ? 64 : 128;
+  p.tg = taps == 9 ? 3 : 1;
+  p.ma = Cout <= 64 ? 1 : 2;
+  int dev = 0, sms = 152;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int npix = B * H * W;
-  const int chunks = (npix + 63) / 64;
-  const int tiles = ((Cout + 127) / 128) * ((Cin + BN - 1) / BN) * ((taps + TG - 1) / TG);
-  splits = (2 * sms + tiles - 1) / tiles;
-  splits = max(1, min(splits, (chunks + 7) / 8));
-  chunks_per_cta = (chunks + splits - 1) / splits;
-  splits = (chunks + chunks_per_cta - 1) / chunks_per_cta;
+  const int per_sm = p.bn <= 64 && p.ma == 1 ? 2 : 1;
+  const int tiles = ((Cout + 127) / 128) * ((Cin + p.bn - 1) / p.bn) * (taps / p.tg);
+  p.splits = max(1, min(per_sm * sms / tiles, p.chunks / 4));
+  p.chunks_per_cta = (p.chunks + p.splits - 1) / p.splits;
+  p.splits = (p.chunks + p.chunks_per_cta - 1) / p.chunks_per_cta;
+  return p;
 }
 
-template <int BN, int TG>
-cudaError_t launch_wgrad(WgradArgs a, float* gw, size_t ws_floats, cudaStream_t st) {
-  const size_t smem = sizeof(WSmem<BN, TG>) + 1024;
-  cudaError_t e = cudaFuncSetAttribute(k_conv_wgrad<BN, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int MA, int BN, int TG>
+cudaError_t launch_wgrad(const WgradPlan& p, const __nv_bfloat16* x, const __nv_bfloat16* gy, WgradArgs a, float* gw,
+                         cudaStream_t st) {
+  CUtensorMap tmg, tmx;
+  auto map = [&](CUtensorMap* m, const void* base, int C, int pixels) {
+    const cuuint64_t d[4] = {(cuuint64_t)C, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.B};
+    const cuuint64_t s[3] = {(cuuint64_t)C * 2, (cuuint64_t)a.W * C * 2, (cuuint64_t)a.H * a.W * C * 2};
+    const cuuint32_t box[4] = {64, (cuuint32_t)pixels, 1, 1};
+    return make_map_128(m, base, 4, d, s, box);
+  };
+  if (!map(&tmg, gy, a.Cout, a.P) || !map(&tmx, x, a.Cin, a.P + TG - 1)) return cudaErrorInvalidValue;
+  const size_t smem = sizeof(WSmem<MA, (BN > 64 ? 2 : 1)>) + 1024;
+  auto kernel = k_conv_wgrad<MA, BN, TG>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  int splits = 1;
-  wgrad_split<BN, TG>(a.B, a.H, a.W, a.Cin, a.Cout, a.taps, splits, a.chunks_per_cta);
-  const long long n = (long long)a.Cout * a.taps * a.Cin;
-  if ((size_t)splits * (size_t)n > ws_floats) return cudaErrorInvalidValue;
-  dim3 grid(splits, (a.Cout + 127) / 128, ((a.Cin + BN - 1) / BN) * ((a.taps + TG - 1) / TG));
-  k_conv_wgrad<BN, TG><<<grid, kThreads, smem, st>>>(a);
-  const long long blocks = (n + 255) / 256;
-  k_wgrad_reduce<<<(int)(blocks < 1024 ? blocks : 1024), 256, 0, st>>>(a.ws, splits, n, gw);
+  const dim3 grid(p.splits, (a.Cout + 127) / 128, ((a.Cin + BN - 1) / BN) * (a.taps / TG));
+  kernel<<<grid, kTileThreads, smem, st>>>(a, tmg, tmx);
+  const long long n = (long long)a.Cout * a.taps * a.Cin, blocks = (n + 255) / 256;
+  k_wgrad_reduce<<<(int)(blocks < 1024 ? blocks : 1024), 256, 0, st>>>(a.ws, p.splits, n, gw);
   return cudaGetLastError();
-}
-
-template <int BN, int TG>
-size_t wgrad_ws(int B, int H, int W, int Cin, int Cout, int taps) {
-  int splits = 1, cpc = 1;
-  wgrad_split<BN, TG>(B, H, W, Cin, Cout, taps, splits, cpc);
-  return (size_t)splits * Cout * taps * Cin;
 }
 
 // wt[ci][8 - t][co] = w[co][t][ci] (taps 9) or wt[ci][0][co] = w[co][0][ci]: the weights
@@ -694,25 +715,29 @@ bool wgrad_args_ok(int B, int H, int W, int Cin, int Cout, int taps) {
 
 size_t conv_wgrad_workspace(int B, int H, int W, int Cin, int Cout, int taps) {
   if (!wgrad_args_ok(B, H, W, Cin, Cout, taps)) return 0;
-  if (taps == 1)
-    return Cin <= 32 ? wgrad_ws<32, 1>(B, H, W, Cin, Cout, taps)
-                     : Cin <= 64 ? wgrad_ws<64, 1>(B, H, W, Cin, Cout, taps) : wgrad_ws<128, 1>(B, H, W, Cin, Cout, taps);
-  return Cin <= 32 ? wgrad_ws<32, 9>(B, H, W, Cin, Cout, taps)
-                   : Cin <= 64 ? wgrad_ws<64, 3>(B, H, W, Cin, Cout, taps) : wgrad_ws<128, 3>(B, H, W, Cin, Cout, taps);
+  return (size_t)wgrad_plan(B, H, W, Cin, Cout, taps).splits * Cout * taps * Cin;
 }
 
 int conv_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* gy, int B, int H, int W, int Cin, int Cout, int taps,
                float* gw, float* ws, size_t ws_floats, cudaStream_t st) {
   if (!x || !gy || !gw || !ws || !wgrad_args_ok(B, H, W, Cin, Cout, taps)) return 1;
-  if (ws_floats < conv_wgrad_workspace(B, H, W, Cin, Cout, taps)) return 1;
-  WgradArgs a{x, gy, ws, B, H, W, Cin, Cout, taps, 1};
+  const WgradPlan p = wgrad_plan(B, H, W, Cin, Cout, taps);
+  if (ws_floats < (size_t)p.splits * Cout * taps * Cin) return 1;
+  const WgradArgs a{ws, B, H, W, Cin, Cout, taps, p.P, p.nx, p.chunks, p.chunks_per_cta};
+  auto launch = [&](auto ma, auto tg) {
+    constexpr int MA = decltype(ma)::value, TG = decltype(tg)::value;
+    if (p.bn == 32) return launch_wgrad<MA, 32, TG>(p, x, gy, a, gw, st);
+    if (p.bn == 64) return launch_wgrad<MA, 64, TG>(p, x, gy, a, gw, st);
+    return launch_wgrad<MA, 128, TG>(p, x, gy, a, gw, st);
+  };
+  using std::integral_constant;
   cudaError_t e;
   if (taps == 1)
-    e = Cin <= 32 ? launch_wgrad<32, 1>(a, gw, ws_floats, st)
-                  : Cin <= 64 ? launch_wgrad<64, 1>(a, gw, ws_floats, st) : launch_wgrad<128, 1>(a, gw, ws_floats, st);
+    e = p.ma == 1 ? launch(integral_constant<int, 1>(), integral_constant<int, 1>())
+                  : launch(integral_constant<int, 2>(), integral_constant<int, 1>());
   else
-    e = Cin <= 32 ? launch_wgrad<32, 9>(a, gw, ws_floats, st)
-                  : Cin <= 64 ? launch_wgrad<64, 3>(a, gw, ws_floats, st) : launch_wgrad<128, 3>(a, gw, ws_floats, st);
+    e = p.ma == 1 ? launch(integral_constant<int, 1>(), integral_constant<int, 3>())
+                  : launch(integral_constant<int, 2>(), integral_constant<int, 3>());
   return e == cudaSuccess ? 0 : 2;
 }
 

@@ -35,6 +35,15 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
+// The same for an operand whose M (N) index is contiguous in memory ("MN-major") with the 128-byte
+// swizzle: atoms of 64 M/N elements (128 bytes) x 8 K rows, 1024 bytes, as a TMA box of 64 channels x
+// pixels leaves them; `lbo` bytes between atoms along M/N, 1024 between atoms along K.  The buffer
+// starts on a 1024-byte boundary; a start address moved by r 128-byte rows reads the K rows from r on
+// (the swizzle follows the address).
+__device__ __forceinline__ uint64_t make_desc_mn128(uint32_t saddr, uint32_t lbo) {
+  return make_desc(saddr, lbo, 1024) | ((uint64_t)2 << 61);
+}
+
 // Instruction descriptor of kind::f16: BF16 x BF16 -> FP32, both operands K-major,
 // M x N tile (M = 64 or 128, N a multiple of 8 up to 256 for M = 128).
 __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N) {
@@ -43,6 +52,11 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N) {
          | (1u << 10)                       // B format: BF16
          | ((uint32_t)(N >> 3) << 17)       // N / 8
          | ((uint32_t)(M >> 4) << 24);      // M / 16
+}
+
+// The same with both operands MN-major.
+__host__ __device__ constexpr uint32_t make_idesc_bf16_mn(int M, int N) {
+  return make_idesc_bf16(M, N) | (1u << 15) | (1u << 16);
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
