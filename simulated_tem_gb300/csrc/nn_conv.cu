@@ -8,12 +8,12 @@
 // touches the operands: one thread moves them, one issues the MMAs, four warps drain TMEM.
 //
 // Per chunk of KC input channels the producer loads a halo tile: the input rows y - 1 ..
-// y + R (R output rows; from y for 1 x 1), pixels x0 - 1 .. x0 + 128, as (KC / 8) slabs
-// of 130 rows x 16 bytes (8 channels) per input row; output row y + q reads the input
-// rows from y - 1 + q, and every row's MMAs read each weight slot.  In such a slab the rows are 16 bytes apart, so
-// the K-major core matrices (8 rows x 16 bytes) of the pixels shifted by dx start 16 dx
-// bytes further: all nine taps read the same tile through shifted descriptors (LBO =
-// slab pitch between 8-channel groups, SBO = 128 between 8-pixel groups).  Outside the
+// y + R (R output rows; from y for 1 x 1), pixels x0 - 1 .. x0 + 128, one box of 130 pixels x KC
+// channels per input row, swizzled by its row of 2 KC bytes; output row y + q reads the input
+// rows from y - 1 + q, and every row's MMAs read each weight slot.  The pixels shifted by dx start
+// 2 KC dx bytes further, so all nine taps read the same tile through shifted descriptors.  (Boxes
+// of 8 channels, unswizzled slabs of 16-byte rows, moved half-used 32-byte sectors and four times
+// the rows: 568 x 568 pixels, 192 to 64 channels 126 -> 109 us.)  Outside the
 // image the TMA box is zero-filled: the padding.  The weights of each (tap, chunk) come
 // into a ring of B slots ([BN rows][16 bytes] per 8-channel group) as one contiguous bulk
 // copy: before the convolution a small kernel writes the weights in exactly that order
@@ -54,7 +54,7 @@ constexpr int kTileThreads = 192;          // forward and weight-gradient kernel
 constexpr uint32_t kWaitLimit = 1u << 20;  // polls of an mbarrier before giving up (about a second)
 constexpr int kTileX = 128;                // output pixels per tile (one image row)
 constexpr int kHalo = kTileX + 2;          // input pixels per halo row
-constexpr int kSlab = 2176;                // bytes per (input row, 8 channels) slab: 130 x 16 rounded to 128
+constexpr int kSlab = 2176;                // bytes per input row and 8 channels: 130 x 16 rounded to 128
 // weight ring depth: as many slots as leave room for two CTAs per SM (TMEM allows two at
 // BN = 128); each slot holds KC/16 MMAs of work, and the ring must cover the latency of
 // the TMA loads that refill it
@@ -167,9 +167,8 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_fwd(const ConvArgs a, con
           tc::mbar_arrive_expect_tx(fa, kBytesA);
           ++na[sa];
           for (int r = 0; r < kInRows; ++r)
-            for (int g = 0; g < kG; ++g)
-              tc::tma_load_4d(tc::smem_addr(S.a[sa] + (r * kG + g) * kSlab), &tmx, c * KC + 8 * g,
-                              tl.xt * kTileX - 1, tl.y + r - (NR == 3 ? 1 : 0), tl.img, fa);
+            tc::tma_load_4d(tc::smem_addr(S.a[sa] + r * kG * kSlab), &tmx, c * KC, tl.xt * kTileX - 1,
+                            tl.y + r - (NR == 3 ? 1 : 0), tl.img, fa);
           for (int tap = 0; tap < kTaps; ++tap) {
             if (rb >= 1 && !wait_or_abort(tc::smem_addr(&S.b_empty[sb]), (rb - 1) & 1, abort)) {
               ok = false;
@@ -214,7 +213,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_fwd(const ConvArgs a, con
             ok = false;
             break;
           }
-          const uint64_t adesc0 = tc::make_desc(tc::smem_addr(S.a[sa]), kSlab, 128);
+          const uint64_t adesc0 = tc::make_desc_k(tc::smem_addr(S.a[sa]), 2 * KC);
           for (int tap = 0; tap < kTaps; ++tap) {
             if (!wait_or_abort(tc::smem_addr(&S.b_full[sb]), rb & 1, abort)) {
               ok = false;
@@ -223,8 +222,8 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_fwd(const ConvArgs a, con
             tc::fence_after_sync();
             const int dy = NR == 3 ? tap / 3 : 0, dx = NR == 3 ? tap % 3 : 1;  // halo row / column offset
             // start addresses in 16-byte units (descriptor bits 0-13); output row q reads
-            // halo rows dy + q, one row group (kG slabs) further
-            uint64_t ad = adesc0 + (uint64_t)(dy * kG * (kSlab / 16) + dx);
+            // halo rows dy + q, a pixel is 2 KC bytes, 16 channels are 32
+            uint64_t ad = adesc0 + (uint64_t)(dy * kG * (kSlab / 16) + dx * (KC / 8));
             uint64_t bd = tc::make_desc(tc::smem_addr(S.b[sb]), BN * 16, 128);
             const uint32_t first = (c == 0 && tap == 0) ? 0u : 1u;
 #pragma unroll
@@ -233,7 +232,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_fwd(const ConvArgs a, con
               for (int q = 0; q < kRowsPerTile; ++q)
                 tc::mma_bf16(acc + (uint32_t)(q * BN), ad + (uint64_t)(q * kG * (kSlab / 16)), bd, idesc,
                              (s == 0) ? first : 1u);
-              ad += 2 * kSlab / 16;
+              ad += 2;
               bd += 2 * BN;
             }
             tc::mma_commit(tc::smem_addr(&S.b_empty[sb]));
@@ -347,14 +346,17 @@ bool make_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The same with the 128-byte swizzle (a box of 64 BF16 innermost).
-bool make_map_128(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
-                  const cuuint32_t* box) {
+// The same, swizzled by the width of the box's innermost extent (16, 32 or 64 BF16).
+bool make_map_swizzled(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims,
+                       const cuuint64_t* strides_bytes, const cuuint32_t* box) {
   PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
   if (!fn) return false;
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUtensorMapSwizzle sw = box[0] == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                                : box[0] == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                               : CU_TENSOR_MAP_SWIZZLE_32B;
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides_bytes, box,
-            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -423,8 +425,8 @@ cudaError_t launch_fwd(const __nv_bfloat16* x, const __nv_bfloat16* w, ConvArgs 
   CUtensorMap tmx;
   const cuuint64_t xd[4] = {(cuuint64_t)a.Cin, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.B};
   const cuuint64_t xs[3] = {(cuuint64_t)a.Cin * 2, (cuuint64_t)a.W * a.Cin * 2, (cuuint64_t)a.H * a.W * a.Cin * 2};
-  const cuuint32_t xb[4] = {8, kHalo, 1, 1};
-  if (!make_map(&tmx, x, 4, xd, xs, xb)) return cudaErrorInvalidValue;
+  const cuuint32_t xb[4] = {KC, kHalo, 1, 1};
+  if (!make_map_swizzled(&tmx, x, 4, xd, xs, xb)) return cudaErrorInvalidValue;
   if (a.taps != (NR == 3 ? 9 : 1) || a.Cin % KC != 0) return cudaErrorInvalidValue;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -678,7 +680,7 @@ cudaError_t launch_wgrad(const WgradPlan& p, const __nv_bfloat16* x, const __nv_
     const cuuint64_t d[4] = {(cuuint64_t)C, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.B};
     const cuuint64_t s[3] = {(cuuint64_t)C * 2, (cuuint64_t)a.W * C * 2, (cuuint64_t)a.H * a.W * C * 2};
     const cuuint32_t box[4] = {64, (cuuint32_t)pixels, 1, 1};
-    return make_map_128(m, base, 4, d, s, box);
+    return make_map_swizzled(m, base, 4, d, s, box);
   };
   if (!map(&tmg, gy, a.Cout, a.P) || !map(&tmx, x, a.Cin, a.P + TG - 1)) return cudaErrorInvalidValue;
   const size_t smem = sizeof(WSmem<MA, (BN > 64 ? 2 : 1)>) + 1024;

@@ -35,6 +35,15 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
+// The same for a K-major tile whose rows are row_bytes = 32, 64 or 128 bytes long and swizzled by that
+// width, as a TMA box of row_bytes / 2 channels x rows leaves them: 8 rows are one repeat of the
+// pattern (the buffer starts on a multiple of 8 row_bytes).  A start address moved by r rows reads the
+// rows from r on, one moved by 32 bytes the next 16 channels (the swizzle follows the address).
+__device__ __forceinline__ uint64_t make_desc_k(uint32_t saddr, uint32_t row_bytes) {
+  const uint64_t mode = row_bytes == 128 ? 2 : row_bytes == 64 ? 4 : 6;
+  return make_desc(saddr, 16, 8 * row_bytes) | mode << 61;
+}
+
 // The same for an operand whose M (N) index is contiguous in memory ("MN-major") with the 128-byte
 // swizzle: atoms of 64 M/N elements (128 bytes) x 8 K rows, 1024 bytes, as a TMA box of 64 channels x
 // pixels leaves them; `lbo` bytes between atoms along M/N, 1024 between atoms along K.  The buffer
