@@ -37,6 +37,7 @@
 #include <cudaTypedefs.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -636,13 +637,36 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_wgrad(const WgradArgs a, 
   if (warp == 5) tc::tmem_dealloc(tmem, kCols);
 }
 
-// gw[i] += sum over splits s (in order) of ws[s][i]
-__global__ void k_wgrad_reduce(const float* __restrict__ ws, int splits, long long n, float* __restrict__ gw) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+// gw[i] += sum over splits s of ws[s][i]: Q = 4 threads per value, a quarter of the splits each in order,
+// then the quarters in order; one thread where the splits are few (64 x 64 channels, 100 splits 12.6 ->
+// 7.6 us with four; 256 x 256, 6 splits 8 us slower with four).
+template <int Q>
+__global__ void __launch_bounds__(256) k_wgrad_reduce(const float* __restrict__ ws, int splits, long long n,
+                                                      float* __restrict__ gw) {
+  constexpr int kVals = 256 / Q;
+  __shared__ float part[Q][kVals];
+  const int c = threadIdx.x % kVals, q = threadIdx.x / kVals;
+  const int per = (splits + Q - 1) / Q, k0 = min(splits, q * per), k1 = min(splits, k0 + per);
+  for (long long i0 = (long long)blockIdx.x * kVals; i0 < n; i0 += (long long)gridDim.x * kVals) {
+    const long long i = i0 + c;
     float s = 0.f;
+    if (i < n) {
 #pragma unroll 8
-    for (int k = 0; k < splits; ++k) s += ws[(size_t)k * n + i];
-    gw[i] += s;
+      for (int k = k0; k < k1; ++k) s += ws[(size_t)k * n + i];
+    }
+    if constexpr (Q == 1) {
+      if (i < n) gw[i] += s;
+    } else {
+      part[q][c] = s;
+      __syncthreads();
+      if (q == 0 && i < n) {
+        float t = part[0][c];
+#pragma unroll
+        for (int k = 1; k < Q; ++k) t += part[k][c];
+        gw[i] += t;
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -689,8 +713,11 @@ cudaError_t launch_wgrad(const WgradPlan& p, const __nv_bfloat16* x, const __nv_
   if (e != cudaSuccess) return e;
   const dim3 grid(p.splits, (a.Cout + 127) / 128, ((a.Cin + BN - 1) / BN) * (a.taps / TG));
   kernel<<<grid, kTileThreads, smem, st>>>(a, tmg, tmx);
-  const long long n = (long long)a.Cout * a.taps * a.Cin, blocks = (n + 255) / 256;
-  k_wgrad_reduce<<<(int)(blocks < 1024 ? blocks : 1024), 256, 0, st>>>(a.ws, p.splits, n, gw);
+  const long long n = (long long)a.Cout * a.taps * a.Cin;
+  if (p.splits >= 32)
+    k_wgrad_reduce<4><<<(int)std::min<long long>((n + 63) / 64, 2048), 256, 0, st>>>(a.ws, p.splits, n, gw);
+  else
+    k_wgrad_reduce<1><<<(int)std::min<long long>((n + 255) / 256, 2048), 256, 0, st>>>(a.ws, p.splits, n, gw);
   return cudaGetLastError();
 }
 
