@@ -65,7 +65,7 @@ def build(verbose=False, ptxas_info=False):
     libs = [
         (LIB, LIB_SOURCES, [os.path.join(CSRC, "internal.h"), os.path.join(CSRC, "parse_number.cuh"),
                             os.path.join(CSRC, "fp64_column.cuh"), os.path.join(CSRC, "slab_ring.cuh"),
-                            os.path.join(CSRC, "host_geom.h"),
+                            os.path.join(CSRC, "rounded_product.h"), os.path.join(CSRC, "host_geom.h"),
                             os.path.join(inc, "stem.h"),
                             os.path.join(inc, "stem_host.h")]),
         (NN_LIB, NN_SOURCES, [os.path.join(CSRC, "nn.h"), os.path.join(CSRC, "tc_sm100.cuh"), os.path.join(CSRC, "nn_conv_strip.cuh"),

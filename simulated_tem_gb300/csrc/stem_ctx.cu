@@ -34,7 +34,7 @@ struct st_ctx {
   size_t cap_x = 0;
   double* d_img = nullptr;
   size_t cap_img = 0;
-  double* d_blur = nullptr;  // in, tmp (+w_stripe), out
+  double* d_blur = nullptr;  // in, tmp (+ weight sums of columns and rows), out
   size_t cap_blur = 0;
   double* d_kern = nullptr;
   size_t cap_kern = 0;
@@ -1404,7 +1404,7 @@ extern "C" int st_blur_device(st_ctx* c, const double* d_in, int32_t nx, int32_t
   std::vector<double> k;
   const int nk = blur_kernel(t, k);
   const size_t n = (size_t)nx * ny;
-  cudaError_t e = ensure(c->d_blur, c->cap_blur, 3 * n + nx);
+  cudaError_t e = ensure(c->d_blur, c->cap_blur, 3 * n + nx + ny);
   if (e == cudaSuccess) e = ensure(c->d_kern, c->cap_kern, (size_t)nk + 1);
   if (e != cudaSuccess) return cuda_fail(c, e, "allocating blur buffers");
   e = cudaMemcpyAsync(c->d_kern, k.data(), (nk + 1) * sizeof(double), cudaMemcpyHostToDevice, st);
@@ -1419,12 +1419,12 @@ extern "C" int st_blur(st_ctx* c, const double* in, int32_t nx, int32_t ny, doub
   if (!in || !out || nx < 1 || ny < 1) return fail(c, ST_ERR_ARG, "invalid blur arguments");
   cudaSetDevice(c->device);
   const size_t n = (size_t)nx * ny;
-  cudaError_t e = ensure(c->d_blur, c->cap_blur, 3 * n + nx);
+  cudaError_t e = ensure(c->d_blur, c->cap_blur, 3 * n + nx + ny);
   if (e != cudaSuccess) return cuda_fail(c, e, "allocating blur buffers");
   e = cudaMemcpyAsync(c->d_blur, in, n * sizeof(double), cudaMemcpyHostToDevice, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "copying blur input");
-  // input at d_blur[0, n), scratch at [n, 2n + nx), output at [2n + nx, 3n + nx)
-  double* d_out = c->d_blur + 2 * n + nx;
+  // input at d_blur[0, n), scratch at [n, 2n + nx + ny), then the output
+  double* d_out = c->d_blur + 2 * n + nx + ny;
   int rc = st_blur_device(c, c->d_blur, nx, ny, t, d_out, c->stream);
   if (rc != ST_OK) return rc;
   e = cudaMemcpyAsync(out, d_out, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
@@ -1474,14 +1474,14 @@ extern "C" int st_write_png(st_ctx* c, const char* path, const double* img, int3
   if (!path || !img || nx < 1 || ny < 1) return fail(c, ST_ERR_ARG, "invalid PNG arguments");
   cudaSetDevice(c->device);
   const size_t n = (size_t)nx * ny;
-  cudaError_t e = ensure(c->d_blur, c->cap_blur, 3 * n + nx);
+  cudaError_t e = ensure(c->d_blur, c->cap_blur, 3 * n + nx + ny);
   if (e == cudaSuccess) e = ensure(c->d_levels, c->cap_levels, n);
   if (e != cudaSuccess) return cuda_fail(c, e, "allocating PNG buffers");
   e = cudaMemcpyAsync(c->d_blur, img, n * sizeof(double), cudaMemcpyHostToDevice, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "copying the PNG image");
   const double* src = c->d_blur;
   if (blur_t > 0) {  // outputImgAsPng blurs first when png_blur > 0
-    double* d_out = c->d_blur + 2 * n + nx;
+    double* d_out = c->d_blur + 2 * n + nx + ny;
     const int rc = st_blur_device(c, c->d_blur, nx, ny, blur_t, d_out, c->stream);
     if (rc != ST_OK) return rc;
     src = d_out;
