@@ -3,13 +3,18 @@
 // line is ignored).
 //
 // The block's bytes are in device memory.  Line starts: each block of threads owns a
-// 16 KB segment and counts its newlines (16-byte loads, coalesced); an exclusive scan over
-// the segments gives each segment's first line number; each segment then writes the starts
-// of its lines (the byte after each newline) in order, 4 KB per step with a block-wide scan
-// of the threads' newline counts.  Then one thread per atom line reads five tokens (from shared
-// memory, where each block copies its lines with 16-byte loads: bytes read one by one from global
-// memory cost a sector per lane): two integers and three reals, each correctly rounded (parse_number.cuh), separated by
-// blanks or commas.  A line with fewer than five tokens, a malformed token or a number
+// 16 KB segment and counts its newlines (64 bytes per thread, all loads in flight at once); an
+// exclusive scan over the segments gives each segment's first line number; each segment then writes
+// the starts of its lines (the byte after each newline) in order, from one block-wide scan of the
+// threads' newline counts.  Then one thread per atom line reads five tokens: two integers and three
+// reals, each correctly rounded (parse_number.cuh), separated by blanks or commas.  Instruction issue
+// bounds that kernel, so the usual form of a line is read by offsets in shared memory, where each block
+// copies its lines with 16-byte loads (bytes read one by one from global memory cost a sector per
+// lane), and everything else is left to the general routine, out of line: its registers would leave
+// four blocks per SM.  17 MB with 300k lines: count 9.5, scan 4.4, starts 10.5, lines 43 us; 239 us for
+// the lines with the general routine from global memory and every rounding by exact comparisons, 74 us
+// with it from shared memory.
+// A line with fewer than five tokens, a malformed token or a number
 // outside the exact parser's range records its line number (the smallest such line wins)
 // and nothing is guessed.
 #include <cuda_runtime.h>
@@ -21,8 +26,8 @@
 namespace stem {
 namespace {
 
-constexpr int kSeg = 16384;   // bytes per segment (one block)
-constexpr int kChunk = 4096;  // bytes per block-wide step: 256 threads x 16 bytes
+constexpr int kSeg = 16384;  // bytes per segment (one block)
+constexpr int kPer = kSeg / 256 / 16;  // 16-byte words per thread
 
 // newlines among the 16 bytes at t[i0, i0 + 16) (bytes at or past n are not newlines),
 // as a bit mask (bit k: byte i0 + k)
@@ -32,8 +37,8 @@ __device__ __forceinline__ unsigned newline_mask(const char* __restrict__ t, int
     const uint4 v = *reinterpret_cast<const uint4*>(t + i0);
     const unsigned w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int k = 0; k < 16; ++k)
-      if (((w[k >> 2] >> (8 * (k & 3))) & 0xFFu) == (unsigned)'\n') m |= 1u << k;
+    for (int k = 0; k < 4; ++k)  // the multiplication gathers bits 0, 8, 16 and 24 in bits 24 to 27
+      m |= (((__vcmpeq4(w[k], 0x0A0A0A0Au) & 0x01010101u) * 0x01020408u) >> 24) << (4 * k);
   } else {  // the end of the text, or an unaligned buffer
     for (int k = 0; k < 16 && i0 + k < n; ++k)
       if (t[i0 + k] == '\n') m |= 1u << k;
@@ -46,8 +51,9 @@ __global__ void __launch_bounds__(256) k_count_lines(const char* __restrict__ t,
   __shared__ int part[8];
   for (int64_t sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
     int c = 0;
-    for (int ch = 0; ch < kSeg / kChunk; ++ch) {
-      const int64_t i0 = sg * kSeg + (int64_t)ch * kChunk + 16 * threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int64_t i0 = sg * kSeg + 16 * (j * 256 + (int)threadIdx.x);
       if (i0 < n) c += __popc(newline_mask(t, n, i0));
     }
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
@@ -91,39 +97,37 @@ __global__ void __launch_bounds__(1024) k_scan_segments(long long* __restrict__ 
 }
 
 // starts[k] = byte offset of line k (k < n_lines; the rest stay -1); line 0 starts at 0.
-// Per 4 KB step every thread holds the newline mask of its 16 bytes; a block-wide scan of
-// the counts gives each newline its line number.
+// Every thread holds the newline masks of its 64 bytes; a block-wide scan of the counts gives each
+// newline its line number.
 __global__ void __launch_bounds__(256) k_line_starts(const char* __restrict__ t, int64_t n, int64_t nseg,
                                                      const long long* __restrict__ seg_base, int64_t n_lines,
                                                      long long* __restrict__ starts) {
   __shared__ int wsum[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int64_t sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
-    long long base = seg_base[sg];  // newlines before this step
-    for (int ch = 0; ch < kSeg / kChunk; ++ch) {
-      const int64_t c0 = sg * kSeg + (int64_t)ch * kChunk;
-      if (c0 >= n) break;  // block-uniform
-      const int64_t i0 = c0 + 16 * threadIdx.x;
-      const unsigned m = i0 < n ? newline_mask(t, n, i0) : 0u;
-      const int c = __popc(m);
-      int incl = c;  // inclusive warp scan
-      for (int o = 1; o < 32; o <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += a;
-      }
-      if (lane == 31) wsum[warp] = incl;
-      __syncthreads();
-      int woff = 0, total = 0;
-      for (int w = 0; w < 8; ++w) {
-        if (w < warp) woff += wsum[w];
-        total += wsum[w];
-      }
-      long long k = base + woff + incl - c + 1;  // the line the first newline here starts
-      for (unsigned mm = m; mm; mm &= mm - 1, ++k)
-        if (k < n_lines) starts[k] = i0 + __ffs(mm);  // the byte after the newline
-      base += total;
-      __syncthreads();  // wsum is rewritten by the next step
+    const int64_t i0 = sg * kSeg + 16 * kPer * (int)threadIdx.x;
+    unsigned m[kPer];
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      m[j] = i0 + 16 * j < n ? newline_mask(t, n, i0 + 16 * j) : 0u;
+      c += __popc(m[j]);
     }
+    int incl = c;  // inclusive warp scan
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += a;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    int woff = 0;
+    for (int w = 0; w < warp; ++w) woff += wsum[w];
+    long long k = seg_base[sg] + woff + incl - c + 1;  // the line the first newline here starts
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      for (unsigned mm = m[j]; mm; mm &= mm - 1, ++k)
+        if (k < n_lines) starts[k] = i0 + 16 * j + __ffs(mm);  // the byte after the newline
+    __syncthreads();  // wsum is rewritten by the next segment
     if (sg == 0 && threadIdx.x == 0 && n_lines > 0) starts[0] = 0;
   }
 }
@@ -137,7 +141,7 @@ __device__ __forceinline__ bool token_end(const char* p, const char* end) {
   return p >= end || pn::is_blank(*p) || *p == '\n';
 }
 
-// The five tokens of one atom line.
+// The five tokens of one atom line, in any form the reference reads.
 __device__ __forceinline__ bool parse_atom(const char* p, const char* end, int& type, double* v) {
   long long id = 0, ty = 0;
   int used = 0;
@@ -165,8 +169,65 @@ __device__ __forceinline__ bool parse_atom(const char* p, const char* end, int& 
   return ok;
 }
 
-__device__ __noinline__ bool parse_atom_global(const char* p, const char* end, int& type, double* v) {
+__device__ __noinline__ bool parse_atom_any(const char* p, const char* end, int& type, double* v) {
   return parse_atom(p, end, type, v);
+}
+
+// The usual form of a line in shared memory, from offset o on (the staged line ends with its newline,
+// which stops every loop): numbers of up to 19 digits whose rounding scaled_round decides.  False for
+// anything else, malformed lines among it: parse_atom then says.
+__device__ __forceinline__ bool parse_atom_fast(const char* s, int o, int& type, double* v) {
+  unsigned c = (unsigned char)s[o];
+  auto skip = [&]() {
+    while (pn::is_blank((char)c)) c = (unsigned char)s[++o];
+  };
+  auto ends = [&]() { return c == '\n' || pn::is_blank((char)c); };
+  for (int k = 0; k < 2; ++k) {  // id, type
+    skip();
+    const bool neg = c == '-';
+    if (neg || c == '+') c = (unsigned char)s[++o];
+    const int first = o;
+    unsigned n = 0;
+    for (; c - '0' <= 9u; c = (unsigned char)s[++o]) n = n * 10 + (c - '0');
+    if (o == first || !ends() || (k == 1 && o - first > 9)) return false;
+    type = neg ? -(int)n : (int)n;
+  }
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    skip();
+    const bool neg = c == '-';
+    if (neg || c == '+') c = (unsigned char)s[++o];
+    unsigned long long w = 0;
+    const int first = o;
+    for (; c - '0' <= 9u; c = (unsigned char)s[++o]) w = w * 10 + (c - '0');
+    int nd = o - first, q = 0;
+    if (c == '.') {
+      const int point = o;
+      c = (unsigned char)s[++o];
+      for (; c - '0' <= 9u; c = (unsigned char)s[++o]) w = w * 10 + (c - '0');
+      q = point + 1 - o;
+      nd -= q;
+    }
+    if (nd == 0 || nd > 19) return false;
+    if (c == 'e' || c == 'E' || c == 'd' || c == 'D') {
+      c = (unsigned char)s[++o];
+      const bool eneg = c == '-';
+      if (eneg || c == '+') c = (unsigned char)s[++o];
+      const int ef = o;
+      int ev = 0;
+      for (; c - '0' <= 9u; c = (unsigned char)s[++o]) ev = ev * 10 + (int)(c - '0');
+      if (o == ef || o - ef > 6) return false;
+      q += eneg ? -ev : ev;
+    }
+    if (!ends()) return false;
+    double r = 0.0;
+    if (w != 0 && !(q >= -pn::kPow5 && q <= pn::kPow5 && pn::scaled_round(w, q, r))) return false;
+    r = neg ? -r : r;
+    if (k == 0) v[0] = r;
+    else if (k == 1) v[1] = r;
+    else v[2] = r;
+  }
+  return true;
 }
 
 // One thread per line, kLines lines per block.  A line that the staged bytes hold whole (its successor
@@ -174,7 +235,7 @@ __device__ __noinline__ bool parse_atom_global(const char* p, const char* end, i
 // last line, lines longer than 112 bytes on average) from global memory.
 constexpr int kLines = 128;
 constexpr int kLineBytes = kLines * 112;
-__global__ void __launch_bounds__(kLines) k_parse_atoms(const char* __restrict__ t, int64_t n,
+__global__ void __launch_bounds__(kLines, 8) k_parse_atoms(const char* __restrict__ t, int64_t n,
                                                         const long long* __restrict__ starts, int64_t n_atoms,
                                                         double* __restrict__ x, int64_t ldx, int* __restrict__ types,
                                                         unsigned long long* __restrict__ bad) {
@@ -201,10 +262,16 @@ __global__ void __launch_bounds__(kLines) k_parse_atoms(const char* __restrict__
     int type = 0;
     double v[3] = {0.0, 0.0, 0.0};
     if (ok) {
-      if (next > st && next <= hi)
-        ok = parse_atom(stage + pad + (int)(st - lo), stage + pad + (int)(next - lo), type, v);
-      else
-        ok = parse_atom_global(t + st, t + n, type, v);
+      const bool staged = next > st && next <= hi;
+      if (!staged || !parse_atom_fast(stage, pad + (int)(st - lo), type, v)) {
+        int ty = 0;  // copies: what parse_atom_any takes by address stays out of the registers
+        double u[3] = {0.0, 0.0, 0.0};
+        ok = parse_atom_any(t + st, t + n, ty, u);
+        type = ty;
+        v[0] = u[0];
+        v[1] = u[1];
+        v[2] = u[2];
+      }
     }
     if (!ok) {
       atomicMin(bad, (unsigned long long)i);
