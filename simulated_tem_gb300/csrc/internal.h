@@ -229,10 +229,10 @@ bool ring_variant_same(int variant);  // gives variant 0's image to the last bit
 // 128, 192, 256 atoms; `four`: every job's steps of four slices fit the ring (four_slices_fit);
 // d_gauss: gauss64_table's values.
 constexpr int kGauss64Size = 3 * 1024 + 16;
-constexpr int kField64Blocks = 2;  // CTAs of four warps per SM at tier 0
-void gauss64_table(double* t);
+constexpr int kField64Blocks = 3;  // CTAs of four warps per SM at tier 0
+void gauss64_table(long long* t);
 cudaError_t launch_field64(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, int slab_tier,
-                           bool density, bool masked, bool four, const double* d_gauss, cudaStream_t st);
+                           bool density, bool masked, bool four, const long long* d_gauss, cudaStream_t st);
 // Whether every step of four slices (z = 0, 4, 8 ...) of an image has home z cells that
 // rise by at most one cell without wrapping, so that the cells the step needs (one more on
 // either side) fit the slab ring's four slots.

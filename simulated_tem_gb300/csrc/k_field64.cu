@@ -59,6 +59,14 @@ constexpr int kWarps = 4;
 // error is below 1e-4 for voxels up to a lattice constant; the reject side of the FP32 test always
 // had this margin.
 constexpr float kGuard64 = 1e-3f;
+
+// A number in [-1, 1] in units of 2^-58, as h 2^29 + l, 0 <= l < 2^29: the product of two is three
+// 32 x 32-bit multiply-adds.
+constexpr int kLimb = 29, kLow = (1 << kLimb) - 1;
+struct __align__(8) Fixed {
+  int h, l;
+};
+constexpr int kPass = 32;         // atoms per pass over the lanes
 constexpr int kN = 64;            // step buffer: flushed at 32, before a round of 32 may add more
 constexpr float kOff = -1e30f;    // hmax of a slice the slab does not serve
 
@@ -75,48 +83,112 @@ struct WarpSmem {
   int bin[kRing][kBins + 1];
   int count[kRing];
   alignas(16) float hm[kN][SL];  // per slice: the largest accepted in-plane r^2 (FP32, scaled)
+  alignas(16) unsigned m[kPass][SL];  // of the pass's atoms, per slice: the lanes that accept
+  int sel[kPass];         // their places in the step buffer
   float2 xy[kN];          // X', Y'
   int2 ref[kN];           // kept atom, cell code | slab number within the step << 16
-  double exy[kN][12];     // the patch's 8 column and 4 row factors of the Gaussian
-  double2 be[SL][kN];     // per slice: z factor times (cos, sin)
+  Fixed exy[kPass][12];   // the patch's 8 column and 4 row factors of the Gaussian
+  int4 be[SL][kPass];     // per slice: z factor times (cos, sin); before that, the list of exy's tasks
   double off[12][3];      // k - zi_frac of the patch's columns and rows, k = -1, 0, 1
   double zoff[kRing][SL]; // the same for the step's slices, per slab
   float cx[12];           // X' of the columns, Y' of the rows
   int hc[12];             // their home cells in the atoms' cell code
 };
 
-// exp(-d^2 / 2 sigma^2) for d >= 0, given jf = d / (sigma / 1024) to within about one unit: with
-// d_c = j sigma / 1024 (exact: a power of two and an integer), d^2 - d_c^2 = (d - d_c)(d + d_c)
-// is small, so its exponential is a polynomial, and exp(-d_c^2 / 2 sigma^2) does not depend on
-// sigma: one table for every image, exact to half a unit.  |u| <= 0.003: the degree-4 Taylor
-// polynomial is within 2e-17 where jf is rounded right.  (Table-driven evaluation after Tang,
-// ACM TOMS 15 (1989) 144, here on the distance instead of the exponent.)
-__device__ __forceinline__ double gauss64(double d, float jf, const double* __restrict__ T, double s1024,
-                                          double ni2s2) {
+__device__ __forceinline__ Fixed split58(long long v) { return Fixed{(int)(v >> kLimb), (int)v & kLow}; }
+
+__device__ __forceinline__ long long wide(int a, int b) { return (long long)a * b; }
+
+// A product of two fixed-point numbers.  The low limbs' product, 0 to 1 units, counts as a quarter.
+__device__ __forceinline__ long long mul58(const Fixed& a, const Fixed& b) {
+  return wide(a.h, b.h) + ((wide(a.h, b.l) + wide(a.l, b.h) + (3LL << (kLimb - 2))) >> kLimb);
+}
+
+// x (|x| <= 1) in units of 2^-58, cut off
+__device__ __forceinline__ long long to58(double x) {
+  const long long b = __double_as_longlong(x);
+  const int e = (int)(b >> 52) & 0x7FF;
+  const long long m = (((b & ((1LL << 52) - 1)) | (1LL << 52)) << 6) >> min(63, 1023 - e);
+  return b < 0 ? -m : m;
+}
+
+// exp(-d^2 / 2 sigma^2) for d >= 0 in units of 2^-58, given jf = d / (sigma / 1024) to within about one
+// unit: with d_c = j sigma / 1024 (exact: a power of two and an integer), d^2 - d_c^2 =
+// (d - d_c)(d + d_c) is small, so its exponential is a polynomial, and exp(-d_c^2 / 2 sigma^2) does not
+// depend on sigma: one table for every image, exact to half a unit of FP64.  |u| <= 0.003 where jf is
+// rounded right: the degree-4 Taylor polynomial is within 2e-17.  (Table-driven evaluation after Tang,
+// ACM TOMS 15 (1989) 144, here on the distance instead of the exponent.)  FP64 up to u; a sum with a
+// large constant leaves u as an integer, and the rest is integer arithmetic.  A distance beyond the
+// table's end (no accepted atom has one) gives a meaningless number.
+__device__ __forceinline__ long long gauss64(double d, float jf, const long long* __restrict__ T, double s1024,
+                                             double ni2s2) {
   jf = fminf(rintf(jf), (float)(kGauss64Size - 1));
   const int b = __float_as_int(jf);
   // the FP64 bits of an FP32 integer (a conversion instruction runs on the FP64 pipe); 0 becomes 2^-127
   const double jd = __hiloint2double((b >> 3) + 0x38000000, b << 29);
-  const double t = __ldg(T + (int)jf);
+  const long long t = __ldg(T + (int)jf);
   const double del = DF(-jd, s1024, d);
   const double s = DF(2.0, d, -del);
-  const double u = DM(DM(del, s), ni2s2);
-  double q = DF(u, 1.0 / 24.0, 1.0 / 6.0);
-  q = DF(u, q, 0.5);
-  q = DF(u, q, 1.0);
-  return DF(t, DM(u, q), t);
+  const double v = DF(DM(del, s), ni2s2, 0x1.8p-6);  // u + 3/128: |u| < 1/128, the last bit is 2^-58
+  const long long u = __double_as_longlong(v) - __double_as_longlong(0x1.8p-6);
+  const int uh = (int)(u >> 20), ul = (int)u & 0xFFFFF;                // 2^-38, 2^-58
+  const long long u2 = wide(uh, uh) + (wide(uh, ul) >> 19);            // u^2, 2^-76
+  const int u2h = (int)(u2 >> 30);                                     // 2^-46
+  const int r = (int)((wide(uh, 357913941) + (wide(u2h, 89478485) >> 8)) >> 28);  // u/6 + u^2/24, 2^-41
+  const long long E = u + ((u2 + (wide(u2h, r) >> 10) + (1 << 18)) >> 19);         // exp(u) - 1, 2^-58
+  const int eh = (int)(E >> 20), el = (int)E & 0xFFFFF;
+  const Fixed f = split58(t);
+  return t + ((wide(f.h, eh) + (wide(f.l, eh) >> 29) + (wide(f.h, el) >> 20) + 256) >> 9);
+}
+
+// A sum of products of fixed-point numbers: kFold of them in hh (2^-58) and x (2^-87), then folded into
+// 96 bits, so that no number of atoms overflows.
+constexpr int kFold = 16;
+struct Sum58 {
+  long long hh, x;
+  unsigned long long lo;
+  int hi;
+  __device__ __forceinline__ void clear() {
+    hh = x = 0;
+    lo = 0;
+    hi = 0;
+  }
+  __device__ __forceinline__ void add(const Fixed& a, int h, int l) {
+    hh += wide(a.h, h);
+    x += wide(a.h, l);
+    x += wide(a.l, h);
+  }
+  __device__ __forceinline__ void fold() {
+    const long long v = hh + ((x + (1LL << (kLimb - 1))) >> kLimb);
+    lo += (unsigned long long)v;
+    hi += (int)(v >> 63) + (lo < (unsigned long long)v ? 1 : 0);
+    hh = x = 0;
+  }
+};
+
+// A folded sum times 2^58
+__device__ __forceinline__ double value58(unsigned long long lo, int hi) {
+  if (hi == (int)((long long)lo >> 63)) return __ll2double_rn((long long)lo);
+  return DF((double)hi, 0x1p64, __ull2double_rn(lo));
+}
+
+// S / max(1e-16, |S|) (:1877-1892); one copy of its code for all slices
+__device__ __noinline__ double2 unit58(unsigned long long rl, int rh, unsigned long long il, int ih) {
+  const double sr = value58(rl, rh), si = value58(il, ih);
+  const double inv = rsqrt(fmax(DF(sr, sr, DM(si, si)), 1e-32 * 0x1p116));
+  return make_double2(DM(sr, inv), DM(si, inv));
 }
 
 template <int SL>
 struct Acc {
-  double sr[SL], si[SL];
-  float rm[SL];  // FP32 min of (r^2 - cutoff^2), scaled (density)
+  Sum58 sr[SL], si[SL];
+  float rm[SL];  // FP32 min of r^2 - cutoff^2, scaled (density)
 };
 
 // Exact squared distance of kept atom gi (cell code `code`) and this lane's column at slice k of
 // the step, in the reference's operations; +inf outside the lane's 27 cells.
 template <int CAPS, int SL>
-__device__ __forceinline__ double exact_dd(const ColumnParams& p, const WarpSmem<CAPS, SL>& W, int gi, int code, int us,
+__device__ __noinline__ double exact_dd(const ColumnParams& p, const WarpSmem<CAPS, SL>& W, int gi, int code, int us,
                                            int k, int lane) {
   const int c = lane & 7, r = 8 + (lane >> 3);
   const int kx = (code & 255) - W.hc[c], ky = ((code >> 8) & 255) - W.hc[r];
@@ -128,82 +200,152 @@ __device__ __forceinline__ double exact_dd(const ColumnParams& p, const WarpSmem
   return DA(DA(DM(d0, d0), DM(d1, d1)), DM(d2, d2));
 }
 
-// The buffered atoms: their Gaussian factors (tasks over the lanes), then every lane's sums.
+// The buffered atoms: which lanes accept them, in passes of up to 32 that some lane accepts; their
+// Gaussian factors (tasks over the lanes), where an accepting lane needs them; then every lane's sums.
 template <int CAPS, int SL, bool kDens>
 __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL>& W, int n, float Xv, float Yv,
-                                        float cut2f, const double* __restrict__ T, double s1024, double ni2s2,
+                                        float cut2f, const long long* __restrict__ T, double s1024, double ni2s2,
                                         Acc<SL>& A, unsigned& n_acc, int lane) {
   constexpr float kGrid = 1.1774100225f * 1024.f;  // scaled length -> sigma / 1024
-  __syncwarp();
-  for (int t = lane; t < 12 * n; t += 32) {
-    const int i = t / 12, c = t - 12 * i;
-    const bool x = c < 8;
-    const int2 r = W.ref[i];
-    const int k = min(1, max(-1, (x ? r.y & 255 : (r.y >> 8) & 255) - W.hc[c]));
-    const double f = reinterpret_cast<const double*>(p.f64 + r.x)[x ? 0 : 1];
-    const float2 q = W.xy[i];
-    const float df = fabsf((x ? q.x : q.y) - W.cx[c]);
-    const double d = fabs(DM(x ? p.a11 : p.a22, DA(f, W.off[c][k + 1])));
-    W.exy[i][c] = gauss64(d, df * kGrid, T, s1024, ni2s2);
-  }
-  for (int t = lane; t < SL * n; t += 32) {
-    const int i = t / SL, k = t - SL * i;
-    const int2 r = W.ref[i];
-    const double f = reinterpret_cast<const double*>(p.f64 + r.x)[2];
-    const double2 cs = p.cs64[r.x];
-    const float df = sqrtf(fmaxf(0.f, cut2f - W.hm[i][k]));
-    const double d = fabs(DM(p.a33, DA(f, W.zoff[r.y >> 16][k])));
-    const double e = gauss64(d, df * kGrid, T, s1024, ni2s2);
-    W.be[k][i] = make_double2(DM(e, cs.x), DM(e, cs.y));
-  }
+  constexpr int U = 1;  // atoms at once
   __syncwarp();
   const int c = lane & 7, row = 8 + (lane >> 3);
-  for (int i = 0; i < n; ++i) {
-    const float2 q = W.xy[i];
-    const float dx = q.x - Xv, dy = q.y - Yv;
-    const float h = fmaf(dx, dx, dy * dy);
-    bool acc[SL], near = false;
-    float g[SL];
+  for (int i = 0; i < n;) {
+    int cnt = 0;
+    for (; i < n && cnt <= kPass - U; i += U) {
+      bool acc[U][SL], near = false;
+      float g[U][SL];
 #pragma unroll
-    for (int k = 0; k < SL; ++k) {
-      g[k] = h - W.hm[i][k];
-      acc[k] = g[k] <= 0.f;
-      near = near || fabsf(g[k]) <= kGuard64;
-    }
-    if (__any_sync(0xffffffffu, near)) {
-      if (near) {
-        const int2 r = W.ref[i];
+      for (int j = 0; j < U; ++j) {
+        const int a = min(i + j, n - 1);
+        const float2 q = W.xy[a];
+        const float dx = q.x - Xv, dy = q.y - Yv;
+        // past the last atom: its distances (written, so finite), far outside every cutoff
+        const float h = i + j < n ? fmaf(dx, dx, dy * dy) : 3e30f;
 #pragma unroll
-        for (int k = 0; k < SL; ++k)
-          if (fabsf(g[k]) <= kGuard64) acc[k] = exact_dd(p, W, r.x, r.y, r.y >> 16, k, lane) <= p.cut2;
+        for (int k = 0; k < SL; ++k) {
+          g[j][k] = h - W.hm[a][k];
+          acc[j][k] = g[j][k] <= 0.f;
+          near = near || fabsf(g[j][k]) <= kGuard64;
+        }
       }
-      __syncwarp();
-    }
-    unsigned m[SL], any = 0;
+      if (__any_sync(0xffffffffu, near)) {
+        if (near) {
 #pragma unroll
-    for (int k = 0; k < SL; ++k) {
-      m[k] = __ballot_sync(0xffffffffu, acc[k]);
-      any |= m[k];
-    }
-    if (!any) continue;
-    const double w = DM(W.exy[i][c], W.exy[i][row]);
+          for (int j = 0; j < U; ++j)
 #pragma unroll
-    for (int k = 0; k < SL; ++k) {
-      if (m[k]) {  // the same branch in every lane: a slice no lane accepts costs no FP64
-        const double2 e = W.be[k][i];
-        const double wk = acc[k] ? w : 0.0;
-        A.sr[k] = DF(wk, e.x, A.sr[k]);
-        A.si[k] = DF(wk, e.y, A.si[k]);
-        n_acc += acc[k];
-        if (kDens) A.rm[k] = fminf(A.rm[k], acc[k] ? g[k] : 0.f);
+            for (int k = 0; k < SL; ++k)
+              if (fabsf(g[j][k]) <= kGuard64) {
+                const int2 r = W.ref[i + j];
+                acc[j][k] = exact_dd(p, W, r.x, r.y, r.y >> 16, k, lane) <= p.cut2;
+              }
+        }
+        __syncwarp();
+      }
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        unsigned m[SL], any = 0;
+#pragma unroll
+        for (int k = 0; k < SL; ++k) {
+          m[k] = __ballot_sync(0xffffffffu, acc[j][k]);
+          any |= m[k];
+          n_acc += acc[j][k];
+          if (kDens) A.rm[k] = fminf(A.rm[k], g[j][k]);
+        }
+        if (any) {
+          if (lane == 0) {
+            W.sel[cnt] = i + j;
+            if constexpr (SL == 4) *reinterpret_cast<uint4*>(W.m[cnt]) = make_uint4(m[0], m[1], m[2], m[3]);
+            else *reinterpret_cast<uint2*>(W.m[cnt]) = make_uint2(m[0], m[1]);
+          }
+          ++cnt;
+        }
       }
     }
+    if (cnt == 0) continue;
+    __syncwarp();
+    // the list of the columns and rows that some lane needs
+    unsigned short* list = reinterpret_cast<unsigned short*>(&W.be[0][0]);
+    int tasks;
+    {
+      unsigned need = 0;
+      if (lane < cnt) {
+        unsigned any = 0;
+#pragma unroll
+        for (int k = 0; k < SL; ++k) any |= W.m[lane][k];
+        need = (any | any >> 16);
+        need = (need | need >> 8) & 255u;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) need |= (any >> (8 * r) & 255u) ? 256u << r : 0u;
+      }
+      const int c0 = __popc(need);
+      int incl = c0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      tasks = __shfl_sync(0xffffffffu, incl, 31);
+      int at = incl - c0;
+      for (unsigned b = need; b; b &= b - 1) list[at++] = (unsigned short)(lane << 4 | (__ffs(b) - 1));
+    }
+    __syncwarp();
+    for (int t = lane; t < tasks; t += 32) {
+      const int e = list[t], j = e >> 4, c = e & 15, i = W.sel[j];
+      const bool x = c < 8;
+      const int2 r = W.ref[i];
+      const int k = min(1, max(-1, (x ? r.y & 255 : (r.y >> 8) & 255) - W.hc[c]));
+      const double f = reinterpret_cast<const double*>(p.f64 + r.x)[x ? 0 : 1];
+      const float2 q = W.xy[i];
+      const float df = fabsf((x ? q.x : q.y) - W.cx[c]);
+      const double d = fabs(DM(x ? p.a11 : p.a22, DA(f, W.off[c][k + 1])));
+      W.exy[j][c] = split58(gauss64(d, df * kGrid, T, s1024, ni2s2));
+    }
+    __syncwarp();
+    for (int t = lane; t < SL * cnt; t += 32) {
+      const int j = t / SL, k = t - SL * j, i = W.sel[j];
+      const int2 r = W.ref[i];
+      const double f = reinterpret_cast<const double*>(p.f64 + r.x)[2];
+      const double2 cs = p.cs64[r.x];
+      const float df = sqrtf(fmaxf(0.f, cut2f - W.hm[i][k]));
+      const double d = fabs(DM(p.a33, DA(f, W.zoff[r.y >> 16][k])));
+      const Fixed e = split58(gauss64(d, df * kGrid, T, s1024, ni2s2));
+      const Fixed re = split58(mul58(e, split58(to58(cs.x)))), im = split58(mul58(e, split58(to58(cs.y))));
+      W.be[k][j] = make_int4(re.h, re.l, im.h, im.l);
+    }
+    __syncwarp();
+    for (int j0 = 0; j0 < cnt; j0 += kFold) {
+      const int j1 = min(cnt, j0 + kFold);
+#pragma unroll 1
+      for (int j = j0; j < j1; ++j) {
+        const Fixed w = split58(mul58(W.exy[j][c], W.exy[j][row]));
+        alignas(16) unsigned ms[SL];
+        if constexpr (SL == 4) *reinterpret_cast<uint4*>(ms) = *reinterpret_cast<const uint4*>(W.m[j]);
+        else *reinterpret_cast<uint2*>(ms) = *reinterpret_cast<const uint2*>(W.m[j]);
+#pragma unroll
+        for (int k = 0; k < SL; ++k) {
+          const unsigned m = ms[k];
+          if (m) {  // the same branch in every lane
+            const int4 e = W.be[k][j];
+            const bool acc = m >> lane & 1;
+            const Fixed wk{acc ? w.h : 0, acc ? w.l : 0};
+            A.sr[k].add(wk, e.x, e.y);
+            A.si[k].add(wk, e.z, e.w);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < SL; ++k) {
+        A.sr[k].fold();
+        A.si[k].fold();
+      }
+    }
+    __syncwarp();
   }
-  __syncwarp();
 }
 
 // rho of convertScaledRangeToRho (:1973-1994), the reference's operations.
-__device__ __forceinline__ double rho64(double r2min, double sig) {
+__device__ __noinline__ double rho64(double r2min, double sig) {
   if (r2min < DM(sig, sig)) return 1.0;
   if (r2min > DM(DM(4.0, sig), sig)) return 0.0;
   const double xx = DS(__ddiv_rn(__dsqrt_rn(r2min), sig), 1.0);
@@ -216,7 +358,7 @@ __device__ __forceinline__ double rho64(double r2min, double sig) {
 template <int CAPS, int SL, bool kDens, bool kMasked>
 __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL>& W, int tile, int z_lo, int z_hi,
                                         double2* __restrict__ out, double* __restrict__ out_rho,
-                                        const double* __restrict__ T, int lane) {
+                                        const long long* __restrict__ T, int lane) {
   constexpr int TX = 8, TY = 4;
   const int Wd = p.ix1 - p.ix0;
   const int tiles_x = (Wd + TX - 1) / TX;
@@ -310,7 +452,8 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
     Acc<SL> A;
 #pragma unroll
     for (int k = 0; k < SL; ++k) {
-      A.sr[k] = A.si[k] = 0.0;
+      A.sr[k].clear();
+      A.si[k].clear();
       A.rm[k] = FLT_MAX;
     }
     int nb = 0;
@@ -334,15 +477,16 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
       lo = W.bin[slot][max(0, min(kBins, (int)floorf((w_lo - r3) * inv_bin)))];
       hi = W.bin[slot][max(0, min(kBins, (int)ceilf((w_hi + r3) * inv_bin)))];
     };
-    for (int u = need_lo; u <= need_hi; ++u) {
-      const int slot = u & (kRing - 1);
-      float t[SL];
-      bool v[SL];
-      int lo, hi;
-      window(u, t, v, lo, hi);
-      for (int b = lo; b < hi; b += 32) {
+    // one loop over slabs and rounds of 32 atoms, so that there is one copy of consume
+    float t[SL];
+    bool v[SL];
+    int u = need_lo - 1, b = 0, hi = 0;
+    for (;;) {
+      while (b >= hi && u < need_hi) window(++u, t, v, b, hi);
+      const bool more = b < hi;
+      if (more) {
         // one atom per lane: kept if some column of the patch can accept it at some slice
-        const int j = b + lane;
+        const int slot = u & (kRing - 1), j = b + lane;
         bool keep = false;
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
         float hm[SL];
@@ -368,16 +512,14 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
           for (int k = 0; k < SL; ++k) W.hm[d][k] = hm[k];
         }
         nb += __popc(m);
-        if (nb >= kN - 32) {
-          consume<CAPS, SL, kDens>(p, W, nb, Xv, Yv, cut2f, T, s1024, ni2s2, A, n_acc, lane);
-          n_tst += (unsigned long long)nb;
-          nb = 0;
-        }
+        b += 32;
       }
-    }
-    if (nb > 0) {
-      consume<CAPS, SL, kDens>(p, W, nb, Xv, Yv, cut2f, T, s1024, ni2s2, A, n_acc, lane);
-      n_tst += (unsigned long long)nb;
+      if (nb > (more ? kN - 33 : 0)) {
+        consume<CAPS, SL, kDens>(p, W, nb, Xv, Yv, cut2f, T, s1024, ni2s2, A, n_acc, lane);
+        n_tst += (unsigned long long)nb;
+        nb = 0;
+      }
+      if (!more) break;
     }
     // density: where the FP32 minimum lies in rho's range, the exact minimum over the atoms the
     // FP32 distance cannot tell from the nearest
@@ -396,8 +538,6 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
         for (int k = 0; k < SL; ++k) best[k] = DBL_MAX;
         for (int u = need_lo; u <= need_hi; ++u) {
           const int slot = u & (kRing - 1);
-          float t[SL];
-          bool v[SL];
           int lo, hi;
           window(u, t, v, lo, hi);
           for (int j = lo; j < hi; ++j) {
@@ -424,13 +564,14 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
 #pragma unroll
     for (int k = 0; k < SL; ++k) {
       if (z0 + k >= z_hi) break;
-      // x = S / max(1e-16, |S|) (:1877-1892); with density, rho x and rho are stored
-      double inv = rsqrt(fmax(DF(A.sr[k], A.sr[k], DM(A.si[k], A.si[k])), 1e-32));
+      // with density, rho x and rho are stored
+      double2 x = unit58(A.sr[k].lo, A.sr[k].hi, A.si[k].lo, A.si[k].hi);
       if constexpr (kDens) {
-        inv = DM(inv, rho[k]);
+        x.x = DM(x.x, rho[k]);
+        x.y = DM(x.y, rho[k]);
         out_rho[((int64_t)(z0 + k) << 5) + lane] = rho[k];
       }
-      out[((int64_t)(z0 + k) << 5) + lane] = make_double2(DM(A.sr[k], inv), DM(A.si[k], inv));
+      out[((int64_t)(z0 + k) << 5) + lane] = x;
     }
   }
   if (p.want_stats) {
@@ -449,7 +590,7 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
 
 template <int CAPS, int SL, bool kDens, bool kMasked, int kMinBlocks>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks)
-    k_field64(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R, const double* __restrict__ T) {
+    k_field64(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R, const long long* __restrict__ T) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpSmem<CAPS, SL>& W = reinterpret_cast<WarpSmem<CAPS, SL>*>(smem_raw)[warp];
@@ -579,7 +720,7 @@ __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict
 }
 
 template <int CAPS, int SL, bool kDens, bool kMasked, int B>
-cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, const double* T, cudaStream_t st) {
+cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, const long long* T, cudaStream_t st) {
   const size_t smem = sizeof(WarpSmem<CAPS, SL>) * kWarps;
   auto kernel = k_field64<CAPS, SL, kDens, kMasked, B>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -592,7 +733,7 @@ cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, const
 }
 
 template <int SL, bool kDens, bool kMasked>
-cudaError_t launch_tier(int tier, const ColumnJob* jobs, int n_jobs, const FieldRange& R, const double* T,
+cudaError_t launch_tier(int tier, const ColumnJob* jobs, int n_jobs, const FieldRange& R, const long long* T,
                         cudaStream_t st) {
   if (tier >= 2) return launch<256, SL, kDens, kMasked, 1>(jobs, n_jobs, R, T, st);
   if (tier == 1) return launch<192, SL, kDens, kMasked, 1>(jobs, n_jobs, R, T, st);
@@ -606,14 +747,15 @@ int field64_patches(const ColumnParams& p) {
   return Wd <= 0 || Hd <= 0 ? 0 : ((Wd + 7) / 8) * ((Hd + 3) / 4);
 }
 
-// exp(-(j / 1024)^2 / 2), j = 0 .. kGauss64Size - 1 (the library's exp: correctly rounded but for
-// one value in a few thousand)
-void gauss64_table(double* t) {
-  for (int j = 0; j < kGauss64Size; ++j) t[j] = std::exp(-0.5 * ((double)j / 1024.0) * ((double)j / 1024.0));
+// exp(-(j / 1024)^2 / 2) in units of 2^-58, j = 0 .. kGauss64Size - 1 (the library's exp: correctly
+// rounded but for one value in a few thousand)
+void gauss64_table(long long* t) {
+  for (int j = 0; j < kGauss64Size; ++j)
+    t[j] = std::llrint(std::ldexp(std::exp(-0.5 * ((double)j / 1024.0) * ((double)j / 1024.0)), 58));
 }
 
 cudaError_t launch_field64(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, int slab_tier,
-                           bool density, bool masked, bool four, const double* d_gauss, cudaStream_t st) {
+                           bool density, bool masked, bool four, const long long* d_gauss, cudaStream_t st) {
   using namespace field64;
   cudaError_t e = cudaSuccess;
   if (R.units() <= 0) return e;

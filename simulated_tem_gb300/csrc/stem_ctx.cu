@@ -42,7 +42,7 @@ struct st_ctx {
   size_t cap_tab = 0;
   void* d_samples = nullptr;  // field samples of one range of patches
   size_t cap_samples = 0;     // bytes
-  double* d_gauss = nullptr;  // gauss64_table
+  long long* d_gauss = nullptr;  // gauss64_table
   double* d_bx = nullptr;  // st_batch: packed atoms of the distinct atom arrays
   size_t cap_bx = 0;
   double* d_bimg = nullptr;  // st_batch: images
@@ -963,11 +963,11 @@ extern "C" int st_create(st_ctx** out, int device) {
   c->fp64_general = kv64 && std::strcmp(kv64, "general") == 0;
   const char* ks = std::getenv("STEM_RING_SLABS");
   c->min_slab_tier = !ks ? 0 : std::strcmp(ks, "256") == 0 ? 2 : std::strcmp(ks, "192") == 0 ? 1 : 0;
-  std::vector<double> gauss(kGauss64Size);
+  std::vector<long long> gauss(kGauss64Size);
   gauss64_table(gauss.data());
-  e = cudaMalloc((void**)&c->d_gauss, gauss.size() * sizeof(double));
+  e = cudaMalloc((void**)&c->d_gauss, gauss.size() * sizeof(long long));
   if (e == cudaSuccess)
-    e = cudaMemcpy(c->d_gauss, gauss.data(), gauss.size() * sizeof(double), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(c->d_gauss, gauss.data(), gauss.size() * sizeof(long long), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     st_destroy(c);
     return ST_ERR_CUDA;
