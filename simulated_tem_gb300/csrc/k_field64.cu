@@ -86,7 +86,7 @@ struct WarpSmem {
   alignas(16) unsigned m[kPass][SL];  // of the pass's atoms, per slice: the lanes that accept
   int sel[kPass];         // their places in the step buffer
   float2 xy[kN];          // X', Y'
-  int2 ref[kN];           // kept atom, cell code | slab number within the step << 16
+  int2 ref[kN];           // kept atom, cell code | slab number within the step << 16 | place in the slab << 18
   Fixed exy[kPass][12];   // the patch's 8 column and 4 row factors of the Gaussian
   int4 be[SL][kPass];     // per slice: z factor times (cos, sin); before that, the list of exy's tasks
   double off[12][3];      // k - zi_frac of the patch's columns and rows, k = -1, 0, 1
@@ -182,7 +182,9 @@ __device__ __noinline__ double2 unit58(unsigned long long rl, int rh, unsigned l
 template <int SL>
 struct Acc {
   Sum58 sr[SL], si[SL];
-  float rm[SL];  // FP32 min of r^2 - cutoff^2, scaled (density)
+  // density: the FP32 minimum of r^2 - cutoff^2 (scaled), the next one, and the minimum's atom
+  float rm[SL], next[SL];
+  int id[SL];
 };
 
 // Exact squared distance of kept atom gi (cell code `code`) and this lane's column at slice k of
@@ -205,20 +207,23 @@ __device__ __noinline__ double exact_dd(const ColumnParams& p, const WarpSmem<CA
 template <int CAPS, int SL, bool kDens>
 __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL>& W, int n, float Xv, float Yv,
                                         float cut2f, const long long* __restrict__ T, double s1024, double ni2s2,
-                                        Acc<SL>& A, unsigned& n_acc, int lane) {
+                                        Acc<SL>& A, unsigned act, unsigned& n_acc, int lane) {
   constexpr float kGrid = 1.1774100225f * 1024.f;  // scaled length -> sigma / 1024
   constexpr int U = 1;  // atoms at once
   __syncwarp();
   const int c = lane & 7, row = 8 + (lane >> 3);
+  const unsigned bit = 1u << lane;
   for (int i = 0; i < n;) {
     int cnt = 0;
     for (; i < n && cnt <= kPass - U; i += U) {
       bool acc[U][SL], near = false;
       float g[U][SL];
+      int id[U];
 #pragma unroll
       for (int j = 0; j < U; ++j) {
         const int a = min(i + j, n - 1);
         const float2 q = W.xy[a];
+        if (kDens) id[j] = W.ref[a].y >> 16;
         const float dx = q.x - Xv, dy = q.y - Yv;
         // past the last atom: its distances (written, so finite), far outside every cutoff
         const float h = i + j < n ? fmaf(dx, dx, dy * dy) : 3e30f;
@@ -237,7 +242,7 @@ __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL
             for (int k = 0; k < SL; ++k)
               if (fabsf(g[j][k]) <= kGuard64) {
                 const int2 r = W.ref[i + j];
-                acc[j][k] = exact_dd(p, W, r.x, r.y, r.y >> 16, k, lane) <= p.cut2;
+                acc[j][k] = exact_dd(p, W, r.x, r.y, (r.y >> 16) & 3, k, lane) <= p.cut2;
               }
         }
         __syncwarp();
@@ -249,8 +254,12 @@ __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL
         for (int k = 0; k < SL; ++k) {
           m[k] = __ballot_sync(0xffffffffu, acc[j][k]);
           any |= m[k];
-          n_acc += acc[j][k];
-          if (kDens) A.rm[k] = fminf(A.rm[k], g[j][k]);
+          if (kDens) {
+            const float v = g[j][k];
+            A.next[k] = fminf(A.next[k], fmaxf(v, A.rm[k]));
+            if (v < A.rm[k]) A.id[k] = id[j];
+            A.rm[k] = fminf(A.rm[k], v);
+          }
         }
         if (any) {
           if (lane == 0) {
@@ -264,7 +273,7 @@ __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL
     }
     if (cnt == 0) continue;
     __syncwarp();
-    // the list of the columns and rows that some lane needs
+    // the list of the columns and rows that some lane needs: place in the buffer, in the pass, column
     unsigned short* list = reinterpret_cast<unsigned short*>(&W.be[0][0]);
     int tasks;
     {
@@ -272,7 +281,10 @@ __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL
       if (lane < cnt) {
         unsigned any = 0;
 #pragma unroll
-        for (int k = 0; k < SL; ++k) any |= W.m[lane][k];
+        for (int k = 0; k < SL; ++k) {
+          any |= W.m[lane][k];
+          n_acc += __popc(W.m[lane][k] & act);
+        }
         need = (any | any >> 16);
         need = (need | need >> 8) & 255u;
 #pragma unroll
@@ -287,11 +299,12 @@ __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL
       }
       tasks = __shfl_sync(0xffffffffu, incl, 31);
       int at = incl - c0;
-      for (unsigned b = need; b; b &= b - 1) list[at++] = (unsigned short)(lane << 4 | (__ffs(b) - 1));
+      const int e0 = lane << 4 | (lane < cnt ? W.sel[lane] << 9 : 0);
+      for (unsigned b = need; b; b &= b - 1) list[at++] = (unsigned short)(e0 | (__ffs(b) - 1));
     }
     __syncwarp();
     for (int t = lane; t < tasks; t += 32) {
-      const int e = list[t], j = e >> 4, c = e & 15, i = W.sel[j];
+      const int e = list[t], j = (e >> 4) & 31, c = e & 15, i = e >> 9;
       const bool x = c < 8;
       const int2 r = W.ref[i];
       const int k = min(1, max(-1, (x ? r.y & 255 : (r.y >> 8) & 255) - W.hc[c]));
@@ -308,7 +321,7 @@ __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL
       const double f = reinterpret_cast<const double*>(p.f64 + r.x)[2];
       const double2 cs = p.cs64[r.x];
       const float df = sqrtf(fmaxf(0.f, cut2f - W.hm[i][k]));
-      const double d = fabs(DM(p.a33, DA(f, W.zoff[r.y >> 16][k])));
+      const double d = fabs(DM(p.a33, DA(f, W.zoff[(r.y >> 16) & 3][k])));
       const Fixed e = split58(gauss64(d, df * kGrid, T, s1024, ni2s2));
       const Fixed re = split58(mul58(e, split58(to58(cs.x)))), im = split58(mul58(e, split58(to58(cs.y))));
       W.be[k][j] = make_int4(re.h, re.l, im.h, im.l);
@@ -318,21 +331,21 @@ __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL
       const int j1 = min(cnt, j0 + kFold);
 #pragma unroll 1
       for (int j = j0; j < j1; ++j) {
-        const Fixed w = split58(mul58(W.exy[j][c], W.exy[j][row]));
+        // every load first: the products of w hide their latency
+        const Fixed gx = W.exy[j][c], gy = W.exy[j][row];
         alignas(16) unsigned ms[SL];
         if constexpr (SL == 4) *reinterpret_cast<uint4*>(ms) = *reinterpret_cast<const uint4*>(W.m[j]);
         else *reinterpret_cast<uint2*>(ms) = *reinterpret_cast<const uint2*>(W.m[j]);
+        int4 e[SL];
 #pragma unroll
-        for (int k = 0; k < SL; ++k) {
-          const unsigned m = ms[k];
-          if (m) {  // the same branch in every lane
-            const int4 e = W.be[k][j];
-            const bool acc = m >> lane & 1;
-            const Fixed wk{acc ? w.h : 0, acc ? w.l : 0};
-            A.sr[k].add(wk, e.x, e.y);
-            A.si[k].add(wk, e.z, e.w);
+        for (int k = 0; k < SL; ++k) e[k] = W.be[k][j];
+        const Fixed w = split58(mul58(gx, gy));
+#pragma unroll
+        for (int k = 0; k < SL; ++k)
+          if (ms[k] & bit) {
+            A.sr[k].add(w, e[k].x, e[k].y);
+            A.si[k].add(w, e[k].z, e[k].w);
           }
-        }
       }
 #pragma unroll
       for (int k = 0; k < SL; ++k) {
@@ -403,7 +416,8 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
   const float rm_lo = sig2 - cut2f - kGuard64, rm_hi = 4.f * sig2 - cut2f + kGuard64;
 
   int ring_lo = 1 << 30, ring_hi = (1 << 30) - 1;
-  unsigned n_acc = 0;
+  const unsigned act = __ballot_sync(0xffffffffu, active);
+  unsigned n_acc = 0;  // accepted by the tile's columns, of the atoms that this lane counts
   unsigned long long n_tst = 0;
   for (int z0 = z_lo; z0 < z_hi; z0 += SL) {
     // the step's slices: home z cells, FP32 depths in the frame of home cell hz[0] (the
@@ -454,7 +468,8 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
     for (int k = 0; k < SL; ++k) {
       A.sr[k].clear();
       A.si[k].clear();
-      A.rm[k] = FLT_MAX;
+      A.rm[k] = A.next[k] = FLT_MAX;
+      A.id[k] = 0;
     }
     int nb = 0;
     // per slab of the step: the bins that overlap the depth window of the slices it serves
@@ -507,7 +522,7 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
         if (keep) {
           const int d = nb + __popc(m & lt);
           W.xy[d] = make_float2(q.x, q.y);
-          W.ref[d] = make_int2(W.gi[slot][j], __float_as_int(q.w) | ((u - need_lo) << 16));
+          W.ref[d] = make_int2(W.gi[slot][j], __float_as_int(q.w) | ((u - need_lo) << 16) | (j << 18));
 #pragma unroll
           for (int k = 0; k < SL; ++k) W.hm[d][k] = hm[k];
         }
@@ -515,41 +530,50 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
         b += 32;
       }
       if (nb > (more ? kN - 33 : 0)) {
-        consume<CAPS, SL, kDens>(p, W, nb, Xv, Yv, cut2f, T, s1024, ni2s2, A, n_acc, lane);
+        consume<CAPS, SL, kDens>(p, W, nb, Xv, Yv, cut2f, T, s1024, ni2s2, A, act, n_acc, lane);
         n_tst += (unsigned long long)nb;
         nb = 0;
       }
       if (!more) break;
     }
-    // density: where the FP32 minimum lies in rho's range, the exact minimum over the atoms the
-    // FP32 distance cannot tell from the nearest
+    // density: where the FP32 minimum lies in rho's range, the exact distance of its atom; where the
+    // FP32 distance cannot tell the nearest from the next, the exact minimum over all that it cannot
     double rho[SL];
     if constexpr (kDens) {
-      bool want[SL], any = false;
+      bool want[SL], any = false, tie = false;
 #pragma unroll
       for (int k = 0; k < SL; ++k) {
         rho[k] = !p.use_density || A.rm[k] < rm_lo ? 1.0 : 0.0;
         want[k] = active && has[k] && p.use_density && A.rm[k] >= rm_lo && A.rm[k] <= fminf(rm_hi, 0.f);
         any = any || want[k];
+        tie = tie || (want[k] && A.next[k] <= A.rm[k] + 2.f * kGuard64);
       }
       if (__any_sync(0xffffffffu, any)) {
         double best[SL];
 #pragma unroll
-        for (int k = 0; k < SL; ++k) best[k] = DBL_MAX;
-        for (int u = need_lo; u <= need_hi; ++u) {
-          const int slot = u & (kRing - 1);
-          int lo, hi;
-          window(u, t, v, lo, hi);
-          for (int j = lo; j < hi; ++j) {
-            const float4 q = W.p[slot][j];
-            const float dx = q.x - Xv, dy = q.y - Yv;
-            const float h = fmaf(dx, dx, dy * dy);
+        for (int k = 0; k < SL; ++k) {
+          best[k] = DBL_MAX;
+          if (want[k]) {
+            const int us = A.id[k] & 3, slot = (need_lo + us) & (kRing - 1), j = A.id[k] >> 2;
+            best[k] = exact_dd(p, W, W.gi[slot][j], __float_as_int(W.p[slot][j].w), us, k, lane);
+          }
+        }
+        if (__any_sync(0xffffffffu, tie)) {
+          for (int u = need_lo; u <= need_hi; ++u) {
+            const int slot = u & (kRing - 1);
+            int lo, hi;
+            window(u, t, v, lo, hi);
+            for (int j = lo; j < hi; ++j) {
+              const float4 q = W.p[slot][j];
+              const float dx = q.x - Xv, dy = q.y - Yv;
+              const float h = fmaf(dx, dx, dy * dy);
 #pragma unroll
-            for (int k = 0; k < SL; ++k) {
-              const float dz = q.z - t[k];
-              if (want[k] && v[k] && h + dz * dz - cut2f <= A.rm[k] + 2.f * kGuard64) {
-                const double dd = exact_dd(p, W, W.gi[slot][j], __float_as_int(q.w), u - need_lo, k, lane);
-                if (dd <= p.cut2 && dd < best[k]) best[k] = dd;
+              for (int k = 0; k < SL; ++k) {
+                const float dz = q.z - t[k];
+                if (want[k] && v[k] && h + dz * dz - cut2f <= A.rm[k] + 2.f * kGuard64) {
+                  const double dd = exact_dd(p, W, W.gi[slot][j], __float_as_int(q.w), u - need_lo, k, lane);
+                  if (dd <= p.cut2 && dd < best[k]) best[k] = dd;
+                }
               }
             }
           }
@@ -575,7 +599,7 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
     }
   }
   if (p.want_stats) {
-    unsigned long long acc_w = active ? n_acc : 0u, tst_w = active ? (unsigned long long)SL * n_tst : 0u;
+    unsigned long long acc_w = n_acc, tst_w = active ? (unsigned long long)SL * n_tst : 0u;
     for (int o = 16; o > 0; o >>= 1) {
       acc_w += __shfl_xor_sync(0xffffffffu, acc_w, o);
       tst_w += __shfl_xor_sync(0xffffffffu, tst_w, o);
