@@ -111,6 +111,9 @@ struct ColumnParams {
   double i2s2;           // 1 / (2 sigma^2)
   double sigma;
   double b0, bg, dz;
+  // the FP64 path's fixed-point integrator: dz times b0, bg and 1 times 2^fx_shift; fx_shift < 0: FP64
+  double fx_b0, fx_bg, fx_a;
+  int fx_shift;
   // FP32 scaled lengths (s = sqrt(log2 e / 2 sigma^2)): s, the link-cell sides, (3 sigma)^2, and back to A^2
   float scale, a11s, a22s, a33s, cut2s, r2_to_A2;
   const int* cell_start;

@@ -172,11 +172,23 @@ __device__ __forceinline__ double value58(unsigned long long lo, int hi) {
   return DF((double)hi, 0x1p64, __ull2double_rn(lo));
 }
 
-// S / max(1e-16, |S|) (:1877-1892); one copy of its code for all slices
-__device__ __noinline__ double2 unit58(unsigned long long rl, int rh, unsigned long long il, int ih) {
+// x (|x| <= 1) in units of 2^-60, cut off
+__device__ __forceinline__ long long to60(double x) {
+  const long long b = __double_as_longlong(x);
+  const int e = (int)(b >> 52) & 0x7FF;
+  const long long m = (((b & ((1LL << 52) - 1)) | (1LL << 52)) << 8) >> min(63, 1023 - e);
+  return b < 0 ? -m : m;
+}
+
+// The sample of a voxel: f S / max(1e-16, |S|) (:1877-1892), the bits of an FP64 number or, for the
+// fixed-point integrator, units of 2^-60; one copy of its code for all slices.
+__device__ __noinline__ longlong2 sample(unsigned long long rl, int rh, unsigned long long il, int ih, double f,
+                                         bool fixed) {
   const double sr = value58(rl, rh), si = value58(il, ih);
   const double inv = rsqrt(fmax(DF(sr, sr, DM(si, si)), 1e-32 * 0x1p116));
-  return make_double2(DM(sr, inv), DM(si, inv));
+  const double x = DM(DM(sr, inv), f), y = DM(DM(si, inv), f);
+  if (fixed) return make_longlong2(to60(x), to60(y));
+  return make_longlong2(__double_as_longlong(x), __double_as_longlong(y));
 }
 
 template <int SL>
@@ -370,7 +382,7 @@ __device__ __noinline__ double rho64(double r2min, double sig) {
 // (slice z, lane at out[(z << 5) + lane]).  False when a slab overflows its staging.
 template <int CAPS, int SL, bool kDens, bool kMasked>
 __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL>& W, int tile, int z_lo, int z_hi,
-                                        double2* __restrict__ out, double* __restrict__ out_rho,
+                                        longlong2* __restrict__ out, long long* __restrict__ out_rho,
                                         const long long* __restrict__ T, int lane) {
   constexpr int TX = 8, TY = 4;
   const int Wd = p.ix1 - p.ix0;
@@ -588,14 +600,15 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
 #pragma unroll
     for (int k = 0; k < SL; ++k) {
       if (z0 + k >= z_hi) break;
-      // with density, rho x and rho are stored
-      double2 x = unit58(A.sr[k].lo, A.sr[k].hi, A.si[k].lo, A.si[k].hi);
+      // with density, rho x and rho are stored; the fixed-point integrator's coefficients where it runs
+      const bool fixed = p.fx_shift >= 0;
+      double f = fixed ? p.fx_bg : 1.0;
       if constexpr (kDens) {
-        x.x = DM(x.x, rho[k]);
-        x.y = DM(x.y, rho[k]);
-        out_rho[((int64_t)(z0 + k) << 5) + lane] = rho[k];
+        f = DM(f, rho[k]);
+        out_rho[((int64_t)(z0 + k) << 5) + lane] =
+            fixed ? to60(DM(rho[k], p.fx_b0)) : __double_as_longlong(rho[k]);
       }
-      out[((int64_t)(z0 + k) << 5) + lane] = x;
+      out[((int64_t)(z0 + k) << 5) + lane] = sample(A.sr[k].lo, A.sr[k].hi, A.si[k].lo, A.si[k].hi, f, fixed);
     }
   }
   if (p.want_stats) {
@@ -630,7 +643,8 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks)
     const int z_lo = unit % R.n_chunks * R.chunk, z_hi = min(J.p.Mz, z_lo + R.chunk);
     if (z_lo >= z_hi) continue;  // an image less deep than the batch's deepest
     const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32;
-    if (!field_tile<CAPS, SL, kDens, kMasked>(J.p, W, patch, z_lo, z_hi, (double2*)R.samples + o, R.rho64 + o, T, lane))
+    if (!field_tile<CAPS, SL, kDens, kMasked>(J.p, W, patch, z_lo, z_hi, (longlong2*)R.samples + o, (long long*)R.rho64 + o, T,
+                                               lane))
       break;
   }
 }
@@ -677,11 +691,76 @@ __device__ __forceinline__ void rk4_64(const S64& s0, const S64& s1, const S64& 
   }
 }
 
+// The same in fixed point: numbers in units of 2^-60 as h 2^30 + l, 0 <= l < 2^30.
+constexpr int kLimb60 = 30;
+__device__ __forceinline__ Fixed split60(long long v) {
+  return Fixed{(int)(v >> kLimb60), (int)v & ((1 << kLimb60) - 1)};
+}
+
+struct SFix {
+  Fixed c0, ca, cgr, cgi, ngi;  // times dz 2^shift; ngi = -cgi
+};
+
+// (a x + b y + c z) 2^-shift, rounded (the low limbs' products, below one unit before the shift, left out)
+__device__ __forceinline__ long long row60(const Fixed& a, const Fixed& x, const Fixed& b, const Fixed& y,
+                                           const Fixed& c, const Fixed& z, long long half, int shift) {
+  long long hh = half, m = 0;
+  hh += wide(a.h, x.h);
+  hh += wide(b.h, y.h);
+  hh += wide(c.h, z.h);
+  m += wide(a.h, x.l);
+  m += wide(a.l, x.h);
+  m += wide(b.h, y.l);
+  m += wide(b.l, y.h);
+  m += wide(c.h, z.l);
+  m += wide(c.l, z.h);
+  return (hh + (m >> kLimb60)) >> shift;
+}
+
+// dz d/dz (phi_0, phi_g), as deriv64
+__device__ __forceinline__ void deriv60(const SFix& s, const long long* v, long long half, int shift, long long* d) {
+  Fixed p[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) p[i] = split60(v[i]);
+  d[0] = -row60(s.c0, p[1], s.cgi, p[2], s.cgr, p[3], half, shift);
+  d[1] = row60(s.c0, p[0], s.cgr, p[2], s.ngi, p[3], half, shift);
+  d[2] = -row60(s.ca, p[3], s.cgr, p[1], s.ngi, p[0], half, shift);
+  d[3] = row60(s.ca, p[2], s.cgi, p[1], s.cgr, p[0], half, shift);
+}
+
+__device__ __forceinline__ void rk4_60(const SFix& s0, const SFix& s1, const SFix& s2, long long half, int shift,
+                                       long long* ph) {
+  long long k1[4], ks[4], k[4], q[4];
+  deriv60(s0, ph, half, shift, k1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) q[i] = ph[i] + k1[i];
+  deriv60(s1, q, half, shift, ks);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) q[i] = ph[i] + ks[i];
+  deriv60(s1, q, half, shift, k);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    ks[i] += k[i];
+    q[i] = ph[i] + 2 * k[i];
+  }
+  deriv60(s2, q, half, shift, k);
+  const int third = 357913941;  // 2^60 / 3, both limbs
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const Fixed t = split60(k1[i] + k[i] + 2 * ks[i]);
+    ph[i] += wide(t.h, third) + ((wide(t.h, third) + wide(t.l, third) + (3LL << (kLimb60 - 2))) >> kLimb60);
+  }
+}
+
 // A warp per patch and angle (warp w of the CTA takes angles w, w + warps, ...), one lane per
-// column.  Bound by the FP64 pipe: about 90 operations per double step.  The equations are
-// linear, so the reference's renormalisation after every double step (:2466-2472) only
-// scales phi: it is done every 8 steps, and at the end through the quotient (every step when a
-// step could grow phi by more than a small factor).
+// column.  FP64 takes about 90 operations per double step, at 76 cycles each; in fixed point they are
+// 156 multiply-adds of 4 cycles and as much again of additions and shifts.  The host takes
+// fixed point where 2^-60 is no coarser than FP64 for these amplitudes (fixed_integrator): the steps
+// are short, so that no number exceeds 1.3 and the norm stays (each step loses less than 2e-6 of it),
+// and |phi_g| is not small against 1.
+// In FP64, the equations being linear, the reference's renormalisation after every double step
+// (:2466-2472) only scales phi: it is done every 8 steps, and at the end through the quotient (every
+// step when a step could grow phi by more than a small factor).
 template <bool kDens>
 __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R) {
   __shared__ double part[8][32];
@@ -701,7 +780,7 @@ __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict
   const double2* __restrict__ X = (const double2*)R.samples + o;
   const double* __restrict__ RH = R.rho64 + o;
   const double dz = p.dz, dz3h = __ddiv_rn(dz, 3.0), dz3l = __ddiv_rn(DF(-3.0, dz3h, dz), 3.0);
-  auto sample = [&](int z) {
+  auto coef = [&](int z) {
     const double2 x = X[(int64_t)z << 5];
     const double c0 = kDens ? DM(p.b0, RH[(int64_t)z << 5]) : p.b0;
     return S64{c0, DM(p.bg, x.x), DM(p.bg, x.y)};
@@ -709,14 +788,46 @@ __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict
   double total = 0.0;
   for (int k0 = 0; k0 < p.n_prec; k0 += nw) {
     const int k = k0 + warp;
-    if (k < p.n_prec) {
+    if (k < p.n_prec && p.fx_shift >= 0) {
+      const longlong2* __restrict__ XF = (const longlong2*)X;
+      const long long* __restrict__ RF = (const long long*)RH;
+      const int shift = p.fx_shift;
+      const long long half = (1LL << shift) >> 1, b0 = to60(p.fx_b0), a = to60(DM(p.aa[k], p.fx_a));
+      auto coef60 = [&](const longlong2& x, long long c0) {
+        const Fixed gi = split60(x.y);
+        return SFix{split60(c0), split60(c0 + a), split60(x.x), gi, Fixed{-gi.h, -gi.l}};
+      };
+      long long ph[4] = {1LL << 60, 0, 0, 0};
+      SFix s0 = coef60(XF[0], kDens ? RF[0] : b0);
+      // the samples of the next double step are loaded ahead
+      auto at = [&](int z) { return (int64_t)(z < p.Mz ? z : 0) << 5; };
+      longlong2 x1 = XF[at(1)], x2 = XF[at(2)];
+      long long r1 = kDens ? RF[at(1)] : b0, r2 = kDens ? RF[at(2)] : b0;
+#pragma unroll 1
+      for (int z = 2; z <= p.Mz; z += 2) {
+        const SFix s1 = coef60(x1, r1), s2 = coef60(x2, r2);
+        x1 = XF[at(z + 1)];
+        x2 = XF[at(z + 2)];
+        if (kDens) {
+          r1 = RF[at(z + 1)];
+          r2 = RF[at(z + 2)];
+        }
+        rk4_60(s0, s1, s2, half, shift, ph);
+        s0 = s2;
+      }
+      double v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = __ll2double_rn(ph[i]);
+      const double ig = DF(v[2], v[2], DM(v[3], v[3]));
+      part[warp][lane] = __ddiv_rn(ig, DF(v[0], v[0], DF(v[1], v[1], ig)));
+    } else if (k < p.n_prec) {
       const double a = p.aa[k];
       const int every = 2.0 * dz * (fabs(p.b0) + fabs(p.bg) + fabs(a)) < 1.0 ? 8 : 1;
       double ph[4] = {1.0, 0.0, 0.0, 0.0};
-      S64 s0 = sample(0);
+      S64 s0 = coef(0);
       int n = 0;
       for (int z = 2; z <= p.Mz; z += 2) {  // the last sample of an even column is the first (:1898-1899)
-        const S64 s1 = sample(z - 1), s2 = sample(z < p.Mz ? z : 0);
+        const S64 s1 = coef(z - 1), s2 = coef(z < p.Mz ? z : 0);
         rk4_64(s0, s1, s2, a, dz, dz3h, dz3l, ph);
         s0 = s2;
         if (++n == every) {

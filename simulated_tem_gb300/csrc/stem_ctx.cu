@@ -319,6 +319,31 @@ void point_at_kept(const st_ctx* c, ColumnParams& cp) {
   cp.ph32 = c->b.ph32;
 }
 
+// Whether the FP64 path's integrator runs in fixed point (units of 2^-60; FIX_TIMES), and
+// its coefficients: where it is no less precise than FP64.  The double steps are short (so that no
+// intermediate exceeds 1.3 and the norm is kept without renormalisation), and |phi_g| is not small
+// against 1: neither by a weak reflection (|phi_g| up to the thickness times bg) nor by excitation
+// errors (up to bg / a).  The coefficients are scaled up to use their limbs.
+void fixed_integrator(ColumnParams& cp, const double* aa) {
+  cp.fx_shift = -1;
+  double a = 0.0;
+  for (int k = 0; k < cp.n_prec; ++k) {
+    if (!std::isfinite(aa[k])) return;
+    a = std::max(a, std::fabs(aa[k]));
+  }
+  const double b0 = std::fabs(cp.b0), bg = std::fabs(cp.bg);
+  if (!(cp.dz > 0.0) || !(2.0 * cp.dz * (b0 + bg + a) <= 0.25) || !(bg * 32.0 >= a) ||
+      !(cp.Mz * cp.dz * bg >= 1.0 / 16.0) || cp.Mz > 50000)
+    return;
+  int e = 0;
+  std::frexp(cp.dz * std::max(b0 + a, bg), &e);  // below 2^e <= 1/4
+  if (e < -24) return;
+  cp.fx_shift = -e;
+  cp.fx_a = std::ldexp(cp.dz, -e);
+  cp.fx_b0 = cp.b0 * cp.fx_a;
+  cp.fx_bg = cp.bg * cp.fx_a;
+}
+
 ColumnParams column_params(st_ctx* c, const Job& j, int64_t cell_base, size_t xoff, size_t yoff, size_t zoff,
                            size_t aoff, int flags) {
   const st_geom* g = j.g;
@@ -346,6 +371,7 @@ ColumnParams column_params(st_ctx* c, const Job& j, int64_t cell_base, size_t xo
   cp.b0 = g->b0;
   cp.bg = g->bg;
   cp.dz = g->deltaz;
+  fixed_integrator(cp, j.aa);
   const double sd = length_scale(g);
   cp.scale = (float)sd;
   cp.a11s = (float)(cp.a11 * sd);
