@@ -12,10 +12,11 @@
 // step (two where some image's steps of four do not fit the ring), the atoms of the link-cell
 // slabs staged in warp-private shared memory and ordered by z bin (slab_ring.cuh).
 //
-// What bounds it is the FP64 pipe: one warp instruction per 76 cycles and SM sub-partition
-// (measured; predicated-off lanes, fully predicated-off instructions and FP64 <-> FP32
-// conversions cost the same), against one FP32 or integer instruction per cycle.  So FP64 is
-// spent only where the result needs it:
+// The FP64 pipe takes one warp instruction per 76 cycles and SM sub-partition (measured;
+// predicated-off lanes, fully predicated-off instructions and FP64 <-> FP32 conversions cost the
+// same), against 2 for an FP32 or integer instruction and 4 for a 32 x 32 -> 64-bit multiply-add,
+// which run beside it.  So FP64 is spent only where the result needs it, and sums and products of
+// bounded numbers are fixed-point:
 // * The accept decision is the reference's, d.d <= (3 sigma)^2 in its rounded operations
 //   (d_a = a_aa (f_a + (k_a - zi_frac_a)), the fractions f of the FP64 binning, the unwrapped
 //   27-cell offsets k).  An FP32 distance decides every pair further than kGuard64 from the
@@ -23,20 +24,26 @@
 //   set equals the reference's.
 // * The weight is a product of three Gaussians, one per axis: exp(-d_x^2 / 2 sigma^2) depends on
 //   the atom and one of the patch's 8 columns, the y factor on one of its 4 rows, the z factor
-//   (times the phasor) on the slice.  The warp evaluates these 16 values per buffered atom as
-//   one flat list of tasks over its lanes instead of one exp per lane.
-// * The Gaussian itself is a table value times a short polynomial (gauss64): 9 FP64 operations.
-// * A lane then spends one multiplication per atom and two fused multiply-adds per slice that
-//   some lane of the warp accepts.
-// Measured (GB300, whole calls): 128k atoms with density 29.0 -> 7.4 ms, 28k atoms 6.75 -> 0.86 ms,
-// 16k atoms with six precession angles 13.6 -> 1.35 ms (before: one exp, the divisions of the
-// reference's integrator and hypot in every lane, a whole column per warp, the field once per four
-// angles).
+//   (times the phasor) on the slice.  The warp evaluates the values that an accepting lane needs
+//   as one flat list of tasks over its lanes instead of one exp per lane.
+// * The Gaussian itself is a table value times a short polynomial (gauss64): six FP64 operations
+//   for the distance, the rest integers.
+// * A lane then multiplies two 58-bit numbers per atom, and adds two products per slice, six
+//   32 x 32-bit multiply-adds.  An accepted weight lies in [exp(-4.5), 1], so that 2^-58 is no
+//   coarser than FP64, and the sums do not round.
+// Now latency bounds it (12 warps per SM, limited by their staging; 0.45 instructions per cycle and
+// sub-partition), and code size: with two copies of the consuming code, or two atoms per iteration, the
+// instruction fetches cost 128k atoms with density a fifth.
+// Measured (GB300, whole calls): 128k atoms with density 29.0 ms with one exp, the divisions of the
+// reference's integrator and hypot in every lane, 7.2 with all of this in FP64, 4.83 now; 28k atoms
+// 6.75, 0.83, 0.53; 16k atoms with six precession angles 13.6, 1.32, 0.71.  128k atoms: field 4.33 ms
+// (a third of it the sums, a fifth the tests and the density's nearest atoms, a fifth the Gaussians),
+// integrator 0.20.
 //
-// Precision: gauss64 is within 2.4 units of 2^-53 of the exact value (root mean square 0.57;
+// Precision: the Gaussians are within 2.4 units of 2^-53 of the exact value (root mean square 0.57;
 // exp of the rounded d.d / 2 sigma^2, up to 4.5, is within 13.5, 2.1 in the mean square: the rounding of
-// its argument); the weight takes two more products, the sums and the integrator are fused.  Images
-// against a 64-bit evaluation of the same sums: relative 2-norm 0.4 to 1.2e-15 (before 0.5 to 1.6e-15).
+// its argument).  Images against a 64-bit evaluation of the same sums: relative 2-norm 0.3 to 1.0e-15
+// (before 0.5 to 1.6e-15).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -221,66 +228,51 @@ __device__ __forceinline__ void consume(const ColumnParams& p, WarpSmem<CAPS, SL
                                         float cut2f, const long long* __restrict__ T, double s1024, double ni2s2,
                                         Acc<SL>& A, unsigned act, unsigned& n_acc, int lane) {
   constexpr float kGrid = 1.1774100225f * 1024.f;  // scaled length -> sigma / 1024
-  constexpr int U = 1;  // atoms at once
   __syncwarp();
   const int c = lane & 7, row = 8 + (lane >> 3);
   const unsigned bit = 1u << lane;
   for (int i = 0; i < n;) {
     int cnt = 0;
-    for (; i < n && cnt <= kPass - U; i += U) {
-      bool acc[U][SL], near = false;
-      float g[U][SL];
-      int id[U];
+    for (; i < n && cnt < kPass; ++i) {
+      const float2 q = W.xy[i];
+      const float dx = q.x - Xv, dy = q.y - Yv;
+      const float h = fmaf(dx, dx, dy * dy);
+      bool acc[SL], near = false;
+      float g[SL];
 #pragma unroll
-      for (int j = 0; j < U; ++j) {
-        const int a = min(i + j, n - 1);
-        const float2 q = W.xy[a];
-        if (kDens) id[j] = W.ref[a].y >> 16;
-        const float dx = q.x - Xv, dy = q.y - Yv;
-        // past the last atom: its distances (written, so finite), far outside every cutoff
-        const float h = i + j < n ? fmaf(dx, dx, dy * dy) : 3e30f;
-#pragma unroll
-        for (int k = 0; k < SL; ++k) {
-          g[j][k] = h - W.hm[a][k];
-          acc[j][k] = g[j][k] <= 0.f;
-          near = near || fabsf(g[j][k]) <= kGuard64;
-        }
+      for (int k = 0; k < SL; ++k) {
+        g[k] = h - W.hm[i][k];
+        acc[k] = g[k] <= 0.f;
+        near = near || fabsf(g[k]) <= kGuard64;
       }
       if (__any_sync(0xffffffffu, near)) {
         if (near) {
+          const int2 r = W.ref[i];
 #pragma unroll
-          for (int j = 0; j < U; ++j)
-#pragma unroll
-            for (int k = 0; k < SL; ++k)
-              if (fabsf(g[j][k]) <= kGuard64) {
-                const int2 r = W.ref[i + j];
-                acc[j][k] = exact_dd(p, W, r.x, r.y, (r.y >> 16) & 3, k, lane) <= p.cut2;
-              }
+          for (int k = 0; k < SL; ++k)
+            if (fabsf(g[k]) <= kGuard64) acc[k] = exact_dd(p, W, r.x, r.y, (r.y >> 16) & 3, k, lane) <= p.cut2;
         }
         __syncwarp();
       }
+      unsigned m[SL], any = 0;
+      const int id = kDens ? W.ref[i].y >> 16 : 0;
 #pragma unroll
-      for (int j = 0; j < U; ++j) {
-        unsigned m[SL], any = 0;
-#pragma unroll
-        for (int k = 0; k < SL; ++k) {
-          m[k] = __ballot_sync(0xffffffffu, acc[j][k]);
-          any |= m[k];
-          if (kDens) {
-            const float v = g[j][k];
-            A.next[k] = fminf(A.next[k], fmaxf(v, A.rm[k]));
-            if (v < A.rm[k]) A.id[k] = id[j];
-            A.rm[k] = fminf(A.rm[k], v);
-          }
+      for (int k = 0; k < SL; ++k) {
+        m[k] = __ballot_sync(0xffffffffu, acc[k]);
+        any |= m[k];
+        if (kDens) {
+          A.next[k] = fminf(A.next[k], fmaxf(g[k], A.rm[k]));
+          if (g[k] < A.rm[k]) A.id[k] = id;
+          A.rm[k] = fminf(A.rm[k], g[k]);
         }
-        if (any) {
-          if (lane == 0) {
-            W.sel[cnt] = i + j;
-            if constexpr (SL == 4) *reinterpret_cast<uint4*>(W.m[cnt]) = make_uint4(m[0], m[1], m[2], m[3]);
-            else *reinterpret_cast<uint2*>(W.m[cnt]) = make_uint2(m[0], m[1]);
-          }
-          ++cnt;
+      }
+      if (any) {
+        if (lane == 0) {
+          W.sel[cnt] = i;
+          if constexpr (SL == 4) *reinterpret_cast<uint4*>(W.m[cnt]) = make_uint4(m[0], m[1], m[2], m[3]);
+          else *reinterpret_cast<uint2*>(W.m[cnt]) = make_uint2(m[0], m[1]);
         }
+        ++cnt;
       }
     }
     if (cnt == 0) continue;

@@ -319,8 +319,8 @@ void point_at_kept(const st_ctx* c, ColumnParams& cp) {
   cp.ph32 = c->b.ph32;
 }
 
-// Whether the FP64 path's integrator runs in fixed point (units of 2^-60; FIX_TIMES), and
-// its coefficients: where it is no less precise than FP64.  The double steps are short (so that no
+// Whether the FP64 path's integrator runs in fixed point (units of 2^-60; 16k atoms and
+// six angles 146 us instead of 505, 128k atoms with density 198 instead of 710), and its coefficients: where it is no less precise than FP64.  The double steps are short (so that no
 // intermediate exceeds 1.3 and the norm is kept without renormalisation), and |phi_g| is not small
 // against 1: neither by a weak reflection (|phi_g| up to the thickness times bg) nor by excitation
 // errors (up to bg / a).  The coefficients are scaled up to use their limbs.
