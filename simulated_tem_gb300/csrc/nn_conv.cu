@@ -38,6 +38,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <mutex>
 #include <type_traits>
 
@@ -74,6 +75,10 @@ struct ConvArgs {
   int xtiles, n_tiles;        // tiles: (x tile, row group, image, channel tile)
 };
 
+// 16-byte output pieces per pixel and pass of the epilogue: what two CTAs per SM leave room for
+template <int BN>
+constexpr int kStagePieces = BN >= 128 ? 2 : BN >= 32 ? 4 : BN / 8;
+
 template <int BN, int KC, int NR>
 struct TSmem {
   static constexpr int kBSlots = b_slots(BN);
@@ -83,6 +88,9 @@ struct TSmem {
       acc_empty[2], done;
   uint32_t tmem;
   int abort;
+  alignas(16) uint4 stage[4][32 * kStagePieces<BN>];  // the epilogue warps' output pieces
+  // without the padding at the end, which at BN = 128 would cost the second CTA
+  static constexpr size_t bytes() { return offsetof(TSmem, stage) + sizeof(stage); }
 };
 
 // bounded wait that gives up early when another role has aborted
@@ -93,6 +101,17 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t mbar, uint32_t parity, vo
   }
   *abort = 1;
   return false;
+}
+
+// Eight channels, zero where the mask is not positive
+__device__ __forceinline__ uint4 masked(uint4 q, const uint4& m) {
+  const __nv_bfloat162* v = reinterpret_cast<const __nv_bfloat162*>(&m);
+  const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+  q.x &= __hgt2_mask(v[0], zero);
+  q.y &= __hgt2_mask(v[1], zero);
+  q.z &= __hgt2_mask(v[2], zero);
+  q.w &= __hgt2_mask(v[3], zero);
+  return q;
 }
 
 struct Tile {
@@ -257,10 +276,28 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_fwd(const ConvArgs a, con
     for (int tt = blockIdx.x; tt < a.n_tiles; tt += gridDim.x, ++k) {
       const Tile tl = tile_of(a, tt, BN);
       const int buf = k & 1;
+      const bool staged = tl.n0 + BN <= a.Cout && !a.y_fp32;
+      constexpr int kNC = kStagePieces<BN>;
+      // the mask's values are loaded before the accumulators are waited for (BN <= 64: the registers
+      // allow it; 568 x 568 pixels, 192 to 64 channels 116 -> 105 us)
+      constexpr bool kAhead = BN <= 64;
+      uint4 mk[kAhead ? BN / 8 : 1];
+      auto load_mask = [&](int q) {
+        const int x32 = tl.xt * kTileX + 32 * warp;
+        const size_t row = ((size_t)tl.img * a.H + tl.y + q) * a.W + x32;
+#pragma unroll
+        for (int c = 0; c < (kAhead ? BN / 8 : 0); ++c) {
+          const int px = 32 * (c % kNC) / kNC + lane / kNC, n = tl.n0 + 8 * (c / kNC * kNC + lane % kNC);
+          if (x32 + px < a.W && tl.y + q < a.H)
+            mk[c] = *reinterpret_cast<const uint4*>(a.mask + (row + px) * a.Cout + n);
+        }
+      };
+      if (kAhead && a.mask && staged) load_mask(0);
       if (!wait_or_abort(tc::smem_addr(&S.acc_full[buf]), (k >> 1) & 1, abort)) break;
       tc::fence_after_sync();
 #pragma unroll 1
       for (int q = 0; q < kRowsPerTile; ++q) {
+      if (kAhead && q > 0 && a.mask && staged) load_mask(q);
       float v[BN];
       {
         uint32_t reg[BN];
@@ -280,8 +317,49 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_fwd(const ConvArgs a, con
         if (lane == 0)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_addr(&S.acc_empty[buf])) : "memory");
       }
-      const int xw = tl.xt * kTileX + 32 * warp + lane;
-      if (xw < a.W && tl.y + q < a.H) {
+      const int x32 = tl.xt * kTileX + 32 * warp, xw = x32 + lane;
+      if (staged) {
+        // whole sectors per store, through shared memory (as in the strip kernel): 568 x 568 pixels, 192 to
+        // 64 channels 112 -> 100 us, 8 x 128 x 128, 128 to 128 channels 68 -> 60
+        uint4* stage = S.stage[warp];
+        auto place = [](int px, int ch) { return px * kNC + (ch ^ (kNC == 4 ? (px >> 1) & 3 : 0)); };
+        const size_t row = ((size_t)tl.img * a.H + tl.y + q) * a.W + x32;
+#pragma unroll
+        for (int c0 = 0; c0 < BN; c0 += 8 * kNC) {
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < kNC; ++c) {
+            const int n = tl.n0 + c0 + 8 * c;
+            __align__(16) __nv_bfloat162 h[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float x = v[c0 + 8 * c + 2 * i], y = v[c0 + 8 * c + 2 * i + 1];
+              if (a.bias) {
+                x += a.bias[n + 2 * i];
+                y += a.bias[n + 2 * i + 1];
+              }
+              if (a.relu) {
+                x = fmaxf(x, 0.f);
+                y = fmaxf(y, 0.f);
+              }
+              h[i] = __floats2bfloat162_rn(x, y);
+            }
+            stage[place(lane, c)] = *reinterpret_cast<const uint4*>(h);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < kNC; ++c) {
+            const int px = 32 * c / kNC + lane / kNC;
+            if (x32 + px < a.W && tl.y + q < a.H) {
+              const size_t at = (row + px) * a.Cout + tl.n0 + c0 + 8 * (lane % kNC);
+              uint4 o = stage[place(px, lane % kNC)];
+              if (a.mask)
+                o = masked(o, kAhead ? mk[kAhead ? c0 / 8 + c : 0] : *reinterpret_cast<const uint4*>(a.mask + at));
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.y) + at) = o;
+            }
+          }
+        }
+      } else if (xw < a.W && tl.y + q < a.H) {
         const size_t p = ((size_t)tl.img * a.H + tl.y + q) * a.W + xw;
 #pragma unroll
         for (int col = 0; col < BN; col += 8) {
@@ -440,7 +518,7 @@ cudaError_t launch_fwd(const __nv_bfloat16* x, const __nv_bfloat16* w, ConvArgs 
   a.wb = bw.p;
   // CTAs per SM: shared memory, and TMEM (2 kRowsPerTile BN columns each, 512 per SM)
   constexpr int kRowsPerTile = rows_per_tile(BN);
-  const size_t per_sm = 232448, need = sizeof(TSmem<BN, KC, NR>) + 1024;
+  const size_t per_sm = 232448, need = TSmem<BN, KC, NR>::bytes() + 1024;
   int ctas = (int)(per_sm / (need + 1024));
   ctas = ctas < 1 ? 1 : ctas;
   if (ctas * 2 * kRowsPerTile * BN > 512) ctas = 512 / (2 * kRowsPerTile * BN);
