@@ -479,16 +479,21 @@ cudaError_t sample_workspace(st_ctx* c, size_t want, size_t least, size_t& room)
 
 // Slices per unit of work (a multiple of 4) of `tiles` tiles up to `deepest` slices deep, `per_sm` of
 // which an SM works on at a time, when a unit costs `fixed` slices beside its own (the slabs it
-// stages before its first step): the number of pieces with the shortest whole waves of units.  On the
-// 128k-atom image (435 tiles, 160 slices) 32 slices in 2.9 waves instead of 20 in 4.6.
-int depth_chunk(int64_t tiles, int deepest, int per_sm, int fixed) {
+// stages before its first step): the number of pieces with the shortest waves of units.  The FP32
+// field's units, a CTA each, end together, so that whole waves count: on the 128k-atom image (435
+// tiles, 160 slices) 32 slices in 2.9 waves instead of 20 in 4.6.  The FP64 field's, a warp each, differ,
+// and up to two waves of them wait for the longest, more even out: the same image with density (1653
+// patches) 4766 us with 160 slices in 0.9 waves, 4512 with 40 in 3.6, 4352 with 20 in 7.2, 4530 with 8.
+int depth_chunk(int64_t tiles, int deepest, int per_sm, int fixed, bool in_step) {
   const int64_t full = (int64_t)sm_count() * per_sm;
   int best = (deepest + 3) & ~3;
-  int64_t best_cost = -1;
+  double best_cost = -1;
   for (int pieces = 1; pieces <= (deepest + 3) / 4 && pieces <= 64; ++pieces) {
     const int chunk = ((deepest + pieces - 1) / pieces + 3) & ~3;
     const int64_t units = tiles * ((deepest + chunk - 1) / chunk);
-    const int64_t cost = (units + full - 1) / full * (chunk + fixed);
+    const double w = (double)units / (double)full;
+    const double waves = in_step ? std::ceil(w) : w <= 2.0 ? 1.08 * std::ceil(w) : w + 0.5;
+    const double cost = waves * (chunk + fixed);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best = chunk;
@@ -725,8 +730,8 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     const int lo = grp ? n_four : 0, hi = grp ? n_ring : n_four;
     std::vector<FieldRange> part;
     field_ranges(cj.data() + lo, hi - lo, (int)total_patches[grp], n_room, align,
-                 fp32 ? depth_chunk(total_patches[grp] / 4, deepest[grp], kField32Blocks, 8)
-                      : depth_chunk(total_patches[grp], deepest[grp], 4 * kField64Blocks, 1),
+                 fp32 ? depth_chunk(total_patches[grp] / 4, deepest[grp], kField32Blocks, 8, true)
+                      : depth_chunk(total_patches[grp], deepest[grp], 4 * kField64Blocks, 1, false),
                  deepest[grp], part);
     for (FieldRange& R : part) {
       R.job_lo = lo;
