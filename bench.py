@@ -142,9 +142,9 @@ def path_roofline(peaks, n_acc, n_kept, n_atoms, voxels, voxel_prec, pixels, den
 
 
 SWEEP_G = ((1, 1, 0), (2, 0, 0), (2, 1, 1))
-# DRAM bytes (read + write) of one k_column_fp32_v3 launch on the 1.2M-atom image, from an
-# ncu capture of `python bench.py --ncu-case fp32` (51.59 MB read + 2.36 MB written)
-COLUMN_TRAFFIC_BYTES = 5.395e7
+# DRAM bytes (read + write) of the column stage on the 1.2M-atom image, from an ncu capture: k_field32
+# (53.5 MB read + 563.1 MB written: the field samples) and k_integrate32 (622.1 + 4.6 MB)
+COLUMN_TRAFFIC_BYTES = 1.2433e9
 
 
 def sweep_specs(cell, n_tomo=41, n_prec=16, gs=SWEEP_G):
@@ -270,7 +270,7 @@ def batched_legs(ctx, cell, stream, flush, steps, warmup, peaks=None, cpu=True):
         pix = sum((G.ix1 - G.ix0) * (G.iy1 - G.iy0) for G in specs_g[0])
         r = path_roofline(peaks, st.n_accepted, st.n_kept, n_atoms, vox, vp, pix, False, t_col)
         if r:
-            r["kernel"] = "k_column_fp32_v3 (every column launch of the batch)"
+            r["kernel"] = "k_field32 and k_integrate32 (every column launch of the batch)"
             r["frac_batch"] = r["t_roof_ms"] / t_batch
             r["executed"] = {"tests": st.n_tests, "tests_per_voxel": st.n_tests / max(vox, 1)}
         return r
@@ -930,23 +930,23 @@ def run_gpu(args):
     roof = path_roofline(peaks, n_acc, n_kept, len(x), V, V * n_prec, pix, False, col_avg)
     if roof:
         c_tests = reference_candidate_tests(ctx, G, x)
-        roof.update({"kernel": "k_column_fp32_v3",
+        roof.update({"kernel": "k_field32 + k_integrate32",
                      "peak_source": "measured live in this run by the project's pipe microbenchmarks "
                                     "(libstem_peaks.so: FP32 FMA, FP64 FMA, MUFU ex2 and sin); HBM from "
                                     + hbm_peak()[1],
-                     "traffic": COLUMN_TRAFFIC_BYTES, "traffic_unit": "bytes per launch",
-                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_column_fp32_v3 on "
-                                       "this image (profiles/k_column_fp32_v3_1p2m_screw.md)",
+                     "traffic": COLUMN_TRAFFIC_BYTES, "traffic_unit": "bytes per image",
+                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the two kernels on "
+                                       "this image (profiles/kernels_of_the_workloads.md)",
                      "frac_step": roof["t_roof_ms"] / ms,
                      "executed": {"tests": n_tst, "tests_per_voxel": n_tst / V,
                                   "reference_tests_per_voxel": c_tests / V,
                                   "accepted_per_voxel": n_acc / V,
-                                  "ex2_issued": n_tst / 2, "ex2_frac_of_peak":
-                                      n_tst / 2 / (col_avg * 1e-3) / (peaks["mufu_ex2_gops"] * 1e9),
+                                  "ex2_issued": n_tst / 4, "ex2_frac_of_peak":
+                                      n_tst / 4 / (col_avg * 1e-3) / (peaks["mufu_ex2_gops"] * 1e9),
                                   "note": "work the kernel executes: tests counts each buffered atom once per "
                                           "column and slice; the in-plane weight is one ex2 per atom and column "
-                                          "for both slices of a step (ex2_issued), the depth factor one per atom "
-                                          "and slice for the whole warp; the reference's own 27-cell search "
+                                          "for the four slices of a step (ex2_issued), the depth factor one per atom "
+                                          "and slice for the whole block; the reference's own 27-cell search "
                                           "tests reference_tests_per_voxel candidates per voxel"}})
     acc = {"max_abs_dI_fp32_vs_fp64": float(np.abs(d).max()), "rms_dI_fp32_vs_fp64": float(np.sqrt((d ** 2).mean()))}
     line = {"metric": METRIC, "value": value, "unit": "images/s", "n_gpus": ws, "steps": args.steps,

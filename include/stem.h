@@ -113,16 +113,16 @@ int st_image(st_ctx* ctx, const st_geom* geom, const double* x, int64_t ldx, int
 int st_image_device(st_ctx* ctx, const st_geom* geom, const double* d_x, int64_t ldx, int64_t nAtoms,
                     const double* aa, int32_t nPrec, int32_t flags, double* d_img, void* stream);
 
-/* Launch tuning of the slab-ring FP32 kernel.  Its variants differ in the warp
- * tile's shape (8 x 4, 4 x 8 or 16 x 2 pixel columns), the slab capacity of
+/* Launch tuning of the slab-ring FP32 kernel.  Its variants differ in the warp's
+ * patch (8 x 4, 4 x 8 or 16 x 2 pixel columns), the slab capacity of
  * the first staging tier (128 or 96 atoms) and with it the CTAs per SM; the
- * images of variants of one tile shape are identical, those of different
+ * images of variants of one patch shape are identical, those of different
  * shapes agree to FP32 rounding (their atoms are summed in different orders).
- * ST_TUNE_AUTO (the default): the first pass of each kind (angles per pass,
- * density) on images of each shape (image and link-cell dimensions) in a
- * context, with at least 4,096 warp tiles, times every variant on the real
- * work, keeps the fastest for the context's later calls on that kind and
- * shape, and leaves that variant's own images.  ST_TUNE_OFF: variant 0 always.
+ * ST_TUNE_AUTO (the default): the first pass of each kind (several angles or
+ * one, density) on images of each shape (image and link-cell dimensions) in a
+ * context, with at least 4,096 patches, times the 8 x 4 variants on the real
+ * work and keeps the faster for the context's later calls on that kind and
+ * shape: the images do not depend on the timing.  ST_TUNE_OFF: variant 0 always.
  * mode >= 0: that variant always.  No counterpart in the reference. */
 #define ST_TUNE_AUTO (-1)
 #define ST_TUNE_OFF (-2)

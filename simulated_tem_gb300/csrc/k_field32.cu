@@ -8,27 +8,33 @@
 // column's depth over CTAs where an image has few columns, and runs once however many precession
 // angles integrate over it.
 //
-// The field kernel: a CTA of four warps owns 16 x 8 pixel columns and a range of slices, each
-// warp 32 of the columns (8 x 4, 4 x 8 or 16 x 2: the tuning variants), one lane per column, four
-// slices per step (two where some image's steps of four do not fit the ring).  What bounds it is
-// instruction issue, then the FP32 pipe; so everything that does not depend on the column is done
-// once for the four warps:
+// The field kernel: a CTA of four warps owns 16 x 8 pixel columns and a range of slices, each warp 32
+// of the columns (8 x 4, 4 x 8 or 16 x 2: the tuning variants), four slices per step (two where some
+// image's steps of four do not fit the ring).  Instruction issue bounds it (0.65 to 0.7 per cycle and
+// sub-partition), then the shared-memory loads of the atoms and the FP32 pipe; so everything that does
+// not depend on the column is done once for the four warps, and an atom's values are loaded for two columns:
 // * The atoms of a link-cell slab (one z cell; a ring of four) within 3 sigma of the tile are
 //   gathered into shared memory once per slab (a tile of one warp would gather 2.3 times as
 //   many per column).
-// * Per step and slab, one thread per atom computes what depends on the atom and the depth
-//   alone: the largest in-plane r^2 each slice still accepts (hmax_k = (3 sigma)^2 - dz_k^2, or kOff
-//   where the reference's 27-cell rule excludes the slab for that slice) and the Gaussian's depth
-//   factor times the phasor, ex2(-dz_k^2) (cos, sin).  Two buffers, so that one slab's values are
-//   made while the previous slab's are consumed.
+// * Per step, one thread per atom computes what depends on the atom and the depth alone, for the
+//   atoms of the step's depth window (counted first, so that they lie densely): the largest in-plane r^2
+//   each slice still accepts (hmax_k = (3 sigma)^2 - dz_k^2, or kOff where the reference's 27-cell
+//   rule excludes the slab for that slice) and the Gaussian's depth factor times the phasor,
+//   ex2(-dz_k^2) (cos, sin).
 // * Each warp lists the atoms that some column of its patch accepts at some slice (distance to
 //   the patch's sample rectangle against the largest hmax), ballot + popc, order kept.
-// * The lanes then take the listed atoms in pairs: the in-plane distance (four FP32x2
-//   operations for the pair), one ex2 per atom for all four slices (the Gaussian is separable),
-//   and per slice the inclusive cutoff dxy^2 <= hmax_k and one FP32x2 multiply-add of the weight into
-//   (cos, sin).
-// Sums run in slab order, then in the gather's order, whatever the patch shape, the depth range or
-// the slab capacity: all of them give the same image to the last bit.
+// * A lane then takes two columns, and the two groups of 16 lanes take different listed atoms: the
+//   in-plane distances (FP32x2), one ex2 per atom and column for all four slices (the Gaussian is
+//   separable), and per slice the inclusive cutoff dxy^2 <= hmax_k and one FP32x2 multiply-add of the
+//   weight into (cos, sin); the groups' sums are added at the end of the step.
+// Measured on the 1.2M-atom image (566 x 566 x 240): 2.84 ms for the kernel before (a warp's own
+// slabs, two slices per step, the integrator in the same kernel), 2.09 ms field + 0.16 ms integrator
+// now; of the field 0.87 ms are the lists' sums (0.65 at the FP32 pipe's rate), 0.30 the depth terms, 0.29
+// the gather, 0.26 the step's fixed cost, 0.16 the lists, 0.13 the exact recheck.  One column per lane
+// ran 2.55 ms (the loads), four columns 2.22, six CTAs per SM instead of five 2.33, a producer warp per CTA
+// 2.55, slabs per warp 2.35.
+// Images of one patch shape are the same to the last bit whatever the slab capacity; the shapes
+// distribute a list over the groups of lanes differently, so between shapes they agree to FP32 rounding.
 // Lengths are scaled by s = sqrt(log2 e / 2 sigma^2), so a weight is ex2(-r'^2).
 //
 // Precision: FP32 throughout; the weight is the product of two ex2 values (a few ulp).  The FP32
@@ -65,7 +71,7 @@ struct Smem {
   float2 cs[kRing * CAP]; // (cos, sin) of the phase
   // the atoms of the step's depth window; entry WCAP accepts nothing (pads a list)
   float4 r[WCAP + 1];     // X', Y', the largest hmax with the margin of the patch test, kept atom
-  float4 h[WCAP + 1];     // hmax per slice
+  typename std::conditional<SL == 4, float4, float2>::type h[WCAP + 1];  // hmax per slice
   float4 e0[WCAP + 1];    // ex2(-dz^2) (cos, sin) of slices 0 and 1
   float4 e1[SL == 4 ? WCAP + 1 : 1];  // of slices 2 and 3
   int4 seg[kSegs];        // the footprint's cell runs: first cell in the plane, cells, x shift, row
@@ -235,8 +241,14 @@ __device__ __noinline__ Fix<W_::SL> exact_fix(const ColumnParams& p, const W_& W
     const float4 e = W.r[W.li[warp][i] >> 4];
     const float dx = __fadd_rn(e.x, -C.X), dy = __fadd_rn(e.y, -C.Y);
     const float h = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
-    const float4 hm4 = W.h[W.li[warp][i] >> 4];
-    const float hm[4] = {hm4.x, hm4.y, hm4.z, hm4.w};
+    float hm[SL];
+    const auto hv = W.h[W.li[warp][i] >> 4];
+    hm[0] = hv.x;
+    hm[1] = hv.y;
+    if constexpr (SL == 4) {
+      hm[2] = hv.z;
+      hm[3] = hv.w;
+    }
 #pragma unroll
     for (int k = 0; k < SL; ++k) {
       if (!(want >> k & 1) || fabsf(h - hm[k]) > kGuard) continue;
@@ -487,7 +499,8 @@ __device__ __forceinline__ bool field_tile(const ColumnParams& p, W_& W, int pat
         }
         // margin: the lanes' own rounding of dxy^2 must not reach below the rectangle's
         W.r[d] = make_float4(q4.x, q4.y, fmaf(hmax, 1.0001f, 1e-4f), q4.w);
-        W.h[d] = make_float4(hm[0], hm[1], hm[2], hm[3]);
+        if constexpr (SL == 4) W.h[d] = make_float4(hm[0], hm[1], hm[2], hm[3]);
+        else W.h[d] = make_float2(hm[0], hm[1]);
         W.e0[d] = make_float4(w[0] * cs.x, w[0] * cs.y, w[1] * cs.x, w[1] * cs.y);
         if constexpr (SL == 4) W.e1[d] = make_float4(w[2] * cs.x, w[2] * cs.y, w[3] * cs.x, w[3] * cs.y);
       }
@@ -534,7 +547,14 @@ __device__ __forceinline__ bool field_tile(const ColumnParams& p, W_& W, int pat
     for (int i = 0; i < n; i += CPL) {
       const unsigned o = L[i + grp];
       const float2 q = *reinterpret_cast<const float2*>(RB + o);
-      const float4 hm = *reinterpret_cast<const float4*>(HB + o);
+      float4 hm = make_float4(kOff, kOff, kOff, kOff);
+      if constexpr (SL == 4) {
+        hm = *reinterpret_cast<const float4*>(HB + o);
+      } else {
+        const float2 h2 = *reinterpret_cast<const float2*>(HB + (o >> 1));
+        hm.x = h2.x;
+        hm.y = h2.y;
+      }
       const float4 ea = *reinterpret_cast<const float4*>(E0 + o);
       float4 eb = make_float4(0.f, 0.f, 0.f, 0.f);
       if constexpr (SL == 4) eb = *reinterpret_cast<const float4*>(E1 + o);
@@ -657,7 +677,8 @@ __global__ void __launch_bounds__(W_::NW * 32, kMinBlocks)
   if ((int64_t)R.counters[0] > R.cap) return;  // the binning overflowed: the host retries
   if (threadIdx.x == 0) {
     W.r[W_::WCAP] = make_float4(0.f, 0.f, kOff, 0.f);
-    W.h[W_::WCAP] = make_float4(kOff, kOff, kOff, kOff);
+    if constexpr (W_::SL == 4) W.h[W_::WCAP] = make_float4(kOff, kOff, kOff, kOff);
+    else W.h[W_::WCAP] = make_float2(kOff, kOff);
     W.e0[W_::WCAP] = make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (W_::SL == 4) W.e1[W_::WCAP] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -915,8 +936,10 @@ cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, int m
 template <int SL, bool kDens, bool kStats, bool kMasked>
 cudaError_t dispatch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, int max_np, int variant, int tier,
                      cudaStream_t st) {
+  // denser slabs, or coarser voxels: a step of two slices needs less window, so that four CTAs fit; the
+  // last tier has one warp per tile, a quarter of the atoms
   if (tier >= 2) return launch<256, 512, 1, SL, 8, kDens, kStats, kMasked, 4>(jobs, n_jobs, R, max_np, st);
-  if (tier == 1) return launch<352, 704, 4, SL, 8, kDens, kStats, kMasked, 2>(jobs, n_jobs, R, max_np, st);
+  if (tier == 1) return launch<SL == 2 ? 320 : 352, SL == 2 ? 512 : 704, 4, SL, 8, kDens, kStats, kMasked, SL == 2 ? 4 : 2>(jobs, n_jobs, R, max_np, st);
   if constexpr (SL == 4 && !kStats) {
     switch (variant) {
       case 1: return launch<160, 288, 4, SL, 8, kDens, kStats, kMasked, kField32Blocks>(jobs, n_jobs, R, max_np, st);

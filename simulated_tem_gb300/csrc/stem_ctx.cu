@@ -195,6 +195,11 @@ void depth_table(const st_geom* g, int2* tab, const double* fv) {
   }
 }
 
+// Voxels so coarse in depth (more than 0.7 sigma a slice) that a step of four slices, whose lists hold
+// the atoms of any of them, costs the FP32 field more than two steps of two (and twice
+// the shared memory for its window): 4.8M atoms at one sigma a slice 4.75 ms with four, 3.92 with two.
+bool coarse_slices(const ColumnParams& p) { return p.dz > 0.7 * p.sigma; }
+
 bool four_slices_fit(const st_geom* g) {
   std::vector<int2> tab((size_t)g->Mz);
   std::vector<double> fv((size_t)g->Mz);
@@ -606,9 +611,8 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   if (cap > total_cand + 1) cap = total_cand + 1;
   if (!alloc_kept(c, (size_t)cap)) return cuda_fail(c, cudaErrorMemoryAllocation, "allocating binning buffers");
 
-  // ---- column parameters. On the FP32 path every image whose link cells allow it goes
-  // to the persistent slab-ring kernel (passes of 16 precession angles); the others,
-  // and every image of the FP64 path, get per-image launches.
+  // ---- column parameters.  Every image whose link cells allow it goes to the field kernel of its path
+  // (one launch for all of them) and the integrator (all angles); the others get per-image launches.
   std::vector<ColumnParams> cps(n);
   std::vector<int> ring_jobs;  // images of the persistent launch
   std::vector<char> on_ring(n, 0);
@@ -639,7 +643,10 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   // images whose steps of four slices fit the slab ring first: the others march two per step, in
   // launches of their own, so that an image's result does not depend on the rest of its batch
   const int n_four = (int)(std::stable_partition(ring_jobs.begin(), ring_jobs.end(),
-                                                 [&](int i) { return four_slices_fit(jobs[i].g); }) -
+                                                 [&](int i) {
+                                                   return four_slices_fit(jobs[i].g) &&
+                                                          !(fp32 && coarse_slices(cps[i]));
+                                                 }) -
                            ring_jobs.begin());
   const bool ring = !ring_jobs.empty();
   const int n_ring = (int)ring_jobs.size();
@@ -716,6 +723,9 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   if (!c->ev_stage) cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming);
   if (c->ev_stage) cudaEventRecord(c->ev_stage, st);
 
+  bool masked = false;  // tile-masked ring jobs take the masked kernel instances
+  for (int r : ring_jobs) masked = masked || cps[r].tile_mask != nullptr;
+
   // ---- ranges of patches whose field samples share one workspace
   std::vector<FieldRange> ranges;
   for (int grp = 0; grp < 2; ++grp) {
@@ -729,9 +739,13 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     const int64_t n_room = (int64_t)(room / per) & ~(int64_t)31;
     const int lo = grp ? n_four : 0, hi = grp ? n_ring : n_four;
     std::vector<FieldRange> part;
+    // of a tile-masked image few patches are wanted (a sixteenth, say): their columns are split further
+    // (4.8M atoms, 2263 x 2263 pixels, 7 % of the tiles: 5.9 ms, 9.2 with whole columns)
+    int64_t at_once = std::min(total_patches[grp], n_room / (32 * (int64_t)deepest[grp])) / align;
+    at_once = std::max<int64_t>(1, masked ? at_once / 16 : at_once);
     field_ranges(cj.data() + lo, hi - lo, (int)total_patches[grp], n_room, align,
-                 fp32 ? depth_chunk(total_patches[grp] / 4, deepest[grp], kField32Blocks, 8, true)
-                      : depth_chunk(total_patches[grp], deepest[grp], 4 * kField64Blocks, 1, false),
+                 fp32 ? depth_chunk(at_once, deepest[grp], kField32Blocks, 8, true)
+                      : depth_chunk(at_once, deepest[grp], 4 * kField64Blocks, 1, false),
                  deepest[grp], part);
     for (FieldRange& R : part) {
       R.job_lo = lo;
@@ -803,8 +817,6 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   }
   int big = c->min_slab_tier;  // slab tier: 128, 192, 256 atoms
   if (auto it = c->ring_big.find(key); it != c->ring_big.end()) big = std::max(big, it->second);
-  bool masked = false;  // tile-masked ring jobs take the masked kernel instances
-  for (int r : ring_jobs) masked = masked || cps[r].tile_mask != nullptr;
   // with_bin false: the column phase only, on the binning already in place
   auto enqueue = [&](bool capturing, bool with_bin) -> cudaError_t {
     cudaError_t ce = cudaSuccess;

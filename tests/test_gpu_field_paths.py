@@ -79,6 +79,22 @@ def test_windows_equal_the_general_kernels(ctx, general, fp32, density):
         assert np.abs(got - want).max() <= (FP32_TOL if fp32 else FP64_TOL)
 
 
+@pytest.mark.parametrize("lattice,M", [("bcc", 2), ("bcc", 3), ("fcc", 2), ("fcc", 4), ("sc", 5)])
+def test_coarse_voxels_and_dense_slabs(ctx, general, lattice, M):
+    """Slices of up to a sigma (two per step in FP32) and every slab capacity, against the general kernels."""
+    base = {"bcc": [[0, 0, 0], [0.5, 0.5, 0.5]], "sc": [[0, 0, 0]],
+            "fcc": [[0, 0, 0], [0.5, 0.5, 0], [0.5, 0, 0.5], [0, 0.5, 0.5]]}[lattice]
+    n, a0 = np.array([10, 9, 8]), 3.6
+    sites = np.stack(np.meshgrid(*[np.arange(k) for k in n], indexing="ij"), -1).reshape(-1, 1, 3)
+    pos = (sites + np.array(base)).reshape(-1, 3) * a0
+    pos = pos + np.random.default_rng(M).normal(0.0, 0.05, pos.shape)
+    t, x, _ = imaging.d2bi_condition(np.diag(n * a0), a0, (0, 0, 1), (1, 1, 0) if lattice == "bcc" else (2, 0, 0), pos,
+                                     sg=0.01, lattice=lattice, M=(M, M))
+    G, aa = t.image_geometry(len(x))
+    for flags, tol in ((_lib.ST_FLAG_FP32, FP32_TOL), (0, FP64_TOL)):
+        assert np.abs(ctx.image(G, x, aa, flags=flags) - general.image(G, x, aa, flags=flags)).max() <= tol
+
+
 @pytest.mark.parametrize("count", [1, 4, 24])
 def test_batches_about_the_cell_scans_limit(ctx, count):
     """One block scans up to 16,384 cells; batches on both sides equal the single images."""
