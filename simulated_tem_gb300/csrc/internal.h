@@ -217,8 +217,8 @@ inline int sm_count() {
 }
 // The FP32 path's field and integration of one range (k_field32.cu).  `variant` 0 ..
 // ring_variant_count() - 1 selects the patch shape and the slab capacity of tier 0 (named per 8 x 4
-// patch: "slab96" stages 160 atoms per 16 x 8 tile, "slab128" 192); `slab_tier` 1: 352 atoms per tile,
-// 2: 256 atoms per patch, the tiles split into their patches.  Variants of
+// patch: "slab96" stages 160 atoms per 16 x 8 tile, "slab128" 192); `slab_tier` 1: 352 atoms per tile (320
+// with two slices per step), 2: 256 atoms per patch, the tiles split into their patches.  Variants of
 // one patch shape give the same image to the last bit; the shapes agree to FP32 rounding.  `four` as
 // below; `masked`: some jobs carry a tile mask (then stats must be false).
 constexpr int kField32Blocks = 5;  // CTAs of four warps per SM at tier 0

@@ -15,7 +15,7 @@
 // writes them transposed, so that the second pass reads lines again.  The 8-byte stores of 32 lines
 // meet in the L2 cache, which holds the intermediate image at the sizes d2bi produces.
 // 1132 x 1131 pixels at t = 6.97 (71 taps): 1095 us with the sums of the weights and the products on
-// the FP64 unit, 427 us now (whole call; the additions alone need 370).  300 x 200 at t = 3.3: 76 and
+// the FP64 unit, 419 us now (whole call; the additions alone need 370).  300 x 200 at t = 3.3: 76 and
 // 58 us, 70 x 61 at t = 6.9: 70 and 62 us, most of them the copy of the weights and the launches.
 #include <cuda_runtime.h>
 

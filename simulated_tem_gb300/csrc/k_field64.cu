@@ -35,8 +35,8 @@
 // sub-partition), and code size: with two copies of the consuming code, or two atoms per iteration, the
 // instruction fetches cost 128k atoms with density a fifth.
 // Measured (GB300, whole calls): 128k atoms with density 29.0 ms with one exp, the divisions of the
-// reference's integrator and hypot in every lane, 7.2 with all of this in FP64, 4.83 now; 28k atoms
-// 6.75, 0.83, 0.53; 16k atoms with six precession angles 13.6, 1.32, 0.71.  128k atoms: field 4.33 ms
+// reference's integrator and hypot in every lane, 7.2 with all of this in FP64, 4.35 now; 28k atoms
+// 6.75, 0.83, 0.54; 16k atoms with six precession angles 13.6, 1.32, 0.71.  128k atoms: field 3.95 ms
 // (a third of it the sums, a fifth the tests and the density's nearest atoms, a fifth the Gaussians),
 // integrator 0.20.
 //
