@@ -327,10 +327,11 @@ __device__ __forceinline__ bool field_tile(const ColumnParams& p, W_& W, int pat
     if (!__syncthreads_or(work)) return true;
   }
 
-  // the frame is the 16 x 8 tile's for any NW, so that the staged values do not depend on it
+  // the frame is the 16 x 8 tile's for any NW, so that the staged values do not depend on it, from
+  // the cell of its middle: coordinates half as large round half as coarsely
   Geo G;
-  G.ux_ref = p.xtab[x0].x;
-  G.uy_ref = p.ytab[y0].x;
+  G.ux_ref = p.xtab[min(x0 + kTileX / 2, p.ix1 - 1)].x;
+  G.uy_ref = p.ytab[min(y0 + kTileY / 2, p.iy1 - 1)].x;
   G.scale = p.scale;
   G.a11s = p.a11s;
   G.a22s = p.a22s;
