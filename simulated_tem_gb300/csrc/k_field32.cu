@@ -28,7 +28,7 @@
 //   separable), and per slice the inclusive cutoff dxy^2 <= hmax_k and one FP32x2 multiply-add of the
 //   weight into (cos, sin); the groups' sums are added at the end of the step.
 // Measured on the 1.2M-atom image (566 x 566 x 240): 2.84 ms for the kernel before (a warp's own
-// slabs, two slices per step, the integrator in the same kernel), 2.09 ms field + 0.16 ms integrator
+// slabs, two slices per step, the integrator in the same kernel), 2.12 ms field + 0.16 ms integrator
 // now; of the field 0.87 ms are the lists' sums (0.65 at the FP32 pipe's rate), 0.30 the depth terms, 0.29
 // the gather, 0.26 the step's fixed cost, 0.16 the lists, 0.13 the exact recheck.  One column per lane
 // ran 2.55 ms (the loads), four columns 2.22, six CTAs per SM instead of five 2.33, a producer warp per CTA
