@@ -1,0 +1,111 @@
+// The host's plan of a call's field: ranges of patches whose samples share one workspace.  Plain C++:
+// the allocations and the split in depth are the caller's.
+#pragma once
+
+#include <stddef.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <vector>
+
+#ifdef __CUDACC__
+#define FP_HD __host__ __device__
+#else
+#define FP_HD
+#endif
+
+namespace stem {
+
+// The voxel field of a range of patches (warp tiles of 32 columns) of a batch, in a workspace of
+// samples: patch by patch in job order, slice by slice, 32 lanes.  The work is handed out in units
+// of one patch and `chunk` slices, so that few patches still fill the GPU.
+struct FieldRange {
+  void* samples = nullptr;  // the field x of a voxel (times rho with density): float2 or double2
+  float* rho32 = nullptr;   // with density: rho
+  double* rho64 = nullptr;
+  int64_t origin = 0;       // index of the workspace's first sample in the batch's sample sequence
+  int patch_lo = 0, patch_hi = 0;
+  int n_chunks = 1;         // per patch: ceil(deepest image / chunk)
+  int chunk = 0;            // slices per unit, a multiple of 4
+  int job_lo = 0, n_jobs = 0;  // the range's jobs in the call's job table
+  bool four = true;         // four slices per step (else two)
+  int64_t rho_at = 0;       // where rho starts in the workspace, in values
+  unsigned* work = nullptr;  // units handed out: zero before the field kernel, zeroed again by the integrator
+  const unsigned long long* counters = nullptr;
+  int64_t cap = 0;
+  FP_HD int units() const { return (patch_hi - patch_lo) * n_chunks; }
+};
+
+// Splits the patches of a batch into ranges of at most `samples` samples, cut at multiples of
+// `align` patches of an image.
+template <typename Job>
+void field_ranges(const Job* jobs, int n_jobs, int patches, int64_t samples, int align, int chunk, int deepest,
+                  std::vector<FieldRange>& out) {
+  out.clear();
+  int job = 0;
+  for (int lo = 0; lo < patches;) {
+    FieldRange R;
+    R.patch_lo = lo;
+    R.chunk = chunk;
+    R.n_chunks = (deepest + chunk - 1) / chunk;
+    auto end_of = [&](int j) { return j + 1 < n_jobs ? jobs[j + 1].patch_base : patches; };
+    while (end_of(job) <= lo) ++job;
+    R.origin = jobs[job].sample_base + (int64_t)(lo - jobs[job].patch_base) * jobs[job].p.Mz * 32;
+    int64_t left = samples;
+    int hi = lo;
+    for (int j = job; j < n_jobs; ++j) {
+      const int64_t per = (int64_t)jobs[j].p.Mz * 32;
+      const int begin = std::max(lo, jobs[j].patch_base), n = end_of(j) - begin;
+      const int64_t fit = std::min<int64_t>(n, left / per / align * align);
+      hi = begin + (int)fit;
+      left -= fit * per;
+      if (fit < n) break;
+    }
+    R.patch_hi = std::max(hi, lo + align);  // the workspace holds at least `align` of the deepest
+    lo = R.patch_hi;
+    out.push_back(R);
+  }
+}
+
+// The images of one group: those that march four slices per step, or two.
+struct FieldGroup {
+  int job_lo = 0, n_jobs = 0;
+  int64_t patches = 0, samples = 0;
+  int deepest = 1;
+};
+
+// The ranges of both groups.  `room(want, least)` gives the workspace's bytes, at least `least` and at most
+// about `want`, or 0; it is asked once, for both groups, since a second answer may be a smaller buffer
+// than the first one's ranges were laid out in.  `chunk(at_once, deepest)`: slices per unit when
+// `at_once` groups of `align` patches are in the workspace together.  False when there is no room.
+template <typename Job, typename Room, typename Chunk>
+bool plan_ranges(const Job* jobs, const FieldGroup (&groups)[2], int align, size_t bytes_per_sample, Room room,
+                 Chunk chunk, std::vector<FieldRange>& out) {
+  out.clear();
+  const size_t want = (size_t)std::max(groups[0].samples, groups[1].samples) * bytes_per_sample;
+  size_t least = 0;
+  for (const FieldGroup& g : groups)
+    if (g.samples) least = std::max(least, (size_t)g.deepest * 32 * align * bytes_per_sample);
+  if (least == 0) return true;
+  const size_t got = room(want, least);
+  if (got < least) return false;
+  const int64_t n_room = (int64_t)(got / bytes_per_sample) & ~(int64_t)31;
+  std::vector<FieldRange> part;
+  for (int i = 0; i < 2; ++i) {
+    const FieldGroup& g = groups[i];
+    if (g.samples == 0) continue;
+    const int64_t at_once = std::min(g.patches, n_room / (32 * (int64_t)g.deepest)) / align;
+    field_ranges(jobs + g.job_lo, g.n_jobs, (int)g.patches, n_room, align,
+                 chunk(std::max<int64_t>(1, at_once), g.deepest), g.deepest, part);
+    for (FieldRange& R : part) {
+      R.job_lo = g.job_lo;
+      R.n_jobs = g.n_jobs;
+      R.four = i == 0;
+      R.rho_at = 2 * n_room;
+      out.push_back(R);
+    }
+  }
+  return true;
+}
+
+}  // namespace stem

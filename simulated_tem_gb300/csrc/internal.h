@@ -7,6 +7,7 @@
 #include <string>
 
 #include "../../include/stem.h"
+#include "field_plan.h"
 
 namespace stem {
 
@@ -176,25 +177,6 @@ struct ColumnJob {
 int field32_patches(const ColumnParams& p);  // 16 x 8 tiles of four patches
 int field64_patches(const ColumnParams& p);  // 8 x 4 patches
 cudaError_t launch_column_fp64(const ColumnParams& p, cudaStream_t st);
-// The voxel field of a range of patches (warp tiles of 32 columns) of a batch, in a workspace of
-// samples: patch by patch in job order, slice by slice, 32 lanes.  The work is handed out in units
-// of one patch and `chunk` slices, so that few patches still fill the GPU.
-struct FieldRange {
-  void* samples = nullptr;  // the field x of a voxel (times rho with density): float2 or double2
-  float* rho32 = nullptr;   // with density: rho
-  double* rho64 = nullptr;
-  int64_t origin = 0;       // index of the workspace's first sample in the batch's sample sequence
-  int patch_lo = 0, patch_hi = 0;
-  int n_chunks = 1;         // per patch: ceil(deepest image / chunk)
-  int chunk = 0;            // slices per unit, a multiple of 4
-  int job_lo = 0, n_jobs = 0;  // the range's jobs in the call's job table
-  bool four = true;         // four slices per step (else two)
-  int64_t rho_at = 0;       // where rho starts in the workspace, in values
-  unsigned* work = nullptr;  // units handed out: zero before the field kernel, zeroed again by the integrator
-  const unsigned long long* counters = nullptr;
-  int64_t cap = 0;
-  __host__ __device__ int units() const { return (patch_hi - patch_lo) * n_chunks; }
-};
 // The job of patch `g` of the batch's patch sequence and its number in the job.
 __device__ __forceinline__ const ColumnJob& field_patch(const ColumnJob* __restrict__ jobs, int n_jobs, int g,
                                                         int& patch) {

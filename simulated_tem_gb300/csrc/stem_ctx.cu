@@ -507,36 +507,6 @@ int depth_chunk(int64_t tiles, int deepest, int per_sm, int fixed, bool in_step)
   return best;
 }
 
-// Splits the patches of a batch into ranges of at most `samples` samples, cut at multiples of
-// `align` patches of an image.
-void field_ranges(const ColumnJob* jobs, int n_jobs, int patches, int64_t samples, int align, int chunk,
-                  int deepest, std::vector<FieldRange>& out) {
-  out.clear();
-  int job = 0;
-  for (int lo = 0; lo < patches;) {
-    FieldRange R;
-    R.patch_lo = lo;
-    R.chunk = chunk;
-    R.n_chunks = (deepest + chunk - 1) / chunk;
-    auto end_of = [&](int j) { return j + 1 < n_jobs ? jobs[j + 1].patch_base : patches; };
-    while (end_of(job) <= lo) ++job;
-    R.origin = jobs[job].sample_base + (int64_t)(lo - jobs[job].patch_base) * jobs[job].p.Mz * 32;
-    int64_t left = samples;
-    int hi = lo;
-    for (int j = job; j < n_jobs; ++j) {
-      const int64_t per = (int64_t)jobs[j].p.Mz * 32;
-      const int begin = std::max(lo, jobs[j].patch_base), n = end_of(j) - begin;
-      const int64_t fit = std::min<int64_t>(n, left / per / align * align);
-      hi = begin + (int)fit;
-      left -= fit * per;
-      if (fit < n) break;
-    }
-    R.patch_hi = std::max(hi, lo + align);  // the workspace holds at least `align` of the deepest
-    lo = R.patch_hi;
-    out.push_back(R);
-  }
-}
-
 // A recorded call (st_plan): the instantiated graph and what its kernels were recorded with.
 struct GraphOut {
   cudaGraphExec_t exec = nullptr;
@@ -654,8 +624,9 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   // takes all angles of an image at once
   std::vector<ColumnJob> cj;
   int64_t tune_tiles = 0;  // 8 x 4 tiles
-  int64_t total_samples[2] = {0, 0}, total_patches[2] = {0, 0};  // four, two slices per step
-  int deepest[2] = {1, 1};
+  FieldGroup groups[2];    // four, two slices per step
+  groups[0].n_jobs = groups[1].job_lo = n_four;
+  groups[1].n_jobs = n_ring - n_four;
   if (ring) {
     // the density variant of the kernel serves every image of the launch when any image uses it;
     // an image without the density field then gets rho = 1 from use_density = 0 in the sample
@@ -669,14 +640,14 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
       J.p.fin_scale = (double)J.p.n_prec;
       J.p.fin_bright = (flags & ST_FLAG_BRIGHT) ? 1 : 0;
       J.pad = 0;
-      const int grp = r < n_four ? 0 : 1;
-      J.patch_base = (int)total_patches[grp];
-      J.sample_base = total_samples[grp];
+      FieldGroup& grp = groups[r < n_four ? 0 : 1];
+      J.patch_base = (int)grp.patches;
+      J.sample_base = grp.samples;
       const int np = fp32 ? field32_patches(J.p) : field64_patches(J.p);
-      total_patches[grp] += np;
+      grp.patches += np;
       tune_tiles += field64_patches(J.p);
-      total_samples[grp] += (int64_t)np * J.p.Mz * 32;
-      deepest[grp] = std::max(deepest[grp], J.p.Mz);
+      grp.samples += (int64_t)np * J.p.Mz * 32;
+      grp.deepest = std::max(grp.deepest, J.p.Mz);
     }
   }
 
@@ -728,32 +699,24 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
 
   // ---- ranges of patches whose field samples share one workspace
   std::vector<FieldRange> ranges;
-  for (int grp = 0; grp < 2; ++grp) {
-    if (total_samples[grp] == 0) continue;
-    const size_t value = fp32 ? sizeof(float) : sizeof(double), per = (dens ? 3 : 2) * value;
-    const int align = fp32 ? 4 : 1;  // patches of an FP32 tile stay together
-    const size_t least = (size_t)deepest[grp] * 32 * align * per;
-    size_t room = 0;
-    e = sample_workspace(c, (size_t)std::max(total_samples[0], total_samples[1]) * per, least, room);
-    if (e != cudaSuccess) return cuda_fail(c, e, "allocating field samples");
-    const int64_t n_room = (int64_t)(room / per) & ~(int64_t)31;
-    const int lo = grp ? n_four : 0, hi = grp ? n_ring : n_four;
-    std::vector<FieldRange> part;
+  {
+    const size_t per = (dens ? 3 : 2) * (fp32 ? sizeof(float) : sizeof(double));
+    cudaError_t we = cudaSuccess;
+    auto room = [&](size_t want, size_t least) {
+      size_t got = 0;
+      we = sample_workspace(c, want, least, got);
+      return we == cudaSuccess ? got : 0;
+    };
     // of a tile-masked image few patches are wanted (a sixteenth, say): their columns are split further
     // (4.8M atoms, 2263 x 2263 pixels, 7 % of the tiles: 5.9 ms, 9.2 with whole columns)
-    int64_t at_once = std::min(total_patches[grp], n_room / (32 * (int64_t)deepest[grp])) / align;
-    at_once = std::max<int64_t>(1, masked ? at_once / 16 : at_once);
-    field_ranges(cj.data() + lo, hi - lo, (int)total_patches[grp], n_room, align,
-                 fp32 ? depth_chunk(at_once, deepest[grp], kField32Blocks, 8, true)
-                      : depth_chunk(at_once, deepest[grp], 4 * kField64Blocks, 1, false),
-                 deepest[grp], part);
-    for (FieldRange& R : part) {
-      R.job_lo = lo;
-      R.n_jobs = hi - lo;
-      R.four = grp == 0;
-      R.rho_at = 2 * n_room;
-      ranges.push_back(R);
-    }
+    auto chunk = [&](int64_t at_once, int deep) {
+      if (masked) at_once = std::max<int64_t>(1, at_once / 16);
+      return fp32 ? depth_chunk(at_once, deep, kField32Blocks, 8, true)
+                  : depth_chunk(at_once, deep, 4 * kField64Blocks, 1, false);
+    };
+    // (patches of an FP32 tile stay together)
+    if (!plan_ranges(cj.data(), groups, fp32 ? 4 : 1, per, room, chunk, ranges))
+      return cuda_fail(c, we, "allocating field samples");
   }
 
   // ---- per-image column launches (general FP32 or FP64 kernel), epilogues, image clearing

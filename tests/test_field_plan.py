@@ -1,0 +1,91 @@
+"""The plan of a call's field samples (field_plan.h): every range of patches lies in the buffer that is held
+when the call runs, whatever the allocator gives, and the ranges cover all patches once."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "simulated_tem_gb300", "csrc")
+
+RANGES = r"""
+#include "field_plan.h"
+#include <cstdio>
+#include <random>
+struct Params { int Mz; };
+struct Job { Params p; int patch_base; int64_t sample_base; };
+#define CHECK(c) do { if (!(c)) { std::printf("line %d: " #c "\n", __LINE__); return 1; } } while (0)
+int main() {
+  std::mt19937 rng(7);
+  auto below = [&](int n) { return (int)(rng() % (unsigned)n); };
+  for (int trial = 0; trial < 3000; ++trial) {
+    const int align = trial % 2 ? 4 : 1;
+    const size_t per = trial % 3 ? 8 : 24;
+    std::vector<Job> jobs;
+    stem::FieldGroup g[2];
+    for (int i = 0; i < 2; ++i) {
+      g[i].job_lo = (int)jobs.size();
+      g[i].n_jobs = below(4);
+      for (int j = 0; j < g[i].n_jobs; ++j) {
+        const int mz = 1 + below(300), np = align * below(40);
+        jobs.push_back({{mz}, (int)g[i].patches, g[i].samples});
+        g[i].patches += np;
+        g[i].samples += (int64_t)np * mz * 32;
+        g[i].deepest = std::max(g[i].deepest, mz);
+      }
+    }
+    // an allocator whose every answer is less than the one before
+    size_t held = 0, scale = 1 + below(64);
+    auto room = [&](size_t want, size_t least) {
+      held = std::max(least, want / scale);
+      scale *= 2;
+      return held;
+    };
+    std::vector<stem::FieldRange> out;
+    CHECK(stem::plan_ranges(jobs.data(), g, align, per, room, [](int64_t, int) { return 8; }, out));
+    int next[2] = {0, 0};
+    for (const stem::FieldRange& R : out) {
+      const int i = R.four ? 0 : 1;
+      CHECK(R.patch_lo == next[i] && R.patch_hi > R.patch_lo && R.n_chunks * R.chunk >= g[i].deepest);
+      CHECK(R.job_lo == g[i].job_lo && R.n_jobs == g[i].n_jobs);
+      next[i] = R.patch_hi;
+      int64_t end = 0;  // samples of the range, from the workspace's start
+      for (int j = g[i].job_lo; j < g[i].job_lo + g[i].n_jobs; ++j) {
+        const int stop = j + 1 < g[i].job_lo + g[i].n_jobs ? jobs[j + 1].patch_base : (int)g[i].patches;
+        const int lo = std::max(R.patch_lo, jobs[j].patch_base), hi = std::min(R.patch_hi, stop);
+        if (lo >= hi) continue;
+        const int64_t o = jobs[j].sample_base - R.origin;
+        CHECK(o + (int64_t)(lo - jobs[j].patch_base) * jobs[j].p.Mz * 32 >= 0);
+        end = std::max(end, o + (int64_t)(hi - jobs[j].patch_base) * jobs[j].p.Mz * 32);
+      }
+      CHECK(2 * end <= R.rho_at);                       // the field before rho,
+      CHECK((size_t)(R.rho_at / 2) * per <= held);      // and all of it in what is held now
+    }
+    CHECK(next[0] == g[0].patches && next[1] == g[1].patches);
+  }
+  std::vector<stem::FieldRange> out;
+  Job one{{10}, 0, 0};
+  stem::FieldGroup g[2];
+  g[0].n_jobs = 1;
+  g[0].patches = 4;
+  g[0].samples = 4 * 320;
+  g[0].deepest = 10;
+  CHECK(!stem::plan_ranges(&one, g, 4, 8, [](size_t, size_t) { return (size_t)0; }, [](int64_t, int) { return 8; }, out));
+  std::puts("ok");
+  return 0;
+}
+"""
+
+
+def run(tmp_path, source):
+    if not shutil.which("g++"):
+        pytest.skip("no C++ compiler")
+    src = tmp_path / "t.cpp"
+    src.write_text(source)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-I", CSRC, str(src), "-o", str(tmp_path / "t")], check=True)
+    r = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout
+
+
+def test_ranges_lie_in_the_buffer_that_is_held(tmp_path):
+    run(tmp_path, RANGES)
