@@ -94,7 +94,12 @@ typedef struct st_stats {
   int32_t n_launches;    /* kernels the call launched (all attempts; autotuning trials included) */
 } st_stats;
 
-/* Context on CUDA device `device` (made current for the calls). */
+/* Context on CUDA device `device` (made current for the calls).  Besides buffers of the size of its largest
+ * call it holds, until it is destroyed, a workspace of field samples: 8 to 24 bytes per voxel of the largest
+ * image or batch, at most 2 GiB (the bytes in the environment variable STEM_SAMPLE_BYTES when that is set
+ * at the context's creation; a larger image then runs in ranges of columns, and 0 means none: the
+ * general kernels).  On a full device it makes do with less.  A plan's private contexts each hold
+ * their own. */
 int st_create(st_ctx** ctx, int device);
 void st_destroy(st_ctx* ctx);
 const char* st_last_error(const st_ctx* ctx);

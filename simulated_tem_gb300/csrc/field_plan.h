@@ -16,6 +16,51 @@
 
 namespace stem {
 
+// Device memory that a context keeps for field samples.
+struct SampleMemory {
+  void* p = nullptr;
+  size_t cap = 0;    // bytes
+  int patience = 0;  // calls that make do with what is held before more is asked for again
+};
+
+// The bytes a call may lay its samples out in: `want`, at most `most` (an image's or batch's columns then
+// run in several ranges), less on a full device, but at least `least`, one patch; 0: not even that.
+// What is held and holds `least` is given up only for a larger buffer, and after a refusal the next
+// kPatience calls do with it: a free, a failing allocation and a synchronisation of the device per call
+// cost more than the further ranges.
+constexpr int kPatience = 63;
+template <typename Alloc, typename Release>
+size_t sample_room(SampleMemory& m, size_t want, size_t least, size_t most, Alloc alloc, Release release) {
+  if (most == 0) return 0;
+  want = std::max(std::min(want, most), least);
+  if (m.p && m.cap >= want) return want;
+  if (m.p && m.cap >= least) {
+    if (m.patience > 0) {
+      --m.patience;
+      return m.cap;
+    }
+    if (void* p = alloc(want)) {
+      release(m.p);
+      m.p = p;
+      m.cap = want;
+    } else {
+      m.patience = kPatience;
+    }
+    return m.cap;
+  }
+  if (m.p) release(m.p);
+  m = SampleMemory();
+  for (size_t n = want;; n = std::max(n / 2, least)) {
+    if (void* p = alloc(n)) {
+      m.p = p;
+      m.cap = n;
+      m.patience = n < want ? kPatience : 0;
+      return n;
+    }
+    if (n <= least) return 0;
+  }
+}
+
 // The voxel field of a range of patches (warp tiles of 32 columns) of a batch, in a workspace of
 // samples: patch by patch in job order, slice by slice, 32 lanes.  The work is handed out in units
 // of one patch and `chunk` slices, so that few patches still fill the GPU.

@@ -40,8 +40,8 @@ struct st_ctx {
   size_t cap_kern = 0;
   unsigned char* d_tab = nullptr;  // the call's tables and job descriptors, one copy from h_stage
   size_t cap_tab = 0;
-  void* d_samples = nullptr;  // field samples of one range of patches
-  size_t cap_samples = 0;     // bytes
+  SampleMemory samples;  // field samples of one range of patches
+  size_t sample_limit = (size_t)2 << 30;  // bytes of them; STEM_SAMPLE_BYTES
   long long* d_gauss = nullptr;  // gauss64_table
   double* d_bx = nullptr;  // st_batch: packed atoms of the distinct atom arrays
   size_t cap_bx = 0;
@@ -461,25 +461,17 @@ bool ring_eligible(const ColumnParams& cp, bool stats) {
   return cp.a11 >= r3 && cp.a22 >= r3 && cp.Ez <= cp.Mz;
 }
 
-// The sample workspace: `want` bytes, at most kSampleBytes (an image's or batch's columns then run
-// in several ranges); less where the device has no room for that, but at least `least`, one patch.
-constexpr size_t kSampleBytes = (size_t)2 << 30, kMinSampleBytes = (size_t)32 << 20;
-cudaError_t sample_workspace(st_ctx* c, size_t want, size_t least, size_t& room) {
-  room = std::max(std::min(want, kSampleBytes), least);
-  if (c->d_samples && c->cap_samples >= room) return cudaSuccess;
-  if (c->d_samples) cudaFree(c->d_samples);
-  c->d_samples = nullptr;
-  c->cap_samples = 0;
-  for (;;) {
-    const cudaError_t e = cudaMalloc(&c->d_samples, room);
-    if (e == cudaSuccess) {
-      c->cap_samples = room;
-      return e;
-    }
-    if (e != cudaErrorMemoryAllocation || room <= std::max(kMinSampleBytes, least)) return e;
+// sample_room with the context's memory; 0 without an error: the device is full.
+size_t sample_workspace(st_ctx* c, size_t want, size_t least, cudaError_t& e) {
+  auto alloc = [&](size_t n) -> void* {
+    void* p = nullptr;
+    const cudaError_t ae = cudaMalloc(&p, n);
+    if (ae == cudaSuccess) return p;
     cudaGetLastError();
-    room = std::max(room / 2, least);
-  }
+    if (ae != cudaErrorMemoryAllocation) e = ae;
+    return nullptr;
+  };
+  return sample_room(c->samples, want, least, c->sample_limit, alloc, [](void* p) { cudaFree(p); });
 }
 
 // Slices per unit of work (a multiple of 4) of `tiles` tiles up to `deepest` slices deep, `per_sm` of
@@ -699,14 +691,11 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
 
   // ---- ranges of patches whose field samples share one workspace
   std::vector<FieldRange> ranges;
+  bool planned = false;  // else no memory for samples: the general kernels, which need none
   {
     const size_t per = (dens ? 3 : 2) * (fp32 ? sizeof(float) : sizeof(double));
     cudaError_t we = cudaSuccess;
-    auto room = [&](size_t want, size_t least) {
-      size_t got = 0;
-      we = sample_workspace(c, want, least, got);
-      return we == cudaSuccess ? got : 0;
-    };
+    auto room = [&](size_t want, size_t least) { return sample_workspace(c, want, least, we); };
     // of a tile-masked image few patches are wanted (a sixteenth, say): their columns are split further
     // (4.8M atoms, 2263 x 2263 pixels, 7 % of the tiles: 5.9 ms, 9.2 with whole columns)
     auto chunk = [&](int64_t at_once, int deep) {
@@ -715,8 +704,8 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
                   : depth_chunk(at_once, deep, 4 * kField64Blocks, 1, false);
     };
     // (patches of an FP32 tile stay together)
-    if (!plan_ranges(cj.data(), groups, fp32 ? 4 : 1, per, room, chunk, ranges))
-      return cuda_fail(c, we, "allocating field samples");
+    planned = plan_ranges(cj.data(), groups, fp32 ? 4 : 1, per, room, chunk, ranges);
+    if (we != cudaSuccess) return cuda_fail(c, we, "allocating field samples");
   }
 
   // ---- per-image column launches (general FP32 or FP64 kernel), epilogues, image clearing
@@ -736,7 +725,7 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     }
     return ce;
   };
-  bool ring_ok = ring;  // false once a slab overflowed even 256-atom staging: the general kernel
+  bool ring_ok = ring && planned;  // false also once a slab overflowed even 256-atom staging: the general kernel
   auto epilogues = [&]() -> cudaError_t {
     cudaError_t ce = cudaSuccess;
     if (!(flags & ST_FLAG_AVERAGE)) return ce;
@@ -793,9 +782,9 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     auto ring_launch = [&](int v) {
       cudaError_t le = cudaSuccess;
       for (FieldRange R : ranges) {
-        R.samples = c->d_samples;
-        R.rho32 = (float*)c->d_samples + R.rho_at;
-        R.rho64 = (double*)c->d_samples + R.rho_at;
+        R.samples = c->samples.p;
+        R.rho32 = (float*)c->samples.p + R.rho_at;
+        R.rho64 = (double*)c->samples.p + R.rho_at;
         R.work = (unsigned*)(c->s.counters + 5);
         R.counters = c->s.counters;
         R.cap = cap;
@@ -969,6 +958,7 @@ extern "C" int st_create(st_ctx** out, int device) {
   c->fp64_general = kv64 && std::strcmp(kv64, "general") == 0;
   const char* ks = std::getenv("STEM_RING_SLABS");
   c->min_slab_tier = !ks ? 0 : std::strcmp(ks, "256") == 0 ? 2 : std::strcmp(ks, "192") == 0 ? 1 : 0;
+  if (const char* kb = std::getenv("STEM_SAMPLE_BYTES")) c->sample_limit = (size_t)std::strtoull(kb, nullptr, 10);
   std::vector<long long> gauss(kGauss64Size);
   gauss64_table(gauss.data());
   e = cudaMalloc((void**)&c->d_gauss, gauss.size() * sizeof(long long));
@@ -988,7 +978,7 @@ extern "C" void st_destroy(st_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* dev_ptrs[] = {c->s.tmp_key, c->s.tmp_cell, c->s.tmp_slot, c->s.tmp_f, c->s.perm, c->s.block_sums,
                       c->s.counters, c->d_tab, c->b.cell_start, c->b.cell_count, c->b.f64, c->b.cs64, c->b.p32, c->b.cs32,
-                      c->b.fr32, c->b.ph32, c->d_x, c->d_img, c->d_blur, c->d_kern, c->d_samples, c->d_gauss, c->d_bx, c->d_bimg,
+                      c->b.fr32, c->b.ph32, c->d_x, c->d_img, c->d_blur, c->d_kern, c->samples.p, c->d_gauss, c->d_bx, c->d_bimg,
                       c->d_lvaux, c->d_levels, c->d_text, c->d_pseg, c->d_pstart, c->d_pbad, c->d_geom, c->d_tilt, c->d_keys, c->d_species};
   for (void* p : dev_ptrs)
     if (p) cudaFree(p);

@@ -76,6 +76,63 @@ int main() {
 }
 """
 
+ROOM = r"""
+#include "field_plan.h"
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+#define CHECK(c) do { if (!(c)) { std::printf("line %d: " #c "\n", __LINE__); return 1; } } while (0)
+int main() {
+  const size_t M = 1 << 20;
+  size_t free_bytes = 100 * M, next = 64;
+  std::map<void*, size_t> live;
+  int calls = 0;
+  auto alloc = [&](size_t n) -> void* {
+    ++calls;
+    if (n > free_bytes) return nullptr;
+    free_bytes -= n;
+    void* p = (void*)(next += 64);
+    live[p] = n;
+    return p;
+  };
+  auto release = [&](void* p) {
+    ++calls;
+    free_bytes += live.at(p);
+    live.erase(p);
+  };
+  stem::SampleMemory m;
+  auto room = [&](size_t want, size_t least, size_t most) {
+    const size_t got = stem::sample_room(m, want, least, most, alloc, release);
+    if (got && !(m.p && live.at(m.p) == m.cap && got <= m.cap)) std::abort();
+    return got;
+  };
+  CHECK(room(10 * M, M, 64 * M) == 10 * M && room(4 * M, M, 64 * M) == 4 * M && calls == 1);
+  CHECK(room(200 * M, M, 64 * M) == 64 * M && live.size() == 1);   // bounded, and the smaller one given back
+  CHECK(room(200 * M, 70 * M, 64 * M) == 70 * M);                   // one patch takes more than the bound
+  // a full device: half, then what is held call after call, and no allocator call in them
+  release(m.p);
+  m = stem::SampleMemory();
+  free_bytes = 40 * M;
+  CHECK(room(64 * M, M, 64 * M) == 32 * M);
+  calls = 0;
+  for (int i = 0; i < stem::kPatience; ++i) CHECK(room(64 * M, M, 64 * M) == 32 * M);
+  CHECK(calls == 0);
+  CHECK(room(64 * M, M, 64 * M) == 32 * M && calls == 1 && live.size() == 1);  // asked again, refused, kept
+  free_bytes = 100 * M;
+  for (int i = 0; i < stem::kPatience; ++i) CHECK(room(64 * M, M, 64 * M) == 32 * M);
+  CHECK(room(64 * M, M, 64 * M) == 64 * M);                         // and again, with the memory there
+  // down to one patch, and nothing
+  release(m.p);
+  m = stem::SampleMemory();
+  free_bytes = 2040;
+  CHECK(room(64 * M, 2000, 64 * M) == 2000);
+  CHECK(room(64 * M, 5001, 64 * M) == 0 && live.empty() && !m.p && m.cap == 0);
+  CHECK(room(64 * M, 1000, 0) == 0);
+  std::puts("ok");
+  return 0;
+}
+"""
+
 
 def run(tmp_path, source):
     if not shutil.which("g++"):
@@ -89,3 +146,7 @@ def run(tmp_path, source):
 
 def test_ranges_lie_in_the_buffer_that_is_held(tmp_path):
     run(tmp_path, RANGES)
+
+
+def test_the_memory_held_for_samples(tmp_path):
+    run(tmp_path, ROOM)
