@@ -115,6 +115,7 @@ struct ColumnParams {
   // the FP64 path's fixed-point integrator: dz times b0, bg and 1 times 2^fx_shift; fx_shift < 0: FP64
   double fx_b0, fx_bg, fx_a;
   int fx_shift;
+  int renorm32;  // the FP32 integrator renormalises after so many double steps (every step: they are long)
   // FP32 scaled lengths (s = sqrt(log2 e / 2 sigma^2)): s, the link-cell sides, (3 sigma)^2, and back to A^2
   float scale, a11s, a22s, a33s, cut2s, r2_to_A2;
   const int* cell_start;

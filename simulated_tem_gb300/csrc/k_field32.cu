@@ -839,10 +839,6 @@ __device__ __forceinline__ void write_pixel(const ColumnParams& p, int64_t o, do
   p.img[o] = v;
 }
 
-__device__ __forceinline__ int renorm_every(const ColumnParams& p, float a_max) {
-  return 2.f * (float)p.dz * (fabsf((float)p.b0) + fabsf((float)p.bg) + a_max) < 1.f ? 8 : 1;
-}
-
 // Every image with one angle: a warp per patch, four patches per CTA.
 template <int TX, bool kDens>
 __global__ void __launch_bounds__(128) k_integrate32(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R) {
@@ -857,7 +853,7 @@ __global__ void __launch_bounds__(128) k_integrate32(const ColumnJob* __restrict
   const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32 + lane;
   const float a = J.p.aaf[0];
   float ig;
-  integrate<float, 1, kDens>(J.p, (const float2*)R.samples + o, R.rho32 + o, &a, renorm_every(J.p, fabsf(a)), &ig);
+  integrate<float, 1, kDens>(J.p, (const float2*)R.samples + o, R.rho32 + o, &a, J.p.renorm32, &ig);
   if (wanted) write_pixel(J.p, px, (double)ig);
 }
 
@@ -882,13 +878,11 @@ __global__ void __launch_bounds__(128) k_integrate32_multi(const ColumnJob* __re
     const int np = min(16, p.n_prec - k0);
     for (int k = 2 * NH * warp; k < np; k += 2 * NH * blockDim.y) {
       float2 a[NH];  // the table is padded to an even count
-      float am = 0.f, ig[2 * NH];
+      float ig[2 * NH];
 #pragma unroll
-      for (int i = 0; i < NH; ++i) {
+      for (int i = 0; i < NH; ++i)
         a[i] = k + 2 * i < np ? make_float2(p.aaf[k0 + k + 2 * i], p.aaf[k0 + k + 2 * i + 1]) : make_float2(0.f, 0.f);
-        am = fmaxf(am, fmaxf(fabsf(a[i].x), fabsf(a[i].y)));
-      }
-      integrate<float2, NH, kDens>(p, (const float2*)R.samples + o, R.rho32 + o, a, renorm_every(p, am), ig);
+      integrate<float2, NH, kDens>(p, (const float2*)R.samples + o, R.rho32 + o, a, p.renorm32, ig);
 #pragma unroll
       for (int i = 0; i < 2 * NH; ++i)
         if (k + i < np) part[k + i][lane] = ig[i];

@@ -349,6 +349,15 @@ void fixed_integrator(ColumnParams& cp, const double* aa) {
   cp.fx_bg = cp.bg * cp.fx_a;
 }
 
+// Double steps between two renormalisations of the FP32 integrator: 8, or 1 when a step could grow phi by
+// more than a small factor.  Of all the image's angles, so that it does not depend on which share a
+// thread, and an image is the same beside any other images of a batch.
+int renorm_every32(const ColumnParams& cp, const double* aa) {
+  float a = 0.f;
+  for (int k = 0; k < cp.n_prec; ++k) a = std::max(a, std::fabs((float)aa[k]));
+  return 2.f * (float)cp.dz * (std::fabs((float)cp.b0) + std::fabs((float)cp.bg) + a) < 1.f ? 8 : 1;
+}
+
 ColumnParams column_params(st_ctx* c, const Job& j, int64_t cell_base, size_t xoff, size_t yoff, size_t zoff,
                            size_t aoff, int flags) {
   const st_geom* g = j.g;
@@ -377,6 +386,7 @@ ColumnParams column_params(st_ctx* c, const Job& j, int64_t cell_base, size_t xo
   cp.bg = g->bg;
   cp.dz = g->deltaz;
   fixed_integrator(cp, j.aa);
+  cp.renorm32 = renorm_every32(cp, j.aa);
   const double sd = length_scale(g);
   cp.scale = (float)sd;
   cp.a11s = (float)(cp.a11 * sd);
