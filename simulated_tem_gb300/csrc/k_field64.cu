@@ -52,6 +52,7 @@
 
 #include "internal.h"
 #include "slab_ring.cuh"
+#include "two_beam64.h"
 
 namespace stem {
 namespace field64 {
@@ -67,12 +68,8 @@ constexpr int kWarps = 4;
 // had this margin.
 constexpr float kGuard64 = 1e-3f;
 
-// A number in [-1, 1] in units of 2^-58, as h 2^29 + l, 0 <= l < 2^29: the product of two is three
-// 32 x 32-bit multiply-adds.
+// A number in [-1, 1] in units of 2^-58, as two limbs of 29 bits.
 constexpr int kLimb = 29, kLow = (1 << kLimb) - 1;
-struct __align__(8) Fixed {
-  int h, l;
-};
 constexpr int kPass = 32;         // atoms per pass over the lanes
 constexpr int kN = 64;            // step buffer: flushed at 32, before a round of 32 may add more
 constexpr float kOff = -1e30f;    // hmax of a slice the slab does not serve
@@ -103,8 +100,6 @@ struct WarpSmem {
 };
 
 __device__ __forceinline__ Fixed split58(long long v) { return Fixed{(int)(v >> kLimb), (int)v & kLow}; }
-
-__device__ __forceinline__ long long wide(int a, int b) { return (long long)a * b; }
 
 // A product of two fixed-point numbers.  The low limbs' product, 0 to 1 units, counts as a quarter.
 __device__ __forceinline__ long long mul58(const Fixed& a, const Fixed& b) {
@@ -179,16 +174,8 @@ __device__ __forceinline__ double value58(unsigned long long lo, int hi) {
   return DF((double)hi, 0x1p64, __ull2double_rn(lo));
 }
 
-// x (|x| <= 1) in units of 2^-60, cut off
-__device__ __forceinline__ long long to60(double x) {
-  const long long b = __double_as_longlong(x);
-  const int e = (int)(b >> 52) & 0x7FF;
-  const long long m = (((b & ((1LL << 52) - 1)) | (1LL << 52)) << 8) >> min(63, 1023 - e);
-  return b < 0 ? -m : m;
-}
-
-// The sample of a voxel: f S / max(1e-16, |S|) (:1877-1892), the bits of an FP64 number or, for the
-// fixed-point integrator, units of 2^-60; one copy of its code for all slices.
+// The sample of a voxel: f S / max(1e-16, |S|) (:1877-1892), the bits of an FP64 number or
+// units of 2^-60; one copy of its code for all slices.
 __device__ __noinline__ longlong2 sample(unsigned long long rl, int rh, unsigned long long il, int ih, double f,
                                          bool fixed) {
   const double sr = value58(rl, rh), si = value58(il, ih);
@@ -592,15 +579,15 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
 #pragma unroll
     for (int k = 0; k < SL; ++k) {
       if (z0 + k >= z_hi) break;
-      // with density, rho x and rho are stored; the fixed-point integrator's coefficients where it runs
+      // with density, rho x and rho are stored; for the fixed-point integrator times its coefficients
       const bool fixed = p.fx_shift >= 0;
       double f = fixed ? p.fx_bg : 1.0;
       if constexpr (kDens) {
         f = DM(f, rho[k]);
-        out_rho[((int64_t)(z0 + k) << 5) + lane] =
-            fixed ? to60(DM(rho[k], p.fx_b0)) : __double_as_longlong(rho[k]);
+        out_rho[((int64_t)(z0 + k) << 5) + lane] = __double_as_longlong(fixed ? DM(rho[k], p.fx_b0) : rho[k]);
       }
-      out[((int64_t)(z0 + k) << 5) + lane] = sample(A.sr[k].lo, A.sr[k].hi, A.si[k].lo, A.si[k].hi, f, fixed);
+      out[((int64_t)(z0 + k) << 5) + lane] =
+          sample(A.sr[k].lo, A.sr[k].hi, A.si[k].lo, A.si[k].hi, f, !kDens && fixed);
     }
   }
   if (p.want_stats) {
@@ -645,114 +632,34 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks)
 // The column integrator
 // ------------------------------------------------------------------------------------------
 
-struct S64 {
-  double c0, cgr, cgi;
+// A column's samples for column60: with density FP64, of which sparse columns need every bit, else units of
+// 2^-60, exact to bg's own bits.
+template <bool kDens>
+struct FixedSamples {
+  const longlong2* x;
+  const long long* r;
+  long long b0, a;
+  struct Raw {
+    longlong2 x;
+    long long r;
+  };
+  __device__ __forceinline__ Raw load(int z) const {
+    return Raw{x[(int64_t)z << 5], kDens ? r[(int64_t)z << 5] : b0};
+  }
+  __device__ __forceinline__ SFix coef(const Raw& s) const {
+    if constexpr (kDens)
+      return sfix(to60(__longlong_as_double(s.r)), to60(__longlong_as_double(s.x.x)),
+                  to60(__longlong_as_double(s.x.y)), a);
+    else
+      return sfix(s.r, s.x.x, s.x.y, a);
+  }
 };
-
-// d/dz (phi_0, phi_g) of the two-beam equations (:2375-2380, 2393-2396), fused
-__device__ __forceinline__ void deriv64(const S64& s, double ca, const double* ph, double* d) {
-  d[0] = DF(-s.cgr, ph[3], DF(-s.cgi, ph[2], -DM(s.c0, ph[1])));
-  d[1] = DF(-s.cgi, ph[3], DF(s.cgr, ph[2], DM(s.c0, ph[0])));
-  d[2] = DF(-ca, ph[3], DF(-s.cgr, ph[1], DM(s.cgi, ph[0])));
-  d[3] = DF(ca, ph[2], DF(s.cgi, ph[1], DM(s.cgr, ph[0])));
-}
-
-// One RK4 double step (:2389-2464): phi + dz/3 (k1 + 2 k2 + 2 k3 + k4), dz/3 in two parts so
-// that its rounding does not add up along the column.
-__device__ __forceinline__ void rk4_64(const S64& s0, const S64& s1, const S64& s2, double a, double dz, double dz3h,
-                                       double dz3l, double* ph) {
-  double k1[4], k2[4], k[4], q[4];
-  const double ca1 = DA(s1.c0, a);
-  deriv64(s0, DA(s0.c0, a), ph, k1);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) q[i] = DF(k1[i], dz, ph[i]);
-  deriv64(s1, ca1, q, k2);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) q[i] = DF(k2[i], dz, ph[i]);
-  deriv64(s1, ca1, q, k);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    k2[i] = DA(k2[i], k[i]);
-    q[i] = DF(k[i], 2.0 * dz, ph[i]);
-  }
-  deriv64(s2, DA(s2.c0, a), q, k);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const double t = DF(2.0, k2[i], DA(k1[i], k[i]));
-    ph[i] = DF(t, dz3h, DF(t, dz3l, ph[i]));
-  }
-}
-
-// The same in fixed point: numbers in units of 2^-60 as h 2^30 + l, 0 <= l < 2^30.
-constexpr int kLimb60 = 30;
-__device__ __forceinline__ Fixed split60(long long v) {
-  return Fixed{(int)(v >> kLimb60), (int)v & ((1 << kLimb60) - 1)};
-}
-
-struct SFix {
-  Fixed c0, ca, cgr, cgi, ngi;  // times dz 2^shift; ngi = -cgi
-};
-
-// (a x + b y + c z) 2^-shift, rounded (the low limbs' products, below one unit before the shift, left out)
-__device__ __forceinline__ long long row60(const Fixed& a, const Fixed& x, const Fixed& b, const Fixed& y,
-                                           const Fixed& c, const Fixed& z, long long half, int shift) {
-  long long hh = half, m = 0;
-  hh += wide(a.h, x.h);
-  hh += wide(b.h, y.h);
-  hh += wide(c.h, z.h);
-  m += wide(a.h, x.l);
-  m += wide(a.l, x.h);
-  m += wide(b.h, y.l);
-  m += wide(b.l, y.h);
-  m += wide(c.h, z.l);
-  m += wide(c.l, z.h);
-  return (hh + (m >> kLimb60)) >> shift;
-}
-
-// dz d/dz (phi_0, phi_g), as deriv64
-__device__ __forceinline__ void deriv60(const SFix& s, const long long* v, long long half, int shift, long long* d) {
-  Fixed p[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) p[i] = split60(v[i]);
-  d[0] = -row60(s.c0, p[1], s.cgi, p[2], s.cgr, p[3], half, shift);
-  d[1] = row60(s.c0, p[0], s.cgr, p[2], s.ngi, p[3], half, shift);
-  d[2] = -row60(s.ca, p[3], s.cgr, p[1], s.ngi, p[0], half, shift);
-  d[3] = row60(s.ca, p[2], s.cgi, p[1], s.cgr, p[0], half, shift);
-}
-
-__device__ __forceinline__ void rk4_60(const SFix& s0, const SFix& s1, const SFix& s2, long long half, int shift,
-                                       long long* ph) {
-  long long k1[4], ks[4], k[4], q[4];
-  deriv60(s0, ph, half, shift, k1);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) q[i] = ph[i] + k1[i];
-  deriv60(s1, q, half, shift, ks);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) q[i] = ph[i] + ks[i];
-  deriv60(s1, q, half, shift, k);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    ks[i] += k[i];
-    q[i] = ph[i] + 2 * k[i];
-  }
-  deriv60(s2, q, half, shift, k);
-  const int third = 357913941;  // 2^60 / 3, both limbs
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const Fixed t = split60(k1[i] + k[i] + 2 * ks[i]);
-    ph[i] += wide(t.h, third) + ((wide(t.h, third) + wide(t.l, third) + (3LL << (kLimb60 - 2))) >> kLimb60);
-  }
-}
 
 // A warp per patch and angle (warp w of the CTA takes angles w, w + warps, ...), one lane per
 // column.  FP64 takes about 90 operations per double step, at 76 cycles each; in fixed point they are
 // 156 multiply-adds of 4 cycles and as much again of additions and shifts.  The host takes
-// fixed point where 2^-60 is no coarser than FP64 for these amplitudes (fixed_integrator): the steps
-// are short, so that no number exceeds 1.3 and the norm stays (each step loses less than 2e-6 of it),
-// and |phi_g| is not small against 1.
-// In FP64, the equations being linear, the reference's renormalisation after every double step
-// (:2466-2472) only scales phi: it is done every 8 steps, and at the end through the quotient (every
-// step when a step could grow phi by more than a small factor).
+// fixed point where 2^-60 is no coarser than FP64 for these amplitudes (fixed_rule), and a warp with
+// columns that turn out too weak for it (column60) repeats those in FP64.
 template <bool kDens>
 __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict__ jobs, int n_jobs, FieldRange R) {
   __shared__ double part[8][32];
@@ -771,66 +678,35 @@ __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict
   const int64_t o = J.sample_base - R.origin + (int64_t)patch * p.Mz * 32 + lane;
   const double2* __restrict__ X = (const double2*)R.samples + o;
   const double* __restrict__ RH = R.rho64 + o;
-  const double dz = p.dz, dz3h = __ddiv_rn(dz, 3.0), dz3l = __ddiv_rn(DF(-3.0, dz3h, dz), 3.0);
-  auto coef = [&](int z) {
-    const double2 x = X[(int64_t)z << 5];
-    const double c0 = kDens ? DM(p.b0, RH[(int64_t)z << 5]) : p.b0;
-    return S64{c0, DM(p.bg, x.x), DM(p.bg, x.y)};
-  };
+  const double reach0 = fabs(p.b0) + fabs(p.bg);
   double total = 0.0;
   for (int k0 = 0; k0 < p.n_prec; k0 += nw) {
     const int k = k0 + warp;
-    if (k < p.n_prec && p.fx_shift >= 0) {
-      const longlong2* __restrict__ XF = (const longlong2*)X;
-      const long long* __restrict__ RF = (const long long*)RH;
-      const int shift = p.fx_shift;
-      const long long half = (1LL << shift) >> 1, b0 = to60(p.fx_b0), a = to60(DM(p.aa[k], p.fx_a));
-      auto coef60 = [&](const longlong2& x, long long c0) {
-        const Fixed gi = split60(x.y);
-        return SFix{split60(c0), split60(c0 + a), split60(x.x), gi, Fixed{-gi.h, -gi.l}};
-      };
-      long long ph[4] = {1LL << 60, 0, 0, 0};
-      SFix s0 = coef60(XF[0], kDens ? RF[0] : b0);
-      // the samples of the next double step are loaded ahead
-      auto at = [&](int z) { return (int64_t)(z < p.Mz ? z : 0) << 5; };
-      longlong2 x1 = XF[at(1)], x2 = XF[at(2)];
-      long long r1 = kDens ? RF[at(1)] : b0, r2 = kDens ? RF[at(2)] : b0;
-#pragma unroll 1
-      for (int z = 2; z <= p.Mz; z += 2) {
-        const SFix s1 = coef60(x1, r1), s2 = coef60(x2, r2);
-        x1 = XF[at(z + 1)];
-        x2 = XF[at(z + 2)];
-        if (kDens) {
-          r1 = RF[at(z + 1)];
-          r2 = RF[at(z + 2)];
-        }
-        rk4_60(s0, s1, s2, half, shift, ph);
-        s0 = s2;
-      }
-      double v[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = __ll2double_rn(ph[i]);
-      const double ig = DF(v[2], v[2], DM(v[3], v[3]));
-      part[warp][lane] = __ddiv_rn(ig, DF(v[0], v[0], DF(v[1], v[1], ig)));
-    } else if (k < p.n_prec) {
+    if (k < p.n_prec) {
       const double a = p.aa[k];
-      const int every = 2.0 * dz * (fabs(p.b0) + fabs(p.bg) + fabs(a)) < 1.0 ? 8 : 1;
-      double ph[4] = {1.0, 0.0, 0.0, 0.0};
-      S64 s0 = coef(0);
-      int n = 0;
-      for (int z = 2; z <= p.Mz; z += 2) {  // the last sample of an even column is the first (:1898-1899)
-        const S64 s1 = coef(z - 1), s2 = coef(z < p.Mz ? z : 0);
-        rk4_64(s0, s1, s2, a, dz, dz3h, dz3l, ph);
-        s0 = s2;
-        if (++n == every) {
-          n = 0;
-          const double inv = rsqrt(DF(ph[3], ph[3], DF(ph[2], ph[2], DF(ph[1], ph[1], DM(ph[0], ph[0])))));
-#pragma unroll
-          for (int i = 0; i < 4; ++i) ph[i] = DM(ph[i], inv);
-        }
+      const bool fixed = p.fx_shift >= 0;
+      bool repeat = !fixed;
+      if (fixed) {
+        const FixedSamples<kDens> src{(const longlong2*)X, (const long long*)RH, to60(p.fx_b0), to60(DM(a, p.fx_a))};
+        part[warp][lane] = column60(p.Mz, p.fx_shift, src, repeat);
+        repeat = repeat && wanted;
       }
-      const double ig = DF(ph[2], ph[2], DM(ph[3], ph[3]));
-      part[warp][lane] = __ddiv_rn(ig, DF(ph[0], ph[0], DF(ph[1], ph[1], ig)));
+      if (__any_sync(0xffffffffu, repeat)) {
+        // the stored samples are rho x and rho, or those times the fixed-point coefficients (in units of
+        // 2^-60 without density)
+        const double inv = fixed ? __ddiv_rn(1.0, p.fx_a) : 1.0;
+        auto coef = [&](int z) {
+          const double2 x = X[(int64_t)z << 5];
+          const double r = kDens ? RH[(int64_t)z << 5] : 1.0;
+          if (!fixed) return S64{kDens ? DM(p.b0, r) : p.b0, DM(p.bg, x.x), DM(p.bg, x.y)};
+          if constexpr (kDens) return S64{DM(r, inv), DM(x.x, inv), DM(x.y, inv)};
+          const double u = DM(inv, 0x1p-60);
+          return S64{p.b0, DM(__ll2double_rn(__double_as_longlong(x.x)), u),
+                     DM(__ll2double_rn(__double_as_longlong(x.y)), u)};
+        };
+        const double ig = column64(p.Mz, p.dz, a, reach0 + fabs(a), coef);
+        if (repeat) part[warp][lane] = ig;
+      }
     }
     __syncthreads();
     if (warp == 0)

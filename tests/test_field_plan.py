@@ -139,7 +139,7 @@ def run(tmp_path, source):
         pytest.skip("no C++ compiler")
     src = tmp_path / "t.cpp"
     src.write_text(source)
-    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-I", CSRC, str(src), "-o", str(tmp_path / "t")], check=True)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-ffp-contract=off", "-Wall", "-Wno-unknown-pragmas", "-I", CSRC, str(src), "-o", str(tmp_path / "t")], check=True)
     r = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout
 

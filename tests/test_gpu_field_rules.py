@@ -32,3 +32,33 @@ def test_fp32_steps_about_the_renormalisation_rule(ctx):
     got = ctx.batch([(G, x, six), (G, x, sixteen)], _lib.ST_FLAG_FP32)
     assert np.array_equal(got[0], want)
     assert np.array_equal(got[1], ctx.image(G, x, sixteen, flags=_lib.ST_FLAG_FP32))
+
+
+@pytest.fixture(scope="module")
+def general():
+    """A context that takes the general kernels (one column per thread, any cells)."""
+    with pytest.MonkeyPatch.context() as m:
+        m.setenv("STEM_FP64_KERNEL", "general")
+        m.setenv("STEM_FP32_KERNEL", "general")
+        c = imaging.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("density", [False, True])
+@pytest.mark.parametrize("n_prec", [1, 5])
+def test_fp64_sparse_columns(ctx, general, density, n_prec):
+    """A dilute gas in a deep box: most columns hold a weak field or none, down to the rim of one atom's density.
+    Each intensity is as accurate, relative to itself, as the general kernel's in FP64."""
+    a0 = synth.A0_FE
+    box = np.array([9, 8, 14]) * a0
+    pos = np.random.default_rng(3).uniform(0.0, 1.0, (70, 3)) * box
+    pos[:8] = np.array([[i, j, k] for i in (0, 1 - 1e-9) for j in (0, 1 - 1e-9) for k in (0, 1 - 1e-9)]) * box
+    t, x, _ = imaging.d2bi_condition(np.diag(box), a0, (0, 0, 1), (1, 1, 0), pos, sg=0.01, density=density)
+    G, aa = t.image_geometry(len(x), prec_angle=0.005, n_prec=n_prec)
+    got, want = ctx.image(G, x, aa), general.image(G, x, aa)
+    assert ctx.stats().column_kernel == 4 and general.stats().column_kernel == 3
+    assert (want < 1e-12).any() or not density
+    assert (want > 1e-3).any()
+    # 40 double steps and sums of a few terms: some tens of units of 2^-53
+    assert (np.abs(got - want) <= 1e-12 * want + 1e-36).all()
