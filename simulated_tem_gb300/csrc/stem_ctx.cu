@@ -439,8 +439,6 @@ cudaError_t tune_ring(st_ctx* c, F&& launch_variant, int64_t cap, cudaStream_t s
   return e;
 }
 
-// The slab-ring FP32 kernel needs cells of at least 3 sigma (no truncated
-// search) and at least one voxel thick in z.
 // The slab ring needs link cells of at least 3 sigma in x and y: then every atom within
 // 3 sigma of a column lies in its 9 cells around it in x-y.  The reference's grid makes them
 // so (Dx + 2 deltaM voxels over floor(Dx / deltaM + 2) cells, deltaM = ceil(3 sigma / the
@@ -450,6 +448,13 @@ bool ring_eligible(const ColumnParams& cp, bool stats) {
   if (cp.tile_mask && (cp.n_prec != 1 || stats)) return false;  // masked ring: one angle, no statistics
   const double r3 = 3 * cp.sigma * (1.0 - 1e-9);
   return cp.a11 >= r3 && cp.a22 >= r3 && cp.Ez <= cp.Mz;
+}
+
+// What the FP64 field needs besides: finite g (its phasors are fixed-point numbers, which hold no NaN).
+bool field64_eligible(const ColumnParams& cp, const st_geom* g) {
+  for (double v : g->g)
+    if (!(std::fabs(v) < 1e200)) return false;
+  return true;
 }
 
 // sample_room with the context's memory; 0 without an error: the device is full.
@@ -574,7 +579,8 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
   for (int i = 0; i < n; ++i) {
     cps[i] = column_params(c, jobs[i], cell_base[i], xoff[i], yoff[i], zoff[i], aoff[i], flags);
     max_np = std::max(max_np, jobs[i].n_prec);
-    if (!(fp32 ? c->fp32_general : c->fp64_general) && ring_eligible(cps[i], (flags & ST_FLAG_STATS) != 0)) {
+    if (!(fp32 ? c->fp32_general : c->fp64_general) && ring_eligible(cps[i], (flags & ST_FLAG_STATS) != 0) &&
+        (fp32 || field64_eligible(cps[i], jobs[i].g))) {
       on_ring[i] = 1;
       ring_jobs.push_back(i);
       dens = dens || cps[i].use_density;

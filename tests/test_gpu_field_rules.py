@@ -62,3 +62,15 @@ def test_fp64_sparse_columns(ctx, general, density, n_prec):
     assert (want > 1e-3).any()
     # 40 double steps and sums of a few terms: some tens of units of 2^-53
     assert (np.abs(got - want) <= 1e-12 * want + 1e-36).all()
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_fp64_reflections_that_are_not_finite(ctx, general, axis, bad):
+    """A g-vector that is not finite gives an image that is not, as the general kernel says."""
+    t, _, x = setup_both(cell_of((6, 5, 5)), sg=0.01)
+    G, aa = t.image_geometry(len(x))
+    G.g[axis] = bad
+    got, want = ctx.image(G, x, aa), general.image(G, x, aa)
+    assert np.isnan(want).any()
+    assert np.array_equal(got, want, equal_nan=True)
