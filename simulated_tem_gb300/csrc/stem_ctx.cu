@@ -450,11 +450,16 @@ bool ring_eligible(const ColumnParams& cp, bool stats) {
   return cp.a11 >= r3 && cp.a22 >= r3 && cp.Ez <= cp.Mz;
 }
 
-// What the FP64 field needs besides: finite g (its phasors are fixed-point numbers, which hold no NaN).
+// What the FP64 field needs besides: finite g (its phasors are fixed-point numbers, which hold no NaN), and
+// FP32 distances that decide every pair further than its guard, 1e-3 of scaled r^2, from the cutoff.  Of
+// coordinates up to F from the patch's reference cell they are within 3.2e-6 F: 7e-5 for voxels of a lattice
+// constant, the coarsest that a reference grid has, 8e-4 at F = 256 (the atoms' cell codes reach there too: at
+// most 101 cells of 3 sigma).
 bool field64_eligible(const ColumnParams& cp, const st_geom* g) {
   for (double v : g->g)
     if (!(std::fabs(v) < 1e200)) return false;
-  return true;
+  const double patch = 8 * std::max(std::fabs(g->a_vox[0]), std::fabs(g->a_vox[4])) + 3 * std::max(cp.a11, cp.a22);
+  return length_scale(g) * std::max(patch, 4 * cp.a33) <= 256.0;
 }
 
 // sample_room with the context's memory; 0 without an error: the device is full.

@@ -74,3 +74,35 @@ def test_fp64_reflections_that_are_not_finite(ctx, general, axis, bad):
     got, want = ctx.image(G, x, aa), general.image(G, x, aa)
     assert np.isnan(want).any()
     assert np.array_equal(got, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("side,kernel", [(20.0, 4), (35.0, 4), (40.0, 3), (110.0, 3)])
+def test_fp64_coarse_voxels_of_a_dilute_gas(ctx, general, side, kernel):
+    """Voxels far beyond a lattice constant, a few atoms about each: the distances to a patch's reference cell grow
+    until FP32 no longer decides (and the cells until their numbers leave a byte)."""
+    t, _, x = setup_both(cell_of((6, 5, 5)), sg=0.01)
+    G, aa = t.image_geometry(len(x))
+    vox, n, cell = (side, 1.0, 1.0), (8, 4, 8), 3.2
+    count = [int(np.ceil(vox[i] * (n[i] - 1) / cell)) + 3 for i in range(3)]
+    rng = np.random.default_rng(2)
+    x = np.concatenate([rng.uniform(-1.5, 1.5, (12, 3)) + [side * i, 1.5, 3.5] for i in range(n[0])])
+    x[:, 2] += rng.uniform(-3.0, 3.0, len(x))
+    G.sigma, G.nuvw, G.useDensity, G.nMax0 = 1.0, 1, 0, 0
+    G.Mx, G.My, G.Mz = n
+    G.ix0, G.ix1, G.iy0, G.iy1 = 0, n[0], 0, n[1]
+    G.Ex, G.Ey, G.Ez = count
+    for k in range(9):
+        i, diag = k // 3, k % 4 == 0
+        G.RU[k] = 1.0 if diag else 0.0
+        G.a_col[k] = cell if diag else 0.0
+        G.ia_col[k] = 1.0 / cell if diag else 0.0
+        G.a_vox[k] = vox[i] if diag else 0.0
+    for k in range(3):
+        G.delta[k] = G.Ruvw[k] = 0.0
+        G.lc_delta[k] = -cell
+        G.g[k] = 0.7 * k
+    G.deltaz = 1.0
+    got, want = ctx.image(G, x, aa), general.image(G, x, aa)
+    assert ctx.stats().column_kernel == kernel and ctx.stats().n_kept == len(x)
+    assert (want > 1e-4).sum() >= 20
+    assert np.abs(got - want).max() <= FP64_TOL
