@@ -396,11 +396,16 @@ int launch_strip(const __nv_bfloat16* x, const __nv_bfloat16* w, StripArgs a, cu
   const int slots = ctas * sms;
   // bands of rows: the number with the shortest whole waves of strips (a strip costs its rows and
   // about four more, its halo and the weights).  Just enough bands to reach the slots left 8 of 160
-  // strips for a second wave on 152 SMs: 8 x 256 x 256 pixels of 64 channels 100 -> 68 us.
+  // strips for a second wave on 152 SMs: 8 x 256 x 256 pixels of 64 channels 100 -> 68 us.  For each number of
+  // waves the fewest rows; tried in up to 64, since more even out (one per row of the image took the host 33 us
+  // for 5,000 rows, longer than the kernel).
   long long best = -1;
-  for (int bands = 1; bands <= a.H && bands <= 4096; ++bands) {
-    const int rows = ((a.H + bands - 1) / bands + RP - 1) / RP * RP, nb = (a.H + rows - 1) / rows;
-    const long long waves = ((long long)a.xtiles * nb * a.B + slots - 1) / slots, cost = waves * (rows + 4);
+  const long long columns = (long long)a.xtiles * a.B;
+  const long long first = (columns + slots - 1) / slots, last = (columns * ((a.H + RP - 1) / RP) + slots - 1) / slots;
+  for (long long w = first; w <= last && w < first + 64; ++w) {
+    const long long most = w * slots / columns;  // bands in w waves
+    const int rows = (int)((a.H + most - 1) / most + RP - 1) / RP * RP, nb = (a.H + rows - 1) / rows;
+    const long long waves = (columns * nb + slots - 1) / slots, cost = waves * (rows + 4);
     if (best < 0 || cost < best) {
       best = cost;
       a.rows_per_band = rows;
