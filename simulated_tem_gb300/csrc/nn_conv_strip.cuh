@@ -1,15 +1,15 @@
 // Strip-persistent convolution for the corrector's wide, shallow layers (Cout <= 64,
-// Cin 16, 32 or 64: the full- and half-resolution levels of the U-Net).  A 96-channel input
+// Cin 16, 32, 48 or 64: the full- and half-resolution levels of the U-Net).  A 96-channel input
 // (dec0a) holds 231 KB here, one CTA per SM, and measured 6 % faster on the halo-tile
 // kernel (two-row tiles, two CTAs per SM), which takes every wider input.
 //
 // A CTA walks down a band of image rows in one 128-pixel column strip, RP output rows per
 // step.  Its weights (all taps, all input channels, BN <= 64 output channels) are loaded
 // once by TMA and stay in shared memory.  Input rows live in a ring of 2 RP + 2 row slots,
-// each holding all Cin channels (16, 32 or 64) of pixels x0 - 1 .. x0 + 128 as one TMA box,
-// swizzled by its row of 2 Cin bytes: output rows y .. y + RP - 1 read input rows y - 1 .. y + RP
+// each holding all Cin channels of pixels x0 - 1 .. x0 + 128 as one TMA box, swizzled by its row of
+// 2 Cin bytes (48 channels, which no swizzle is as wide as: three boxes of 16): output rows y .. y + RP - 1 read input rows y - 1 .. y + RP
 // from the ring, and the next step's RP new rows load meanwhile.  The nine taps read a row
-// through descriptors shifted by 2 Cin bytes per pixel, as in the halo-tile kernel, and TMA
+// through descriptors shifted by one box row per pixel, as in the halo-tile kernel, and TMA
 // zero-fills outside the image.
 //
 // With N = BN <= 64 one MMA is little work, and MMAs that accumulate into the same TMEM
@@ -85,6 +85,9 @@ __device__ __forceinline__ Strip strip_of(const StripArgs& a, int s) {
   return r;
 }
 
+// Channels per TMA box of an input row
+__host__ __device__ __forceinline__ int box_channels(int Cin) { return Cin == 48 ? 16 : Cin; }
+
 constexpr int kBarBytes = (sizeof(Bars) + 15) & ~15;
 
 // NR = 3 (3 x 3 convolution) or 1 (1 x 1); RP output rows per step
@@ -92,7 +95,8 @@ template <int BN, int NR, int RP>
 __global__ void __launch_bounds__(kThreads) k_conv_strip(const StripArgs a, const __grid_constant__ CUtensorMap tmx,
                                                          const __grid_constant__ CUtensorMap tmw) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* base = smem_raw + ((1024 - ((uintptr_t)smem_raw & 1023)) & 1023);
+  const int align = 16 * box_channels(a.Cin);  // eight box rows: one repeat of the swizzle
+  unsigned char* base = smem_raw + ((align - ((uintptr_t)smem_raw & (align - 1))) & (align - 1));
   static_assert(RP % kIssuers == 0, "rows per step shared by the issuers");
   constexpr int kTaps = NR == 3 ? 9 : 1;
   constexpr uint32_t kCols = 2 * RP * BN;  // two sets of RP accumulators
@@ -151,7 +155,9 @@ __global__ void __launch_bounds__(kThreads) k_conv_strip(const StripArgs a, cons
           tc::mbar_arrive_expect_tx(rf, (uint32_t)(G * kHalo * 16));
           ++armed[slot];
           const int yin = sp.y0 - (NR == 3 ? 1 : 0) + i;
-          tc::tma_load_4d(tc::smem_addr(ring + slot * G * kSlab), &tmx, 0, sp.xt * kTileX - 1, yin, sp.img, rf);
+          for (int c = 0; c < a.Cin; c += box_channels(a.Cin))
+            tc::tma_load_4d(tc::smem_addr(ring + (slot * G + c / 8) * kSlab), &tmx, c, sp.xt * kTileX - 1, yin, sp.img,
+                            rf);
         }
       }
       // every load issued has landed before the CTA may leave
@@ -172,7 +178,8 @@ __global__ void __launch_bounds__(kThreads) k_conv_strip(const StripArgs a, cons
       // address (field bits 0-13, bytes / 16) moves by a fixed amount
       const uint64_t wdesc0 = tc::make_desc(tc::smem_addr(wsm), BN * 16, 128);
       const uint32_t wstep_tap = (uint32_t)(G * BN), wstep_k = (uint32_t)(2 * BN);  // in 16-byte units
-      const uint32_t pixel = (uint32_t)(G);  // 2 Cin bytes, in 16-byte units
+      const uint32_t pixel = (uint32_t)(box_channels(a.Cin) / 8);  // a box row, in 16-byte units
+      const uint32_t astep_k = a.Cin == 48 ? 2 * kSlab / 16 : 2;      // 16 channels: the next box, or 32 bytes
       int li = 0;  // ring position of the strip's first input row
       int k = 0;   // steps issued by this CTA (accumulator set sequence)
       for (int s = blockIdx.x; s < a.n_strips && ok; s += gridDim.x) {
@@ -195,7 +202,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_strip(const StripArgs a, cons
           uint64_t rowdesc[RP + NR - 1];
 #pragma unroll
           for (int d = 0; d < RP + NR - 1; ++d)
-            rowdesc[d] = tc::make_desc_k(rb + (uint32_t)((li + j * RP + d) % R) * row_bytes, (uint32_t)(16 * G));
+            rowdesc[d] = tc::make_desc_k(rb + (uint32_t)((li + j * RP + d) % R) * row_bytes, 16 * pixel);
 #pragma unroll
           for (int r = ri; r < RP; r += kIssuers) {
             const uint32_t acc = tmem + (uint32_t)((buf * RP + r) * BN);
@@ -206,7 +213,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_strip(const StripArgs a, cons
               uint64_t bd = wdesc0 + (uint64_t)(tap * wstep_tap);
               for (int s2 = 0; s2 < G / 2; ++s2) {
                 tc::mma_bf16(acc, ad, bd, idesc, (tap == 0 && s2 == 0) ? 0u : 1u);
-                ad += 2;  // 16 channels
+                ad += astep_k;
                 bd += wstep_k;
               }
             }
@@ -362,7 +369,7 @@ template <int BN, int NR>
 size_t strip_smem(int Cin, int ring) {
   const int G = Cin / 8;
   const size_t w = ((size_t)(NR == 3 ? 9 : 1) * G * BN * 16 + 1023) & ~(size_t)1023;
-  return 1024 + w + (size_t)ring * G * kSlab + kBarBytes + 4 * 32 * (BN / 8) * 16;
+  return 16 * box_channels(Cin) + w + (size_t)ring * G * kSlab + kBarBytes + 4 * 32 * (BN / 8) * 16;
 }
 
 template <int BN, int NR, int RP>
@@ -376,7 +383,7 @@ int launch_strip(const __nv_bfloat16* x, const __nv_bfloat16* w, StripArgs a, cu
   const int taps = NR == 3 ? 9 : 1;
   const cuuint64_t xd[4] = {(cuuint64_t)a.Cin, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.B};
   const cuuint64_t xs[3] = {(cuuint64_t)a.Cin * 2, (cuuint64_t)a.W * a.Cin * 2, (cuuint64_t)a.H * a.W * a.Cin * 2};
-  const cuuint32_t xb[4] = {(cuuint32_t)a.Cin, kHalo, 1, 1};
+  const cuuint32_t xb[4] = {(cuuint32_t)box_channels(a.Cin), kHalo, 1, 1};
   const cuuint64_t wd[3] = {(cuuint64_t)a.Cin, (cuuint64_t)taps, (cuuint64_t)a.Cout};
   const cuuint64_t wsd[2] = {(cuuint64_t)a.Cin * 2, (cuuint64_t)taps * a.Cin * 2};
   const cuuint32_t wbx[3] = {8, 1, (cuuint32_t)BN};
@@ -422,7 +429,7 @@ int launch_strip(const __nv_bfloat16* x, const __nv_bfloat16* w, StripArgs a, cu
 
 int conv_fwd_strip(const __nv_bfloat16* x, int B, int H, int W, int Cin, const __nv_bfloat16* w, int Cout, int taps,
                    const float* bias, int relu, const __nv_bfloat16* mask, void* y, int y_fp32, cudaStream_t st) {
-  if (Cout > 64 || (Cin != 16 && Cin != 32 && Cin != 64) || Cout % 8 != 0 || (taps != 1 && taps != 9)) return -1;
+  if (Cout > 64 || Cin > 64 || Cin % 16 != 0 || Cout % 8 != 0 || (taps != 1 && taps != 9)) return -1;
   strip::StripArgs a{bias, mask, y, B, H, W, Cin, Cout, relu, y_fp32, 0, 0, 0, 0, 0};
   using namespace strip;
   // two rows per step (four measured no faster: fewer CTAs fit)
