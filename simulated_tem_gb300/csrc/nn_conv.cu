@@ -580,7 +580,9 @@ namespace {
 // 256 pixels and 64 x 64 channels, this takes 61: 630 TFLOP/s).  A chunk is P consecutive pixels of a row
 // (P a multiple of 16 up to 64); for a 3 x 3 convolution a CTA owns one tap row dy: its x tile is row
 // y + dy, pixels x0 - 1 .. x0 + P, and the three taps read it shifted by 0, 1, 2 pixels (128 bytes
-// each).  Outside the image the boxes are zero-filled, in gy past the row's end, in x on every side.
+// each).  Outside the image the boxes are zero-filled, in gy past the row's end, in x on every side.  Where
+// a row's last chunk reaches past its end, the left tap would multiply the first pixel there, zero in gy, by the
+// row's last pixel: a NaN if that is not finite.  Its x tile then is a second box, of an image one pixel narrower.
 // A CTA owns 128 output channels (one 64-channel atom twice when Cout <= 64: the upper half of
 // the accumulator is not read) x BN input channels x TG taps (TG BN TMEM columns) for a range of
 // chunks.  Partial sums over the CTA's pixels go to its slice of a workspace (one slice per pixel
@@ -599,10 +601,11 @@ constexpr int kWAtom = 8192;   // 64 pixels x 128 bytes
 constexpr int kWAtomB = 9216;  // 66 pixels, rounded to the swizzle's 1024 bytes
 
 // MA, NB: 64-channel atoms of the output and input channels
-template <int MA, int NB>
+template <int MA, int NB, int TG>
 struct WSmem {
   alignas(1024) unsigned char a[kWStages][MA * kWAtom];
   alignas(1024) unsigned char b[kWStages][NB * kWAtomB];
+  alignas(1024) unsigned char left[TG == 3 ? kWStages : 1][NB * kWAtom];  // the left tap's tile at a ragged row end
   alignas(8) unsigned long long full[kWStages], empty[kWStages], done;
   uint32_t tmem;
   int abort;
@@ -613,10 +616,11 @@ __host__ __device__ constexpr int tmem_cols(int n) { return n <= 32 ? 32 : n <= 
 // BN = 32, 64 or 128 input channels, TG taps (3: a tap row; 1: a 1 x 1 convolution)
 template <int MA, int BN, int TG>
 __global__ void __launch_bounds__(kTileThreads) k_conv_wgrad(const WgradArgs a, const __grid_constant__ CUtensorMap tmg,
-                                                             const __grid_constant__ CUtensorMap tmx) {
+                                                             const __grid_constant__ CUtensorMap tmx,
+                                                             const __grid_constant__ CUtensorMap tml) {
   constexpr int NB = BN > 64 ? 2 : 1;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  WSmem<MA, NB>& S = *reinterpret_cast<WSmem<MA, NB>*>(smem_raw + ((1024 - ((uintptr_t)smem_raw & 1023)) & 1023));
+  WSmem<MA, NB, TG>& S = *reinterpret_cast<WSmem<MA, NB, TG>*>(smem_raw + ((1024 - ((uintptr_t)smem_raw & 1023)) & 1023));
   constexpr uint32_t kCols = tmem_cols(TG * BN);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   volatile int* abort = &S.abort;
@@ -626,6 +630,9 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_wgrad(const WgradArgs a, 
   const int dyi = blockIdx.z / n_ctiles;              // tap row
   const int chunk0 = blockIdx.x * a.chunks_per_cta;
   const int n = max(0, min(a.chunks_per_cta, a.chunks - chunk0));
+  // the chunk of a row that reaches past its end, if any (counted along: divisions by the issuing threads, one per
+  // chunk, cost 32 channels of 1136 x 1136 pixels a tenth)
+  const int x_ragged = TG == 3 && a.W < a.nx * a.P ? a.nx - 1 : -1;
 
   if (warp == 5) tc::tmem_alloc(tc::smem_addr(&S.tmem), kCols);
   if (t == 0) {
@@ -646,18 +653,28 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_wgrad(const WgradArgs a, 
     if (lane == 0) {
       // ---- producer
       const uint32_t bytes = (uint32_t)(MA * a.P + NB * (a.P + TG - 1)) * 128u;
-      int armed = 0;
+      int armed = 0, xi = chunk0 % a.nx, y = chunk0 / a.nx % a.H, img = chunk0 / a.nx / a.H;
       for (int c = 0; c < n; ++c, ++armed) {
         const int st = c % kWStages;
         if (c >= kWStages && !wait_or_abort(tc::smem_addr(&S.empty[st]), (c / kWStages - 1) & 1, abort)) break;
-        const int ch = chunk0 + c, xi = ch % a.nx, row = ch / a.nx, y = row % a.H, img = row / a.H;
         const uint32_t f = tc::smem_addr(&S.full[st]);
-        tc::mbar_arrive_expect_tx(f, bytes);
+        tc::mbar_arrive_expect_tx(f, xi == x_ragged ? bytes + (uint32_t)(NB * a.P) * 128u : bytes);
+        if (xi == x_ragged)  // (a row of one pixel: nothing to its left, a box outside the image)
+          for (int j = 0; j < NB; ++j)
+            tc::tma_load_4d(tc::smem_addr(S.left[st] + j * kWAtom), &tml, c0 + 64 * j, a.W > 1 ? xi * a.P - 1 : 1,
+                            y + dyi - 1, img, f);
         for (int j = 0; j < MA; ++j)
           tc::tma_load_4d(tc::smem_addr(S.a[st] + j * kWAtom), &tmg, m0 + 64 * j, xi * a.P, y, img, f);
         for (int j = 0; j < NB; ++j)
           tc::tma_load_4d(tc::smem_addr(S.b[st] + j * kWAtomB), &tmx, c0 + 64 * j, xi * a.P - (TG == 3 ? 1 : 0),
                           y + (TG == 3 ? dyi - 1 : 0), img, f);
+        if (++xi == a.nx) {
+          xi = 0;
+          if (++y == a.H) {
+            y = 0;
+            ++img;
+          }
+        }
       }
       // every load issued has landed before the CTA may leave (bounded)
       for (int st = 0; st < kWStages; ++st)
@@ -668,6 +685,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_wgrad(const WgradArgs a, 
     if (lane == 0) {
       // ---- MMA issuer
       constexpr uint32_t idesc = tc::make_idesc_bf16_mn(128, BN);
+      int xi = chunk0 % a.nx;
       for (int c = 0; c < n; ++c) {
         const int st = c % kWStages;
         if (!wait_or_abort(tc::smem_addr(&S.full[st]), (c / kWStages) & 1, abort)) break;
@@ -675,15 +693,19 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_wgrad(const WgradArgs a, 
         // start addresses in 16-byte units: 16 pixels are 2048 bytes, one pixel 128.  With one atom of
         // output channels the second one's rows (any shared memory behind it) are not read back.
         uint64_t ad = tc::make_desc_mn128(tc::smem_addr(S.a[st]), kWAtom);
-        uint64_t bd = tc::make_desc_mn128(tc::smem_addr(S.b[st]), kWAtomB);
+        uint64_t bd = tc::make_desc_mn128(tc::smem_addr(S.b[st]), kWAtomB), bl = bd;
+        if (xi == x_ragged) bl = tc::make_desc_mn128(tc::smem_addr(S.left[st]), kWAtom);
         for (int s = 0; s < a.P / 16; ++s) {
 #pragma unroll
           for (int tap = 0; tap < TG; ++tap)
-            tc::mma_bf16(tmem + (uint32_t)(tap * BN), ad, bd + (uint64_t)(8 * tap), idesc, (c > 0 || s > 0) ? 1u : 0u);
+            tc::mma_bf16(tmem + (uint32_t)(tap * BN), ad, tap == 0 ? bl : bd + (uint64_t)(8 * tap), idesc,
+                         (c > 0 || s > 0) ? 1u : 0u);
           ad += 128;
           bd += 128;
+          bl += 128;
         }
         tc::mma_commit(tc::smem_addr(&S.empty[st]));
+        xi = xi + 1 == a.nx ? 0 : xi + 1;
       }
       tc::mma_commit(tc::smem_addr(&S.done));  // arrives when every MMA issued above has completed
       if (!tc::mbar_wait(tc::smem_addr(&S.done), 0, kWaitLimit)) *abort = 1;
@@ -777,20 +799,22 @@ WgradPlan wgrad_plan(int B, int H, int W, int Cin, int Cout, int taps) {
 template <int MA, int BN, int TG>
 cudaError_t launch_wgrad(const WgradPlan& p, const __nv_bfloat16* x, const __nv_bfloat16* gy, WgradArgs a, float* gw,
                          cudaStream_t st) {
-  CUtensorMap tmg, tmx;
-  auto map = [&](CUtensorMap* m, const void* base, int C, int pixels) {
-    const cuuint64_t d[4] = {(cuuint64_t)C, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.B};
+  CUtensorMap tmg, tmx, tml;
+  auto map = [&](CUtensorMap* m, const void* base, int C, int pixels, int W) {
+    const cuuint64_t d[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)a.H, (cuuint64_t)a.B};
     const cuuint64_t s[3] = {(cuuint64_t)C * 2, (cuuint64_t)a.W * C * 2, (cuuint64_t)a.H * a.W * C * 2};
     const cuuint32_t box[4] = {64, (cuuint32_t)pixels, 1, 1};
     return make_map_swizzled(m, base, 4, d, s, box);
   };
-  if (!map(&tmg, gy, a.Cout, a.P) || !map(&tmx, x, a.Cin, a.P + TG - 1)) return cudaErrorInvalidValue;
-  const size_t smem = sizeof(WSmem<MA, (BN > 64 ? 2 : 1)>) + 1024;
+  if (!map(&tmg, gy, a.Cout, a.P, a.W) || !map(&tmx, x, a.Cin, a.P + TG - 1, a.W) ||
+      !map(&tml, x, a.Cin, a.P, a.W > 1 ? a.W - 1 : 1))
+    return cudaErrorInvalidValue;
+  const size_t smem = sizeof(WSmem<MA, (BN > 64 ? 2 : 1), TG>) + 1024;
   auto kernel = k_conv_wgrad<MA, BN, TG>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const dim3 grid(p.splits, (a.Cout + 127) / 128, ((a.Cin + BN - 1) / BN) * (a.taps / TG));
-  kernel<<<grid, kTileThreads, smem, st>>>(a, tmg, tmx);
+  kernel<<<grid, kTileThreads, smem, st>>>(a, tmg, tmx, tml);
   const long long n = (long long)a.Cout * a.taps * a.Cin;
   if (p.splits >= 32)
     k_wgrad_reduce<4><<<(int)std::min<long long>((n + 63) / 64, 2048), 256, 0, st>>>(a.ws, p.splits, n, gw);
