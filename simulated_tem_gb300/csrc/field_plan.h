@@ -2,6 +2,7 @@
 // the allocations and the split in depth are the caller's.
 #pragma once
 
+#include <math.h>
 #include <stddef.h>
 #include <stdint.h>
 
@@ -75,6 +76,11 @@ struct FieldRange {
   int job_lo = 0, n_jobs = 0;  // the range's jobs in the call's job table
   bool four = true;         // four slices per step (else two)
   int64_t rho_at = 0;       // where rho starts in the workspace, in values
+  // of a tile-masked image, which is alone: the tiles that have a wanted column, in any order, and their number;
+  // patches and samples are then counted along this list, and the split in depth follows the number
+  const int* list = nullptr;
+  const unsigned long long* n_list = nullptr;
+  int slots = 0;            // units that the GPU works on at a time
   unsigned* work = nullptr;  // units handed out: zero before the field kernel, zeroed again by the integrator
   const unsigned long long* counters = nullptr;
   int64_t cap = 0;
@@ -110,6 +116,40 @@ void field_ranges(const Job* jobs, int n_jobs, int patches, int64_t samples, int
     lo = R.patch_hi;
     out.push_back(R);
   }
+}
+
+// Slices per unit of work (a multiple of 4) of `tiles` tiles up to `deepest` slices deep, `slots` of
+// which the GPU works on at a time, when a unit costs `fixed` slices beside its own (the slabs it
+// stages before its first step): the number of pieces with the shortest waves of units.  The FP32
+// field's units, a CTA each, end together, so that whole waves count: on the 128k-atom image (435
+// tiles, 160 slices) 32 slices in 2.9 waves instead of 20 in 4.6.  The FP64 field's, a warp each, differ,
+// and up to two waves of them wait for the longest, more even out: the same image with density (1653
+// patches) 4766 us with 160 slices in 0.9 waves, 4512 with 40 in 3.6, 4352 with 20 in 7.2, 4530 with 8.
+constexpr int kPieces = 64;
+struct DepthRule {
+  int fixed;
+  bool whole_waves;
+};
+constexpr DepthRule kRule32{8, true}, kRule64{1, false};
+template <typename F>
+FP_HD F depth_cost(int64_t tiles, int deepest, int slots, DepthRule rule, int pieces, int& chunk) {
+  chunk = ((deepest + pieces - 1) / pieces + 3) & ~3;
+  const F w = (F)(tiles * ((deepest + chunk - 1) / chunk)) / (F)slots;
+  const F waves = rule.whole_waves ? ceil(w) : w <= (F)2.0 ? (F)1.08 * ceil(w) : w + (F)0.5;
+  return waves * (F)(chunk + rule.fixed);
+}
+inline int depth_chunk(int64_t tiles, int deepest, int slots, DepthRule rule) {
+  int best = (deepest + 3) & ~3;
+  double best_cost = -1;
+  for (int pieces = 1; pieces <= (deepest + 3) / 4 && pieces <= kPieces; ++pieces) {
+    int chunk;
+    const double cost = depth_cost<double>(tiles, deepest, slots, rule, pieces, chunk);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = chunk;
+    }
+  }
+  return best;
 }
 
 // The images of one group: those that march four slices per step, or two.

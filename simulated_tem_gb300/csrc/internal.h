@@ -78,7 +78,7 @@ struct Scratch {
   double4_32a* tmp_f = nullptr; // fx, fy, fz, g.y (FP64 path); Rec32 (FP32 path)
   int* perm = nullptr;      // position-in-cell -> tmp index
   int* block_sums = nullptr;
-  unsigned long long* counters = nullptr;  // [0] kept, [1] max cell count, [2] tests, [3] accepted, [4] slab overflow, [5] units of field work handed out
+  unsigned long long* counters = nullptr;  // [0] kept, [1] max cell count, [2] tests, [3] accepted, [4] slab overflow, [5] units of field work handed out, [6] tiles wanted by a mask
   size_t cap_candidates = 0;
   size_t cap_cells = 0;
   size_t cap_blocks = 0;
@@ -192,6 +192,43 @@ __device__ __forceinline__ const ColumnJob& field_patch(const ColumnJob* __restr
   patch = g - jobs[lo].patch_base;
   return jobs[lo];
 }
+#ifdef __CUDACC__
+// A tile-masked image: the patches of the range that are listed, `align` per tile, and their slices per
+// unit, by one warp (every lane gets them).
+__device__ __forceinline__ int listed_patches(const FieldRange& R, int align) {
+  const int64_t n = (int64_t)*R.n_list * align - R.patch_lo;
+  return (int)max((int64_t)0, min(n, (int64_t)(R.patch_hi - R.patch_lo)));
+}
+__device__ __forceinline__ int listed_patch(const FieldRange& R, int align, int patch) {
+  return R.list[patch / align] * align + patch % align;
+}
+__device__ __forceinline__ int warp_depth_chunk(int64_t tiles, int deepest, int slots, DepthRule rule) {
+  const int lane = threadIdx.x & 31;
+  float best = 3.0e38f;
+  int chunk = (deepest + 3) & ~3;
+  for (int pieces = lane + 1; pieces <= (deepest + 3) / 4 && pieces <= kPieces; pieces += 32) {
+    int c;
+    const float cost = depth_cost<float>(tiles, deepest, slots, rule, pieces, c);
+    if (cost < best) {
+      best = cost;
+      chunk = c;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {  // of equal costs the larger chunk
+    const float other = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oc = __shfl_xor_sync(0xffffffffu, chunk, o);
+    if (other < best || (other == best && oc > chunk)) {
+      best = other;
+      chunk = oc;
+    }
+  }
+  return chunk;
+}
+#endif
+// The tiles of tx x ty pixels of a tile-masked image that have a wanted one, to `list`; their number to *count
+// (zero before).
+cudaError_t launch_wanted_tiles(const ColumnJob* d_job, int tiles, int tx, int ty, int* list, unsigned long long* count,
+                                cudaStream_t st);
 inline int sm_count() {
   int dev = 0, sms = 152;
   cudaGetDevice(&dev);

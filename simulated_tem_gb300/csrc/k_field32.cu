@@ -321,10 +321,16 @@ __device__ __forceinline__ bool field_tile(const ColumnParams& p, W_& W, int pat
     if (p.tile_mask) wanted = active && p.tile_mask[(iy / p.mask_T) * p.mask_ntx + ix / p.mask_T] != 0;
   }
   const bool work = __any_sync(0xffffffffu, wanted);
+  unsigned patches = 15;  // of the tile, with a wanted column
   if constexpr (NW == 1) {
     if (!work) return true;
-  } else {
-    if (!__syncthreads_or(work)) return true;
+  } else if constexpr (kMasked) {
+    if (lane == 0) W.wcnt[warp] = work;
+    sync<NW>();
+    patches = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) patches |= W.wcnt[w] ? 1u << w : 0u;
+    if (!patches) return true;
   }
 
   // the frame is the 16 x 8 tile's for any NW, so that the staged values do not depend on it, from
@@ -364,8 +370,26 @@ __device__ __forceinline__ bool field_tile(const ColumnParams& p, W_& W, int pat
     pyc = 0.5f * (y_lo + y_hi);
     pxh = 0.5f * (x_hi - x_lo) + 2e-5f;  // the centre's rounding
     pyh = 0.5f * (y_hi - y_lo) + 2e-5f;
-    // the gather's rectangle and cells: the tile's, or for one warp the patch's
+    // the gather's rectangle and cells: the tile's, or for one warp the patch's, or about the wanted patches
     int gx0 = x0, gx1 = min(x0 + kTileX, p.ix1) - 1, gy0 = y0, gy1 = min(y0 + kTileY, p.iy1) - 1;
+    if (kMasked && NW > 1 && patches != 15) {
+      int lx = 1 << 30, ly = 1 << 30, ux = 0, uy = 0;
+#pragma unroll
+      for (int w = 0; w < 4; ++w)
+        if (patches >> w & 1) {
+          int cx, cy;
+          patch_column<TX>(x0, y0, w, 0, cx, cy);
+          lx = min(lx, cx);
+          ly = min(ly, cy);
+          patch_column<TX>(x0, y0, w, 31, cx, cy);
+          ux = max(ux, cx);
+          uy = max(uy, cy);
+        }
+      gx0 = lx;
+      gy0 = ly;
+      gx1 = min(gx1, ux);
+      gy1 = min(gy1, uy);
+    }
     if constexpr (NW == 1) {
       gx0 = xa;
       gy0 = ya;
@@ -683,7 +707,13 @@ __global__ void __launch_bounds__(W_::NW * 32, kMinBlocks)
     W.e0[W_::WCAP] = make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (W_::SL == 4) W.e1[W_::WCAP] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  const int units = R.units() / NW;
+  int chunk = R.chunk, n_chunks = R.n_chunks, units = R.units() / NW;
+  if constexpr (kMasked) {
+    const int n = listed_patches(R, 4), deep = jobs[0].p.Mz;
+    chunk = warp_depth_chunk((n + 3) / 4, deep, R.slots, kRule32);
+    n_chunks = (deep + chunk - 1) / chunk;
+    units = n / NW * n_chunks;
+  }
   for (;;) {
     sync<NW>();
     // a slab overflowed: the host recomputes with larger slabs
@@ -692,10 +722,11 @@ __global__ void __launch_bounds__(W_::NW * 32, kMinBlocks)
     const int unit = W.unit;
     if (unit >= units) break;
     int patch;
-    const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + unit / R.n_chunks * NW, patch);
-    const int z_lo = unit % R.n_chunks * R.chunk, z_hi = min(J.p.Mz, z_lo + R.chunk);
+    const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + unit / n_chunks * NW, patch);
+    const int z_lo = unit % n_chunks * chunk, z_hi = min(J.p.Mz, z_lo + chunk);
     if (z_lo >= z_hi) continue;  // an image less deep than the batch's deepest
     const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32;
+    if constexpr (kMasked) patch = listed_patch(R, 4, patch);
     if (!field_tile<CPL, TX, kDens, kStats, kMasked>(J.p, W, patch, z_lo, z_hi, (float2*)R.samples + o, R.rho32 + o))
       break;
   }
@@ -845,12 +876,14 @@ __global__ void __launch_bounds__(128) k_integrate32(const ColumnJob* __restrict
   const int lane = threadIdx.x, g = R.patch_lo + blockIdx.x * 4 + threadIdx.y;
   if (g == R.patch_lo && lane == 0) *R.work = 0;  // for the next field kernel
   if ((int64_t)R.counters[0] > R.cap || R.counters[4] != 0 || g >= R.patch_hi) return;
+  if (R.list && g - R.patch_lo >= listed_patches(R, 4)) return;
   int patch;
   const ColumnJob& J = field_patch(jobs, n_jobs, g, patch);
+  const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32 + lane;
+  if (R.list) patch = listed_patch(R, 4, patch);
   int64_t px;
   const bool wanted = patch_pixel<TX>(J.p, patch, lane, px);
   if (!__any_sync(0xffffffffu, wanted)) return;
-  const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32 + lane;
   const float a = J.p.aaf[0];
   float ig;
   integrate<float, 1, kDens>(J.p, (const float2*)R.samples + o, R.rho32 + o, &a, J.p.renorm32, &ig);
@@ -917,7 +950,7 @@ cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, int m
   auto kernel = k_field32<W, kCPL, TX, kDens, kStats, kMasked, B>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(W));
   if (e != cudaSuccess) return e;
-  const int grid = std::max(1, std::min(sm_count() * B, R.units() / NW));
+  const int grid = std::max(1, std::min(sm_count() * B, R.list ? R.patch_hi - R.patch_lo : R.units() / NW));
   ++launch_count();
   kernel<<<grid, NW * 32, sizeof(W), st>>>(jobs, n_jobs, R);
   e = cudaGetLastError();
@@ -966,6 +999,35 @@ int field32_patches(const ColumnParams& p) {
   const int Wd = p.ix1 - p.ix0, Hd = p.iy1 - p.iy0;
   if (Wd <= 0 || Hd <= 0) return 0;
   return 4 * ((Wd + field32::kTileX - 1) / field32::kTileX) * ((Hd + field32::kTileY - 1) / field32::kTileY);
+}
+
+namespace {
+__global__ void __launch_bounds__(256) k_wanted_tiles(const ColumnJob* __restrict__ job, int tiles, int tx, int ty,
+                                                      int* __restrict__ list, unsigned long long* __restrict__ count) {
+  const ColumnParams& p = job->p;
+  const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31;
+  bool want = false;
+  if (i < tiles) {
+    const int across = (p.ix1 - p.ix0 + tx - 1) / tx;
+    const int x0 = p.ix0 + i % across * tx, y0 = p.iy0 + i / across * ty;
+    const int x1 = min(x0 + tx, p.ix1) - 1, y1 = min(y0 + ty, p.iy1) - 1;
+    for (int my = y0 / p.mask_T; my <= y1 / p.mask_T; ++my)
+      for (int mx = x0 / p.mask_T; mx <= x1 / p.mask_T; ++mx) want = want || p.tile_mask[my * p.mask_ntx + mx] != 0;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  if (!m) return;
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(count, (unsigned long long)__popc(m));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (want) list[base + __popc(m & ((1u << lane) - 1))] = i;
+}
+}  // namespace
+
+cudaError_t launch_wanted_tiles(const ColumnJob* d_job, int tiles, int tx, int ty, int* list, unsigned long long* count,
+                                cudaStream_t st) {
+  ++launch_count();
+  k_wanted_tiles<<<(tiles + 255) / 256, 256, 0, st>>>(d_job, tiles, tx, ty, list, count);
+  return cudaGetLastError();
 }
 
 int ring_variant_count() { return field32::kVariants; }

@@ -610,17 +610,25 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpSmem<CAPS, SL>& W = reinterpret_cast<WarpSmem<CAPS, SL>*>(smem_raw)[warp];
   if ((int64_t)R.counters[0] > R.cap) return;  // the binning overflowed: the host retries
+  int chunk = R.chunk, n_chunks = R.n_chunks, units = R.units();
+  if constexpr (kMasked) {
+    const int n = listed_patches(R, 1), deep = jobs[0].p.Mz;
+    chunk = warp_depth_chunk(n, deep, R.slots, kRule64);
+    n_chunks = (deep + chunk - 1) / chunk;
+    units = n * n_chunks;
+  }
   for (;;) {
     int unit = 0;
     if (lane == 0) unit = (int)atomicAdd(R.work, 1u);
     unit = __shfl_sync(0xffffffffu, unit, 0);
-    if (unit >= R.units()) break;
+    if (unit >= units) break;
     if (R.counters[4] != 0) break;  // a slab overflowed: the host recomputes with larger slabs
     int patch;
-    const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + unit / R.n_chunks, patch);
-    const int z_lo = unit % R.n_chunks * R.chunk, z_hi = min(J.p.Mz, z_lo + R.chunk);
+    const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + unit / n_chunks, patch);
+    const int z_lo = unit % n_chunks * chunk, z_hi = min(J.p.Mz, z_lo + chunk);
     if (z_lo >= z_hi) continue;  // an image less deep than the batch's deepest
     const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32;
+    if constexpr (kMasked) patch = listed_patch(R, 1, patch);
     if (!field_tile<CAPS, SL, kDens, kMasked>(J.p, W, patch, z_lo, z_hi, (longlong2*)R.samples + o, (long long*)R.rho64 + o, T,
                                                lane))
       break;
@@ -665,16 +673,18 @@ __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict
   const int lane = threadIdx.x, warp = threadIdx.y, nw = blockDim.y;
   if (blockIdx.x == 0 && warp == 0 && lane == 0) *R.work = 0;  // for the next field kernel
   if ((int64_t)R.counters[0] > R.cap || R.counters[4] != 0) return;
+  if (R.list && (int)blockIdx.x >= listed_patches(R, 1)) return;
   int patch;
   const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + blockIdx.x, patch);
   const ColumnParams& p = J.p;
+  const int64_t o = J.sample_base - R.origin + (int64_t)patch * p.Mz * 32 + lane;
+  if (R.list) patch = listed_patch(R, 1, patch);
   const int tiles_x = (p.ix1 - p.ix0 + 7) / 8;
   const int ix = p.ix0 + (patch % tiles_x) * 8 + (lane & 7), iy = p.iy0 + (patch / tiles_x) * 4 + (lane >> 3);
   const bool active = ix < p.ix1 && iy < p.iy1;
   bool wanted = active;
   if (p.tile_mask) wanted = active && p.tile_mask[(iy / p.mask_T) * p.mask_ntx + ix / p.mask_T] != 0;
   if (!__any_sync(0xffffffffu, wanted)) return;
-  const int64_t o = J.sample_base - R.origin + (int64_t)patch * p.Mz * 32 + lane;
   const double2* __restrict__ X = (const double2*)R.samples + o;
   const double* __restrict__ RH = R.rho64 + o;
   const double reach0 = fabs(p.b0) + fabs(p.bg);
@@ -728,7 +738,7 @@ cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, const
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int grid = sm_count() * B;
-  grid = std::max(1, std::min(grid, (R.units() + kWarps - 1) / kWarps));
+  if (!R.list) grid = std::max(1, std::min(grid, (R.units() + kWarps - 1) / kWarps));
   ++launch_count();
   kernel<<<grid, kWarps * 32, smem, st>>>(jobs, n_jobs, R, T);
   return cudaGetLastError();

@@ -43,6 +43,8 @@ struct st_ctx {
   size_t cap_tab = 0;
   SampleMemory samples;  // field samples of one range of patches
   size_t sample_limit = (size_t)2 << 30;  // bytes of them; STEM_SAMPLE_BYTES
+  int* d_list = nullptr;  // the wanted tiles of a tile-masked image
+  size_t cap_list = 0;
   long long* d_gauss = nullptr;  // gauss64_table
   double* d_bx = nullptr;  // st_batch: packed atoms of the distinct atom arrays
   size_t cap_bx = 0;
@@ -475,31 +477,6 @@ size_t sample_workspace(st_ctx* c, size_t want, size_t least, cudaError_t& e) {
   return sample_room(c->samples, want, least, c->sample_limit, alloc, [](void* p) { cudaFree(p); });
 }
 
-// Slices per unit of work (a multiple of 4) of `tiles` tiles up to `deepest` slices deep, `per_sm` of
-// which an SM works on at a time, when a unit costs `fixed` slices beside its own (the slabs it
-// stages before its first step): the number of pieces with the shortest waves of units.  The FP32
-// field's units, a CTA each, end together, so that whole waves count: on the 128k-atom image (435
-// tiles, 160 slices) 32 slices in 2.9 waves instead of 20 in 4.6.  The FP64 field's, a warp each, differ,
-// and up to two waves of them wait for the longest, more even out: the same image with density (1653
-// patches) 4766 us with 160 slices in 0.9 waves, 4512 with 40 in 3.6, 4352 with 20 in 7.2, 4530 with 8.
-int depth_chunk(int64_t tiles, int deepest, int per_sm, int fixed, bool in_step) {
-  const int64_t full = (int64_t)sm_count() * per_sm;
-  int best = (deepest + 3) & ~3;
-  double best_cost = -1;
-  for (int pieces = 1; pieces <= (deepest + 3) / 4 && pieces <= 64; ++pieces) {
-    const int chunk = ((deepest + pieces - 1) / pieces + 3) & ~3;
-    const int64_t units = tiles * ((deepest + chunk - 1) / chunk);
-    const double w = (double)units / (double)full;
-    const double waves = in_step ? std::ceil(w) : w <= 2.0 ? 1.08 * std::ceil(w) : w + 0.5;
-    const double cost = waves * (chunk + fixed);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best = chunk;
-    }
-  }
-  return best;
-}
-
 // A recorded call (st_plan): the instantiated graph and what its kernels were recorded with.
 struct GraphOut {
   cudaGraphExec_t exec = nullptr;
@@ -693,21 +670,29 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
 
   // ---- ranges of patches whose field samples share one workspace
   std::vector<FieldRange> ranges;
+  int wanted_tiles = 0;  // of a tile-masked image, at most
   bool planned = false;  // else no memory for samples: the general kernels, which need none
   {
     const size_t per = (dens ? 3 : 2) * (fp32 ? sizeof(float) : sizeof(double));
     cudaError_t we = cudaSuccess;
     auto room = [&](size_t want, size_t least) { return sample_workspace(c, want, least, we); };
-    // of a tile-masked image few patches are wanted (a sixteenth, say): their columns are split further
-    // (4.8M atoms, 2263 x 2263 pixels, 7 % of the tiles: 5.9 ms, 9.2 with whole columns)
-    auto chunk = [&](int64_t at_once, int deep) {
-      if (masked) at_once = std::max<int64_t>(1, at_once / 16);
-      return fp32 ? depth_chunk(at_once, deep, kField32Blocks, 8, true)
-                  : depth_chunk(at_once, deep, 4 * kField64Blocks, 1, false);
+    const int slots = sm_count() * (fp32 ? kField32Blocks : 4 * kField64Blocks);
+    auto chunk = [&](int64_t at_once, int deep) {  // (of a tile-masked image the kernel decides)
+      return depth_chunk(at_once, deep, slots, fp32 ? kRule32 : kRule64);
     };
     // (patches of an FP32 tile stay together)
     planned = plan_ranges(cj.data(), groups, fp32 ? 4 : 1, per, room, chunk, ranges);
     if (we != cudaSuccess) return cuda_fail(c, we, "allocating field samples");
+    if (masked && planned) {  // (st_image_device_masked images one)
+      wanted_tiles = (int)(groups[0].patches + groups[1].patches) / (fp32 ? 4 : 1);
+      e = ensure(c->d_list, c->cap_list, (size_t)wanted_tiles);
+      if (e != cudaSuccess) return cuda_fail(c, e, "allocating the list of wanted tiles");
+      for (FieldRange& R : ranges) {
+        R.list = c->d_list;
+        R.n_list = c->s.counters + 6;
+        R.slots = slots;
+      }
+    }
   }
 
   // ---- per-image column launches (general FP32 or FP64 kernel), epilogues, image clearing
@@ -781,6 +766,10 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     }
     if (ce == cudaSuccess) ce = clear_images();
     if (!capturing) cudaEventRecord(c->ev[1], st);
+    if (ring_ok && wanted_tiles > 0 && ce == cudaSuccess) {
+      cudaMemsetAsync(c->s.counters + 6, 0, sizeof(unsigned long long), st);
+      ce = launch_wanted_tiles(d_coljobs, wanted_tiles, fp32 ? 16 : 8, fp32 ? 8 : 4, c->d_list, c->s.counters + 6, st);
+    }
     auto ring_launch = [&](int v) {
       cudaError_t le = cudaSuccess;
       for (FieldRange R : ranges) {
@@ -980,7 +969,7 @@ extern "C" void st_destroy(st_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* dev_ptrs[] = {c->s.tmp_key, c->s.tmp_cell, c->s.tmp_slot, c->s.tmp_f, c->s.perm, c->s.block_sums,
                       c->s.counters, c->d_tab, c->b.cell_start, c->b.cell_count, c->b.f64, c->b.cs64, c->b.p32, c->b.cs32,
-                      c->b.fr32, c->b.ph32, c->d_x, c->d_img, c->d_blur, c->d_kern, c->samples.p, c->d_gauss, c->d_bx, c->d_bimg,
+                      c->b.fr32, c->b.ph32, c->d_x, c->d_img, c->d_blur, c->d_kern, c->samples.p, c->d_list, c->d_gauss, c->d_bx, c->d_bimg,
                       c->d_lvaux, c->d_levels, c->d_text, c->d_pseg, c->d_pstart, c->d_pbad, c->d_geom, c->d_tilt, c->d_keys, c->d_species};
   for (void* p : dev_ptrs)
     if (p) cudaFree(p);
