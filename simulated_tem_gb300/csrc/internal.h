@@ -237,10 +237,14 @@ inline int sm_count() {
 }
 // The FP32 path's field and integration of one range (k_field32.cu).  `variant` 0 ..
 // ring_variant_count() - 1 selects the patch shape and the slab capacity of tier 0 (named per 8 x 4
-// patch: "slab96" stages 160 atoms per 16 x 8 tile, "slab128" 192); `slab_tier` 1: 352 atoms per tile (320
-// with two slices per step), 2: 256 atoms per patch, the tiles split into their patches.  Variants of
-// one patch shape give the same image to the last bit; the shapes agree to FP32 rounding.  `four` as
+// patch: "slab96" stages 160 atoms per 16 x 8 tile, "slab128" 192); `slab_tier` 1, 2: 288 and 416 atoms per
+// tile (320 and 512 with two slices per step), 3, 4: 256 atoms per patch, the tiles split into their patches, with
+// a larger window at 4.  Variants of
+// one patch shape give the same image to the last bit, at any tier; the shapes agree to FP32 rounding.  `four` as
 // below; `masked`: some jobs carry a tile mask (then stats must be false).
+constexpr int kField32Tiers = 5;
+// STEM_RING_SLABS' names of the tiers (the first three by what a patch of 8 x 4 columns can hold)
+constexpr const char* kSlabTierNames[kField32Tiers] = {"128", "192", "256", "patch", "patch1024"};
 constexpr int kField32Blocks = 5;  // CTAs of four warps per SM at tier 0
 cudaError_t launch_field32(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, bool density,
                            bool stats, bool masked, bool four, int variant, int slab_tier, cudaStream_t st);
@@ -252,6 +256,7 @@ bool ring_variant_same(int variant);  // gives variant 0's image to the last bit
 // 128, 192, 256 atoms; `four`: every job's steps of four slices fit the ring (four_slices_fit);
 // d_gauss: gauss64_table's values.
 constexpr int kGauss64Size = 3 * 1024 + 16;
+constexpr int kField64Tiers = 3;
 constexpr int kField64Blocks = 3;  // CTAs of four warps per SM at tier 0
 void gauss64_table(long long* t);
 cudaError_t launch_field64(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, int slab_tier,

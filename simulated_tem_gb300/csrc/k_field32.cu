@@ -946,6 +946,7 @@ cudaError_t launch_integrate(const ColumnJob* jobs, int n_jobs, const FieldRange
 
 template <int CAP, int WCAP, int NW, int SL, int TX, bool kDens, bool kStats, bool kMasked, int B>
 cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, int max_np, cudaStream_t st) {
+  static_assert((sizeof(Smem<CAP, WCAP, NW, SL>) + 1024) * B <= 232448, "shared memory of B CTAs");
   using W = Smem<CAP, WCAP, NW, SL>;
   auto kernel = k_field32<W, kCPL, TX, kDens, kStats, kMasked, B>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(W));
@@ -964,10 +965,21 @@ cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, int m
 template <int SL, bool kDens, bool kStats, bool kMasked>
 cudaError_t dispatch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, int max_np, int variant, int tier,
                      cudaStream_t st) {
-  // denser slabs, or coarser voxels: a step of two slices needs less window, so that four CTAs fit; the
-  // last tier has one warp per tile, a quarter of the atoms
-  if (tier >= 2) return launch<256, 512, 1, SL, 8, kDens, kStats, kMasked, 4>(jobs, n_jobs, R, max_np, st);
-  if (tier == 1) return launch<SL == 2 ? 320 : 352, SL == 2 ? 512 : 704, 4, SL, 8, kDens, kStats, kMasked, SL == 2 ? 4 : 2>(jobs, n_jobs, R, max_np, st);
+  // Denser slabs, or coarser voxels: as much staging as three and as two CTAs per SM leave (four with two
+  // slices per step, whose window entries are smaller), then one warp per patch, and at last a window that holds
+  // all of its slabs.  With 352 / 704 atoms at two CTAs and then a warp per patch, 400k atoms of two interpenetrating
+  // bcc cells at 1.2 A voxels took 1.98 ms (0.84 with slabs per warp before, 0.89 now), 0.6 A 2.71 (2.31, 2.34), 800k of
+  // two fcc cells at 0.72 A 4.76 (2.20, 1.75), 400k fcc atoms at 0.9 A 0.83 (0.83, 0.69).
+  if (tier >= 4) return launch<256, 1024, 1, SL, 8, kDens, kStats, kMasked, 2>(jobs, n_jobs, R, max_np, st);
+  if (tier == 3) return launch<256, 512, 1, SL, 8, kDens, kStats, kMasked, SL == 2 ? 4 : 3>(jobs, n_jobs, R, max_np, st);
+  if constexpr (SL == 4) {
+    if (tier == 2) return launch<416, 960, 4, SL, 8, kDens, kStats, kMasked, 2>(jobs, n_jobs, R, max_np, st);
+    if (tier == 1) return launch<288, 608, 4, SL, 8, kDens, kStats, kMasked, 3>(jobs, n_jobs, R, max_np, st);
+  } else {
+    if (tier == 2) return launch<512, 1024, 4, SL, 8, kDens, kStats, kMasked, 2>(jobs, n_jobs, R, max_np, st);
+    if (tier == 1) return launch<320, 512, 4, SL, 8, kDens, kStats, kMasked, 4>(jobs, n_jobs, R, max_np, st);
+    return launch<192, 384, 4, SL, 8, kDens, kStats, kMasked, 4>(jobs, n_jobs, R, max_np, st);
+  }
   if constexpr (SL == 4 && !kStats) {
     switch (variant) {
       case 1: return launch<160, 288, 4, SL, 8, kDens, kStats, kMasked, kField32Blocks>(jobs, n_jobs, R, max_np, st);

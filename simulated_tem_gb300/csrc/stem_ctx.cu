@@ -59,7 +59,7 @@ struct st_ctx {
   int64_t last_kept = 0;       // kept atoms of the previous call: sizes the next one
   bool fp32_general = false;   // STEM_FP32_KERNEL=general: always use k_column_fp32
   bool fp64_general = false;   // STEM_FP64_KERNEL=general: always use k_column_fp64
-  int min_slab_tier = 0;       // STEM_RING_SLABS=192 or 256: start the slab ring at that capacity
+  int min_slab_tier = 0;       // STEM_RING_SLABS: start the slab ring at that tier
   int last_column_kernel = 0;  // 1 general FP32, 2 slab-ring FP32, 3 general FP64, 4 slab-ring FP64
   int tune_mode = ST_TUNE_AUTO;
   std::map<uint64_t, int> ring_tuned;  // (pass kind, image and link-cell shape) -> fastest slab-ring variant
@@ -754,7 +754,7 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     const int dims[6] = {g->Mx, g->My, g->Mz, g->Ex, g->Ey, g->Ez};
     for (int d : dims) key = key * 1000003ull + (uint64_t)d;
   }
-  int big = c->min_slab_tier;  // slab tier: 128, 192, 256 atoms
+  int big = c->min_slab_tier;  // slab tier
   if (auto it = c->ring_big.find(key); it != c->ring_big.end()) big = std::max(big, it->second);
   // with_bin false: the column phase only, on the binning already in place
   auto enqueue = [&](bool capturing, bool with_bin) -> cudaError_t {
@@ -840,10 +840,9 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
       cap = (int64_t)c->h_counters[0] + (int64_t)c->h_counters[0] / 8 + 1024;  // grow and redo
       continue;
     }
-    while (ring_ok && c->h_counters[4] != 0 && big < 2) {
-      // a slab held more atoms than this tier stages: the column phase again with the next
-      // (192, then 256 atoms), and this context keeps it for these kinds of pass on images
-      // of this shape
+    while (ring_ok && c->h_counters[4] != 0 && big < (fp32 ? kField32Tiers : kField64Tiers) - 1) {
+      // a slab or a step's window held more atoms than this tier stages: the column phase again with the
+      // next, and this context keeps it for these kinds of pass on images of this shape
       ++big;
       c->ring_big[key] = big;
       cudaMemsetAsync(c->s.counters + 2, 0, 4 * sizeof(unsigned long long), st);
@@ -948,7 +947,9 @@ extern "C" int st_create(st_ctx** out, int device) {
   const char* kv64 = std::getenv("STEM_FP64_KERNEL");
   c->fp64_general = kv64 && std::strcmp(kv64, "general") == 0;
   const char* ks = std::getenv("STEM_RING_SLABS");
-  c->min_slab_tier = !ks ? 0 : std::strcmp(ks, "256") == 0 ? 2 : std::strcmp(ks, "192") == 0 ? 1 : 0;
+  if (ks)
+    for (int i = 0; i < kField32Tiers; ++i)
+      if (std::strcmp(ks, kSlabTierNames[i]) == 0) c->min_slab_tier = i;
   if (const char* kb = std::getenv("STEM_SAMPLE_BYTES")) c->sample_limit = (size_t)std::strtoull(kb, nullptr, 10);
   std::vector<long long> gauss(kGauss64Size);
   gauss64_table(gauss.data());
