@@ -71,8 +71,9 @@ struct FieldRange {
   double* rho64 = nullptr;
   int64_t origin = 0;       // index of the workspace's first sample in the batch's sample sequence
   int patch_lo = 0, patch_hi = 0;
-  int n_chunks = 1;         // per patch: ceil(deepest image / chunk)
-  int chunk = 0;            // slices per unit, a multiple of 4
+  int deepest = 1;          // slices of the deepest image
+  int n_chunks = 1;         // per patch: ceil(deepest / chunk)
+  int chunk = 0;            // slices per unit, a multiple of 4 (split_depth)
   int job_lo = 0, n_jobs = 0;  // the range's jobs in the call's job table
   bool four = true;         // four slices per step (else two)
   int64_t rho_at = 0;       // where rho starts in the workspace, in values
@@ -80,7 +81,7 @@ struct FieldRange {
   // patches and samples are then counted along this list, and the split in depth follows the number
   const int* list = nullptr;
   const unsigned long long* n_list = nullptr;
-  int slots = 0;            // units that the GPU works on at a time
+  int slots = 1;            // units that the GPU works on at a time
   unsigned* work = nullptr;  // units handed out: zero before the field kernel, zeroed again by the integrator
   const unsigned long long* counters = nullptr;
   int64_t cap = 0;
@@ -90,15 +91,14 @@ struct FieldRange {
 // Splits the patches of a batch into ranges of at most `samples` samples, cut at multiples of
 // `align` patches of an image.
 template <typename Job>
-void field_ranges(const Job* jobs, int n_jobs, int patches, int64_t samples, int align, int chunk, int deepest,
+void field_ranges(const Job* jobs, int n_jobs, int patches, int64_t samples, int align, int deepest,
                   std::vector<FieldRange>& out) {
   out.clear();
   int job = 0;
   for (int lo = 0; lo < patches;) {
     FieldRange R;
     R.patch_lo = lo;
-    R.chunk = chunk;
-    R.n_chunks = (deepest + chunk - 1) / chunk;
+    R.deepest = R.chunk = deepest;
     auto end_of = [&](int j) { return j + 1 < n_jobs ? jobs[j + 1].patch_base : patches; };
     while (end_of(job) <= lo) ++job;
     R.origin = jobs[job].sample_base + (int64_t)(lo - jobs[job].patch_base) * jobs[job].p.Mz * 32;
@@ -119,26 +119,34 @@ void field_ranges(const Job* jobs, int n_jobs, int patches, int64_t samples, int
 }
 
 // Slices per unit of work (a multiple of 4) of `tiles` tiles up to `deepest` slices deep, `slots` of
-// which the GPU works on at a time, when a unit costs `fixed` slices beside its own (the slabs it
-// stages before its first step): the number of pieces with the shortest waves of units.  The FP32
-// field's units, a CTA each, end together, so that whole waves count: on the 128k-atom image (435
-// tiles, 160 slices) 32 slices in 2.9 waves instead of 20 in 4.6.  The FP64 field's, a warp each, differ,
-// and up to two waves of them wait for the longest, more even out: the same image with density (1653
-// patches) 4766 us with 160 slices in 0.9 waves, 4512 with 40 in 3.6, 4352 with 20 in 7.2, 4530 with 8.
+// which the GPU works on at a time (the CTAs of the instance that runs), when a unit costs `fixed` slices beside
+// its own (the slabs it stages before its first step): of up to kPieces pieces the number with the shortest waves
+// of units, the last one partly filled.  In the FP32 field a unit, a CTA each, that is left alone in its SM at the
+// end runs faster, which leaves a tail of 0.7 waves: over 28 images and instances (45 to 2,556 tiles, 40 to 240 slices, one
+// to five CTAs per SM) the pieces are within 1.5 % of the fastest in the mean, 5 % at worst; whole
+// waves of five CTAs, whatever the instance, 10 and 43 % (648 tiles of 120 slices, four CTAs: 1.21 ms in one piece,
+// 0.87 in five).  The FP64 field's units, a warp each, differ, and up to two waves of them wait for the
+// longest, more even out: 128k atoms with density (1653 patches, 160 slices) 4766 us with 160 slices in 0.9 waves,
+// 4512 with 40 in 3.6, 4352 with 20 in 7.2, 4530 with 8.
 constexpr int kPieces = 64;
 struct DepthRule {
   int fixed;
-  bool whole_waves;
+  float tail;
+  bool two_whole;  // up to two waves are whole ones
 };
-constexpr DepthRule kRule32{8, true}, kRule64{1, false};
+constexpr DepthRule kRule32{4, 0.7f, false}, kRule64{1, 0.5f, true};
 template <typename F>
 FP_HD F depth_cost(int64_t tiles, int deepest, int slots, DepthRule rule, int pieces, int& chunk) {
   chunk = ((deepest + pieces - 1) / pieces + 3) & ~3;
   const F w = (F)(tiles * ((deepest + chunk - 1) / chunk)) / (F)slots;
-  const F waves = rule.whole_waves ? ceil(w) : w <= (F)2.0 ? (F)1.08 * ceil(w) : w + (F)0.5;
+  const F waves = rule.two_whole && w <= (F)2.0 ? (F)1.08 * ceil(w) : w + (F)rule.tail;
   return waves * (F)(chunk + rule.fixed);
 }
-inline int depth_chunk(int64_t tiles, int deepest, int slots, DepthRule rule) {
+// The range split for a kernel whose units are `align` patches and of which `slots` run at a time.
+inline void split_depth(FieldRange& R, int align, int slots, DepthRule rule) {
+  const int deepest = R.deepest;
+  const int64_t tiles = std::max(1, (R.patch_hi - R.patch_lo) / align);
+  R.slots = slots;
   int best = (deepest + 3) & ~3;
   double best_cost = -1;
   for (int pieces = 1; pieces <= (deepest + 3) / 4 && pieces <= kPieces; ++pieces) {
@@ -149,7 +157,8 @@ inline int depth_chunk(int64_t tiles, int deepest, int slots, DepthRule rule) {
       best = chunk;
     }
   }
-  return best;
+  R.chunk = best;
+  R.n_chunks = (deepest + best - 1) / best;
 }
 
 // The images of one group: those that march four slices per step, or two.
@@ -161,11 +170,10 @@ struct FieldGroup {
 
 // The ranges of both groups.  `room(want, least)` gives the workspace's bytes, at least `least` and at most
 // about `want`, or 0; it is asked once, for both groups, since a second answer may be a smaller buffer
-// than the first one's ranges were laid out in.  `chunk(at_once, deepest)`: slices per unit when
-// `at_once` groups of `align` patches are in the workspace together.  False when there is no room.
-template <typename Job, typename Room, typename Chunk>
+// than the first one's ranges were laid out in.  False when there is no room.
+template <typename Job, typename Room>
 bool plan_ranges(const Job* jobs, const FieldGroup (&groups)[2], int align, size_t bytes_per_sample, Room room,
-                 Chunk chunk, std::vector<FieldRange>& out) {
+                 std::vector<FieldRange>& out) {
   out.clear();
   const size_t want = (size_t)std::max(groups[0].samples, groups[1].samples) * bytes_per_sample;
   size_t least = 0;
@@ -179,9 +187,7 @@ bool plan_ranges(const Job* jobs, const FieldGroup (&groups)[2], int align, size
   for (int i = 0; i < 2; ++i) {
     const FieldGroup& g = groups[i];
     if (g.samples == 0) continue;
-    const int64_t at_once = std::min(g.patches, n_room / (32 * (int64_t)g.deepest)) / align;
-    field_ranges(jobs + g.job_lo, g.n_jobs, (int)g.patches, n_room, align,
-                 chunk(std::max<int64_t>(1, at_once), g.deepest), g.deepest, part);
+    field_ranges(jobs + g.job_lo, g.n_jobs, (int)g.patches, n_room, align, g.deepest, part);
     for (FieldRange& R : part) {
       R.job_lo = g.job_lo;
       R.n_jobs = g.n_jobs;

@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(W_::NW * 32, kMinBlocks)
   int chunk = R.chunk, n_chunks = R.n_chunks, units = R.units() / NW;
   if constexpr (kMasked) {
     const int n = listed_patches(R, 4), deep = jobs[0].p.Mz;
-    chunk = warp_depth_chunk((n + 3) / 4, deep, R.slots, kRule32);
+    chunk = warp_depth_chunk((n + NW - 1) / NW, deep, R.slots, kRule32);
     n_chunks = (deep + chunk - 1) / chunk;
     units = n / NW * n_chunks;
   }
@@ -945,12 +945,13 @@ cudaError_t launch_integrate(const ColumnJob* jobs, int n_jobs, const FieldRange
 }
 
 template <int CAP, int WCAP, int NW, int SL, int TX, bool kDens, bool kStats, bool kMasked, int B>
-cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, int max_np, cudaStream_t st) {
+cudaError_t launch(const ColumnJob* jobs, int n_jobs, FieldRange R, int max_np, cudaStream_t st) {
   static_assert((sizeof(Smem<CAP, WCAP, NW, SL>) + 1024) * B <= 232448, "shared memory of B CTAs");
   using W = Smem<CAP, WCAP, NW, SL>;
   auto kernel = k_field32<W, kCPL, TX, kDens, kStats, kMasked, B>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(W));
   if (e != cudaSuccess) return e;
+  split_depth(R, NW, sm_count() * B, kRule32);
   const int grid = std::max(1, std::min(sm_count() * B, R.list ? R.patch_hi - R.patch_lo : R.units() / NW));
   ++launch_count();
   kernel<<<grid, NW * 32, sizeof(W), st>>>(jobs, n_jobs, R);

@@ -732,12 +732,13 @@ __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict
 }
 
 template <int CAPS, int SL, bool kDens, bool kMasked, int B>
-cudaError_t launch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, const long long* T, cudaStream_t st) {
+cudaError_t launch(const ColumnJob* jobs, int n_jobs, FieldRange R, const long long* T, cudaStream_t st) {
   const size_t smem = sizeof(WarpSmem<CAPS, SL>) * kWarps;
   auto kernel = k_field64<CAPS, SL, kDens, kMasked, B>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int grid = sm_count() * B;
+  split_depth(R, 1, kWarps * grid, kRule64);
   if (!R.list) grid = std::max(1, std::min(grid, (R.units() + kWarps - 1) / kWarps));
   ++launch_count();
   kernel<<<grid, kWarps * 32, smem, st>>>(jobs, n_jobs, R, T);

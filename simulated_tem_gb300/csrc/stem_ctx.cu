@@ -676,12 +676,8 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     const size_t per = (dens ? 3 : 2) * (fp32 ? sizeof(float) : sizeof(double));
     cudaError_t we = cudaSuccess;
     auto room = [&](size_t want, size_t least) { return sample_workspace(c, want, least, we); };
-    const int slots = sm_count() * (fp32 ? kField32Blocks : 4 * kField64Blocks);
-    auto chunk = [&](int64_t at_once, int deep) {  // (of a tile-masked image the kernel decides)
-      return depth_chunk(at_once, deep, slots, fp32 ? kRule32 : kRule64);
-    };
     // (patches of an FP32 tile stay together)
-    planned = plan_ranges(cj.data(), groups, fp32 ? 4 : 1, per, room, chunk, ranges);
+    planned = plan_ranges(cj.data(), groups, fp32 ? 4 : 1, per, room, ranges);
     if (we != cudaSuccess) return cuda_fail(c, we, "allocating field samples");
     if (masked && planned) {  // (st_image_device_masked images one)
       wanted_tiles = (int)(groups[0].patches + groups[1].patches) / (fp32 ? 4 : 1);
@@ -690,7 +686,6 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
       for (FieldRange& R : ranges) {
         R.list = c->d_list;
         R.n_list = c->s.counters + 6;
-        R.slots = slots;
       }
     }
   }

@@ -42,11 +42,13 @@ int main() {
       return held;
     };
     std::vector<stem::FieldRange> out;
-    CHECK(stem::plan_ranges(jobs.data(), g, align, per, room, [](int64_t, int) { return 8; }, out));
+    CHECK(stem::plan_ranges(jobs.data(), g, align, per, room, out));
     int next[2] = {0, 0};
-    for (const stem::FieldRange& R : out) {
+    for (stem::FieldRange& R : out) {
+      stem::split_depth(R, align, 1 + below(3000), trial % 5 ? stem::kRule32 : stem::kRule64);
+      CHECK(R.chunk >= 4 && R.chunk % 4 == 0 && R.n_chunks * R.chunk >= R.deepest && (R.n_chunks - 1) * R.chunk < R.deepest);
       const int i = R.four ? 0 : 1;
-      CHECK(R.patch_lo == next[i] && R.patch_hi > R.patch_lo && R.n_chunks * R.chunk >= g[i].deepest);
+      CHECK(R.patch_lo == next[i] && R.patch_hi > R.patch_lo && R.deepest == g[i].deepest);
       CHECK(R.job_lo == g[i].job_lo && R.n_jobs == g[i].n_jobs);
       next[i] = R.patch_hi;
       int64_t end = 0;  // samples of the range, from the workspace's start
@@ -70,7 +72,7 @@ int main() {
   g[0].patches = 4;
   g[0].samples = 4 * 320;
   g[0].deepest = 10;
-  CHECK(!stem::plan_ranges(&one, g, 4, 8, [](size_t, size_t) { return (size_t)0; }, [](int64_t, int) { return 8; }, out));
+  CHECK(!stem::plan_ranges(&one, g, 4, 8, [](size_t, size_t) { return (size_t)0; }, out));
   std::puts("ok");
   return 0;
 }
