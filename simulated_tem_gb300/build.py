@@ -64,6 +64,7 @@ def build(verbose=False, ptxas_info=False):
     inc = os.path.join(HERE, "..", "include")
     libs = [
         (LIB, LIB_SOURCES, [os.path.join(CSRC, "internal.h"), os.path.join(CSRC, "field_plan.h"), os.path.join(CSRC, "two_beam64.h"),
+                           os.path.join(CSRC, "two_beam32.h"),
                             os.path.join(CSRC, "parse_number.cuh"),
                             os.path.join(CSRC, "fp64_column.cuh"), os.path.join(CSRC, "slab_ring.cuh"),
                             os.path.join(CSRC, "rounded_product.h"), os.path.join(CSRC, "host_geom.h"),

@@ -49,6 +49,7 @@
 
 #include "internal.h"
 #include "slab_ring.cuh"
+#include "two_beam32.h"
 
 namespace stem {
 namespace field32 {
@@ -736,77 +737,6 @@ __global__ void __launch_bounds__(W_::NW * 32, kMinBlocks)
 // The column integrator
 // ------------------------------------------------------------------------------------------
 
-// The RK4 double step in explicitly rounded operations, on one precession angle
-// (float) or two (float2: .x angle k, .y angle k + 1, one FP32x2 instruction per
-// operation).  Both forms round every operation the same way, so an angle's result
-// does not depend on how many angles share a thread.
-__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ float2 fma_(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float2 mul_(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float add_(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float2 add_(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float neg_(float a) { return -a; }
-__device__ __forceinline__ float2 neg_(float2 a) { return make_float2(-a.x, -a.y); }
-template <typename T>
-__device__ __forceinline__ T bc(float v);
-template <>
-__device__ __forceinline__ float bc<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float2 bc<float2>(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float rsq_(float a) { return rsqrtf(a); }
-__device__ __forceinline__ float2 rsq_(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
-
-struct Sample {
-  float c0, cgr, cgi;
-};
-
-// d/dz (phi_0, phi_g) of the reference's two-beam equations (:2375-2380), phases as
-// (Re phi_0, Im phi_0, Re phi_g, Im phi_g)
-template <typename T>
-__device__ __forceinline__ void deriv(const Sample& s, T a, const T* ph, T* d) {
-  const T c0 = bc<T>(s.c0), cgr = bc<T>(s.cgr), cgi = bc<T>(s.cgi), ca = add_(c0, a);
-  d[0] = fma_(neg_(cgr), ph[3], fma_(neg_(cgi), ph[2], mul_(neg_(c0), ph[1])));
-  d[1] = fma_(neg_(cgi), ph[3], fma_(cgr, ph[2], mul_(c0, ph[0])));
-  d[2] = fma_(neg_(ca), ph[3], fma_(neg_(cgr), ph[1], mul_(cgi, ph[0])));
-  d[3] = fma_(ca, ph[2], fma_(cgi, ph[1], mul_(cgr, ph[0])));
-}
-
-// One RK4 double step over samples (z-2, z-1, z) with weights dz/3, 2dz/3 (:2389-2464).
-template <typename T>
-__device__ __forceinline__ void rk4(const Sample& s0, const Sample& s1, const Sample& s2, T a, float dzf, T* ph) {
-  T d[4], p1[4], q[4];
-  const T dz = bc<T>(dzf), dz3 = bc<T>(dzf / 3.f), dz23 = bc<T>(2.f * dzf / 3.f), dz2 = bc<T>(2.f * dzf);
-  deriv(s0, a, ph, d);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    p1[i] = fma_(d[i], dz3, ph[i]);
-    q[i] = fma_(d[i], dz, ph[i]);
-  }
-  deriv(s1, a, q, d);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    q[i] = fma_(d[i], dz, ph[i]);
-    p1[i] = fma_(d[i], dz23, p1[i]);
-  }
-  deriv(s1, a, q, d);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    q[i] = fma_(d[i], dz2, ph[i]);
-    p1[i] = fma_(d[i], dz23, p1[i]);
-  }
-  deriv(s2, a, q, d);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) ph[i] = fma_(d[i], dz3, p1[i]);
-}
-
-template <typename T>
-__device__ __forceinline__ void renormalise(T* ph) {
-  const T inv = rsq_(fma_(ph[3], ph[3], fma_(ph[2], ph[2], fma_(ph[1], ph[1], mul_(ph[0], ph[0])))));
-#pragma unroll
-  for (int i = 0; i < 4; ++i) ph[i] = mul_(ph[i], inv);
-}
-
 // NH angle pairs of one column (T = float: one angle), |phi_g|^2 to out[0 ..].  The equations are
 // linear, so the reference's renormalisation after every double step (:2466-2472) only scales
 // phi: it is done every 8 steps and at the end (every step when a step could grow phi by more
@@ -827,7 +757,10 @@ __device__ __forceinline__ void integrate(const ColumnParams& p, const float2* _
   };
   Sample s0 = sample(0);
   int n = 0;
-#pragma unroll 4
+  // (1.2M atoms, one angle, 165 us with the steps' parts added one by one, 150 now; density, 128k atoms, 55 and 52,
+  // 59 with eight steps unrolled)
+  constexpr int kUnroll = kDens ? 2 : 8;
+#pragma unroll kUnroll
   for (int z = 2; z <= p.Mz; z += 2) {  // the last sample of an even column is the first (:1898-1899)
     const Sample s1 = sample(z - 1), s2 = sample(z < p.Mz ? z : 0);
 #pragma unroll
