@@ -89,8 +89,12 @@ typedef struct st_stats {
   double ms_column;    /* device time of the column kernel (ms) */
   int32_t column_kernel; /* 1 general FP32, 2 slab-ring FP32, 3 general FP64, 4 slab-ring FP64 (the
                             slab ring for at least one image) */
-  int32_t ring_variant;  /* occupancy variant of the last slab-ring launch, -1 if none ran */
-  int32_t ring_slab_atoms; /* staging capacity per slab of the last slab-ring launch (0 if none ran) */
+  int32_t ring_variant;  /* tuning variant in force for the last slab-ring launch, -1 if none ran; 0 where all its
+                            images march two slices per step (voxels deeper than 0.7 sigma), which has one */
+  int32_t ring_slab_atoms; /* staging class of the last slab-ring launch, 0 if none ran: 96 or 128 as the variant's
+                              name says, 192 and 256 the larger tiers of dense images.  It names about what a
+                              patch of 8 x 4 columns may hold of a slab; the FP32 kernels stage 160, 192, 288 and
+                              416 atoms (two slices per step: 192, 320, 512) per tile of four patches */
   int32_t n_launches;    /* kernels the call launched (all attempts; autotuning trials included) */
 } st_stats;
 
@@ -120,7 +124,8 @@ int st_image_device(st_ctx* ctx, const st_geom* geom, const double* d_x, int64_t
 
 /* Launch tuning of the slab-ring FP32 kernel.  Its variants differ in the warp's
  * patch (8 x 4, 4 x 8 or 16 x 2 pixel columns), the slab capacity of
- * the first staging tier (128 or 96 atoms) and with it the CTAs per SM; the
+ * the first staging tier (named 128 or 96 by a patch's share of the tile's 192 or
+ * 160 atoms) and with it the CTAs per SM; the
  * images of variants of one patch shape are identical, those of different
  * shapes agree to FP32 rounding (their atoms are summed in different orders).
  * ST_TUNE_AUTO (the default): the first pass of each kind (several angles or

@@ -786,9 +786,11 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
       bool done = false;
       if (!capturing) {  // a recorded launch replays the eager run's variant
         v = 0;
-        if (c->tune_mode >= 0 && fp32) {
+        // (the FP64 path and the FP32 steps of two slices have one variant)
+        const bool variants = fp32 && groups[0].samples > 0;
+        if (c->tune_mode >= 0 && variants) {
           v = c->tune_mode;
-        } else if (c->tune_mode == ST_TUNE_AUTO && !stats && fp32) {  // the FP64 path has one variant
+        } else if (c->tune_mode == ST_TUNE_AUTO && !stats && variants) {
           auto it = c->ring_tuned.find(key);
           if (it != c->ring_tuned.end()) {
             v = it->second;

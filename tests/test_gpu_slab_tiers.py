@@ -63,3 +63,23 @@ def test_dense_images_stay_on_the_ring(M, reps):
     finally:
         c.close()
         general.close()
+
+
+def test_two_slices_per_step_have_one_variant():
+    """An image of deep voxels alone is not tuned, and reports variant 0 whatever was asked for."""
+    cell = synth.make_cell(100, 100, 8, 13, n_voids=2, void_radius=(5.0, 8.0))
+    t, x, _ = imaging.d2bi_condition(cell.a_super, synth.A0_FE, (0, 0, 1), (1, 1, 0), cell.pos, sg=0.01, M=(4, 1))
+    G, aa = t.image_geometry(len(x))
+    assert ((G.ix1 - G.ix0 + 7) // 8) * ((G.iy1 - G.iy0 + 3) // 4) >= 4096  # large enough to tune
+    c = context()
+    try:
+        c.image(G, x, aa, flags=_lib.ST_FLAG_FP32)  # finds the slab tier
+        launches = []
+        for mode in (_lib.ST_TUNE_AUTO, _lib.ST_TUNE_OFF, 3):
+            c.tune(mode)
+            c.image(G, x, aa, flags=_lib.ST_FLAG_FP32)
+            launches.append(c.stats().n_launches)
+            assert c.stats().column_kernel == 2 and c.stats().ring_variant == 0
+        assert len(set(launches)) == 1
+    finally:
+        c.close()
