@@ -442,7 +442,7 @@ __device__ __noinline__ bool field_tile(const ColumnParams& p, WarpSmem<CAPS, SL
     bool ok = true;
     while (ring_hi < need_hi && ok) {
       ++ring_hi;
-      ok = load_slab<CAPS, true, true>(p, G, ring_hi, W, lane);
+      ok = load_slab<CAPS>(p, G, ring_hi, W, lane);
     }
     if (!ok) {
       if (lane == 0) atomicExch(&p.counters[4], 1ull);

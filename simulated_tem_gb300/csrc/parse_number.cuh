@@ -140,7 +140,6 @@ struct Pow5 {
       lo[kPow5 + k] = b;
       e[kPow5 + k] = -sh;
       // q = -k: the first 128 bits of 1 / 5^k by long division
-      const int bits = 128 - sh;   // of 5^k
       uint64_t qh = 0, ql = 0, rh = 0, rl = 1;  // quotient, remainder (below 5^k)
       int made = 0, p = 0;         // quotient bits from its leading one on; position of the last bit
       if (k == 0) {
@@ -164,7 +163,6 @@ struct Pow5 {
           ++made;
         }
       }
-      (void)bits;
       hi[kPow5 - k] = qh;
       lo[kPow5 - k] = ql;
       e[kPow5 - k] = -p;

@@ -100,20 +100,17 @@ __device__ __forceinline__ bool slab_append(float4* P, int* GI, int& n, bool kee
 // Gather slab u (its cells in the patch footprint, atoms within 3 sigma of the
 // patch rectangle) into its ring slot and order it by z bin in place; false
 // when it holds more than CAPS atoms.
-// kCellCode: the fourth float of an entry holds the atom's unwrapped cell relative to the warp's
-// reference cells, (ux - ux_ref + 8) | (uy - uy_ref + 8) << 8 (the FP64 kernel's exact
-// distances need it), instead of its phase.  WS: any warp-memory layout with the slab
-// arrays p, gi, bin and count.
+// The fourth float of an entry holds the atom's unwrapped cell relative to the warp's
+// reference cells, (ux - ux_ref + 8) | (uy - uy_ref + 8) << 8 (exact distances need it).  WS: any
+// warp-memory layout with the slab arrays p, gi, bin and count.
 //
 // The footprint is rows uy of x runs (a run ends where x wraps): segments of consecutive
-// atoms.  With kJoined and up to 8 segments, the lanes look up all segment ranges at once,
+// atoms.  Up to 8 segments, the lanes look up all segment ranges at once,
 // join them into one index space (the slot's bin array, free until the sort, holds the
 // table) and gather two 32-lane rounds at a time; otherwise row by row, one round at a
-// time (with more than one angle per pass the march's phases leave no registers for a
-// second round: measured, 16 angles spilled more and ran 10 % slower).  Both
-// routes visit the atoms in the same order (rows, runs, atoms), so the slab's contents
+// time.  Both routes visit the atoms in the same order (rows, runs, atoms), so the slab's contents
 // and order do not depend on the route.
-template <int CAPS, bool kCellCode = false, bool kJoined = true, typename WS>
+template <int CAPS, typename WS>
 __device__ bool load_slab(const ColumnParams& p, const Geo& G, int u, WS& W, int lane) {
   const int cz = pos_mod(u, p.Ez);
   const int slot = u & (kRing - 1);
@@ -124,7 +121,7 @@ __device__ bool load_slab(const ColumnParams& p, const Geo& G, int u, WS& W, int
   static_assert(4 * kMaxSeg + 1 <= kBins + 1, "the segment table lives in a slot's bin array");
   const int k_lo = floor_div(G.ux_lo, p.Ex), k_hi = floor_div(G.ux_hi, p.Ex);
   const int n_run = max(0, k_hi - k_lo + 1), n_seg = max(0, G.uy_hi - G.uy_lo + 1) * n_run;
-  if (kJoined && n_seg >= 1 && n_seg <= kMaxSeg) {
+  if (n_seg >= 1 && n_seg <= kMaxSeg) {
     int* seg = W.bin[slot];  // per segment: first index, first atom, x shift, row; then the total
     int len = 0, a_lo = 0, shift = 0, uy = 0;
     if (lane < n_seg) {
@@ -172,7 +169,7 @@ __device__ bool load_slab(const ColumnParams& p, const Geo& G, int u, WS& W, int
         rec[r] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < total) {
           locate(i, j[r], sh, y);
-          keep[r] = slab_candidate<kCellCode>(p, G, j[r], sh, y, rec[r]);
+          keep[r] = slab_candidate<true>(p, G, j[r], sh, y, rec[r]);
         }
       }
 #pragma unroll
@@ -191,7 +188,7 @@ __device__ bool load_slab(const ColumnParams& p, const Geo& G, int u, WS& W, int
           const int j = b + lane;
           bool keep = false;
           float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (j < a_hi) keep = slab_candidate<kCellCode>(p, G, j, shift, uy, rec);
+          if (j < a_hi) keep = slab_candidate<true>(p, G, j, shift, uy, rec);
           if (!slab_append<CAPS>(P, GI, n, keep, rec, j, lane)) return false;
         }
       }

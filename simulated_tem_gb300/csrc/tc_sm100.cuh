@@ -19,11 +19,6 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// Byte offset of element (row, k) of a K-major non-swizzled tile with Kc elements per row.
-__device__ __forceinline__ uint32_t tile_offset(int row, int k, int Kc) {
-  return (uint32_t)((row >> 3) * (Kc * 16) + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
-}
-
 // Shared-memory matrix descriptor: start address, leading (K) and stride (M/N) byte
 // offsets, descriptor version 1, no swizzle.
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
@@ -139,9 +134,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
       : "memory");
 }
 
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 __device__ __forceinline__ void fence_before_sync() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -159,20 +151,8 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// Eight consecutive FP32 accumulator columns of this thread's TMEM lane (warp w of a
-// warpgroup reads lanes 32w .. 32w + 31).
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-  uint32_t r[8];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// 32 consecutive FP32 accumulator columns of this thread's TMEM lane, without the wait:
+// 32 consecutive FP32 accumulator columns of this thread's TMEM lane (warp w of a
+// warpgroup reads lanes 32w .. 32w + 31), without the wait:
 // several loads may be in flight before one tmem_wait_ld().
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
   asm volatile(
