@@ -106,3 +106,35 @@ def test_fp64_coarse_voxels_of_a_dilute_gas(ctx, general, side, kernel):
     assert ctx.stats().column_kernel == kernel and ctx.stats().n_kept == len(x)
     assert (want > 1e-4).sum() >= 20
     assert np.abs(got - want).max() <= FP64_TOL
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("density", [False, True])
+def test_small_windows_on_the_field_kernels(ctx, general, fp32, density):
+    """Pixel windows smaller than a patch, of a patch, of a tile and one more, in the whole image's link cells (a
+    geometry made for a small window has cells too narrow for the field kernels)."""
+    t, _, x = setup_both(cell_of((9, 10, 6)), sg=0.01, density=density)
+    G, aa = t.image_geometry(len(x))
+    flags = _lib.ST_FLAG_FP32 if fp32 else 0
+    for ix0, iy0, dx, dy in ((0, 0, 1, 1), (3, 2, 7, 3), (1, 5, 8, 4), (0, 1, 9, 5), (2, 0, 16, 8), (1, 1, 17, 9),
+                             (G.Mx - 1, G.My - 1, 1, 1), (G.Mx - 9, 0, 9, G.My)):
+        G.ix0, G.ix1, G.iy0, G.iy1 = ix0, ix0 + dx, iy0, iy0 + dy
+        got, want = ctx.image(G, x, aa, flags=flags), general.image(G, x, aa, flags=flags)
+        assert ctx.stats().column_kernel == (2 if fp32 else 4) and general.stats().column_kernel == (1 if fp32 else 3)
+        assert np.abs(got - want).max() <= (FP32_TOL if fp32 else FP64_TOL)
+        inside = np.zeros(got.shape, dtype=bool)
+        inside[ix0:ix0 + dx, iy0:iy0 + dy] = True
+        assert (got[inside] != 0).any() and not got[~inside].any()
+
+
+@pytest.mark.parametrize("n_prec", [1, 3])
+def test_steps_long_enough_to_renormalise_each(ctx, general, n_prec):
+    """2 dz (b0 + bg + |a|) of 1 and more: both integrators renormalise after every double step."""
+    t, _, x = setup_both(cell_of((6, 5, 6)), sg=0.0)
+    G, _ = t.image_geometry(len(x))
+    aa = (np.array([1.05, -1.2, 1.4])[:n_prec]) / (2 * G.deltaz)
+    assert (2 * G.deltaz * (G.b0 + G.bg + np.abs(aa)) >= 1).all()
+    for flags, tol in ((_lib.ST_FLAG_FP32, FP32_TOL), (0, FP64_TOL)):
+        got, want = ctx.image(G, x, aa, flags=flags), general.image(G, x, aa, flags=flags)
+        assert ctx.stats().column_kernel == (2 if flags else 4)
+        assert np.abs(got - want).max() <= tol * n_prec
