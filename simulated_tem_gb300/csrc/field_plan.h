@@ -81,6 +81,7 @@ struct FieldRange {
   // patches and samples are then counted along this list, and the split in depth follows the number
   const int* list = nullptr;
   const unsigned long long* n_list = nullptr;
+  int per_item = 1;         // patches per listed tile (2: the left or right half of an FP32 tile)
   int slots = 1;            // units that the GPU works on at a time
   unsigned* work = nullptr;  // units handed out: zero before the field kernel, zeroed again by the integrator
   const unsigned long long* counters = nullptr;

@@ -193,14 +193,18 @@ __device__ __forceinline__ const ColumnJob& field_patch(const ColumnJob* __restr
   return jobs[lo];
 }
 #ifdef __CUDACC__
-// A tile-masked image: the patches of the range that are listed, `align` per tile, and their slices per
-// unit, by one warp (every lane gets them).
-__device__ __forceinline__ int listed_patches(const FieldRange& R, int align) {
-  const int64_t n = (int64_t)*R.n_list * align - R.patch_lo;
+// A tile-masked image: the patches of the range that are listed; the patch at place `patch` of the list; slices
+// per unit, by one warp (every lane gets them).
+__device__ __forceinline__ int listed_patches(const FieldRange& R) {
+  const int64_t n = (int64_t)*R.n_list * R.per_item - R.patch_lo;
   return (int)max((int64_t)0, min(n, (int64_t)(R.patch_hi - R.patch_lo)));
 }
-__device__ __forceinline__ int listed_patch(const FieldRange& R, int align, int patch) {
-  return R.list[patch / align] * align + patch % align;
+__device__ __forceinline__ int listed_patch(const FieldRange& R, const ColumnParams& p, int patch) {
+  if (R.per_item == 2) {  // a half: patches h and h + 2 of its tile
+    const int i = R.list[patch >> 1], across = 2 * ((p.ix1 - p.ix0 + 15) / 16), hx = i % across;
+    return 4 * (i / across * (across / 2) + (hx >> 1)) + (hx & 1) + 2 * (patch & 1);
+  }
+  return R.list[patch / R.per_item] * R.per_item + patch % R.per_item;
 }
 __device__ __forceinline__ int warp_depth_chunk(int64_t tiles, int deepest, int slots, DepthRule rule) {
   const int lane = threadIdx.x & 31;
@@ -225,10 +229,10 @@ __device__ __forceinline__ int warp_depth_chunk(int64_t tiles, int deepest, int 
   return chunk;
 }
 #endif
-// The tiles of tx x ty pixels of a tile-masked image that have a wanted one, to `list`; their number to *count
-// (zero before).
-cudaError_t launch_wanted_tiles(const ColumnJob* d_job, int tiles, int tx, int ty, int* list, unsigned long long* count,
-                                cudaStream_t st);
+// The tiles of tx x ty pixels, `across` of them per row, of a tile-masked image that have a wanted one, to
+// `list`; their number to *count (zero before).
+cudaError_t launch_wanted_tiles(const ColumnJob* d_job, int tiles, int across, int tx, int ty, int* list,
+                                unsigned long long* count, cudaStream_t st);
 inline int sm_count() {
   int dev = 0, sms = 152;
   cudaGetDevice(&dev);
@@ -248,6 +252,7 @@ constexpr const char* kSlabTierNames[kField32Tiers] = {"128", "192", "256", "pat
 constexpr int kField32Blocks = 5;  // CTAs of four warps per SM at tier 0
 cudaError_t launch_field32(const ColumnJob* d_jobs, int n_jobs, const FieldRange& R, int max_np, bool density,
                            bool stats, bool masked, bool four, int variant, int slab_tier, cudaStream_t st);
+bool field32_halves(int mask_T, int variant, int slab_tier);  // a tile-masked launch by halves of tiles
 int ring_variant_count();
 const char* ring_variant_name(int variant);
 int ring_variant_slab(int variant);  // the capacity in the variant's name

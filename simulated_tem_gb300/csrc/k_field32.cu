@@ -292,7 +292,8 @@ __device__ __forceinline__ void patch_column(int x0, int y0, int w, int lane, in
   iy = y0 + wy + lane / TX;
 }
 
-// The slices [z_lo, z_hi) of one tile (NW = 4: its four patches; NW = 1: patch `patch` of it).
+// The slices [z_lo, z_hi) of one tile (NW = 4: its four patches; NW = 2: `patch` and the one below it; NW = 1:
+// patch `patch` of it).
 // Samples of patch w, slice z to out[((w * Mz + z) << 5) + lane].  False when a slab or a step's
 // window overflows.
 //
@@ -309,7 +310,9 @@ __device__ __forceinline__ bool field_tile(const ColumnParams& p, W_& W, int pat
   constexpr bool kSameX = LPG % TX == 0;  // a lane's columns share x
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int grp = lane / LPG;
-  const int tile = patch >> 2, w4 = NW == 1 ? patch & 3 : warp;
+  const int tile = patch >> 2;
+  auto patch_of = [&](int w) { return NW == 1 ? patch & 3 : NW == 2 ? (patch & 1) + 2 * w : w; };  // within the tile
+  const int w4 = patch_of(warp);
   const int tiles_x = (p.ix1 - p.ix0 + kTileX - 1) / kTileX;
   const int x0 = p.ix0 + tile % tiles_x * kTileX, y0 = p.iy0 + tile / tiles_x * kTileY;
   int ix, iy;
@@ -330,7 +333,7 @@ __device__ __forceinline__ bool field_tile(const ColumnParams& p, W_& W, int pat
     sync<NW>();
     patches = 0;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) patches |= W.wcnt[w] ? 1u << w : 0u;
+    for (int w = 0; w < NW; ++w) patches |= W.wcnt[w] ? 1u << patch_of(w) : 0u;
     if (!patches) return true;
   }
 
@@ -712,7 +715,7 @@ __global__ void __launch_bounds__(W_::NW * 32, kMinBlocks)
   }
   int chunk = R.chunk, n_chunks = R.n_chunks, units = R.units() / NW;
   if constexpr (kMasked) {
-    const int n = listed_patches(R, 4), deep = jobs[0].p.Mz;
+    const int n = listed_patches(R), deep = jobs[0].p.Mz;
     chunk = warp_depth_chunk((n + NW - 1) / NW, deep, R.slots, kRule32);
     n_chunks = (deep + chunk - 1) / chunk;
     units = n / NW * n_chunks;
@@ -729,7 +732,7 @@ __global__ void __launch_bounds__(W_::NW * 32, kMinBlocks)
     const int z_lo = unit % n_chunks * chunk, z_hi = min(J.p.Mz, z_lo + chunk);
     if (z_lo >= z_hi) continue;  // an image less deep than the batch's deepest
     const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32;
-    if constexpr (kMasked) patch = listed_patch(R, 4, patch);
+    if constexpr (kMasked) patch = listed_patch(R, J.p, patch);
     if (!field_tile<CPL, TX, kDens, kStats, kMasked>(J.p, W, patch, z_lo, z_hi, (float2*)R.samples + o, R.rho32 + o))
       break;
   }
@@ -811,11 +814,11 @@ __global__ void __launch_bounds__(128) k_integrate32(const ColumnJob* __restrict
   const int lane = threadIdx.x, g = R.patch_lo + blockIdx.x * 4 + threadIdx.y;
   if (g == R.patch_lo && lane == 0) *R.work = 0;  // for the next field kernel
   if ((int64_t)R.counters[0] > R.cap || R.counters[4] != 0 || g >= R.patch_hi) return;
-  if (R.list && g - R.patch_lo >= listed_patches(R, 4)) return;
+  if (R.list && g - R.patch_lo >= listed_patches(R)) return;
   int patch;
   const ColumnJob& J = field_patch(jobs, n_jobs, g, patch);
   const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32 + lane;
-  if (R.list) patch = listed_patch(R, 4, patch);
+  if (R.list) patch = listed_patch(R, J.p, patch);
   int64_t px;
   const bool wanted = patch_pixel<TX>(J.p, patch, lane, px);
   if (!__any_sync(0xffffffffu, wanted)) return;
@@ -908,6 +911,10 @@ cudaError_t dispatch(const ColumnJob* jobs, int n_jobs, const FieldRange& R, int
   // two fcc cells at 0.72 A 4.76 (2.20, 1.75), 400k fcc atoms at 0.9 A 0.83 (0.83, 0.69).
   if (tier >= 4) return launch<256, 1024, 1, SL, 8, kDens, kStats, kMasked, 2>(jobs, n_jobs, R, max_np, st);
   if (tier == 3) return launch<256, 512, 1, SL, 8, kDens, kStats, kMasked, SL == 2 ? 4 : 3>(jobs, n_jobs, R, max_np, st);
+  if constexpr (kMasked)  // halves of tiles (field32_halves)
+    if (tier == 0 && R.per_item == 2)
+      return launch<SL == 2 ? 128 : 112, SL == 2 ? 240 : 208, 2, SL, 8, kDens, kStats, kMasked, 8>(jobs, n_jobs, R,
+                                                                                                 max_np, st);
   if constexpr (SL == 4) {
     if (tier == 2) return launch<416, 960, 4, SL, 8, kDens, kStats, kMasked, 2>(jobs, n_jobs, R, max_np, st);
     if (tier == 1) return launch<288, 608, 4, SL, 8, kDens, kStats, kMasked, 3>(jobs, n_jobs, R, max_np, st);
@@ -950,14 +957,14 @@ int field32_patches(const ColumnParams& p) {
 }
 
 namespace {
-__global__ void __launch_bounds__(256) k_wanted_tiles(const ColumnJob* __restrict__ job, int tiles, int tx, int ty,
-                                                      int* __restrict__ list, unsigned long long* __restrict__ count) {
+__global__ void __launch_bounds__(256) k_wanted_tiles(const ColumnJob* __restrict__ job, int tiles, int across, int tx,
+                                                      int ty, int* __restrict__ list,
+                                                      unsigned long long* __restrict__ count) {
   const ColumnParams& p = job->p;
   const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31;
   bool want = false;
-  if (i < tiles) {
-    const int across = (p.ix1 - p.ix0 + tx - 1) / tx;
-    const int x0 = p.ix0 + i % across * tx, y0 = p.iy0 + i / across * ty;
+  const int x0 = p.ix0 + i % across * tx, y0 = p.iy0 + i / across * ty;
+  if (i < tiles && x0 < p.ix1) {
     const int x1 = min(x0 + tx, p.ix1) - 1, y1 = min(y0 + ty, p.iy1) - 1;
     for (int my = y0 / p.mask_T; my <= y1 / p.mask_T; ++my)
       for (int mx = x0 / p.mask_T; mx <= x1 / p.mask_T; ++mx) want = want || p.tile_mask[my * p.mask_ntx + mx] != 0;
@@ -971,11 +978,18 @@ __global__ void __launch_bounds__(256) k_wanted_tiles(const ColumnJob* __restric
 }
 }  // namespace
 
-cudaError_t launch_wanted_tiles(const ColumnJob* d_job, int tiles, int tx, int ty, int* list, unsigned long long* count,
-                                cudaStream_t st) {
+cudaError_t launch_wanted_tiles(const ColumnJob* d_job, int tiles, int across, int tx, int ty, int* list,
+                                unsigned long long* count, cudaStream_t st) {
   ++launch_count();
-  k_wanted_tiles<<<(tiles + 255) / 256, 256, 0, st>>>(d_job, tiles, tx, ty, list, count);
+  k_wanted_tiles<<<(tiles + 255) / 256, 256, 0, st>>>(d_job, tiles, across, tx, ty, list, count);
   return cudaGetLastError();
+}
+
+// A mask whose tiles are an odd number of 8 pixels wide often wants one half of a 16 x 8 tile: two warps and the
+// atoms about 8 x 8 pixels then (4.8M atoms, 480 slices, 7 % of the tiles of 8 pixels 4.44 ms, by whole tiles 5.73;
+// all of them 49.3 and 44.0: above some 85 % whole tiles would be the better).
+bool field32_halves(int mask_T, int variant, int slab_tier) {
+  return mask_T % 16 != 0 && ring_variant_same(variant) && slab_tier == 0;
 }
 
 int ring_variant_count() { return field32::kVariants; }

@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks)
   if ((int64_t)R.counters[0] > R.cap) return;  // the binning overflowed: the host retries
   int chunk = R.chunk, n_chunks = R.n_chunks, units = R.units();
   if constexpr (kMasked) {
-    const int n = listed_patches(R, 1), deep = jobs[0].p.Mz;
+    const int n = listed_patches(R), deep = jobs[0].p.Mz;
     chunk = warp_depth_chunk(n, deep, R.slots, kRule64);
     n_chunks = (deep + chunk - 1) / chunk;
     units = n * n_chunks;
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks)
     const int z_lo = unit % n_chunks * chunk, z_hi = min(J.p.Mz, z_lo + chunk);
     if (z_lo >= z_hi) continue;  // an image less deep than the batch's deepest
     const int64_t o = J.sample_base - R.origin + (int64_t)patch * J.p.Mz * 32;
-    if constexpr (kMasked) patch = listed_patch(R, 1, patch);
+    if constexpr (kMasked) patch = listed_patch(R, J.p, patch);
     if (!field_tile<CAPS, SL, kDens, kMasked>(J.p, W, patch, z_lo, z_hi, (longlong2*)R.samples + o, (long long*)R.rho64 + o, T,
                                                lane))
       break;
@@ -673,12 +673,12 @@ __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict
   const int lane = threadIdx.x, warp = threadIdx.y, nw = blockDim.y;
   if (blockIdx.x == 0 && warp == 0 && lane == 0) *R.work = 0;  // for the next field kernel
   if ((int64_t)R.counters[0] > R.cap || R.counters[4] != 0) return;
-  if (R.list && (int)blockIdx.x >= listed_patches(R, 1)) return;
+  if (R.list && (int)blockIdx.x >= listed_patches(R)) return;
   int patch;
   const ColumnJob& J = field_patch(jobs, n_jobs, R.patch_lo + blockIdx.x, patch);
   const ColumnParams& p = J.p;
   const int64_t o = J.sample_base - R.origin + (int64_t)patch * p.Mz * 32 + lane;
-  if (R.list) patch = listed_patch(R, 1, patch);
+  if (R.list) patch = listed_patch(R, J.p, patch);
   const int tiles_x = (p.ix1 - p.ix0 + 7) / 8;
   const int ix = p.ix0 + (patch % tiles_x) * 8 + (lane & 7), iy = p.iy0 + (patch / tiles_x) * 4 + (lane >> 3);
   const bool active = ix < p.ix1 && iy < p.iy1;

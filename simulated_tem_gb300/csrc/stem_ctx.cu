@@ -679,9 +679,9 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     // (patches of an FP32 tile stay together)
     planned = plan_ranges(cj.data(), groups, fp32 ? 4 : 1, per, room, ranges);
     if (we != cudaSuccess) return cuda_fail(c, we, "allocating field samples");
-    if (masked && planned) {  // (st_image_device_masked images one)
+    if (masked && planned) {
       wanted_tiles = (int)(groups[0].patches + groups[1].patches) / (fp32 ? 4 : 1);
-      e = ensure(c->d_list, c->cap_list, (size_t)wanted_tiles);
+      e = ensure(c->d_list, c->cap_list, (size_t)wanted_tiles * 2);  // (or halves of tiles)
       if (e != cudaSuccess) return cuda_fail(c, e, "allocating the list of wanted tiles");
       for (FieldRange& R : ranges) {
         R.list = c->d_list;
@@ -761,12 +761,21 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
     }
     if (ce == cudaSuccess) ce = clear_images();
     if (!capturing) cudaEventRecord(c->ev[1], st);
-    if (ring_ok && wanted_tiles > 0 && ce == cudaSuccess) {
-      cudaMemsetAsync(c->s.counters + 6, 0, sizeof(unsigned long long), st);
-      ce = launch_wanted_tiles(d_coljobs, wanted_tiles, fp32 ? 16 : 8, fp32 ? 8 : 4, c->d_list, c->s.counters + 6, st);
-    }
     auto ring_launch = [&](int v) {
       cudaError_t le = cudaSuccess;
+      int per_item = fp32 ? 4 : 1;
+      if (wanted_tiles > 0) {  // (st_image_device_masked images one)
+        const ColumnParams& p = cj[0].p;
+        int across = (p.ix1 - p.ix0 + (fp32 ? 15 : 7)) / (fp32 ? 16 : 8), tiles = wanted_tiles;
+        if (fp32 && field32_halves(p.mask_T, v, big)) {
+          per_item = 2;
+          across *= 2;
+          tiles *= 2;
+        }
+        cudaMemsetAsync(c->s.counters + 6, 0, sizeof(unsigned long long), st);
+        le = launch_wanted_tiles(d_coljobs, tiles, across, fp32 && per_item == 4 ? 16 : 8, fp32 ? 8 : 4, c->d_list,
+                                 c->s.counters + 6, st);
+      }
       for (FieldRange R : ranges) {
         R.samples = c->samples.p;
         R.rho32 = (float*)c->samples.p + R.rho_at;
@@ -774,6 +783,7 @@ int run_images(st_ctx* c, const std::vector<Job>& jobs, int32_t flags, cudaStrea
         R.work = (unsigned*)(c->s.counters + 5);
         R.counters = c->s.counters;
         R.cap = cap;
+        R.per_item = per_item;
         if (le != cudaSuccess) break;
         const ColumnJob* dj = d_coljobs + R.job_lo;
         le = fp32 ? launch_field32(dj, R.n_jobs, R, ring_np, dens, stats, masked, R.four, v, big, st)
