@@ -144,7 +144,7 @@ def path_roofline(peaks, n_acc, n_kept, n_atoms, voxels, voxel_prec, pixels, den
 SWEEP_G = ((1, 1, 0), (2, 0, 0), (2, 1, 1))
 # DRAM bytes (read + write) of the column stage on the 1.2M-atom image, from an ncu capture: k_field32
 # (53.5 MB read + 563.1 MB written: the field samples) and k_integrate32 (622.1 + 4.6 MB)
-COLUMN_TRAFFIC_BYTES = 1.2433e9
+COLUMN_TRAFFIC_BYTES = 1.2415e9
 
 
 def sweep_specs(cell, n_tomo=41, n_prec=16, gs=SWEEP_G):

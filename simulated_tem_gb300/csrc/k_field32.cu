@@ -10,7 +10,7 @@
 //
 // The field kernel: a CTA of four warps owns 16 x 8 pixel columns and a range of slices, each warp 32
 // of the columns (8 x 4, 4 x 8 or 16 x 2: the tuning variants), four slices per step (two where some
-// image's steps of four do not fit the ring).  Instruction issue bounds it (0.65 to 0.7 per cycle and
+// image's steps of four do not fit the ring).  Instruction issue bounds it (0.64 to 0.7 per cycle and
 // sub-partition), then the shared-memory loads of the atoms and the FP32 pipe; so everything that does
 // not depend on the column is done once for the four warps, and an atom's values are loaded for two columns:
 // * The atoms of a link-cell slab (one z cell; a ring of four) within 3 sigma of the tile are
@@ -28,8 +28,8 @@
 //   separable), and per slice the inclusive cutoff dxy^2 <= hmax_k and one FP32x2 multiply-add of the
 //   weight into (cos, sin); the groups' sums are added at the end of the step.
 // Measured on the 1.2M-atom image (566 x 566 x 240): 2.84 ms for the kernel before (a warp's own
-// slabs, two slices per step, the integrator in the same kernel), 2.12 ms field + 0.16 ms integrator
-// now; of the field 0.87 ms are the lists' sums (0.65 at the FP32 pipe's rate), 0.30 the depth terms, 0.29
+// slabs, two slices per step, the integrator in the same kernel), 2.06 ms field + 0.15 ms integrator
+// now; of a field of 2.12 ms 0.87 were the lists' sums (0.65 at the FP32 pipe's rate), 0.30 the depth terms, 0.29
 // the gather, 0.26 the step's fixed cost, 0.16 the lists, 0.13 the exact recheck.  One column per lane
 // ran 2.55 ms (the loads), four columns 2.22, six CTAs per SM instead of five 2.33, a producer warp per CTA
 // 2.55, slabs per warp 2.35.

@@ -29,8 +29,8 @@
 // * The Gaussian itself is a table value times a short polynomial (gauss64): six FP64 operations
 //   for the distance, the rest integers.
 // * A lane then multiplies two 58-bit numbers per atom, and adds two products per slice, six
-//   32 x 32-bit multiply-adds.  An accepted weight lies in [exp(-4.5), 1], so that 2^-58 is no
-//   coarser than FP64, and the sums do not round.
+//   32 x 32-bit multiply-adds.  The sums do not round.  (FP64's spacing of an accepted weight, exp(-4.5) to 1,
+//   is 2^-59 to 2^-53: 2^-58 is finer but for the smallest weights.)
 // Now latency bounds it (12 warps per SM, limited by their staging; 0.45 instructions per cycle and
 // sub-partition), and code size: with two copies of the consuming code, or two atoms per iteration, the
 // instruction fetches cost 128k atoms with density a fifth.
@@ -38,7 +38,7 @@
 // reference's integrator and hypot in every lane, 7.2 with all of this in FP64, 4.35 now; 28k atoms
 // 6.75, 0.83, 0.54; 16k atoms with six precession angles 13.6, 1.32, 0.71.  128k atoms: field 3.95 ms
 // (a third of it the sums, a fifth the tests and the density's nearest atoms, a fifth the Gaussians),
-// integrator 0.20.
+// integrator 0.21.
 //
 // Precision: the Gaussians are within 2.4 units of 2^-53 of the exact value (root mean square 0.57;
 // exp of the rounded d.d / 2 sigma^2, up to 4.5, is within 13.5, 2.1 in the mean square: the rounding of

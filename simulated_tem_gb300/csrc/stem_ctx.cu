@@ -200,7 +200,7 @@ void depth_table(const st_geom* g, int2* tab, const double* fv) {
 
 // Voxels so coarse in depth (more than 0.7 sigma a slice) that a step of four slices, whose lists hold
 // the atoms of any of them, costs the FP32 field more than two steps of two (and twice
-// the shared memory for its window): 4.8M atoms at one sigma a slice 4.75 ms with four, 3.92 with two.
+// the shared memory for its window): 4.8M atoms at one sigma a slice 4.82 ms with four, 3.93 with two.
 bool coarse_slices(const ColumnParams& p) { return p.dz > 0.7 * p.sigma; }
 
 bool four_slices_fit(const st_geom* g) {
