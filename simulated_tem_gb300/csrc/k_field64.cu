@@ -701,17 +701,18 @@ __global__ void __launch_bounds__(256) k_integrate64(const ColumnJob* __restrict
         repeat = repeat && wanted;
       }
       if (__any_sync(0xffffffffu, repeat)) {
-        // the stored samples are rho x and rho, or those times the fixed-point coefficients (in units of
-        // 2^-60 without density)
+        // the stored samples are rho x and rho, or those times the fixed-point coefficients; of an image without
+        // density in units of 2^-60, whatever the others of its batch have
         const double inv = fixed ? __ddiv_rn(1.0, p.fx_a) : 1.0;
         auto coef = [&](int z) {
           const double2 x = X[(int64_t)z << 5];
           const double r = kDens ? RH[(int64_t)z << 5] : 1.0;
           if (!fixed) return S64{kDens ? DM(p.b0, r) : p.b0, DM(p.bg, x.x), DM(p.bg, x.y)};
-          if constexpr (kDens) return S64{DM(r, inv), DM(x.x, inv), DM(x.y, inv)};
+          if (kDens && p.use_density) return S64{DM(r, inv), DM(x.x, inv), DM(x.y, inv)};
           const double u = DM(inv, 0x1p-60);
-          return S64{p.b0, DM(__ll2double_rn(__double_as_longlong(x.x)), u),
-                     DM(__ll2double_rn(__double_as_longlong(x.y)), u)};
+          const long long xr = kDens ? to60(x.x) : __double_as_longlong(x.x),
+                          xi = kDens ? to60(x.y) : __double_as_longlong(x.y);
+          return S64{p.b0, DM(__ll2double_rn(xr), u), DM(__ll2double_rn(xi), u)};
         };
         const double ig = column64(p.Mz, p.dz, a, reach0 + fabs(a), coef);
         if (repeat) part[warp][lane] = ig;

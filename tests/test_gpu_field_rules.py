@@ -45,23 +45,44 @@ def general():
     c.close()
 
 
+def dilute(density, n_prec=1, **options):
+    """A dilute gas in a deep box."""
+    a0 = synth.A0_FE
+    box = np.array([9, 8, 14]) * a0
+    pos = np.random.default_rng(3).uniform(0.0, 1.0, (70, 3)) * box
+    pos[:8] = np.array([[i, j, k] for i in (0, 1 - 1e-9) for j in (0, 1 - 1e-9) for k in (0, 1 - 1e-9)]) * box
+    t, x, _ = imaging.d2bi_condition(np.diag(box), a0, (0, 0, 1), (1, 1, 0), pos, density=density,
+                                     **{"sg": 0.01, **options})
+    G, aa = t.image_geometry(len(x), prec_angle=0.005, n_prec=n_prec)
+    return G, aa, x
+
+
 @pytest.mark.parametrize("density", [False, True])
 @pytest.mark.parametrize("n_prec", [1, 5])
 def test_fp64_sparse_columns(ctx, general, density, n_prec):
     """A dilute gas in a deep box: most columns hold a weak field or none, down to the rim of one atom's density.
     Each intensity is as accurate, relative to itself, as the general kernel's in FP64."""
-    a0 = synth.A0_FE
-    box = np.array([9, 8, 14]) * a0
-    pos = np.random.default_rng(3).uniform(0.0, 1.0, (70, 3)) * box
-    pos[:8] = np.array([[i, j, k] for i in (0, 1 - 1e-9) for j in (0, 1 - 1e-9) for k in (0, 1 - 1e-9)]) * box
-    t, x, _ = imaging.d2bi_condition(np.diag(box), a0, (0, 0, 1), (1, 1, 0), pos, sg=0.01, density=density)
-    G, aa = t.image_geometry(len(x), prec_angle=0.005, n_prec=n_prec)
+    G, aa, x = dilute(density, n_prec)
     got, want = ctx.image(G, x, aa), general.image(G, x, aa)
     assert ctx.stats().column_kernel == 4 and general.stats().column_kernel == 3
     assert (want < 1e-12).any() or not density
     assert (want > 1e-3).any()
     # 40 double steps and sums of a few terms: some tens of units of 2^-53
     assert (np.abs(got - want) <= 1e-12 * want + 1e-36).all()
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+def test_sparse_image_beside_one_with_density(ctx, fp32):
+    """An image without the density field in a batch with one that has it is the image alone, weak columns included
+    (a reflection that lets one atom's edge reach a few thousandths)."""
+    flags = _lib.ST_FLAG_FP32 if fp32 else 0
+    plain, dens = (dilute(d, sg=0.002, xig=1900.0) for d in (False, True))
+    G, aa, _ = plain
+    assert 32 * G.bg >= abs(aa[0]) and G.Mz * G.deltaz * G.bg >= 1 / 16
+    got = ctx.batch([(g[0], g[2], g[1]) for g in (plain, dens)], flags)
+    assert ((got[0] > 0) & (got[0] < 2.0 ** -13)).any()
+    for image, (G, aa, x) in zip(got, (plain, dens)):
+        assert np.array_equal(image, ctx.image(G, x, aa, flags=flags))
 
 
 @pytest.mark.parametrize("axis", [0, 1, 2])
