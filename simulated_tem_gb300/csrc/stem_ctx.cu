@@ -1271,6 +1271,7 @@ extern "C" int st_plan_create(st_ctx* c, int32_t n_jobs, const st_job* jobs, int
     G.c->ring_tuned = c->ring_tuned;
     G.c->fp32_general = c->fp32_general;
     G.c->fp64_general = c->fp64_general;
+    G.c->sample_limit = c->sample_limit;
     G.jobs.assign(js.begin() + first, js.begin() + last);
     p->groups.push_back(G);
     first = last;

@@ -56,3 +56,29 @@ def test_no_workspace_takes_the_general_kernels(fp32):
     assert kernel == (1 if fp32 else 3)
     for a, b in zip(got, want):
         assert np.abs(a - b).max() <= (FP32_TOL if fp32 else FP64_TOL)
+
+
+def test_a_plan_keeps_its_contexts_bound():
+    """The private contexts of a plan take the bound of the context that it is made from."""
+    with pytest.MonkeyPatch.context() as m:
+        m.setenv("STEM_SAMPLE_BYTES", "100000")
+        c = imaging.Context(0)
+    try:
+        G, aa, x = jobs_of(False)[0]
+        d_x = torch.from_numpy(x).cuda()
+        img = torch.zeros((G.My, G.Mx), dtype=torch.float64, device="cuda")
+        job = [(G, d_x.data_ptr(), len(x), aa, img.data_ptr())]
+        stream = torch.cuda.current_stream().cuda_stream
+        c.batch_device(job, _lib.ST_FLAG_FP32, stream)
+        want, launches = img.clone(), c.stats().n_launches
+        p = c.plan(job, _lib.ST_FLAG_FP32, stream)
+        try:
+            img.zero_()
+            p.launch(stream)
+            p.wait(stream)
+            assert p.stats().n_launches == launches > 8
+            assert torch.equal(img, want)
+        finally:
+            p.close()
+    finally:
+        c.close()
