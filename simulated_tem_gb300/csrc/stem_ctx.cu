@@ -957,7 +957,11 @@ extern "C" int st_create(st_ctx** out, int device) {
   if (ks)
     for (int i = 0; i < kField32Tiers; ++i)
       if (std::strcmp(ks, kSlabTierNames[i]) == 0) c->min_slab_tier = i;
-  if (const char* kb = std::getenv("STEM_SAMPLE_BYTES")) c->sample_limit = (size_t)std::strtoull(kb, nullptr, 10);
+  if (const char* kb = std::getenv("STEM_SAMPLE_BYTES")) {
+    char* end = nullptr;
+    const unsigned long long v = std::strtoull(kb, &end, 10);
+    if (end != kb && *end == 0) c->sample_limit = (size_t)v;  // anything else is no bound
+  }
   std::vector<long long> gauss(kGauss64Size);
   gauss64_table(gauss.data());
   e = cudaMalloc((void**)&c->d_gauss, gauss.size() * sizeof(long long));

@@ -41,9 +41,9 @@ def test_many_ranges_equal_one(fp32, density):
     jobs, flags = jobs_of(density), (_lib.ST_FLAG_FP32 if fp32 else 0) | _lib.ST_FLAG_AVERAGE
     want, kernel, launches = batch(None, jobs, flags)
     assert kernel == (2 if fp32 else 4)
-    for limit in (1, 100_000, 1_000_000):
+    for limit in (1, 100_000, 1_000_000, "", "2G"):  # the last two are no numbers, and no bound
         got, k, n = batch(limit, jobs, flags)
-        assert k == kernel and (n > launches or limit == 1_000_000)
+        assert k == kernel and (n > launches or limit in (1_000_000, "", "2G"))
         for a, b in zip(got, want):
             assert np.array_equal(a, b)
 
